@@ -497,12 +497,12 @@ inline void radix_scatter_shape(int shape, unsigned nb, cudaStream_t s, const K 
   }
 }
 
-// Sorts keys[0..n) (and vals alongside, if given) by bits [0, nbits).
+// Sorts keys[0..n) (and vals alongside, if given) by bits [from, nbits).
 // Buffers are swapped with internal scratch, so the sorted data ends in
 // `keys`/`vals`.  n < 2^32.
 template <typename K>
 inline void radix_sort(DBuf<K> &keys, DBuf<uint32_t> *vals, long long n, int nbits,
-                       cudaStream_t s) {
+                       cudaStream_t s, int from = 0) {
   static_assert(sizeof(K) == 4 || sizeof(K) == 8, "radix sort keys are 32 or 64 bits");
   if (n <= 1 || nbits <= 0) return;
   if (n >= (1LL << 32)) throw Error(TMRG_ERR_ARG, "radix sort size >= 2^32");
@@ -514,7 +514,7 @@ inline void radix_sort(DBuf<K> &keys, DBuf<uint32_t> *vals, long long n, int nbi
   DBuf<uint32_t> hist((size_t)256 * nb + 256, s);
   uint32_t *dtot = hist.p + (size_t)256 * nb;
   constexpr long long KB = sizeof(K);
-  for (int shift = 0; shift < nbits; shift += 8) {
+  for (int shift = from; shift < nbits; shift += 8) {
     prof_bytes(KB * n);
     launch(k_radix_hist<K>, nb, RS_THREADS, 0, s, (const K *)keys.p, n, shift, hist.p, nb);
     prof_bytes(8LL * 256 * nb);

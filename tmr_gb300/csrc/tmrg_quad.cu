@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "tmrg_keyset.cuh"
 #include "tmrg_quad.h"
 #include "tmrg_tree.cuh"
 
@@ -452,18 +453,45 @@ __device__ __forceinline__ int q_refine_target(const QRefineArgs &a, int r, int 
   }
   return level;
 }
-__global__ void k_q_refine_count(long long n, QRefineArgs a, const int16_t *__restrict__ lev,
-                                 unsigned *cnt, int *maxlev) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// state[0]: finest target level, state[1]: some quadrant coarsens or refines
+// by more than one level (the octree's k_refine_levels).
+__global__ void k_q_refine_levels(long long n, QRefineArgs a, const int16_t *__restrict__ lev,
+                                  int *state) {
   int ml = 0;
-  if (i < n) {
+  bool general = false;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
     int reps;
-    int nl = q_refine_target(a, a.ref ? a.ref[i] : 1, lev[i], reps);
-    cnt[i] = (unsigned)(reps * reps);
-    ml = nl;
+    const int l = lev[i], nl = q_refine_target(a, a.ref ? a.ref[i] : 1, l, reps);
+    ml = max(ml, nl);
+    general |= nl < l || reps > 1;
   }
-  for (int o = 16; o > 0; o >>= 1) ml = max(ml, __shfl_down_sync(0xffffffffu, ml, o));
-  if ((threadIdx.x & 31) == 0 && ml > 0) atomicMax(maxlev, ml);
+  ml = __reduce_max_sync(0xffffffffu, ml);
+  general = __any_sync(0xffffffffu, general);
+  if ((threadIdx.x & 31) == 0) {
+    if (ml > 0) atomicMax(state, ml);
+    if (general) atomicOr(state + 1, 1);
+  }
+}
+// Every quadrant stays or becomes the child-0 seed of its refinement, at its
+// own anchor: the order is the one before.
+__global__ void k_q_refine_in_place(long long n, QRefineArgs a, int16_t *lev, int16_t *info) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int reps;
+  const int l = lev[i], nl = q_refine_target(a, a.ref ? a.ref[i] : 1, l, reps);
+  if (nl != l) {
+    lev[i] = (int16_t)nl;
+    info[i] = 0;
+  }
+}
+__global__ void k_q_refine_count(long long n, QRefineArgs a, const int16_t *__restrict__ lev,
+                                 unsigned *cnt) {
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int reps;
+  q_refine_target(a, a.ref ? a.ref[i] : 1, lev[i], reps);
+  cnt[i] = (unsigned)(reps * reps);
 }
 template <typename Key>
 __global__ void k_q_refine_emit(long long n, QRefineArgs a, QKeyT<Key> K,
@@ -559,15 +587,25 @@ void qforest_refine(QForest &f, const int *d_ref, long long nref, int min_level,
   if (n == 0) return;
   cudaStream_t s = f.s;
   QRefineArgs a{d_ref, min_level, max_level};
+  DBuf<int> state(2, s);
+  state.zero();
+  launch(k_q_refine_levels, std::min(blocks_for(n, 256), 152u * 8), 256, 0, s, n, a,
+         (const int16_t *)f.level.p, state.p);
+  const int *dst[2] = {state.p, state.p + 1};
+  int hst[2];
+  read_scalars(dst, hst, s);
+  f.maxlev = std::max(f.maxlev, std::max(hst[0], 0));
+  const QKey K = f.key();
+  // as in the octree's refine: no sort where every quadrant keeps its anchor
+  if (!hst[1]) {
+    launch(k_q_refine_in_place, blocks_for(n, 256), 256, 0, s, n, a, f.level.p, f.info.p);
+    return;
+  }
   DBuf<unsigned> cnt(n + 1, s);
-  DBuf<int> ml(1, s);
-  ml.zero();
   launch(k_q_refine_count, blocks_for(n, 256), 256, 0, s, n, a, (const int16_t *)f.level.p,
-         cnt.p, ml.p);
+         cnt.p);
   exclusive_scan<unsigned>(cnt.p, cnt.p, n, s);
   const unsigned total = read_scalar(cnt.p + n, s);
-  f.maxlev = std::max(f.maxlev, std::max(read_scalar(ml.p, s), 0));
-  const QKey K = f.key();
   if (K.total_bits() > 64)
     q_refine_sort_compact<U128>(f, a, qkey_as<U128>(K), cnt, total);
   else
@@ -747,32 +785,33 @@ __global__ void k_q_level_starts(long long n, const Key *__restrict__ keys, int 
   int l = (int)klo64(keys[i] >> shift);
   if (i == 0 || (int)klo64(keys[i - 1] >> shift) != l) starts[l] = i;
 }
-// children-0 of the parent's edge (and corner) neighbours of family q
+// children-0 of the parent's edge (and corner) neighbours of family q: the
+// parent's 8 neighbours lie in 4 sibling groups (family_target of the
+// octree), bit d of g: the group beyond the outward side of direction d;
+// group 3 is reached by a corner neighbour only
+template <typename F>
+__device__ __forceinline__ void q_family_target(const QConnDev &c, const Quad &q, int g, F &&f) {
+  const Quad p = q_parent(q);
+  const int32_t h = side_of(p.level), bs = 2 * h;
+  Quad r;
+  r.block = p.block;
+  r.level = p.level;
+  r.x = (p.x & ~h) + ((g & 1) ? ((p.x & h) ? bs : -bs) : 0);
+  r.y = (p.y & ~h) + ((g & 2) ? ((p.y & h) ? bs : -bs) : 0);
+  if (q_in_tree(r))
+    f(r);
+  else
+    q_for_images(c, r, bs, g == 3, f);
+}
 template <bool WRITE, typename Key>
 __device__ __forceinline__ unsigned q_gen_family(const QConnDev &c, QPos<Key> P, const Quad &q,
                                                  int corner, Key *out) {
   unsigned cnt = 0;
-  Quad p = q_parent(q);
-  const int32_t bs = 2 * side_of(p.level);
-  auto emit = [&](const Quad &r) {
-    if (WRITE) out[cnt] = P.make(r.block, r.x, r.y);
-    cnt++;
-  };
-  for (int e = 0; e < 4; e++) {
-    Quad r = q_sibling(q_edge_nbr(p, e), 0);
-    if (q_in_tree(r))
-      emit(r);
-    else
-      q_for_images(c, r, bs, false, emit);
-  }
-  if (corner)
-    for (int k = 0; k < 4; k++) {
-      Quad r = q_sibling(q_corner_nbr(p, k), 0);
-      if (q_in_tree(r))
-        emit(r);
-      else
-        q_for_images(c, r, bs, true, emit);
-    }
+  for (int g = 0; g < (corner ? 4 : 3); g++)
+    q_family_target(c, q, g, [&](const Quad &r) {
+      if (WRITE) out[cnt] = P.make(r.block, r.x, r.y);
+      cnt++;
+    });
   return cnt;
 }
 // n bounds the families; *m (device) is their number (entries past it
@@ -960,6 +999,112 @@ static void q_balance_impl(QForest &f, int corner, const QKeyT<Key> K) {
          f.x.p, f.y.p, f.level.p, f.info.p);
 }
 
+// ---------------------------------------------------------------------
+// The balance for 64-bit keys with a hash set of families, as the octree's
+// balance_hashed: one launch per level, one wait in all.
+__global__ void __launch_bounds__(256)
+    k_q_fam_seeds(long long n, QKey K, KeySet S, const int *__restrict__ blk,
+                  const int *__restrict__ xs, const int *__restrict__ ys,
+                  const int16_t *__restrict__ lev) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  auto family = [&](long long k) {
+    const Quad q = q_sibling(Quad{blk[k], xs[k], ys[k], lev[k]}, 0);
+    return K.make(q.block, q.x, q.y, q.level);
+  };
+  uint64_t k = 0;
+  bool on = i < n;
+  if (on) {
+    k = family(i);
+    on = i == 0 || family(i - 1) != k;
+  }
+  S.add(k, on, 0, 0);
+}
+// 4 lanes per family, one group each
+__global__ void __launch_bounds__(256)
+    k_q_fam_close(int level, int gen, int corner, QConnDev c, QKey K, KeySet S) {
+  const unsigned m = S.before(gen);
+  const int g = threadIdx.x & 3;
+  const unsigned stride = gridDim.x * 64;
+  for (unsigned b0 = blockIdx.x * 64; b0 < m; b0 += stride) {  // uniform per block
+    const unsigned i = b0 + (threadIdx.x >> 2);
+    const uint64_t k = i < m ? S.list[i] : 0;
+    const bool mine = i < m && (int)(k & 31) == level && (corner || g != 3);
+    if (!__any_sync(0xffffffffu, mine)) continue;
+    uint64_t first = 0;
+    int cnt = 0;
+    Quad q{0, 0, 0, 0};
+    if (mine) {
+      q = K.decode(k);
+      q_family_target(c, q, g, [&](const Quad &r) {
+        if (cnt++ == 0) first = K.make(r.block, r.x, r.y, r.level);
+      });
+    }
+    S.add(first, cnt > 0, gen, m);
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    for (int j = 1; j < most; j++) {
+      uint64_t key = 0;
+      if (j < cnt) {
+        int at = 0;
+        q_family_target(c, q, g, [&](const Quad &r) {
+          if (at++ == j) key = K.make(r.block, r.x, r.y, r.level);
+        });
+      }
+      S.add(key, j < cnt, gen, m);
+    }
+  }
+}
+__global__ void __launch_bounds__(256)
+    k_q_fam_leaves(int gens, QKey K, KeySet S, uint64_t *out, unsigned cap) {
+  const unsigned m = S.before(gens);
+  const int j = threadIdx.x & 3, lane = threadIdx.x & 31;
+  const unsigned stride = gridDim.x * 64;
+  for (unsigned b0 = blockIdx.x * 64; b0 < m; b0 += stride) {
+    const unsigned i = b0 + (threadIdx.x >> 2);
+    uint64_t key = 0;
+    bool leaf = false;
+    if (i < m) {
+      Quad q = K.decode(S.list[i]);
+      if (q.level > 0) q = q_sibling(q, j);
+      if (q.level > 0 || j == 0) {
+        key = K.make(q.block, q.x, q.y, q.level);
+        leaf = q.level >= TMRG_MAX_LEVEL || !S.contains(key + 1);
+      }
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, leaf);
+    if (b == 0u) continue;
+    unsigned o = 0;
+    if (lane == 0) o = atomicAdd(S.counter(), (unsigned)__popc(b));
+    o = __shfl_sync(0xffffffffu, o, 0) + __popc(b & ((1u << lane) - 1u));
+    if (leaf && o < cap) out[o] = key;
+  }
+}
+static bool q_balance_hashed(QForest &f, int corner, const QKey K) {
+  const long long n = f.n;
+  cudaStream_t s = f.s;
+  const QConnDev c = f.conn->dev;
+  const long long cap = n + n / 4 + 4096;
+  KeySetBuf B(cap, s);
+  const KeySet S = B.set;
+  launch(k_q_fam_seeds, blocks_for(n, 256), 256, 0, s, n, K, S, (const int *)f.block.p,
+         (const int *)f.x.p, (const int *)f.y.p, (const int16_t *)f.level.p);
+  const unsigned grid = std::min(blocks_for(cap, 64), 152u * 8);
+  int gens = 1;
+  for (int l = f.maxlev; l >= 2; l--, gens++)
+    launch(k_q_fam_close, grid, 256, 0, s, l, gens, corner, c, K, S);
+  DBuf<uint64_t> leaves(4 * cap, s);
+  launch(k_q_fam_leaves, grid, 256, 0, s, gens, K, S, leaves.p, (unsigned)(4 * cap));
+  const unsigned *dv[2] = {B.count.p + KEYSET_GENS + 1, B.count.p + KEYSET_GENS};
+  unsigned hv[2];
+  read_scalars(dv, hv, s);
+  if (hv[1]) return false;
+  const long long m = hv[0];
+  radix_sort(leaves, nullptr, m, K.total_bits(), s, 5);  // positions are distinct
+  q_alloc(f, m);
+  launch(k_q_decode<uint64_t>, blocks_for(m, 256), 256, 0, s, m, K, (const uint64_t *)leaves.p,
+         f.block.p, f.x.p, f.y.p, f.level.p, f.info.p);
+  return true;
+}
+
 void qforest_balance(QForest &f, int corner) {
   Stage stage("tmrg_quad_balance");
   if (!f.have_quads)
@@ -967,9 +1112,11 @@ void qforest_balance(QForest &f, int corner) {
   f.free_nodes();
   if (f.n == 0) return;
   const QKey K = f.key();
-  if (K.total_bits() > 64)
+  if (K.total_bits() > 64) {
     q_balance_impl<U128>(f, corner, qkey_as<U128>(K));
-  else
+    return;
+  }
+  if (f.n >= (1LL << 28) || !q_balance_hashed(f, corner, K))
     q_balance_impl<uint64_t>(f, corner, K);
 }
 
