@@ -112,3 +112,36 @@ def test_balance_of_a_set_that_outgrows_its_list(gpu_lib, dim):
     assert abs((2.0 ** (-dim * lev)).sum() - 2.0) < 1e-9
     f.balance(1)
     assert np.array_equal(_cells(f), a)
+
+
+@pytest.mark.parametrize("order,interp", [(2, 1), (3, 1), (4, 1), (3, 2)])
+def test_nodes_of_tiles_equal_nodes_of_entries(gpu_lib, order, interp):
+    # a small forest emits every (element, object); with uniform bricks
+    # beside it the same elements go through tiles, the last one ragged, and
+    # keep their numbers (nodes are numbered in block order)
+    from tmr_gb300 import TMR
+    base = W.rotate_blocks(W.brick(2, 2, 1), 8)
+    got = []
+    for extra in (0, 4):
+        conn = base if not extra else _union([base, W.brick(extra, 2, 1)])
+        f = TMR.OctForest(order=order, interp=interp)
+        f.setConnectivity(conn)
+        f.createTrees(1)
+        for p in range(4):
+            c = _cells(f)
+            flags = np.zeros(len(c), np.intc)
+            mine = c[:, 0] < len(base)
+            flags[mine] = W.uniform(13, p, int(mine.sum())) < (0.45 if p < 3 else 0.0)
+            flags[~mine] = p < 3
+            f.refine(flags, 0, 5)
+            f.balance(1)
+        f.createNodes()
+        c = _cells(f)
+        n = int((c[:, 0] < len(base)).sum())
+        conn = f.getMeshConn()[:n]
+        ptr, dc, dw = f.getDepNodeConn()
+        nd = int(-conn.min())
+        got.append((n, len(c), conn, ptr[:nd + 1], dc[:ptr[nd]], dw[:ptr[nd]]))
+    assert got[0][1] < 16384 <= got[1][1] and got[1][1] % 256 != 0
+    for a, b in zip(got[0][2:], got[1][2:]):
+        assert np.array_equal(a, b)
