@@ -1048,6 +1048,20 @@ __global__ void k_df_split_x(long long n, const double *__restrict__ x, float2 *
   xs[i] = make_float2(hi, lo);
 }
 
+// The same for an odd number of vectors, with one more that is zero, so that
+// the pairs of k_df_apply2 are whole.
+__global__ void k_df_split_odd(long long rows, int nvec, const double *__restrict__ x, float2 *xs,
+                               int *flag) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * (nvec + 1)) return;
+  const long long r = i / (nvec + 1);
+  const int v = (int)(i - r * (nvec + 1));
+  float hi = 0.0f, lo = 0.0f;
+  if (v < nvec && !df_split(__ldg(x + r * nvec + v), DF_X_EMIN, DF_X_ERANGE, hi, lo))
+    atomicOr(flag, 1);
+  xs[i] = make_float2(hi, lo);
+}
+
 // The apply copy of P: 8 lanes per row keep the apply_keeps entries in order.
 // Each kept entry also gets its transpose sort record: key = column,
 // value = its position in the copy, erow = its row (k_t_keys' output).
@@ -2129,54 +2143,105 @@ static void interp_colsum(Interp &I) {
 // input and rebuilds each weight as hi + lo).  With `scale` the result is
 // divided by scale[row] (weight-normalised transpose).
 
-// G lanes per row, lane v accumulates vectors v, v+G, ... in entry order
-// (any number of vectors).
+// Few vectors on a small matrix, in FP64 straight from the caller's vector:
+// 2^LB lanes per row take its entries in turn, each with all NV components,
+// and combine in a fixed tree.  One launch instead of a flag reset, a pass
+// that splits the input and an apply; no window on the values.  The weight is
+// put together from its two floats with integer operations, which leaves the
+// FP64 pipe NV instructions an entry.
+template <int NV>
 __global__ void __launch_bounds__(256)
-    k_df_apply(long long rows, int G, int nvec, const int *__restrict__ rowptr,
+    k_f64_rows(long long rows, int LB, const int *__restrict__ rowptr,
                const int *__restrict__ cols, const float2 *__restrict__ w,
-               const float2 *__restrict__ xs, const double *__restrict__ x,
-               double *__restrict__ y, const double *__restrict__ scale,
-               const int *__restrict__ flags) {
+               const double *__restrict__ x, double *__restrict__ y,
+               const double *__restrict__ scale) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long r = t / G;
-  const int lane = (int)(t - r * G);
-  if (r >= rows) return;
-  const bool f64 = (__ldg(flags) | __ldg(flags + 1)) != 0;
-  const int p0 = __ldg(rowptr + r), p1 = __ldg(rowptr + r + 1);
-  for (int v = lane; v < nvec; v += G) {
-    double acc = 0.0;
-    if (f64) {
-      for (int p = p0; p < p1; p++) {
-        const float2 wv = __ldg(w + p);
-        acc = __fma_rn(__dadd_rn((double)wv.x, (double)wv.y),
-                       __ldg(x + (long long)__ldg(cols + p) * nvec + v), acc);
-      }
-    } else {
-      float sh = 0.0f, sl = 0.0f;
-      int p = p0;
-      for (; p + 4 <= p1; p += 4) {
+  const long long r = t >> LB;
+  const int L = 1 << LB, l = (int)t & (L - 1);
+  const bool have = r < rows;
+  const int p0 = have ? __ldg(rowptr + r) : 0, p1 = have ? __ldg(rowptr + r + 1) : 0;
+  double acc[NV];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const float2 wv = __ldg(w + p + k);
-          const float2 xv = __ldg(xs + (long long)__ldg(cols + p + k) * nvec + v);
-          df_fma(wv.x, wv.y, xv.x, xv.y, sh, sl);
-        }
-        df_renorm(sh, sl);
-      }
-      for (; p < p1; p++) {
-        const float2 wv = __ldg(w + p);
-        const float2 xv = __ldg(xs + (long long)__ldg(cols + p) * nvec + v);
-        df_fma(wv.x, wv.y, xv.x, xv.y, sh, sl);
-      }
-      df_renorm(sh, sl);
-      acc = df_value(sh, sl);
-    }
-    if (scale) {
-      const double sc = scale[r];
-      acc = (sc != 0.0) ? __ddiv_rn(acc, sc) : 0.0;
-    }
-    y[r * nvec + v] = acc;
+  for (int v = 0; v < NV; v++) acc[v] = 0.0;
+#pragma unroll 2
+  for (int p = p0 + l; p < p1; p += L) {
+    const float2 wv = __ldg(w + p);
+    const double *xr = x + (long long)__ldg(cols + p) * NV;
+    const double wd = df_value(wv.x, wv.y);
+#pragma unroll
+    for (int v = 0; v < NV; v++) acc[v] = __fma_rn(wd, __ldg(xr + v), acc[v]);
   }
+  for (int o = L >> 1; o > 0; o >>= 1)
+#pragma unroll
+    for (int v = 0; v < NV; v++)
+      acc[v] = __dadd_rn(acc[v], __shfl_down_sync(0xffffffffu, acc[v], o));
+  if (!have || l != 0) return;
+  const double sc = scale ? scale[r] : 1.0;
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    double a = acc[v];
+    if (scale) a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
+    y[r * NV + v] = a;
+  }
+}
+
+// One vector, in double-float: 2^LB lanes per row in storage order take its
+// entries in turn (a warp's entries are one run of memory) and combine in a
+// fixed tree.  Bound by the latency of the gathers: 117M entries in 0.47 ms
+// (P, mean row 8.5) and 0.59 ms (P^T, 35.5), 3.0 and 2.4 TB/s; one lane per
+// row took 0.54 and 0.83 ms, half-empty vector pairs 0.60 and 0.68 ms.
+__global__ void __launch_bounds__(256)
+    k_df_one(long long rows, int LB, const int *__restrict__ rowptr,
+             const int *__restrict__ cols, const float2 *__restrict__ w,
+             const float2 *__restrict__ xs, const double *__restrict__ x,
+             double *__restrict__ y, const double *__restrict__ scale,
+             const int *__restrict__ flags) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long r = t >> LB;
+  const int L = 1 << LB, l = (int)t & (L - 1);
+  const bool f64 = (__ldg(flags) | __ldg(flags + 1)) != 0;
+  const bool have = r < rows;
+  const int p0 = have ? __ldg(rowptr + r) : 0, p1 = have ? __ldg(rowptr + r + 1) : 0;
+  double acc = 0.0;
+  if (f64) {
+    for (int p = p0 + l; p < p1; p += L) {
+      const float2 wv = __ldg(w + p);
+      acc = __fma_rn(__dadd_rn((double)wv.x, (double)wv.y), __ldg(x + __ldg(cols + p)), acc);
+    }
+    for (int o = L >> 1; o > 0; o >>= 1)
+      acc = __dadd_rn(acc, __shfl_down_sync(0xffffffffu, acc, o));
+  } else {
+    float sh = 0.0f, sl = 0.0f;
+    int p = p0 + l;
+    for (; p + 3 * L < p1; p += 4 * L) {
+      float2 wv[4], xv[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        wv[k] = __ldg(w + p + k * L);
+        xv[k] = __ldg(xs + __ldg(cols + p + k * L));
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) df_fma(wv[k].x, wv[k].y, xv[k].x, xv[k].y, sh, sl);
+      df_renorm(sh, sl);
+    }
+    for (; p < p1; p += L) {
+      const float2 wv = __ldg(w + p), xv = __ldg(xs + __ldg(cols + p));
+      df_fma(wv.x, wv.y, xv.x, xv.y, sh, sl);
+    }
+    df_renorm(sh, sl);
+    for (int o = L >> 1; o > 0; o >>= 1) {
+      const float oh = __shfl_down_sync(0xffffffffu, sh, o);
+      const float ol = __shfl_down_sync(0xffffffffu, sl, o);
+      df_add(sh, sl, oh, ol);
+    }
+    acc = df_value(sh, sl);
+  }
+  if (!have || l != 0) return;
+  if (scale) {
+    const double sc = scale[r];
+    acc = (sc != 0.0) ? __ddiv_rn(acc, sc) : 0.0;
+  }
+  y[r] = acc;
 }
 
 // Vector pairs: LPR lanes per row, lane v holds PPL consecutive vector
@@ -2189,12 +2254,16 @@ __global__ void __launch_bounds__(256)
 // with four pairs per lane) before their arithmetic, so a warp waits for
 // two memory round trips per group; more pairs per lane (PPL) give each
 // wait more arithmetic.
-template <int LPR, int NG, int PPL>
+// An odd number of vectors is carried as one more, zero, in the (hi, lo)
+// input (a lane per vector took 1.70 ms for 3 vectors and 117M entries, whole
+// pairs take 0.96 ms; 7 vectors 3.04 and 1.75 ms); SC: the caller's vectors then have no 16-byte rows (nor has an
+// unaligned buffer) and are read and written value by value.
+template <int LPR, int NG, int PPL, bool SC>
 __global__ void __launch_bounds__(256)
-    k_df_apply2(long long rows, int nvec2, const int *__restrict__ rowptr,
+    k_df_apply2(long long rows, int nvec2, int nvec, const int *__restrict__ rowptr,
                 const int *__restrict__ cols, const float2 *__restrict__ w,
-                const float4 *__restrict__ xs, const double2 *__restrict__ x,
-                double2 *__restrict__ y, const double *__restrict__ scale,
+                const float4 *__restrict__ xs, const double *__restrict__ x,
+                double *__restrict__ y, const double *__restrict__ scale,
                 const int *__restrict__ perm, const int *__restrict__ flags) {
   constexpr int RPW = 32 / (LPR * NG);
   const int lane = threadIdx.x & 31;
@@ -2229,8 +2298,16 @@ __global__ void __launch_bounds__(256)
         const double wd = __dadd_rn((double)wv.x, (double)wv.y);
 #pragma unroll
         for (int j = 0; j < PPL; j++) {
-          const double2 xv = (on && act[j]) ? __ldg(x + (long long)c * nvec2 + q0 + j)
-                                            : make_double2(0.0, 0.0);
+          double2 xv = make_double2(0.0, 0.0);
+          if (on && act[j]) {
+            if (SC) {
+              const double *xp = x + (long long)c * nvec + 2 * (q0 + j);
+              xv.x = __ldg(xp);
+              if (2 * (q0 + j) + 1 < nvec) xv.y = __ldg(xp + 1);
+            } else {
+              xv = __ldg((const double2 *)x + (long long)c * nvec2 + q0 + j);
+            }
+          }
           ax[j] = __fma_rn(wd, xv.x, ax[j]);
           ay[j] = __fma_rn(wd, xv.y, ay[j]);
         }
@@ -2325,7 +2402,13 @@ __global__ void __launch_bounds__(256)
           a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
           b = (sc != 0.0) ? __ddiv_rn(b, sc) : 0.0;
         }
-        y[r * nvec2 + q0 + j] = make_double2(a, b);
+        if (SC) {
+          double *yp = y + r * nvec + 2 * (q0 + j);
+          yp[0] = a;
+          if (2 * (q0 + j) + 1 < nvec) yp[1] = b;
+        } else {
+          ((double2 *)y)[r * nvec2 + q0 + j] = make_double2(a, b);
+        }
       }
     }
   }
@@ -2567,20 +2650,24 @@ static bool tma_apply(long long rows, long long nin, const int *rp, const int *c
 // (k_df_apply_tma); fewer pairs: LPR = pairs rounded down to a power of
 // two, NG 1 or 2
 constexpr int DF2_SHAPES_WIDE = 7, DF2_SHAPES_NARROW = 2;
-static void df_apply2(int shape, long long rows, int nvec2, const int *rp, const int *ci,
+static void df_apply2(int shape, long long rows, int nvec, const int *rp, const int *ci,
                       const float2 *w, const float2 *xs, const double *x, double *y,
                       const double *scale, const int *perm, int *flags, cudaStream_t s,
                       long long nin) {
-  if (shape == 6 && nvec2 == 8 &&
+  const int nvec2 = (nvec + 1) / 2;
+  const bool scalar = nvec % 2 != 0 || ((uintptr_t)x % 16) != 0 || ((uintptr_t)y % 16) != 0;
+  if (shape == 6 && nvec2 == 8 && !scalar &&
       tma_apply(rows, nin, rp, ci, w, xs, x, y, scale, perm, flags, s))
     return;
   const float4 *x4 = (const float4 *)xs;
-  const double2 *x2 = (const double2 *)x;
-  double2 *y2 = (double2 *)y;
-#define TMRG_DF2(L, N, P)                                                                  \
-  launch((k_df_apply2<L, N, P>),                                                           \
+#define TMRG_DF2S(L, N, P, SC)                                                             \
+  launch((k_df_apply2<L, N, P, SC>),                                                       \
          blocks_for(((rows + 32 / ((L) * (N)) - 1) / (32 / ((L) * (N)))) * 32, 256), 256, 0, s, \
-         rows, nvec2, rp, ci, w, x4, x2, y2, scale, perm, flags)
+         rows, nvec2, nvec, rp, ci, w, x4, x, y, scale, perm, flags)
+#define TMRG_DF2(L, N, P)                                     \
+  do {                                                        \
+    if (scalar) TMRG_DF2S(L, N, P, true); else TMRG_DF2S(L, N, P, false); \
+  } while (0)
   if (nvec2 >= 8) {
     switch (shape) {
       case 0: TMRG_DF2(8, 1, 1); break;
@@ -2607,6 +2694,7 @@ static void df_apply2(int shape, long long rows, int nvec2, const int *rp, const
       TMRG_DF2(1, 2, 1);
   }
 #undef TMRG_DF2
+#undef TMRG_DF2S
 }
 // Size class of an apply: direction, vector pairs (8 = 8 or more), log2 of
 // the rows, mean row length in quarters (capped).
@@ -2617,12 +2705,18 @@ static TuneKey df_key(int which, long long rows, long long nnz, int nvec2) {
   return TuneKey{which == 0 ? TUNE_P : TUNE_PT, std::min(nvec2, 8), lr, q, 0, 0};
 }
 
-// The input as (hi, lo) pairs in pool memory, with its window flag.
-static void df_split_input(Interp &I, const double *x, long long n, DBuf<float2> &xs,
-                           cudaStream_t s) {
+// The input as (hi, lo) pairs in pool memory, with its window flag; an odd
+// number of vectors gets one more, zero.
+static void df_split_input(Interp &I, const double *x, long long nrows, int nvec,
+                           DBuf<float2> &xs, cudaStream_t s) {
+  const long long n = nrows * nvec;
   if (n <= 0) return;
   prof_bytes(16 * n);
-  launch(k_df_split_x, blocks_for(n, 256), 256, 0, s, n, x, xs.p, I.dfflag.p + 1);
+  if (nvec % 2 == 0 || nvec == 1)
+    launch(k_df_split_x, blocks_for(n, 256), 256, 0, s, n, x, xs.p, I.dfflag.p + 1);
+  else
+    launch(k_df_split_odd, blocks_for(nrows * (nvec + 1), 256), 256, 0, s, nrows, nvec, x, xs.p,
+           I.dfflag.p + 1);
 }
 
 // Transpose apply with the input in host memory: the input rows are copied
@@ -2684,7 +2778,7 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
              (const double *)(dx + r0 * nvec), xs.p + r0 * nvec, I.dfflag.p + 1);
     const long long a = I.t_chunk[k], n = I.t_chunk[k + 1] - a;
     if (n > 0)
-      df_apply2(shape, n, nvec / 2, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, xs.p, dx, y, sc,
+      df_apply2(shape, n, nvec, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, xs.p, dx, y, sc,
                 I.t_perm.p + a, I.dfflag.p, s, nin);
   }
   TMRG_CUDA(cudaStreamSynchronize(s));
@@ -2797,7 +2891,7 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
     }
     if (r1 > r0) {
       prof_bytes(12 * I.nnz_nz * (r1 - r0) / rows + 4 * (r1 - r0) + 8LL * nvec * (r1 - r0));
-      df_apply2(shape, r1 - r0, n2, I.ap_rowptr(), I.ap_colidx(), I.ap_w.p, xs.p, dx, y,
+      df_apply2(shape, r1 - r0, nvec, I.ap_rowptr(), I.ap_colidx(), I.ap_w.p, xs.p, dx, y,
                 nullptr, I.perm.p + r0, I.dfflag.p, s, nin);
     }
     TMRG_CUDA(cudaEventRecord(ev[k], s));
@@ -2818,6 +2912,41 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
   return true;
 }
 
+// The FP64 apply (k_f64_rows) where it is the faster one: up to 8 vectors and
+// F64_ROWS_MAX entries x vectors, where launches count and the FP64 pipe does
+// not yet.  Measured per apply, split pass and double-float apply against
+// this kernel: 27K entries, 1 to 8 vectors 16-20 -> 10-12 us; 476K entries, 1
+// vector 16 -> 12 us, 2 vectors 19 -> 16 us, 3 vectors 20 -> 19 us, 4 vectors
+// 19 against 23 us; 4.8M entries, 1 vector 37 against 65 us.
+constexpr long long F64_ROWS_MAX = 1000000;
+static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, const int *ci,
+                     const float2 *w, const double *x, double *y, const double *scale,
+                     long long bytes, cudaStream_t s) {
+  if (nvec > 8 || nnz * nvec > F64_ROWS_MAX) return false;
+  // lanes per row: about a third of the mean row length
+  int lb = 0;
+  while (lb < 4 && (6LL << lb) * rows <= 2 * nnz) lb++;
+  prof_bytes(bytes);
+  const unsigned g = blocks_for(rows << lb, 256);
+  switch (nvec) {
+#define TMRG_F64(V)                                                                     \
+  case V:                                                                               \
+    launch(k_f64_rows<V>, g, 256, 0, s, rows, lb, rp, ci, w, x, y, scale);              \
+    break
+    TMRG_F64(1);
+    TMRG_F64(2);
+    TMRG_F64(3);
+    TMRG_F64(4);
+    TMRG_F64(5);
+    TMRG_F64(6);
+    TMRG_F64(7);
+    default:
+      launch(k_f64_rows<8>, g, 256, 0, s, rows, lb, rp, ci, w, x, y, scale);
+#undef TMRG_F64
+  }
+  return true;
+}
+
 void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
   Stage st(which == 0 ? "tmrg_interp_mult" : "tmrg_interp_mult_transpose");
   if (nvec <= 0) throw Error(TMRG_ERR_ARG, "interp apply: nvec <= 0");
@@ -2830,27 +2959,30 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
   const float2 *w = which == 0 ? (const float2 *)I.ap_w.p : (const float2 *)I.t_w.p;
   const double *sc = which == 2 ? (const double *)I.colsum.p : (const double *)nullptr;
   const int *perm = which == 0 ? (const int *)I.perm.p : (const int *)I.t_perm.p;
-  DBuf<float2> xs(nin * nvec + 1, s);
-  TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
-  df_split_input(I, x, nin * nvec, xs, s);
   // compulsory traffic: 12 B per nonzero entry, the row pointers, one read
   // of the input (its (hi, lo) copy) and one write of the output vectors
   const long long bytes = 12 * I.nnz_nz + 4 * (nout + 1) + 8LL * nvec * (nin + nout) +
                           (which == 2 ? 8 * nout : 0);
+  if (f64_rows(nvec, nout, I.nnz_nz, rp, ci, w, x, y, sc, bytes, s)) return;
+  const int n2 = (nvec + 1) / 2;
+  DBuf<float2> xs(nin * (nvec == 1 ? 1 : 2 * n2) + 1, s);
+  TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
+  df_split_input(I, x, nin, nvec, xs, s);
   prof_bytes(bytes);
-  if (nvec % 2 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0) {
-    const int n2 = nvec / 2;
-    tune_run(df_key(which, nout, I.nnz_nz, n2), n2 >= 8 ? DF2_SHAPES_WIDE : DF2_SHAPES_NARROW,
-             [&](int shape) {
-               df_apply2(shape, nout, n2, rp, ci, w, xs.p, x, y, sc, perm, I.dfflag.p, s, nin);
-             },
-             s);
+  if (nvec == 1) {
+    // lanes per row by the mean row length: 1 below 10 entries (8.5: 471 us
+    // against 514 with 2, 117M entries), 2 below 24 (13.9: 35 us against 47
+    // with 1), then 4 (35.5: 593 us against 645 with 2 and 629 with 8)
+    const int lb = I.nnz_nz < 10 * nout ? 0 : I.nnz_nz < 24 * nout ? 1 : 2;
+    launch(k_df_one, blocks_for(nout << lb, 256), 256, 0, s, nout, lb, rp, ci, w,
+           (const float2 *)xs.p, x, y, sc, (const int *)I.dfflag.p);
     return;
   }
-  int G = 1;
-  while (G < nvec && G < 32) G <<= 1;
-  launch(k_df_apply, blocks_for(nout * G, 256), 256, 0, s, nout, G, nvec, rp, ci, w,
-         (const float2 *)xs.p, x, y, sc, (const int *)I.dfflag.p);
+  tune_run(df_key(which, nout, I.nnz_nz, n2), n2 >= 8 ? DF2_SHAPES_WIDE : DF2_SHAPES_NARROW,
+           [&](int shape) {
+             df_apply2(shape, nout, nvec, rp, ci, w, xs.p, x, y, sc, perm, I.dfflag.p, s, nin);
+           },
+           s);
 }
 
 }  // namespace tmrg
