@@ -1,0 +1,89 @@
+"""The mass matrix assembled row by row, against a dense assembly from the
+forest's own connectivity: a node shared by many blocks (rows larger than
+the tables of the first attempts), hanging nodes, and a block size so small
+that no entry is taken from the unit block's."""
+import numpy as np
+import pytest
+
+from tmr_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _fan(k):
+    """k hexahedra around one edge: node 0 (and 0 + layer) on the axis, then
+    2k nodes of the rim per layer."""
+    layer = 2 * k + 1
+    conn = []
+    for i in range(k):
+        a, b, c = 1 + 2 * i, 2 + 2 * i, 1 + (2 * i + 2) % (2 * k)
+        conn.append([0, a, c, b, layer, layer + a, layer + c, layer + b])
+    return np.array(conn, np.intc)
+
+
+def _mass(f, dim, n, block_len):
+    """Dense M, element by element, dependent nodes through their rows."""
+    conn = f.getMeshConn()
+    ptr, dc, dw = f.getDepNodeConn()
+    lev = f.getOctantsArray()[:, 5] if dim == 3 else f.getQuadrantsArray()[:, 4]
+    m1 = np.array([[2.0, 1.0], [1.0, 2.0]]) / 6.0
+    ref = m1
+    for _ in range(dim - 1):
+        ref = np.kron(m1, ref)
+    M = np.zeros((n, n))
+    for e, c in enumerate(conn):
+        S = np.zeros((len(c), n))
+        for a, g in enumerate(c):
+            if g >= 0:
+                S[a, g] = 1.0
+            else:
+                r = slice(ptr[-g - 1], ptr[-g])
+                np.add.at(S[a], dc[r], dw[r])
+        M += (block_len * 0.5 ** lev[e]) ** dim * (S.T @ ref @ S)
+    return M
+
+
+def _check(F, M):
+    rp, c, v, _, _, _ = F.getMatrix()
+    n = len(rp) - 1
+    got = np.zeros((n, n))
+    for i in range(n):
+        cols = c[rp[i]:rp[i + 1]]
+        assert np.all(np.diff(cols) > 0)
+        got[i, cols] = v[rp[i]:rp[i + 1]]
+    # sums of at most a few thousand products
+    np.testing.assert_allclose(got, M, rtol=1e-12, atol=1e-15 * np.abs(M).max())
+
+
+@pytest.mark.parametrize("k", [7, 100, 300])
+def test_rows_of_a_node_in_many_blocks(gpu_lib, k):
+    from tmr_gb300 import TMR
+    f = TMR.OctForest(order=2)
+    f.setConnectivity(_fan(k))
+    f.createTrees(0)
+    f.createNodes()
+    n = int(f.getNodeRange()[1])
+    assert n == 2 * (2 * k + 1)
+    F = TMR.MatrixFilter(0.5, 3, None, [f])
+    _check(F, _mass(f, 3, n, 1.0))
+
+
+@pytest.mark.parametrize("dim", [3, 2])
+@pytest.mark.parametrize("block_len", [1.0, 0.7, 1e-60, 1e-98])
+def test_rows_with_hanging_nodes(gpu_lib, dim, block_len):
+    from tmr_gb300 import TMR
+    if dim == 3:
+        f = TMR.OctForest(order=2)
+        f.setConnectivity(W.rotate_blocks(W.brick(2, 2, 1), 4))
+    else:
+        f = TMR.QuadForest(order=2)
+        f.setConnectivity(W.brick2d(3, 2))
+    f.createTrees(1)
+    for p in range(3):
+        n = f.getNumOctants() if dim == 3 else f.getNumQuadrants()
+        f.refine(W.random_indicator(n, 5, p, 0.25), 0, 5)
+        f.balance(1)
+    f.createNodes()
+    n = int(f.getNodeRange()[1])
+    F = TMR.MatrixFilter(0.1 * block_len, 3, None, [f], block_len=block_len)
+    _check(F, _mass(f, dim, n, block_len))

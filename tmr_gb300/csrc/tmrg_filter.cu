@@ -2,17 +2,20 @@
 //
 // Setup: the consistent mass matrix M of the trilinear (octree) or
 // bilinear (quadtree) elements of an order-2 forest, with dependent nodes
-// condensed onto the independent nodes they interpolate.  Each element
-// first merges its 8x8 (4x4) element
-// matrix, expanded through the dependent-node weights, into a dense
-// block over its distinct independent nodes; the blocks of all elements
-// are then sorted by (row, column) and summed in element order.  Then
+// condensed onto the independent nodes they interpolate.  Each element's
+// matrix, expanded through the dependent-node weights, is a dense block
+// over its distinct independent nodes; a row of M adds the block rows of
+// the elements around its node in element order (assemble_rows).  Orders
+// 3 and 4 sort the blocks' entries by (row, column) instead.  Then
 // D = M 1, Ainv = 1/(1 + r^2/D^(2/3)), B = Ainv r^2/(D^(2/3) D) (in 2-D
 // Ainv = 1/(1 + r^2/D), B = Ainv r^2/(D D)) and Tinv = 1/(F~ 1).
 //
 // Apply: Horner's recurrence out = B.(M out) + t1 (forward) or
 // out = M(B.out) + t1 (transpose), one fused CSR kernel per term over all
 // `vpn` interleaved design components, so M is read once per term.
+#include <string.h>
+
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -101,30 +104,268 @@ __device__ int element_block(const FilterCtx &c, long long e, int *U,
   return K;
 }
 
-__global__ void k_fe_count(long long n, FilterCtx c, unsigned *cnt) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
+// ---------------------------------------------------------------------
+// M by rows (order 2).  Sorting every block entry by (row, column) moves K^2
+// records of 20 bytes per element through 5 or more passes; here only the K
+// block rows of an element are sorted, by their node, and a row adds its
+// block rows into a hash table in shared memory, element after element (the
+// order of the sums is that of the sorted entries, hence the same bits).
+// An element without dependent nodes needs no stored block: its entries are
+// the level's mass over 2^nd, by exponent arithmetic.
+// Bound by the probes and the rank pass of the small rows (1.9 ms for 2.56M
+// rows of 27 columns) and by local memory in the hanging elements' blocks
+// (0.8 ms); building this filter with its restrictions and filtering once
+// went from 23.0 to 13.1 ms, 14.9 of the 23.0 the sort and its passes.
+struct RowAsm {
+  const int *conn;
+  const int16_t *lev;
+  int npe, dim;
+  unsigned long long m0;    // bits of the mass entry of a unit block, nd = 0
+  const unsigned *hoff;     // per element: place among the hanging ones
+  const unsigned *ucnt;     // per hanging element: first of its distinct nodes,
+  const unsigned *boff;     // and of its block
+  const int *unode;
+  const double *block;
+  const unsigned *srp;      // per node: its block rows in `slot`,
+  const uint32_t *slot;     // element << 5 | block row, elements ascending
+  __device__ __forceinline__ bool hanging(unsigned e) const {
+    return hoff[e + 1] != hoff[e];
+  }
+  __device__ __forceinline__ int nodes(unsigned e) const {
+    if (!hanging(e)) return npe;
+    const unsigned h = hoff[e];
+    return (int)(ucnt[h + 1] - ucnt[h]);
+  }
+};
+// Elements with a stored block: those with a dependent node, or with one
+// node twice (a collapsed block), or all of them (`all`).
+__global__ void k_fa_hanging(long long ne, int npe, const int *__restrict__ conn, int all,
+                             unsigned *flag) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  bool h = all != 0;
+  int g[8];
+#pragma unroll
+  for (int a = 0; a < 8; a++) {
+    g[a] = a < npe ? __ldg(conn + e * npe + a) : 0;
+    if (a < npe) h |= g[a] < 0;
+#pragma unroll
+    for (int b = 0; b < a; b++) h |= a < npe && g[a] == g[b];
+  }
+  flag[e] = h ? 1u : 0u;
+}
+__global__ void k_fa_list(long long ne, const unsigned *__restrict__ hoff, unsigned *list) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < ne && hoff[e + 1] != hoff[e]) list[hoff[e]] = (unsigned)e;
+}
+__global__ void k_fa_count(long long nh, FilterCtx c, const unsigned *__restrict__ list,
+                           unsigned *ucnt, unsigned *bcnt) {
+  const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= nh) return;
   int U[FMAXK];
-  int K = element_block(c, e, U, nullptr);
-  cnt[e] = (unsigned)(K * K);
+  const int K = element_block(c, list[h], U, nullptr);
+  ucnt[h] = (unsigned)K;
+  bcnt[h] = (unsigned)(K * K);
 }
 __global__ void __launch_bounds__(64)
-    k_fe_write(long long n, FilterCtx c, int cb, const unsigned *__restrict__ offs,
-               uint64_t *keys, uint32_t *perm, double *vals) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
+    k_fa_blocks(long long nh, FilterCtx c, const unsigned *__restrict__ list,
+                const unsigned *__restrict__ uoff, const unsigned *__restrict__ boff, int *unode,
+                double *block) {
+  const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= nh) return;
   int U[FMAXK];
   double L[FMAXK][FMAXK];
-  int K = element_block(c, e, U, L);
-  unsigned o = offs[e];
-  for (int u = 0; u < K; u++)
-    for (int v = 0; v < K; v++) {
-      keys[o] = ((uint64_t)(uint32_t)U[u] << cb) | (uint64_t)(uint32_t)U[v];
-      perm[o] = o;
-      vals[o] = L[u][v];
-      o++;
-    }
+  const int K = element_block(c, list[h], U, L);
+  const unsigned u0 = uoff[h], b0 = boff[h];
+  for (int u = 0; u < K; u++) {
+    unode[u0 + u] = U[u];
+    for (int v = 0; v < K; v++) block[b0 + u * K + v] = L[u][v];
+  }
 }
+// Block rows of every element (soff: their scanned counts) by node.
+__global__ void k_fa_slot_count(long long ne, RowAsm A, unsigned *cnt) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < ne) cnt[e] = (unsigned)A.nodes((unsigned)e);
+}
+__global__ void k_fa_slots(long long ne, RowAsm A, const unsigned *__restrict__ soff,
+                           uint32_t *keys, uint32_t *vals) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  const unsigned o = soff[e];
+  const int K = (int)(soff[e + 1] - o);
+  const int *U = A.hanging((unsigned)e) ? A.unode + A.ucnt[A.hoff[e]] : A.conn + e * A.npe;
+  for (int u = 0; u < K; u++) {
+    keys[o + u] = (uint32_t)U[u];
+    vals[o + u] = (uint32_t)e << 5 | (uint32_t)u;
+  }
+}
+// first[j] = first sorted block row of a node >= j
+__global__ void k_fa_starts(long long n, long long E, const uint32_t *__restrict__ keys,
+                            unsigned *first) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > E) return;
+  const long long k = i < E ? (long long)keys[i] : n;
+  for (long long j = i ? (long long)keys[i - 1] + 1 : 0; j <= k; j++) first[j] = (unsigned)i;
+}
+// Entries each row has to add; rows with more than FA_SMALL go to `large`.
+constexpr int FA_SMALL = 64;         // 8 elements of 8 nodes
+// A large row's table: slots and rows per block of the first attempt, and of
+// the one that follows where some row has more columns (in a 2:1 balanced
+// forest none has).
+constexpr int FA_LARGE = 512, FA_LARGE_WARPS = 4;
+constexpr int FA_HUGE = 8192, FA_HUGE_WARPS = 1;
+constexpr size_t FA_SLOT_BYTES = sizeof(double) + sizeof(int) + sizeof(uint16_t);
+__global__ void k_fa_candidates(long long n, RowAsm A, unsigned *cand, unsigned *large,
+                                unsigned *nlarge) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned t = 0;
+  if (i < n) {
+    for (unsigned p = A.srp[i]; p < A.srp[i + 1]; p++) t += (unsigned)A.nodes(A.slot[p] >> 5);
+    cand[i] = t;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, t > FA_SMALL);
+  if (m == 0u) return;
+  const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
+  unsigned o = 0;
+  if (lane == lead) o = atomicAdd(nlarge, (unsigned)__popc(m));
+  o = __shfl_sync(0xffffffffu, o, lead);
+  if (t > FA_SMALL) large[o + __popc(m & ((1u << lane) - 1u))] = (unsigned)i;
+}
+// One row by G lanes (the whole warp calls it) over a table of `slots` slots (a
+// power of two): the sorted columns and sums go to col / val, their number
+// is returned; *err = FA_FULL when the row has more columns than the table.
+constexpr int FA_FULL = 2;
+template <int G>
+__device__ __forceinline__ int assemble_row(const RowAsm &A, long long row, bool have,
+                                            int slots, int *tcol, double *tval, uint16_t *tidx, int *col,
+                                            double *val, int *err) {
+  const int lane = threadIdx.x & 31, l = lane & (G - 1);
+  for (int i = l; i < slots; i += G) {
+    tcol[i] = -1;
+    tval[i] = 0.0;
+  }
+  __syncwarp();
+  const unsigned p0 = have ? A.srp[row] : 0, p1 = have ? A.srp[row + 1] : 0;
+  unsigned steps = p1 - p0;
+#pragma unroll
+  for (int o = G; o < 32; o <<= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, o));
+  bool full = false;
+  for (unsigned k = 0; k < steps; k++) {
+    const bool on = p0 + k < p1;
+    unsigned e = 0, u = 0;
+    int K = 0;
+    bool hang = false;
+    if (on) {
+      const unsigned s = __ldg(A.slot + p0 + k);
+      e = s >> 5;
+      u = s & 31u;
+      hang = A.hanging(e);
+      K = A.npe;
+    }
+    const int *U = A.conn + (long long)e * A.npe;
+    const double *B = nullptr;
+    if (hang) {
+      const unsigned h = A.hoff[e], u0 = A.ucnt[h];
+      K = (int)(A.ucnt[h + 1] - u0);
+      U = A.unode + u0;
+      B = A.block + A.boff[h] + u * K;
+    }
+    for (int v = l; v < K; v += G) {  // an element's nodes are distinct
+      const int c = __ldg(U + v);
+      double m;
+      if (hang) {
+        m = __ldg(B + v);
+      } else {
+        const int nd = __popc(u ^ (unsigned)v);
+        m = __longlong_as_double((long long)(
+            A.m0 - ((unsigned long long)(A.dim * __ldg(A.lev + e) + nd) << 52)));
+      }
+      unsigned h = ((unsigned)c * 0x9E3779B1u) >> 16 & (unsigned)(slots - 1);
+      int it = 0;
+      for (; it < slots; it++) {
+        int was = *(volatile int *)(tcol + h);
+        if (was == -1) was = atomicCAS(tcol + h, -1, c);
+        if (was == -1 || was == c) break;
+        h = (h + 1) & (unsigned)(slots - 1);
+      }
+      if (it == slots)
+        full = true;
+      else
+        tval[h] = __dadd_rn(tval[h], m);
+    }
+    __syncwarp();
+  }
+  if (full) atomicExch(err, FA_FULL);
+  // the taken slots, then each one's rank among their columns
+  int n = 0;
+  const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (lane & ~(G - 1));
+  for (int i = l; i < slots; i += G) {
+    const bool taken = tcol[i] >= 0;
+    const unsigned m = __ballot_sync(0xffffffffu, taken) & gmask;
+    if (taken) tidx[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
+    n += __popc(m);
+  }
+  __syncwarp();
+  for (int i = l; i < n; i += G) {
+    const int s = tidx[i], c = tcol[s];
+    int r = 0;
+    for (int j = 0; j < n; j++) r += tcol[tidx[j]] < c;
+    col[r] = c;
+    val[r] = tval[s];
+  }
+  return n;
+}
+// Rows of at most FA_SMALL entries: 8 lanes each (7-8 elements of 8 nodes
+// keep every lane busy).
+__global__ void __launch_bounds__(128)
+    k_fa_rows_small(long long n, RowAsm A, const unsigned *__restrict__ coff, int *col,
+                    double *val, int *len, int *err) {
+  __shared__ int tcol[16][FA_SMALL];
+  __shared__ double tval[16][FA_SMALL];
+  __shared__ uint16_t tidx[16][FA_SMALL];
+  const int g = threadIdx.x >> 3;
+  const long long row = (long long)blockIdx.x * 16 + g;
+  const unsigned o = row < n ? coff[row] : 0, o1 = row < n ? coff[row + 1] : 0;
+  const bool have = row < n && o1 - o <= FA_SMALL;
+  const int m = assemble_row<8>(A, row, have, FA_SMALL, tcol[g], tval[g], tidx[g], col + o,
+                                val + o, err);
+  if (have && (threadIdx.x & 7) == 0) len[row] = m;
+}
+// The others: a warp each, `warps` rows per block.
+__global__ void __launch_bounds__(FA_LARGE_WARPS * 32)
+    k_fa_rows_large(const unsigned *__restrict__ nlarge, const unsigned *__restrict__ list,
+                    int slots, int warps, RowAsm A, const unsigned *__restrict__ coff, int *col,
+                    double *val, int *len, int *err) {
+  extern __shared__ __align__(16) unsigned char fa_smem[];
+  const int w = threadIdx.x >> 5;
+  double *tval = (double *)fa_smem + (size_t)w * slots;
+  int *tcol = (int *)((double *)fa_smem + (size_t)warps * slots) + (size_t)w * slots;
+  uint16_t *tidx = (uint16_t *)((int *)((double *)fa_smem + (size_t)warps * slots) +
+                                (size_t)warps * slots) + (size_t)w * slots;
+  const unsigned m = *nlarge;
+  for (unsigned i = blockIdx.x * warps + w; i < m; i += gridDim.x * warps) {
+    const long long row = list[i];
+    const unsigned o = coff[row];
+    const int c = assemble_row<32>(A, row, true, slots, tcol, tval, tidx, col + o, val + o, err);
+    if ((threadIdx.x & 31) == 0) len[row] = c;
+    __syncwarp();
+  }
+}
+// Rows from their places to CSR, 8 lanes per row.
+__global__ void k_fa_compact(long long n, const unsigned *__restrict__ coff,
+                             const int *__restrict__ rp, const int *__restrict__ col,
+                             const double *__restrict__ val, int *ocol, double *oval) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long row = t >> 3;
+  if (row >= n) return;
+  const unsigned o = coff[row];
+  const int p0 = rp[row], m = rp[row + 1] - p0;
+  for (int k = (int)(t & 7); k < m; k += 8) {
+    ocol[p0 + k] = col[o + k];
+    oval[p0 + k] = val[o + k];
+  }
+}
+
 // Sum each run of equal (row, col) keys in element order.
 __global__ void k_fe_reduce(long long E, const uint64_t *__restrict__ keys,
                             const uint32_t *__restrict__ perm,
@@ -397,6 +638,10 @@ __global__ void k_fe_scalings(long long n, int dim, const int *__restrict__ rp,
 __global__ void k_fe_tinv(long long n, const double *__restrict__ y, double *T) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) T[i] = (y[i] != 0.0) ? __ddiv_rn(1.0, y[i]) : 0.0;
+}
+__global__ void k_fe_ones(long long n, double *a, double *b) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) a[i] = b[i] = 1.0;
 }
 template <typename T>
 __global__ void k_to_f32(long long n, const double *__restrict__ a, T *b) {
@@ -859,77 +1104,58 @@ void filter_create_quad(QForest &f, double len, double r, int N, Filter &F) {
                len, r, N, F);
 }
 
-static void filter_build(const FSource &f, double len, double r, int N, Filter &F) {
+// M with every block entry sorted by (row, column) and equal ones summed in
+// element order (orders 3 and 4).
+static void assemble_sorted(const FSource &f, const FilterCtx &c, int cb, Filter &F) {
   cudaStream_t s = f.s;
-  F.s = s;
-  F.N = N;
-  F.r = r;
   const long long n = f.nn, ne = f.ne;
-  F.n = n;
-  DBuf<int> err(1, s);
-  err.zero();
-  FilterCtx c{f.econn, f.dptr, f.dconn, f.dw, len, f.level, err.p, f.npe, f.dim};
-  const int cb = bits_for(n + 1);
-  if (2 * cb > 64) throw Error(TMRG_ERR_KEY_RANGE, "filter key range");
   long long E = 0;
   DBuf<uint64_t> keys;
   DBuf<uint32_t> perm;
   DBuf<double> ev;
-  if (f.order == 2) {
-    DBuf<unsigned> cnt(ne + 1, s);
-    launch(k_fe_count, blocks_for(ne, 128), 128, 0, s, ne, c, cnt.p);
-    exclusive_scan<unsigned>(cnt.p, cnt.p, ne, s);
-    E = read_scalar(cnt.p + ne, s);
-    keys.alloc(E, s);
-    perm.alloc(E, s);
-    ev.alloc(E, s);
-    launch(k_fe_write, blocks_for(ne, 64), 64, 0, s, ne, c, cb,
-           (const unsigned *)cnt.p, keys.p, perm.p, ev.p);
-  } else {
-    FGen g{};
-    g.o = f.order;
-    g.npe = f.npe;
-    for (int i = 0; i < g.o; i++)
-      for (int j = 0; j < g.o; j++) g.m1[i][j] = bernstein_mass_1d(g.o - 1, i, j);
-    DBuf<int> mx(2, s);
-    mx.zero();
-    launch(k_fe_gen_emax, blocks_for(ne, 256), 256, 0, s, ne, c, g.npe, mx.p);
-    const int emax = read_scalar(mx.p, s);
-    // count pass: the list and its distinct nodes (at most the list length)
-    g.cap = std::max(32, emax);
-    g.kcap = g.cap;
-    g.tcols = 0;
-    const size_t sm_c = fg_layout(g).total * FG_WARPS;
-    if (g.cap > 65535 || sm_c > 200 * 1024)
-      throw Error(TMRG_ERR_UNSUPPORTED, "matrix filter: an element expands to " +
-                                            std::to_string(emax) + " entries");
-    DBuf<long long> cnt(ne + 1, s);
-    TMRG_CUDA(cudaFuncSetAttribute(k_fe_gen_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sm_c));
-    launch(k_fe_gen_count, blocks_for(ne, FG_WARPS), FG_WARPS * 32, sm_c, s, ne, c, g, cnt.p,
-           mx.p + 1);
-    const int kmax = read_scalar(mx.p + 1, s);
-    if (read_scalar(err.p, s))
-      throw Error(TMRG_ERR_UNSUPPORTED, "matrix filter: an element touches too many nodes");
-    exclusive_scan<long long>(cnt.p, cnt.p, ne, s);
-    E = read_scalar(cnt.p + ne, s);
-    if (E >= (1LL << 32))
-      throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
-    // write pass: T over the largest number of distinct nodes
-    g.kcap = std::max(1, kmax);
-    g.tcols = g.kcap;
-    const size_t smem = fg_layout(g).total * FG_WARPS;
-    if (smem > 227 * 1024)
-      throw Error(TMRG_ERR_UNSUPPORTED, "matrix filter: an element touches " +
-                                            std::to_string(kmax) + " independent nodes");
-    keys.alloc(E, s);
-    perm.alloc(E, s);
-    ev.alloc(E, s);
-    TMRG_CUDA(cudaFuncSetAttribute(k_fe_gen_write, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
-    launch(k_fe_gen_write, blocks_for(ne, FG_WARPS), FG_WARPS * 32, smem, s, ne, c, g, cb,
-           (const long long *)cnt.p, keys.p, perm.p, ev.p);
-  }
+  FGen g{};
+  g.o = f.order;
+  g.npe = f.npe;
+  for (int i = 0; i < g.o; i++)
+    for (int j = 0; j < g.o; j++) g.m1[i][j] = bernstein_mass_1d(g.o - 1, i, j);
+  DBuf<int> mx(2, s);
+  mx.zero();
+  launch(k_fe_gen_emax, blocks_for(ne, 256), 256, 0, s, ne, c, g.npe, mx.p);
+  const int emax = read_scalar(mx.p, s);
+  // count pass: the list and its distinct nodes (at most the list length)
+  g.cap = std::max(32, emax);
+  g.kcap = g.cap;
+  g.tcols = 0;
+  const size_t sm_c = fg_layout(g).total * FG_WARPS;
+  if (g.cap > 65535 || sm_c > 200 * 1024)
+    throw Error(TMRG_ERR_UNSUPPORTED, "matrix filter: an element expands to " +
+                                          std::to_string(emax) + " entries");
+  DBuf<long long> cnt(ne + 1, s);
+  TMRG_CUDA(cudaFuncSetAttribute(k_fe_gen_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sm_c));
+  launch(k_fe_gen_count, blocks_for(ne, FG_WARPS), FG_WARPS * 32, sm_c, s, ne, c, g, cnt.p,
+         mx.p + 1);
+  const int kmax = read_scalar(mx.p + 1, s);
+  if (read_scalar(c.err, s))
+    throw Error(TMRG_ERR_UNSUPPORTED, "matrix filter: an element touches too many nodes");
+  exclusive_scan<long long>(cnt.p, cnt.p, ne, s);
+  E = read_scalar(cnt.p + ne, s);
+  if (E >= (1LL << 32))
+    throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
+  // write pass: T over the largest number of distinct nodes
+  g.kcap = std::max(1, kmax);
+  g.tcols = g.kcap;
+  const size_t smem = fg_layout(g).total * FG_WARPS;
+  if (smem > 227 * 1024)
+    throw Error(TMRG_ERR_UNSUPPORTED, "matrix filter: an element touches " +
+                                          std::to_string(kmax) + " independent nodes");
+  keys.alloc(E, s);
+  perm.alloc(E, s);
+  ev.alloc(E, s);
+  TMRG_CUDA(cudaFuncSetAttribute(k_fe_gen_write, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+  launch(k_fe_gen_write, blocks_for(ne, FG_WARPS), FG_WARPS * 32, smem, s, ne, c, g, cb,
+         (const long long *)cnt.p, keys.p, perm.p, ev.p);
   radix_sort(keys, &perm, E, 2 * cb, s);
   DBuf<unsigned> pos(E + 1, s);
   launch(k_fe_first, blocks_for(E, 256), 256, 0, s, E, (const uint64_t *)keys.p,
@@ -949,6 +1175,122 @@ static void filter_build(const FSource &f, double len, double r, int N, Filter &
   ev.release();
   pos.release();
   exclusive_scan<int>(F.rowptr.p, F.rowptr.p, n, s);
+}
+
+// M by rows (order 2; RowAsm).
+static void assemble_rows(const FSource &f, const FilterCtx &c, int cb, Filter &F) {
+  cudaStream_t s = f.s;
+  const long long n = f.nn, ne = f.ne;
+  if (ne >= (1LL << 27)) throw Error(TMRG_ERR_KEY_RANGE, "matrix filter: too many elements");
+  RowAsm A{};
+  A.conn = f.econn;
+  A.lev = f.level;
+  A.npe = f.npe;
+  A.dim = f.dim;
+  const double len = c.block_len;
+  // the mass entry of a unit block: element sides are len over a power of
+  // two, so an element's entry is this one with a smaller exponent
+  const double m0 = f.dim == 3 ? len * len * len / 27.0 : len * len / 9.0;
+  memcpy(&A.m0, &m0, sizeof(m0));
+  // hanging elements: their distinct nodes and blocks
+  DBuf<unsigned> hoff(ne + 1, s);
+  // (far from the ends of the exponent's range, where an entry of a deep
+  // level might not be the scaled one: 3 x 30 levels and nd <= 3)
+  const int ex = (int)((A.m0 >> 52) & 0x7ff);
+  const int all = ex < 128 || ex == 0x7ff;
+  launch(k_fa_hanging, blocks_for(ne, 256), 256, 0, s, ne, f.npe, f.econn, all, hoff.p);
+  exclusive_scan<unsigned>(hoff.p, hoff.p, ne, s);
+  const long long nh = read_scalar(hoff.p + ne, s);
+  DBuf<unsigned> list(nh + 1, s), ucnt(nh + 1, s), boff(nh + 1, s);
+  launch(k_fa_list, blocks_for(ne, 256), 256, 0, s, ne, (const unsigned *)hoff.p, list.p);
+  launch(k_fa_count, blocks_for(nh, 128), 128, 0, s, nh, c, (const unsigned *)list.p, ucnt.p,
+         boff.p);
+  exclusive_scan<unsigned>(ucnt.p, ucnt.p, nh, s);
+  exclusive_scan<unsigned>(boff.p, boff.p, nh, s);
+  const unsigned *hp[2] = {ucnt.p + nh, boff.p + nh};
+  unsigned hv[2];
+  read_scalars(hp, hv, s);
+  DBuf<int> unode((size_t)hv[0] + 1, s);
+  DBuf<double> block((size_t)hv[1] + 1, s);
+  launch(k_fa_blocks, blocks_for(nh, 64), 64, 0, s, nh, c, (const unsigned *)list.p,
+         (const unsigned *)ucnt.p, (const unsigned *)boff.p, unode.p, block.p);
+  list.release();
+  A.hoff = hoff.p;
+  A.ucnt = ucnt.p;
+  A.boff = boff.p;
+  A.unode = unode.p;
+  A.block = block.p;
+  // block rows sorted by node, elements ascending
+  DBuf<unsigned> soff(ne + 1, s);
+  launch(k_fa_slot_count, blocks_for(ne, 256), 256, 0, s, ne, A, soff.p);
+  exclusive_scan<unsigned>(soff.p, soff.p, ne, s);
+  const long long ns = (long long)(ne - nh) * f.npe + hv[0];
+  DBuf<uint32_t> skey(ns, s), slot(ns, s);
+  launch(k_fa_slots, blocks_for(ne, 256), 256, 0, s, ne, A, (const unsigned *)soff.p, skey.p,
+         slot.p);
+  soff.release();
+  radix_sort(skey, &slot, ns, cb, s);
+  DBuf<unsigned> srp(n + 1, s);
+  launch(k_fa_starts, blocks_for(ns + 1, 256), 256, 0, s, n, ns, (const uint32_t *)skey.p, srp.p);
+  skey.release();
+  A.srp = srp.p;
+  A.slot = slot.p;
+  // rows, each at its number of entries before equal columns are added
+  const long long E = (long long)(ne - nh) * f.npe * f.npe + hv[1];
+  if (E >= (1LL << 32))
+    throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
+  DBuf<unsigned> coff(n + 1, s), large(n + 1, s), nlarge(1, s);
+  nlarge.zero();
+  launch(k_fa_candidates, blocks_for(n, 256), 256, 0, s, n, A, coff.p, large.p, nlarge.p);
+  exclusive_scan<unsigned>(coff.p, coff.p, n, s);
+  DBuf<int> col(E + 1, s);
+  DBuf<double> val(E + 1, s);
+  F.rowptr.alloc(n + 1, s);
+  DBuf<int> ncol(n + 1, s);
+  launch(k_fa_rows_small, blocks_for(n, 16), 128, 0, s, n, A, (const unsigned *)coff.p, col.p,
+         val.p, ncol.p, c.err);
+  auto rows = [&](int slots, int warps) {
+    const size_t smem = FA_SLOT_BYTES * slots * warps;
+    TMRG_CUDA(cudaFuncSetAttribute(k_fa_rows_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(FA_SLOT_BYTES * FA_HUGE * FA_HUGE_WARPS)));
+    launch(k_fa_rows_large, std::min(blocks_for(n, warps), 152u * 8), warps * 32, smem, s,
+           (const unsigned *)nlarge.p, (const unsigned *)large.p, slots, warps, A,
+           (const unsigned *)coff.p, col.p, val.p, ncol.p, c.err);
+    exclusive_scan<int>(ncol.p, F.rowptr.p, n, s);
+    const int *pv[2] = {F.rowptr.p + n, c.err};
+    int hv2[2];
+    read_scalars(pv, hv2, s);
+    F.nnz = hv2[0];
+    return hv2[1];
+  };
+  if (rows(FA_LARGE, FA_LARGE_WARPS) == FA_FULL) {
+    TMRG_CUDA(cudaMemsetAsync(c.err, 0, sizeof(int), s));
+    rows(FA_HUGE, FA_HUGE_WARPS);
+  }
+  const long long nnz = F.nnz;
+  F.colidx.alloc(nnz + 1, s);
+  F.vals.alloc(nnz + 1, s);
+  launch(k_fa_compact, blocks_for(n * 8, 256), 256, 0, s, n, (const unsigned *)coff.p,
+         (const int *)F.rowptr.p, (const int *)col.p, (const double *)val.p, F.colidx.p,
+         F.vals.p);
+}
+
+static void filter_build(const FSource &f, double len, double r, int N, Filter &F) {
+  cudaStream_t s = f.s;
+  F.s = s;
+  F.N = N;
+  F.r = r;
+  const long long n = f.nn, ne = f.ne;
+  F.n = n;
+  DBuf<int> err(1, s);
+  err.zero();
+  FilterCtx c{f.econn, f.dptr, f.dconn, f.dw, len, f.level, err.p, f.npe, f.dim};
+  const int cb = bits_for(n + 1);
+  if (2 * cb > 64) throw Error(TMRG_ERR_KEY_RANGE, "filter key range");
+  if (f.order == 2)
+    assemble_rows(f, c, cb, F);
+  else
+    assemble_sorted(f, c, cb, F);
   if (read_scalar(err.p, s))
     throw Error(TMRG_ERR_INTERNAL, "matrix filter: element touches too many nodes");
   F.Ainv.alloc(n, s);
@@ -977,11 +1319,7 @@ static void filter_build(const FSource &f, double len, double r, int N, Filter &
   // Tinv = 1 / (F~ 1) with Tinv = 1 during the evaluation.
   {
     DBuf<double> ones(n, s), y(n, s);
-    std::vector<double> h1(n, 1.0);
-    TMRG_CUDA(cudaMemcpyAsync(ones.p, h1.data(), n * sizeof(double),
-                              cudaMemcpyHostToDevice, s));
-    TMRG_CUDA(cudaMemcpyAsync(F.Tinv.p, h1.data(), n * sizeof(double),
-                              cudaMemcpyHostToDevice, s));
+    launch(k_fe_ones, blocks_for(n, 256), 256, 0, s, n, ones.p, F.Tinv.p);
     filter_apply(F, false, 1, ones.p, y.p);
     launch(k_fe_tinv, blocks_for(n, 256), 256, 0, s, n, (const double *)y.p,
            F.Tinv.p);
