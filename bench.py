@@ -337,7 +337,7 @@ def pipeline_roofline(TMR, conn, W, x_fine, peak):
                            if stages.get(k) else None} for k in b}}
 
 
-TUNE_KINDS = {1: "P apply", 2: "P^T apply", 3: "filter vpn3 FP32", 4: "filter vpn3 FP64",
+TUNE_KINDS = {1: "P apply", 2: "P^T apply",
               5: "radix scatter (key bytes, values, log2 n)"}
 
 

@@ -87,3 +87,88 @@ def test_rows_with_hanging_nodes(gpu_lib, dim, block_len):
     n = int(f.getNodeRange()[1])
     F = TMR.MatrixFilter(0.1 * block_len, 3, None, [f], block_len=block_len)
     _check(F, _mass(f, dim, n, block_len))
+
+
+def _horner(F, N, x, transpose):
+    import scipy.sparse as sp
+    rp, c, v, A, B, T = F.getMatrix()
+    n = len(rp) - 1
+    M = sp.csr_matrix((v, c, rp), shape=(n, n))
+    A, B, T = A[:, None], B[:, None], T[:, None]
+    if not transpose:
+        t1 = A * x
+        y = t1
+        for _ in range(N):
+            y = B * (M @ y) + t1
+        return T * y
+    t1 = T * x
+    y = t1
+    for _ in range(N):
+        y = M @ (B * y) + t1
+    return A * y
+
+
+def _random_filter(TMR, N):
+    f = TMR.OctForest(order=2)
+    f.setConnectivity(W.rotate_blocks(W.brick(2, 2, 1), 4))
+    f.createTrees(1)
+    for p in range(3):
+        f.refine(W.random_indicator(f.getNumOctants(), 5, p, 0.25), 0, 5)
+        f.balance(1)
+    f.createNodes()
+    return TMR.MatrixFilter(0.1, N, None, [f])
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("N,vpn", [(0, 2), (1, 1), (2, 3), (3, 2), (4, 4), (5, 5), (3, 7), (10, 3)])
+def test_terms_of_tiles_match_horner(gpu_lib, dtype, N, vpn):
+    # apart, in place and overlapping by one row; rounding of N + 1 terms of
+    # about 30 products each
+    import torch
+
+    from tmr_gb300 import TMR
+    F = _random_filter(TMR, N)
+    n = F.size()[0]
+    assert n % 256 != 0 and n > 512
+    rng = np.random.default_rng(N)
+    tol = (1e-13 if dtype == "float64" else 4e-6)
+    for transpose in (False, True):
+        x = rng.uniform(0.0, 1.0, (n, vpn))
+        want = _horner(F, N, x.astype(dtype).astype(np.float64), transpose)
+        xd = torch.from_numpy(x.reshape(-1)).cuda().to(getattr(torch, dtype))
+        apply = F.applyTranspose if transpose else F.applyFilter
+        y = torch.empty_like(xd)
+        apply(xd, y, vpn)
+        got = y.cpu().numpy().astype(np.float64).reshape(n, vpn)
+        assert np.abs(got - want).max() <= tol * np.abs(want).max()
+        same = xd.clone()
+        apply(same, same, vpn)
+        assert torch.equal(same, y)
+        both = torch.zeros((n + 1) * vpn, dtype=xd.dtype, device="cuda")
+        both[: n * vpn] = xd
+        apply(both[: n * vpn], both[vpn:], vpn)
+        assert torch.equal(both[vpn:], y)
+
+
+def test_terms_of_a_tile_with_too_many_columns(gpu_lib):
+    # a node in 1100 blocks: its row alone has 4402 columns, more than a tile
+    # may have, and the sliced copy runs
+    import torch
+
+    from tmr_gb300 import TMR
+    f = TMR.OctForest(order=2)
+    f.setConnectivity(_fan(1100))
+    f.createTrees(0)
+    f.createNodes()
+    F = TMR.MatrixFilter(0.5, 4, None, [f])
+    n = F.size()[0]
+    rng = np.random.default_rng(2)
+    for vpn in (1, 3):
+        for transpose in (False, True):
+            x = rng.uniform(0.0, 1.0, (n, vpn))
+            want = _horner(F, 4, x, transpose)
+            y = torch.empty(n * vpn, dtype=torch.float64, device="cuda")
+            (F.applyTranspose if transpose else F.applyFilter)(
+                torch.from_numpy(x.reshape(-1)).cuda(), y, vpn)
+            assert np.abs(y.cpu().numpy().reshape(n, vpn) - want).max() <= (
+                1e-12 * np.abs(want).max())

@@ -11,8 +11,8 @@
 // Ainv = 1/(1 + r^2/D), B = Ainv r^2/(D D)) and Tinv = 1/(F~ 1).
 //
 // Apply: Horner's recurrence out = B.(M out) + t1 (forward) or
-// out = M(B.out) + t1 (transpose), one fused CSR kernel per term over all
-// `vpn` interleaved design components, so M is read once per term.
+// out = M(B.out) + t1 (transpose), one fused kernel per term over up to four
+// of the interleaved design components, so M is read once per term.
 #include <string.h>
 
 #include <algorithm>
@@ -21,6 +21,7 @@
 
 #include "tmrg_quad.h"
 #include "tmrg_tree.cuh"
+#include "tmrg_tsell.cuh"
 
 namespace tmrg {
 
@@ -659,6 +660,16 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ double ffma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
+// four values from shared memory, 16 bytes a load
+__device__ __forceinline__ void lds4(const float *p, float (&v)[4]) {
+  const float4 q = *(const float4 *)p;
+  v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+}
+__device__ __forceinline__ void lds4(const double *p, double (&v)[4]) {
+  const double2 a = ((const double2 *)p)[0], b = ((const double2 *)p)[1];
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
 // t1 = s . in ; returns t1 (the first Horner iterate).
 template <typename T>
 __global__ void k_fe_scale(long long n, int vpn, const T *__restrict__ s,
@@ -758,91 +769,85 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Three components per node (the design fields of the C3 workload) are
-// carried through the Horner terms padded to four: a node's values are one
-// 16-byte (FP32) or two 16-byte (FP64) loads per gathered neighbour instead
-// of three scalar loads.  Only the first scaling reads and only the last
-// term writes the caller's 3-component layout.  Same operation sequence per
-// component as k_fe_sell, so the results are the same bits.
-template <typename T>
-__device__ __forceinline__ void load4(const T *p, T (&v)[4]);
-template <>
-__device__ __forceinline__ void load4<float>(const float *p, float (&v)[4]) {
-  const float4 q = __ldg((const float4 *)p);
-  v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-}
-template <>
-__device__ __forceinline__ void load4<double>(const double *p, double (&v)[4]) {
-  const double2 a = __ldg((const double2 *)p), b = __ldg((const double2 *)p + 1);
-  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
-}
-template <typename T>
-__device__ __forceinline__ void store4(T *p, T a, T b, T c);
-template <>
-__device__ __forceinline__ void store4<float>(float *p, float a, float b, float c) {
-  *(float4 *)p = make_float4(a, b, c, 0.0f);
-}
-template <>
-__device__ __forceinline__ void store4<double>(double *p, double a, double b, double c) {
-  ((double2 *)p)[0] = make_double2(a, b);
-  ((double2 *)p)[1] = make_double2(c, 0.0);
-}
-// t1 (padded) = s . in (3 components)
-template <typename T>
-__global__ void k_fe_scale3p(long long n, const T *__restrict__ s, const T *__restrict__ in,
-                             T *out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const T si = s[i];
-  store4<T>(out + 4 * i, fmul(si, in[3 * i]), fmul(si, in[3 * i + 1]),
-            fmul(si, in[3 * i + 2]));
-}
-// One Horner term, padded input; output padded (ypad) or in the caller's
-// 3-component layout (the last term).
-template <typename T, bool TR>
-__global__ void __launch_bounds__(256)
-    k_fe_sell3p(long long n, const int *__restrict__ perm, const int *__restrict__ srl,
-                const long long *__restrict__ soff, const int *__restrict__ scol,
-                const T *__restrict__ sval, const T *__restrict__ B, const T *__restrict__ t1,
-                const T *__restrict__ x, T *__restrict__ y, bool ypad,
-                const T *__restrict__ post) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const long long i = perm[p];
-  const int len = srl[p];
-  const long long base = soff[p >> 5] + (p & 31);
-  T a0 = T(0), a1 = T(0), a2 = T(0);
+// The same term on the tiled copy (TSell): a block loads its tile's distinct
+// input values into shared memory, the transpose scaled by B there (once per
+// value instead of once per entry), and its rows read them by 16-bit places.
+// FIRST: the term's input is pre.in, formed as it is loaded, and t1 = pre.in
+// is written for the terms that follow.  The same multiplies and FMAs per
+// row, in CSR order, as k_fe_sell after k_fe_scale: the same bits.  VPN
+// components a time (of vpn, from c0).  Three components sit three values
+// apart: consecutive places meet no bank twice (padded to four, a 16-byte
+// load each, the FP32 terms took 127 us instead of 110).
+//
+// Measured with 2.56M rows of 27 and three components, against sliced ELL
+// with 32-bit columns and gathers through L1: FP64 forward 336 -> 342 us a
+// term, transpose 645 -> 357 us, both at the FP64 pipe's 0.6 T FMA/s (the
+// transpose no longer multiplies every entry's input by B); FP32 120 -> 109 and
+// 144 -> 110 us, 3.8 TB/s, bound by the shared-memory reads (3 per entry).
+template <typename T, int VPN, bool TR, bool FIRST>
+__global__ void __launch_bounds__(TS_ROWS)
+    k_fe_tile(TSellView M, int vpn, int c0, const T *__restrict__ val, const T *__restrict__ B,
+              const T *__restrict__ pre, T *t1, const T *__restrict__ x, T *__restrict__ y,
+              const T *__restrict__ post) {
+  extern __shared__ __align__(16) unsigned char fe_smem[];
+  T *sx = (T *)fe_smem;
+  const int t = threadIdx.x;
+  const unsigned u0 = M.uoff[blockIdx.x];
+  const int m = (int)(M.uoff[blockIdx.x + 1] - u0);
+  for (int i = t; i < m; i += TS_ROWS) {
+    const long long j = __ldg(M.ucol + u0 + i);
+    const T sc = FIRST ? __ldg(pre + j) : T(1);
+    const T bj = TR ? __ldg(B + j) : T(1);
+    const T *xj = x + j * vpn + c0;
+#pragma unroll
+    for (int v = 0; v < VPN; v++) {
+      T xv = __ldg(xj + v);
+      if (FIRST) xv = fmul(sc, xv);
+      if (TR) xv = fmul(bj, xv);
+      sx[i * VPN + v] = xv;
+    }
+  }
+  __syncthreads();
+  const long long q = (long long)blockIdx.x * TS_ROWS + t;
+  const int i = M.row[q];
+  if (i < 0) return;
+  const int len = M.len[q];
+  const long long base = (long long)M.soff[q >> 5] * 32 + (t & 31);
+  const uint16_t *ip = M.idx + base;
+  const T *vp = val + base;
+  T acc[VPN];
+#pragma unroll
+  for (int v = 0; v < VPN; v++) acc[v] = T(0);
 #pragma unroll 4
   for (int k = 0; k < len; k++) {
-    const int j = __ldg(scol + base + 32LL * k);
-    const T m = __ldg(sval + base + 32LL * k);
-    T xv[4];
-    load4<T>(x + 4LL * j, xv);
-    if (TR) {
-      const T bj = __ldg(B + j);
-      xv[0] = fmul(bj, xv[0]), xv[1] = fmul(bj, xv[1]), xv[2] = fmul(bj, xv[2]);
+    const T *xv = sx + (int)__ldg(ip + 32LL * k) * VPN;
+    const T mv = __ldg(vp + 32LL * k);
+    if constexpr (VPN == 4) {
+      T xr[4];
+      lds4(xv, xr);
+#pragma unroll
+      for (int v = 0; v < VPN; v++) acc[v] = ffma(mv, xr[v], acc[v]);
+    } else {
+#pragma unroll
+      for (int v = 0; v < VPN; v++) acc[v] = ffma(mv, xv[v], acc[v]);
     }
-    a0 = ffma(m, xv[0], a0);
-    a1 = ffma(m, xv[1], a1);
-    a2 = ffma(m, xv[2], a2);
   }
-  T tv[4];
-  load4<T>(t1 + 4 * i, tv);
-  T r0, r1, r2;
-  if (TR) {
-    r0 = fadd(a0, tv[0]), r1 = fadd(a1, tv[1]), r2 = fadd(a2, tv[2]);
-  } else {
-    const T bi = B[i];
-    r0 = fadd(fmul(bi, a0), tv[0]), r1 = fadd(fmul(bi, a1), tv[1]), r2 = fadd(fmul(bi, a2), tv[2]);
-  }
-  if (post) {
-    const T pi = post[i];
-    r0 = fmul(r0, pi), r1 = fmul(r1, pi), r2 = fmul(r2, pi);
-  }
-  if (ypad) {
-    store4<T>(y + 4 * i, r0, r1, r2);
-  } else {
-    y[3 * i] = r0, y[3 * i + 1] = r1, y[3 * i + 2] = r2;
+  const T bi = TR ? T(1) : B[i];
+  const T si = FIRST ? pre[i] : T(1);
+  const T pi = post ? post[i] : T(1);
+#pragma unroll
+  for (int v = 0; v < VPN; v++) {
+    const long long o = (long long)i * vpn + c0 + v;
+    T tv;
+    if (FIRST) {
+      tv = fmul(si, __ldg(x + o));
+      t1[o] = tv;
+    } else {
+      tv = t1[o];
+    }
+    T r = TR ? fadd(acc[v], tv) : fadd(fmul(bi, acc[v]), tv);
+    if (post) r = fmul(r, pi);
+    y[o] = r;
   }
 }
 
@@ -883,37 +888,77 @@ static void launch_sell(const Filter &F, int vpn, const T *B, const T *t1, const
 #undef TMRG_SELL
 }
 
-// applyFilter / applyTranspose for three components per node, padded
-// (k_fe_sell3p); F.N >= 1.
 template <typename T>
-static void horner3p(Filter &F, bool tr, const T *in, T *out, const T *Ainv, const T *B,
-                     const T *Tinv) {
-  cudaStream_t s = F.s;
-  const long long n = F.n;
-  DBuf<T> t1(4 * n, s), ta(4 * n, s), tb(4 * n, s);
-  const T *pre = tr ? Tinv : Ainv;
-  const T *post = tr ? Ainv : Tinv;
-  prof_bytes((long long)sizeof(T) * (3 * n + 4 * n + n));
-  launch(k_fe_scale3p<T>, blocks_for(n, 256), 256, 0, s, n, pre, in, t1.p);
-  const T *sv = sell_vals<T>(F);
-  const T *x = t1.p;
-  for (int k = 0; k < F.N; k++) {
-    const bool last = (k == F.N - 1);
-    T *y = last ? out : ((k % 2 == 0) ? ta.p : tb.p);
-    // compulsory traffic of one term: M (value + column), B, t1 and one read
-    // of x (padded), one write of y (padded, or 3 components)
-    prof_bytes((long long)(sizeof(T) + 4) * F.nnz + 4 * (n + 1) + (long long)sizeof(T) * n +
-               (long long)sizeof(T) * n * (4 + 4 + (last ? 3 : 4)) +
-               (last ? (long long)sizeof(T) * n : 0));
-    prof_flops(6LL * F.nnz);
-    if (tr)
-      launch((k_fe_sell3p<T, true>), blocks_for(n, 256), 256, 0, s, n, (const int *)F.sperm.p,
-             (const int *)F.srl.p, (const long long *)F.soff.p, (const int *)F.scol.p, sv, B,
-             (const T *)t1.p, x, y, !last, last ? post : (const T *)nullptr);
-    else
-      launch((k_fe_sell3p<T, false>), blocks_for(n, 256), 256, 0, s, n, (const int *)F.sperm.p,
-             (const int *)F.srl.p, (const long long *)F.soff.p, (const int *)F.scol.p, sv, B,
-             (const T *)t1.p, x, y, !last, last ? post : (const T *)nullptr);
+static const T *tile_vals(const Filter &F);
+template <>
+const double *tile_vals<double>(const Filter &F) {
+  return F.tval.p;
+}
+template <>
+const float *tile_vals<float>(const Filter &F) {
+  return F.tval32.p;
+}
+// One Horner term on the tiled copy, VPN components from c0.
+template <typename T, int VPN>
+static void launch_tile_term(const Filter &F, bool tr, bool first, int vpn, int c0, const T *B,
+                             const T *pre, T *t1, const T *x, T *y, const T *post,
+                             cudaStream_t s) {
+  const size_t smem = sizeof(T) * VPN * (size_t)F.tiled.maxu;
+  const unsigned g = (unsigned)F.tiled.tiles;
+  const TSellView M = F.tiled.view();
+  // compulsory traffic of one term: M (value + place), the input, t1 and y
+  // once, B
+  prof_bytes((long long)(sizeof(T) + 2) * F.nnz + (long long)sizeof(T) * F.n * (3LL * VPN + 1));
+  prof_flops(2LL * VPN * F.nnz);
+#define TMRG_TILE(TR, FIRST)                                                                 \
+  do {                                                                                       \
+    if (smem > 48 * 1024)                                                                    \
+      TMRG_CUDA(cudaFuncSetAttribute(k_fe_tile<T, VPN, TR, FIRST>,                           \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    launch((k_fe_tile<T, VPN, TR, FIRST>), g, TS_ROWS, smem, s, M, vpn, c0, tile_vals<T>(F), B, \
+           pre, t1, x, y, post);                                                             \
+  } while (0)
+  if (tr) {
+    if (first) TMRG_TILE(true, true); else TMRG_TILE(true, false);
+  } else {
+    if (first) TMRG_TILE(false, true); else TMRG_TILE(false, false);
+  }
+#undef TMRG_TILE
+}
+static bool overlap(const void *a, const void *b, size_t bytes) {
+  const uintptr_t p = (uintptr_t)a, q = (uintptr_t)b;
+  return p < q + bytes && q < p + bytes;
+}
+// applyFilter / applyTranspose on the tiled copy (F.N > 0); t1 and tmp hold
+// n * vpn values.  Where `in` and `out` overlap t1 is formed before any term
+// writes.
+template <typename T>
+static void horner_tiled(const Filter &F, bool tr, int vpn, const T *in, T *out, T *t1, T *tmp,
+                         const T *Ainv, const T *B, const T *Tinv, cudaStream_t s) {
+  const long long len = F.n * vpn;
+  const T *pre = tr ? Tinv : Ainv, *post = tr ? Ainv : Tinv;
+  const T *x = in;
+  bool first = true;
+  if (overlap(in, out, sizeof(T) * len)) {
+    prof_bytes(2LL * sizeof(T) * len + (long long)sizeof(T) * F.n);
+    launch(k_fe_scale<T>, blocks_for(len, 256), 256, 0, s, F.n, vpn, pre, in, t1);
+    x = t1;
+    first = false;
+  }
+  for (int k = 0; k < F.N; k++, first = false) {
+    const T *last = k == F.N - 1 ? post : nullptr;
+    T *y = ((F.N - 1 - k) % 2 == 0) ? out : tmp;
+    for (int c0 = 0; c0 < vpn; c0 += 4) {
+      const int nc = std::min(4, vpn - c0);
+      if (nc == 1)
+        launch_tile_term<T, 1>(F, tr, first, vpn, c0, B, pre, t1, x, y, last, s);
+      else if (nc == 2)
+        launch_tile_term<T, 2>(F, tr, first, vpn, c0, B, pre, t1, x, y, last, s);
+      else if (nc == 3)
+        launch_tile_term<T, 3>(F, tr, first, vpn, c0, B, pre, t1, x, y, last, s);
+      else
+        launch_tile_term<T, 4>(F, tr, first, vpn, c0, B, pre, t1, x, y, last, s);
+    }
     x = y;
   }
 }
@@ -926,27 +971,11 @@ static void horner_generic(Filter &F, bool tr, int vpn, const T *in, T *out, con
 template <typename T>
 static void horner(Filter &F, bool tr, int vpn, const T *in, T *out, const T *Ainv,
                    const T *B, const T *Tinv) {
-  cudaStream_t s = F.s;
-  const long long n = F.n;
-  if (n == 0) return;
-  if (vpn == 3 && F.N > 0) {
-    // three components: padded (candidate 0) or sliced-ELL with three
-    // scalar loads per neighbour (candidate 1), chosen by the autotuner per
-    // precision and size (both give the same bits)
-    int lr = 0;
-    while ((1LL << (lr + 1)) <= n) lr++;
-    const TuneKey key{sizeof(T) == 4 ? TUNE_FILTER3_F32 : TUNE_FILTER3_F64, lr, (int)tr, 0, 0, 0};
-    auto run = [&](int c) {
-      if (c == 0)
-        horner3p<T>(F, tr, in, out, Ainv, B, Tinv);
-      else
-        horner_generic<T>(F, tr, vpn, in, out, Ainv, B, Tinv);
-    };
-    // tuning runs the apply several times: not on an in-place call
-    if ((const void *)in == (const void *)out)
-      run(tune_lookup(key));
-    else
-      tune_run(key, 2, run, s);
+  const long long len = F.n * vpn;
+  if (len == 0) return;
+  if (F.tiled.ok && F.N > 0) {
+    DBuf<T> t1(len, F.s), tmp(F.N > 1 ? len : 0, F.s);
+    horner_tiled<T>(F, tr, vpn, in, out, t1.p, tmp.p, Ainv, B, Tinv, F.s);
     return;
   }
   horner_generic<T>(F, tr, vpn, in, out, Ainv, B, Tinv);
@@ -1040,6 +1069,10 @@ void filter_apply_static(Filter &F, bool tr, int vpn, const double *in, double *
   double *tmp = t1 + FILTER_STATIC_MAX;
   if (n == 0) return;
   cudaStream_t s = F.s;
+  if (F.tiled.ok && F.N > 0) {
+    horner_tiled<double>(F, tr, vpn, in, out, t1, tmp, F.Ainv.p, F.B.p, F.Tinv.p, s);
+    return;
+  }
   const double *pre = tr ? F.Tinv.p : F.Ainv.p;
   const double *post = tr ? F.Ainv.p : F.Tinv.p;
   prof_bytes(2LL * sizeof(double) * len + (long long)sizeof(double) * n);
@@ -1298,8 +1331,12 @@ static void filter_build(const FSource &f, double len, double r, int N, Filter &
   F.Tinv.alloc(n, s);
   launch(k_fe_scalings, blocks_for(n, 256), 256, 0, s, n, f.dim, (const int *)F.rowptr.p,
          (const double *)F.vals.p, r, F.Ainv.p, F.B.p);
-  // the sliced-ELL copy the Horner steps read
-  {
+  // the copy the Horner steps read: tiled, or sliced with 32-bit columns
+  // where a tile has too many
+  if (tsell_build(F.tiled, n, F.rowptr.p, F.colidx.p, s)) {
+    tsell_values(F.tiled, F.rowptr.p, (const double *)F.vals.p, F.tval, s);
+    tsell_values(F.tiled, F.rowptr.p, (const double *)F.vals.p, F.tval32, s);
+  } else {
     const long long nsl = (n + 31) / 32;
     F.npos = nsl * 32;
     F.sperm.alloc(std::max(1LL, n), s);
@@ -1325,9 +1362,11 @@ static void filter_build(const FSource &f, double len, double r, int N, Filter &
            F.Tinv.p);
     TMRG_CUDA(cudaStreamSynchronize(s));
   }
-  F.sval32.alloc(std::max(1LL, F.nsell), s);
-  launch(k_to_f32<float>, blocks_for(F.nsell, 256), 256, 0, s, F.nsell,
-         (const double *)F.sval.p, F.sval32.p);
+  if (!F.tiled.ok) {
+    F.sval32.alloc(std::max(1LL, F.nsell), s);
+    launch(k_to_f32<float>, blocks_for(F.nsell, 256), 256, 0, s, F.nsell,
+           (const double *)F.sval.p, F.sval32.p);
+  }
   F.Ainv32.alloc(n, s);
   F.B32.alloc(n, s);
   F.Tinv32.alloc(n, s);

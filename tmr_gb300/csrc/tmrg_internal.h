@@ -10,6 +10,7 @@
 
 #include "tmrg_common.cuh"
 #include "tmrg_prims.cuh"
+#include "tmrg_tsell.cuh"
 
 namespace tmrg {
 
@@ -132,6 +133,9 @@ struct Interp {
 
 struct Filter {
   cudaStream_t s = 0;
+  TSell tiled;
+  DBuf<double> tval;
+  DBuf<float> tval32;
   long long n = 0, nnz = 0;
   int N = 10;
   double r = 0.0;
@@ -139,7 +143,8 @@ struct Filter {
   DBuf<double> vals;
   DBuf<double> Ainv, B, Tinv;
   DBuf<float> Ainv32, B32, Tinv32;
-  // M as sliced ELL for the Horner steps: rows in length order inside
+  // M for the Horner steps: tiled (values of both precisions), or where a
+  // tile has too many columns as sliced ELL: rows in length order inside
   // 4096-row windows (sperm, with each position's row length in srl),
   // slices of 32 positions stored entry-major from soff[slice], so a warp
   // reads its rows' k-th entries as one contiguous run

@@ -470,8 +470,6 @@ struct TuneKey {
 enum TuneKind {
   TUNE_P = 1,
   TUNE_PT = 2,
-  TUNE_FILTER3_F32 = 3,
-  TUNE_FILTER3_F64 = 4,
   TUNE_RADIX = 5
 };
 int tune_run(const TuneKey &k, int ncand, const std::function<void(int)> &run,
