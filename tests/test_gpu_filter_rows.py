@@ -151,13 +151,13 @@ def test_terms_of_tiles_match_horner(gpu_lib, dtype, N, vpn):
 
 
 def test_terms_of_a_tile_with_too_many_columns(gpu_lib):
-    # a node in 1100 blocks: its row alone has 4402 columns, more than a tile
+    # a node in 2000 blocks: its row alone has 8002 columns, more than a tile
     # may have, and the sliced copy runs
     import torch
 
     from tmr_gb300 import TMR
     f = TMR.OctForest(order=2)
-    f.setConnectivity(_fan(1100))
+    f.setConnectivity(_fan(2000))
     f.createTrees(0)
     f.createNodes()
     F = TMR.MatrixFilter(0.5, 4, None, [f])

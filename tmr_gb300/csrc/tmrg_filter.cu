@@ -20,12 +20,11 @@
 #include <string>
 
 #include "tmrg_quad.h"
+#include "tmrg_rowasm.cuh"
 #include "tmrg_tree.cuh"
 #include "tmrg_tsell.cuh"
 
 namespace tmrg {
-
-constexpr int FMAXK = 27;  // distinct independent nodes one element touches
 
 struct FilterCtx {
   const int *conn;
@@ -37,335 +36,27 @@ struct FilterCtx {
   int npe, dim;  // 8 and 3 (octree) or 4 and 2 (quadtree)
 };
 
-// Merged element block: distinct nodes U[0..K) in first-appearance order
-// and L[u][v] summed over (a, b, p, q) in loop order.
-__device__ int element_block(const FilterCtx &c, long long e, int *U,
-                             double (*L)[FMAXK]) {
-  const int npe = c.npe;
-  const int *ec = c.conn + e * npe;
-  int ni[8][4];
-  double nw[8][4];
-  int nc[8];
-  int K = 0;
-  for (int a = 0; a < npe; a++) {
-    int g = ec[a];
-    if (g >= 0) {
-      nc[a] = 1;
-      ni[a][0] = g;
-      nw[a][0] = 1.0;
-    } else {
-      int d = -g - 1;
-      int p0 = c.dptr[d], p1 = c.dptr[d + 1];
-      nc[a] = p1 - p0;
-      if (nc[a] > 4) {
-        atomicExch(c.err, 1);
-        nc[a] = 4;
-      }
-      for (int p = 0; p < nc[a]; p++) {
-        ni[a][p] = c.dconn[p0 + p];
-        nw[a][p] = c.dw[p0 + p];
-      }
-    }
-    for (int p = 0; p < nc[a]; p++) {
-      int u = 0;
-      while (u < K && U[u] != ni[a][p]) u++;
-      if (u == K) {
-        if (K == FMAXK) {
-          atomicExch(c.err, 1);
-          return K;
-        }
-        U[K++] = ni[a][p];
-      }
-    }
-  }
-  if (!L) return K;
-  for (int u = 0; u < K; u++)
-    for (int v = 0; v < K; v++) L[u][v] = 0.0;
-  double side = c.block_len / (double)(1 << c.lev[e]);
-  double s3 = __dmul_rn(__dmul_rn(side, side), side);
-  const double s2 = __dmul_rn(side, side);
-  // exact mass of the linear element (corner a = i + 2j + 4k): the 1-D
-  // entries s/3 and s/6 multiplied over the directions, nd of which differ
-  for (int a = 0; a < npe; a++)
-    for (int b = 0; b < npe; b++) {
-      int nd = ((a ^ b) & 1) + (((a ^ b) >> 1) & 1) + ((a ^ b) >> 2);
-      double mab = c.dim == 3 ? __ddiv_rn(s3, 27.0 * (double)(1 << nd))
-                              : __ddiv_rn(s2, 9.0 * (double)(1 << nd));
-      for (int p = 0; p < nc[a]; p++) {
-        int u = 0;
-        while (U[u] != ni[a][p]) u++;
-        double t = __dmul_rn(mab, nw[a][p]);
-        for (int q = 0; q < nc[b]; q++) {
-          int v = 0;
-          while (U[v] != ni[b][q]) v++;
-          L[u][v] = __dadd_rn(L[u][v], __dmul_rn(t, nw[b][q]));
-        }
-      }
-    }
-  return K;
-}
-
-// ---------------------------------------------------------------------
-// M by rows (order 2).  Sorting every block entry by (row, column) moves K^2
-// records of 20 bytes per element through 5 or more passes; here only the K
-// block rows of an element are sorted, by their node, and a row adds its
-// block rows into a hash table in shared memory, element after element (the
-// order of the sums is that of the sorted entries, hence the same bits).
-// An element without dependent nodes needs no stored block: its entries are
-// the level's mass over 2^nd, by exponent arithmetic.
-// Bound by the probes and the rank pass of the small rows (1.9 ms for 2.56M
-// rows of 27 columns) and by local memory in the hanging elements' blocks
-// (0.8 ms); building this filter with its restrictions and filtering once
-// went from 23.0 to 13.1 ms, 14.9 of the 23.0 the sort and its passes.
-struct RowAsm {
-  const int *conn;
+// The entries of M (assemble_rows): the exact mass of the linear element
+// (corner a = i + 2j + 4k), the 1-D entries s/3 and s/6 multiplied over the
+// directions, nd of which differ.  A side is block_len over a power of two,
+// so an element's entry is the unit block's with a smaller exponent.
+struct MassEntry {
+  double block_len;
   const int16_t *lev;
-  int npe, dim;
-  unsigned long long m0;    // bits of the mass entry of a unit block, nd = 0
-  const unsigned *hoff;     // per element: place among the hanging ones
-  const unsigned *ucnt;     // per hanging element: first of its distinct nodes,
-  const unsigned *boff;     // and of its block
-  const int *unode;
-  const double *block;
-  const unsigned *srp;      // per node: its block rows in `slot`,
-  const uint32_t *slot;     // element << 5 | block row, elements ascending
-  __device__ __forceinline__ bool hanging(unsigned e) const {
-    return hoff[e + 1] != hoff[e];
+  int dim;
+  unsigned long long m0;  // bits of the unit block's entry, nd = 0
+  __device__ __forceinline__ double direct(long long e, int a, int b) const {
+    const double side = block_len / (double)(1 << lev[e]);
+    const double s2 = __dmul_rn(side, side);
+    const int nd = __popc((unsigned)(a ^ b));
+    return dim == 3 ? __ddiv_rn(__dmul_rn(s2, side), 27.0 * (double)(1 << nd))
+                    : __ddiv_rn(s2, 9.0 * (double)(1 << nd));
   }
-  __device__ __forceinline__ int nodes(unsigned e) const {
-    if (!hanging(e)) return npe;
-    const unsigned h = hoff[e];
-    return (int)(ucnt[h + 1] - ucnt[h]);
+  __device__ __forceinline__ double regular(unsigned e, unsigned x) const {
+    return __longlong_as_double((long long)(
+        m0 - ((unsigned long long)(dim * __ldg(lev + e) + __popc(x)) << 52)));
   }
 };
-// Elements with a stored block: those with a dependent node, or with one
-// node twice (a collapsed block), or all of them (`all`).
-__global__ void k_fa_hanging(long long ne, int npe, const int *__restrict__ conn, int all,
-                             unsigned *flag) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  bool h = all != 0;
-  int g[8];
-#pragma unroll
-  for (int a = 0; a < 8; a++) {
-    g[a] = a < npe ? __ldg(conn + e * npe + a) : 0;
-    if (a < npe) h |= g[a] < 0;
-#pragma unroll
-    for (int b = 0; b < a; b++) h |= a < npe && g[a] == g[b];
-  }
-  flag[e] = h ? 1u : 0u;
-}
-__global__ void k_fa_list(long long ne, const unsigned *__restrict__ hoff, unsigned *list) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < ne && hoff[e + 1] != hoff[e]) list[hoff[e]] = (unsigned)e;
-}
-__global__ void k_fa_count(long long nh, FilterCtx c, const unsigned *__restrict__ list,
-                           unsigned *ucnt, unsigned *bcnt) {
-  const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= nh) return;
-  int U[FMAXK];
-  const int K = element_block(c, list[h], U, nullptr);
-  ucnt[h] = (unsigned)K;
-  bcnt[h] = (unsigned)(K * K);
-}
-__global__ void __launch_bounds__(64)
-    k_fa_blocks(long long nh, FilterCtx c, const unsigned *__restrict__ list,
-                const unsigned *__restrict__ uoff, const unsigned *__restrict__ boff, int *unode,
-                double *block) {
-  const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= nh) return;
-  int U[FMAXK];
-  double L[FMAXK][FMAXK];
-  const int K = element_block(c, list[h], U, L);
-  const unsigned u0 = uoff[h], b0 = boff[h];
-  for (int u = 0; u < K; u++) {
-    unode[u0 + u] = U[u];
-    for (int v = 0; v < K; v++) block[b0 + u * K + v] = L[u][v];
-  }
-}
-// Block rows of every element (soff: their scanned counts) by node.
-__global__ void k_fa_slot_count(long long ne, RowAsm A, unsigned *cnt) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < ne) cnt[e] = (unsigned)A.nodes((unsigned)e);
-}
-__global__ void k_fa_slots(long long ne, RowAsm A, const unsigned *__restrict__ soff,
-                           uint32_t *keys, uint32_t *vals) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const unsigned o = soff[e];
-  const int K = (int)(soff[e + 1] - o);
-  const int *U = A.hanging((unsigned)e) ? A.unode + A.ucnt[A.hoff[e]] : A.conn + e * A.npe;
-  for (int u = 0; u < K; u++) {
-    keys[o + u] = (uint32_t)U[u];
-    vals[o + u] = (uint32_t)e << 5 | (uint32_t)u;
-  }
-}
-// first[j] = first sorted block row of a node >= j
-__global__ void k_fa_starts(long long n, long long E, const uint32_t *__restrict__ keys,
-                            unsigned *first) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > E) return;
-  const long long k = i < E ? (long long)keys[i] : n;
-  for (long long j = i ? (long long)keys[i - 1] + 1 : 0; j <= k; j++) first[j] = (unsigned)i;
-}
-// Entries each row has to add; rows with more than FA_SMALL go to `large`.
-constexpr int FA_SMALL = 64;         // 8 elements of 8 nodes
-// A large row's table: slots and rows per block of the first attempt, and of
-// the one that follows where some row has more columns (in a 2:1 balanced
-// forest none has).
-constexpr int FA_LARGE = 512, FA_LARGE_WARPS = 4;
-constexpr int FA_HUGE = 8192, FA_HUGE_WARPS = 1;
-constexpr size_t FA_SLOT_BYTES = sizeof(double) + sizeof(int) + sizeof(uint16_t);
-__global__ void k_fa_candidates(long long n, RowAsm A, unsigned *cand, unsigned *large,
-                                unsigned *nlarge) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned t = 0;
-  if (i < n) {
-    for (unsigned p = A.srp[i]; p < A.srp[i + 1]; p++) t += (unsigned)A.nodes(A.slot[p] >> 5);
-    cand[i] = t;
-  }
-  const unsigned m = __ballot_sync(0xffffffffu, t > FA_SMALL);
-  if (m == 0u) return;
-  const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
-  unsigned o = 0;
-  if (lane == lead) o = atomicAdd(nlarge, (unsigned)__popc(m));
-  o = __shfl_sync(0xffffffffu, o, lead);
-  if (t > FA_SMALL) large[o + __popc(m & ((1u << lane) - 1u))] = (unsigned)i;
-}
-// One row by G lanes (the whole warp calls it) over a table of `slots` slots (a
-// power of two): the sorted columns and sums go to col / val, their number
-// is returned; *err = FA_FULL when the row has more columns than the table.
-constexpr int FA_FULL = 2;
-template <int G>
-__device__ __forceinline__ int assemble_row(const RowAsm &A, long long row, bool have,
-                                            int slots, int *tcol, double *tval, uint16_t *tidx, int *col,
-                                            double *val, int *err) {
-  const int lane = threadIdx.x & 31, l = lane & (G - 1);
-  for (int i = l; i < slots; i += G) {
-    tcol[i] = -1;
-    tval[i] = 0.0;
-  }
-  __syncwarp();
-  const unsigned p0 = have ? A.srp[row] : 0, p1 = have ? A.srp[row + 1] : 0;
-  unsigned steps = p1 - p0;
-#pragma unroll
-  for (int o = G; o < 32; o <<= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, o));
-  bool full = false;
-  for (unsigned k = 0; k < steps; k++) {
-    const bool on = p0 + k < p1;
-    unsigned e = 0, u = 0;
-    int K = 0;
-    bool hang = false;
-    if (on) {
-      const unsigned s = __ldg(A.slot + p0 + k);
-      e = s >> 5;
-      u = s & 31u;
-      hang = A.hanging(e);
-      K = A.npe;
-    }
-    const int *U = A.conn + (long long)e * A.npe;
-    const double *B = nullptr;
-    if (hang) {
-      const unsigned h = A.hoff[e], u0 = A.ucnt[h];
-      K = (int)(A.ucnt[h + 1] - u0);
-      U = A.unode + u0;
-      B = A.block + A.boff[h] + u * K;
-    }
-    for (int v = l; v < K; v += G) {  // an element's nodes are distinct
-      const int c = __ldg(U + v);
-      double m;
-      if (hang) {
-        m = __ldg(B + v);
-      } else {
-        const int nd = __popc(u ^ (unsigned)v);
-        m = __longlong_as_double((long long)(
-            A.m0 - ((unsigned long long)(A.dim * __ldg(A.lev + e) + nd) << 52)));
-      }
-      unsigned h = ((unsigned)c * 0x9E3779B1u) >> 16 & (unsigned)(slots - 1);
-      int it = 0;
-      for (; it < slots; it++) {
-        int was = *(volatile int *)(tcol + h);
-        if (was == -1) was = atomicCAS(tcol + h, -1, c);
-        if (was == -1 || was == c) break;
-        h = (h + 1) & (unsigned)(slots - 1);
-      }
-      if (it == slots)
-        full = true;
-      else
-        tval[h] = __dadd_rn(tval[h], m);
-    }
-    __syncwarp();
-  }
-  if (full) atomicExch(err, FA_FULL);
-  // the taken slots, then each one's rank among their columns
-  int n = 0;
-  const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (lane & ~(G - 1));
-  for (int i = l; i < slots; i += G) {
-    const bool taken = tcol[i] >= 0;
-    const unsigned m = __ballot_sync(0xffffffffu, taken) & gmask;
-    if (taken) tidx[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
-    n += __popc(m);
-  }
-  __syncwarp();
-  for (int i = l; i < n; i += G) {
-    const int s = tidx[i], c = tcol[s];
-    int r = 0;
-    for (int j = 0; j < n; j++) r += tcol[tidx[j]] < c;
-    col[r] = c;
-    val[r] = tval[s];
-  }
-  return n;
-}
-// Rows of at most FA_SMALL entries: 8 lanes each (7-8 elements of 8 nodes
-// keep every lane busy).
-__global__ void __launch_bounds__(128)
-    k_fa_rows_small(long long n, RowAsm A, const unsigned *__restrict__ coff, int *col,
-                    double *val, int *len, int *err) {
-  __shared__ int tcol[16][FA_SMALL];
-  __shared__ double tval[16][FA_SMALL];
-  __shared__ uint16_t tidx[16][FA_SMALL];
-  const int g = threadIdx.x >> 3;
-  const long long row = (long long)blockIdx.x * 16 + g;
-  const unsigned o = row < n ? coff[row] : 0, o1 = row < n ? coff[row + 1] : 0;
-  const bool have = row < n && o1 - o <= FA_SMALL;
-  const int m = assemble_row<8>(A, row, have, FA_SMALL, tcol[g], tval[g], tidx[g], col + o,
-                                val + o, err);
-  if (have && (threadIdx.x & 7) == 0) len[row] = m;
-}
-// The others: a warp each, `warps` rows per block.
-__global__ void __launch_bounds__(FA_LARGE_WARPS * 32)
-    k_fa_rows_large(const unsigned *__restrict__ nlarge, const unsigned *__restrict__ list,
-                    int slots, int warps, RowAsm A, const unsigned *__restrict__ coff, int *col,
-                    double *val, int *len, int *err) {
-  extern __shared__ __align__(16) unsigned char fa_smem[];
-  const int w = threadIdx.x >> 5;
-  double *tval = (double *)fa_smem + (size_t)w * slots;
-  int *tcol = (int *)((double *)fa_smem + (size_t)warps * slots) + (size_t)w * slots;
-  uint16_t *tidx = (uint16_t *)((int *)((double *)fa_smem + (size_t)warps * slots) +
-                                (size_t)warps * slots) + (size_t)w * slots;
-  const unsigned m = *nlarge;
-  for (unsigned i = blockIdx.x * warps + w; i < m; i += gridDim.x * warps) {
-    const long long row = list[i];
-    const unsigned o = coff[row];
-    const int c = assemble_row<32>(A, row, true, slots, tcol, tval, tidx, col + o, val + o, err);
-    if ((threadIdx.x & 31) == 0) len[row] = c;
-    __syncwarp();
-  }
-}
-// Rows from their places to CSR, 8 lanes per row.
-__global__ void k_fa_compact(long long n, const unsigned *__restrict__ coff,
-                             const int *__restrict__ rp, const int *__restrict__ col,
-                             const double *__restrict__ val, int *ocol, double *oval) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long row = t >> 3;
-  if (row >= n) return;
-  const unsigned o = coff[row];
-  const int p0 = rp[row], m = rp[row + 1] - p0;
-  for (int k = (int)(t & 7); k < m; k += 8) {
-    ocol[p0 + k] = col[o + k];
-    oval[p0 + k] = val[o + k];
-  }
-}
 
 // Sum each run of equal (row, col) keys in element order.
 __global__ void k_fe_reduce(long long E, const uint64_t *__restrict__ keys,
@@ -1210,104 +901,6 @@ static void assemble_sorted(const FSource &f, const FilterCtx &c, int cb, Filter
   exclusive_scan<int>(F.rowptr.p, F.rowptr.p, n, s);
 }
 
-// M by rows (order 2; RowAsm).
-static void assemble_rows(const FSource &f, const FilterCtx &c, int cb, Filter &F) {
-  cudaStream_t s = f.s;
-  const long long n = f.nn, ne = f.ne;
-  if (ne >= (1LL << 27)) throw Error(TMRG_ERR_KEY_RANGE, "matrix filter: too many elements");
-  RowAsm A{};
-  A.conn = f.econn;
-  A.lev = f.level;
-  A.npe = f.npe;
-  A.dim = f.dim;
-  const double len = c.block_len;
-  // the mass entry of a unit block: element sides are len over a power of
-  // two, so an element's entry is this one with a smaller exponent
-  const double m0 = f.dim == 3 ? len * len * len / 27.0 : len * len / 9.0;
-  memcpy(&A.m0, &m0, sizeof(m0));
-  // hanging elements: their distinct nodes and blocks
-  DBuf<unsigned> hoff(ne + 1, s);
-  // (far from the ends of the exponent's range, where an entry of a deep
-  // level might not be the scaled one: 3 x 30 levels and nd <= 3)
-  const int ex = (int)((A.m0 >> 52) & 0x7ff);
-  const int all = ex < 128 || ex == 0x7ff;
-  launch(k_fa_hanging, blocks_for(ne, 256), 256, 0, s, ne, f.npe, f.econn, all, hoff.p);
-  exclusive_scan<unsigned>(hoff.p, hoff.p, ne, s);
-  const long long nh = read_scalar(hoff.p + ne, s);
-  DBuf<unsigned> list(nh + 1, s), ucnt(nh + 1, s), boff(nh + 1, s);
-  launch(k_fa_list, blocks_for(ne, 256), 256, 0, s, ne, (const unsigned *)hoff.p, list.p);
-  launch(k_fa_count, blocks_for(nh, 128), 128, 0, s, nh, c, (const unsigned *)list.p, ucnt.p,
-         boff.p);
-  exclusive_scan<unsigned>(ucnt.p, ucnt.p, nh, s);
-  exclusive_scan<unsigned>(boff.p, boff.p, nh, s);
-  const unsigned *hp[2] = {ucnt.p + nh, boff.p + nh};
-  unsigned hv[2];
-  read_scalars(hp, hv, s);
-  DBuf<int> unode((size_t)hv[0] + 1, s);
-  DBuf<double> block((size_t)hv[1] + 1, s);
-  launch(k_fa_blocks, blocks_for(nh, 64), 64, 0, s, nh, c, (const unsigned *)list.p,
-         (const unsigned *)ucnt.p, (const unsigned *)boff.p, unode.p, block.p);
-  list.release();
-  A.hoff = hoff.p;
-  A.ucnt = ucnt.p;
-  A.boff = boff.p;
-  A.unode = unode.p;
-  A.block = block.p;
-  // block rows sorted by node, elements ascending
-  DBuf<unsigned> soff(ne + 1, s);
-  launch(k_fa_slot_count, blocks_for(ne, 256), 256, 0, s, ne, A, soff.p);
-  exclusive_scan<unsigned>(soff.p, soff.p, ne, s);
-  const long long ns = (long long)(ne - nh) * f.npe + hv[0];
-  DBuf<uint32_t> skey(ns, s), slot(ns, s);
-  launch(k_fa_slots, blocks_for(ne, 256), 256, 0, s, ne, A, (const unsigned *)soff.p, skey.p,
-         slot.p);
-  soff.release();
-  radix_sort(skey, &slot, ns, cb, s);
-  DBuf<unsigned> srp(n + 1, s);
-  launch(k_fa_starts, blocks_for(ns + 1, 256), 256, 0, s, n, ns, (const uint32_t *)skey.p, srp.p);
-  skey.release();
-  A.srp = srp.p;
-  A.slot = slot.p;
-  // rows, each at its number of entries before equal columns are added
-  const long long E = (long long)(ne - nh) * f.npe * f.npe + hv[1];
-  if (E >= (1LL << 32))
-    throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
-  DBuf<unsigned> coff(n + 1, s), large(n + 1, s), nlarge(1, s);
-  nlarge.zero();
-  launch(k_fa_candidates, blocks_for(n, 256), 256, 0, s, n, A, coff.p, large.p, nlarge.p);
-  exclusive_scan<unsigned>(coff.p, coff.p, n, s);
-  DBuf<int> col(E + 1, s);
-  DBuf<double> val(E + 1, s);
-  F.rowptr.alloc(n + 1, s);
-  DBuf<int> ncol(n + 1, s);
-  launch(k_fa_rows_small, blocks_for(n, 16), 128, 0, s, n, A, (const unsigned *)coff.p, col.p,
-         val.p, ncol.p, c.err);
-  auto rows = [&](int slots, int warps) {
-    const size_t smem = FA_SLOT_BYTES * slots * warps;
-    TMRG_CUDA(cudaFuncSetAttribute(k_fa_rows_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(FA_SLOT_BYTES * FA_HUGE * FA_HUGE_WARPS)));
-    launch(k_fa_rows_large, std::min(blocks_for(n, warps), 152u * 8), warps * 32, smem, s,
-           (const unsigned *)nlarge.p, (const unsigned *)large.p, slots, warps, A,
-           (const unsigned *)coff.p, col.p, val.p, ncol.p, c.err);
-    exclusive_scan<int>(ncol.p, F.rowptr.p, n, s);
-    const int *pv[2] = {F.rowptr.p + n, c.err};
-    int hv2[2];
-    read_scalars(pv, hv2, s);
-    F.nnz = hv2[0];
-    return hv2[1];
-  };
-  if (rows(FA_LARGE, FA_LARGE_WARPS) == FA_FULL) {
-    TMRG_CUDA(cudaMemsetAsync(c.err, 0, sizeof(int), s));
-    rows(FA_HUGE, FA_HUGE_WARPS);
-  }
-  const long long nnz = F.nnz;
-  F.colidx.alloc(nnz + 1, s);
-  F.vals.alloc(nnz + 1, s);
-  launch(k_fa_compact, blocks_for(n * 8, 256), 256, 0, s, n, (const unsigned *)coff.p,
-         (const int *)F.rowptr.p, (const int *)col.p, (const double *)val.p, F.colidx.p,
-         F.vals.p);
-}
-
 static void filter_build(const FSource &f, double len, double r, int N, Filter &F) {
   cudaStream_t s = f.s;
   F.s = s;
@@ -1320,10 +913,22 @@ static void filter_build(const FSource &f, double len, double r, int N, Filter &
   FilterCtx c{f.econn, f.dptr, f.dconn, f.dw, len, f.level, err.p, f.npe, f.dim};
   const int cb = bits_for(n + 1);
   if (2 * cb > 64) throw Error(TMRG_ERR_KEY_RANGE, "filter key range");
-  if (f.order == 2)
-    assemble_rows(f, c, cb, F);
-  else
+  if (f.order == 2) {
+    MassEntry ent{len, f.level, f.dim, 0};
+    const double m0 = f.dim == 3 ? len * len * len / 27.0 : len * len / 9.0;
+    memcpy(&ent.m0, &m0, sizeof(m0));
+    // near the ends of the exponent's range an entry of a deep level might
+    // not be the scaled one (3 x 30 levels and nd <= 3)
+    const int ex = (int)((ent.m0 >> 52) & 0x7ff);
+    if (!assemble_rows(ElemCtx{c.conn, c.dptr, c.dconn, c.dw, c.err, c.npe}, ent, n, ne,
+                       ex < 128 || ex == 0x7ff, F.rowptr, F.colidx, F.vals, F.nnz, s)) {
+      if (read_scalar(err.p, s))
+        throw Error(TMRG_ERR_INTERNAL, "matrix filter: element touches too many nodes");
+      throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
+    }
+  } else {
     assemble_sorted(f, c, cb, F);
+  }
   if (read_scalar(err.p, s))
     throw Error(TMRG_ERR_INTERNAL, "matrix filter: element touches too many nodes");
   F.Ainv.alloc(n, s);

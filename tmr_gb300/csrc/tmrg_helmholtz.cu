@@ -30,13 +30,22 @@
 //   FP32 at 64 times its FP64 rate, and the FP64 outer iteration still
 //   drives the true residual to the reference's tolerance.  The smoother is
 //   Chebyshev on D^-1 K over [lower, 1.1] lmax (lmax from Lanczos; degree
-//   5 and lower 0.05 for order-2 levels, degree 6 and lower 0.1 for order
-//   3, the settings that solved the measured filter hierarchies fastest),
+//   3 and lower 0.2 for order-2 levels, degree 6 and lower 0.1 for order 3;
+//   per solve of 2.1M nodes, degree 5 from 0.05 against 3 from 0.2: r = 2 h
+//   12.3 and 7.5 ms, r = 32 h 12.3 and 8.7 ms, with 7 and 6 or 7 iterations;
+//   on scattered refinement at r = 32 h 4.1 and 4.6 ms, all else faster),
 //   which is parallel where SOR is sequential.  Restriction and prolongation are the forests' own
 //   createInterpolation operators (P^T and P); coarse levels are
 //   rediscretised, as in the reference (use_galerkin = 0).  The coarsest
 //   level is solved with its explicit dense inverse (Gauss-Jordan on the
 //   GPU) when it has at most HM_DENSE_MAX nodes, else by Chebyshev sweeps.
+// * Linear elements on all levels but a dense coarsest one: K is assembled
+//   (assemble_rows) and kept on tiles (TSell), FP32 for the smoother and also
+//   FP64 on the finest level; one kernel then does a product with K and the
+//   Chebyshev or residual update that follows it (k_ht).  27 multiply-adds a
+//   row cost less than the element operator's 140 an element, its slot values
+//   and the scatter: an FP32 step 145 + 25 (update) -> 95 us, an FP64 product
+//   690 -> 123 us at 2.1M nodes.  Quadratic elements keep the element operator.
 // * All design components are solved together: vectors are node-major
 //   with `nvec` interleaved components and every scalar of the iteration is
 //   kept per component.
@@ -47,11 +56,13 @@
 
 #include "tmrg_helmholtz.h"
 #include "tmrg_quad.h"
+#include "tmrg_rowasm.cuh"
+#include "tmrg_tsell.cuh"
 
 namespace tmrg {
 
 constexpr int HM_THREADS = 128;
-constexpr int HM_RED_BLOCKS = 304;  // 2 per SM
+constexpr int HM_RED_BLOCKS = 1216;  // 8 per SM
 constexpr int HM_MAXVEC = 16;
 
 // ---------------------------------------------------------------------
@@ -413,18 +424,201 @@ __global__ void k_h_scatter(long long nn, int nvec, const int *__restrict__ rp,
     out[i] -= s;
 }
 
-// y = A x for a CSR matrix (thread per row and component).
+// y = A x (add: y += A x) for a CSR matrix: 2^LB lanes per row and component
+// take its entries in turn and combine in a fixed tree.
 template <typename T>
-__global__ void k_h_csr(long long nrows, int nvec, const int *__restrict__ rp,
+__global__ void k_h_csr(long long nrows, int nvec, int LB, const int *__restrict__ rp,
                         const int *__restrict__ ci, const T *__restrict__ v,
-                        const T *__restrict__ x, T *y) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nrows * nvec) return;
-  long long j = i / nvec;
-  int c = (int)(i - j * nvec);
+                        const T *__restrict__ x, T *y, int add) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long i = t >> LB;
+  const int L = 1 << LB, l = (int)t & (L - 1);
+  const bool have = i < nrows * nvec;
+  const long long j = nvec == 1 ? i : i / nvec;
+  const int c = (int)(i - j * nvec);
+  const int p0 = have ? rp[j] : 0, p1 = have ? rp[j + 1] : 0;
   T s = T(0);
-  for (int p = rp[j]; p < rp[j + 1]; p++) s = fma(v[p], x[(long long)ci[p] * nvec + c], s);
-  y[i] = s;
+#pragma unroll 2
+  for (int p = p0 + l; p < p1; p += L) s = fma(v[p], x[(long long)ci[p] * nvec + c], s);
+  for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (have && l == 0) y[i] = add ? y[i] + s : s;
+}
+
+// ---------------------------------------------------------------------
+// K on tiles.  Entries of K for assemble_rows (linear elements): V (C0 + cx
+// Cx + cy Cy + cz Cz) with C the products of the 1-D reference entries by
+// the directions in which two corners differ.
+struct HelmEntry {
+  const HGeoT<double> *geo;
+  double C0[8], Cx[8], Cy[8], Cz[8];
+  __device__ __forceinline__ double regular(unsigned e, unsigned x) const {
+    const double2 *g = (const double2 *)(geo + e);
+    const double2 a = __ldg(g), b = __ldg(g + 1);
+    return a.x * fma(a.y, Cx[x], fma(b.x, Cy[x], fma(b.y, Cz[x], C0[x])));
+  }
+  __device__ __forceinline__ double direct(long long e, int a, int b) const {
+    return regular((unsigned)e, (unsigned)(a ^ b));
+  }
+};
+static HelmEntry make_helm_entry(const HLevel &L) {
+  HelmEntry E{};
+  E.geo = (const HGeoT<double> *)L.geo.p;
+  for (int x = 0; x < (1 << L.dim); x++) {
+    const int i = x & 1, j = (x >> 1) & 1, k = x >> 2;
+    const double *M = L.bas.M[0], *K = L.bas.K[0];
+    if (L.dim == 3) {
+      E.C0[x] = M[i] * M[j] * M[k];
+      E.Cx[x] = K[i] * M[j] * M[k];
+      E.Cy[x] = M[i] * K[j] * M[k];
+      E.Cz[x] = M[i] * M[j] * K[k];
+    } else {
+      E.C0[x] = M[i] * M[j];
+      E.Cx[x] = K[i] * M[j];
+      E.Cy[x] = M[i] * K[j];
+    }
+  }
+  return E;
+}
+
+// One product with K and what follows it, VPN components from c0 of nvec:
+//   HT_APPLY   r = K in, and the blocks' parts of in . r
+//   HT_START   zero guess, in = b: d = c1 D^-1 b, x = d, r = b - K d, then the
+//              second Chebyshev step d2 = a d + c D^-1 r, x += d2
+//   HT_START1  the same without the second step (degree 1)
+//   HT_STEP    in = d: r -= K d, d2 = a d + c D^-1 r, x += d2
+//   HT_END     HT_STEP that leaves x only (the last one)
+//   HT_RES     in = d: r -= K d
+//   HT_FROM    in = x: r = b - K x, d2 = c1 D^-1 r, x2 = x + d2 (the first step
+//              from a guess)
+// A block loads its tile's distinct inputs into shared memory (HT_START forms
+// d as it loads) and its rows read them by 16-bit places; d2 and x2 are other
+// buffers than the gathered d and x.  Bound by the matrix (6 or 10 bytes an
+// entry, 5.0 TB/s) on the finest level and by latency on the small ones (8 us
+// for 6,000 nodes).
+enum HtMode { HT_APPLY, HT_START, HT_START1, HT_STEP, HT_END, HT_RES, HT_FROM };
+template <typename T>
+struct HtArgs {
+  const T *in, *b, *dinv;
+  T *r, *d2, *x, *x2;
+  T a, c, c1;
+  double *part;  // HT_APPLY: per block and component, in . r (or null)
+};
+template <typename T, int VPN, int MODE>
+__global__ void __launch_bounds__(TS_ROWS)
+    k_ht(TSellView M, int nvec, int c0, const T *__restrict__ val, HtArgs<T> A) {
+  constexpr bool START = MODE == HT_START || MODE == HT_START1;
+  extern __shared__ __align__(16) unsigned char ht_smem[];
+  T *sx = (T *)ht_smem;
+  const int t = threadIdx.x;
+  // the row's own data is on its way while the tile's inputs are loaded
+  const long long q = (long long)blockIdx.x * TS_ROWS + t;
+  const int i = M.row[q];
+  const int len = M.len[q];
+  const long long base = (long long)M.soff[q >> 5] * 32 + (t & 31);
+  const unsigned u0 = M.uoff[blockIdx.x];
+  const int m = (int)(M.uoff[blockIdx.x + 1] - u0);
+  for (int k = t; k < m; k += TS_ROWS) {
+    const long long j = __ldg(M.ucol + u0 + k);
+    const T dj = START ? A.c1 * __ldg(A.dinv + j) : T(1);
+#pragma unroll
+    for (int v = 0; v < VPN; v++) {
+      const T xv = __ldg(A.in + j * nvec + c0 + v);
+      sx[k * VPN + v] = START ? dj * xv : xv;
+    }
+  }
+  __syncthreads();
+  const uint16_t *ip = M.idx + base;
+  const T *vp = val + base;
+  T acc[VPN];
+#pragma unroll
+  for (int v = 0; v < VPN; v++) acc[v] = T(0);
+#pragma unroll 6
+  for (int k = 0; k < len; k++) {
+    const T *xv = sx + (int)__ldg(ip + 32LL * k) * VPN;
+    const T mv = __ldg(vp + 32LL * k);
+#pragma unroll
+    for (int v = 0; v < VPN; v++) acc[v] = fma(mv, xv[v], acc[v]);
+  }
+  if constexpr (MODE == HT_APPLY) {
+    // the block's part of in . r (FP64), rows in position order
+    __shared__ double s_dot[TS_SLICES];
+#pragma unroll
+    for (int v = 0; v < VPN; v++) {
+      if (i >= 0) A.r[(long long)i * nvec + c0 + v] = acc[v];
+      if (!A.part) continue;
+      double d = i >= 0 ? (double)__ldg(A.in + (long long)i * nvec + c0 + v) * acc[v] : 0.0;
+#pragma unroll
+      for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      if ((t & 31) == 0) s_dot[t >> 5] = d;
+      __syncthreads();
+      if (t == 0) {
+        double s = 0.0;
+        for (int w = 0; w < TS_SLICES; w++) s += s_dot[w];
+        A.part[(long long)blockIdx.x * nvec + c0 + v] = s;
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  if (i < 0) return;
+  const T di = MODE == HT_RES ? T(0) : __ldg(A.dinv + i);
+#pragma unroll
+  for (int v = 0; v < VPN; v++) {
+    const long long o = (long long)i * nvec + c0 + v;
+    if constexpr (START) {
+      const T bo = __ldg(A.in + o), d = A.c1 * di * bo, r = bo - acc[v];
+      A.r[o] = r;
+      if (MODE == HT_START) {
+        const T d2 = fma(A.a, d, A.c * di * r);
+        A.d2[o] = d2;
+        A.x[o] = d + d2;
+      } else {
+        A.x[o] = d;
+      }
+    } else if constexpr (MODE == HT_STEP || MODE == HT_END) {
+      const T r = A.r[o] - acc[v];
+      const T d2 = fma(A.a, __ldg(A.in + o), A.c * di * r);
+      if (MODE == HT_STEP) {
+        A.r[o] = r;
+        A.d2[o] = d2;
+      }
+      A.x[o] += d2;
+    } else if constexpr (MODE == HT_RES) {
+      A.r[o] -= acc[v];
+    } else {
+      const T r = A.b[o] - acc[v];
+      const T d2 = A.c1 * di * r;
+      A.r[o] = r;
+      A.d2[o] = d2;
+      A.x2[o] = __ldg(A.in + o) + d2;
+    }
+  }
+}
+template <typename T, int MODE>
+static void ht_launch(const TSell &M, const T *val, int nvec, const HtArgs<T> &A,
+                      cudaStream_t s) {
+  const TSellView V = M.view();
+  const unsigned g = (unsigned)M.tiles;
+#define TMRG_HT(VPN)                                                                         \
+  do {                                                                                       \
+    const size_t smem = sizeof(T) * VPN * (size_t)M.maxu;                                    \
+    if (smem > 48 * 1024)                                                                    \
+      TMRG_CUDA(cudaFuncSetAttribute(k_ht<T, VPN, MODE>,                                     \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    prof_bytes((long long)(sizeof(T) + 2) * M.entries + (long long)sizeof(T) * M.n *         \
+                                                            (1 + 5LL * VPN));                \
+    prof_flops(sizeof(T) == 8 ? 2LL * VPN * M.entries : 0);                                  \
+    launch((k_ht<T, VPN, MODE>), g, TS_ROWS, smem, s, V, nvec, c0, val, A);                  \
+  } while (0)
+  for (int c0 = 0; c0 < nvec; c0 += 4) {
+    switch (std::min(4, nvec - c0)) {
+      case 1: TMRG_HT(1); break;
+      case 2: TMRG_HT(2); break;
+      case 3: TMRG_HT(3); break;
+      default: TMRG_HT(4);
+    }
+  }
+#undef TMRG_HT
 }
 
 // ---------------------------------------------------------------------
@@ -525,32 +719,28 @@ __global__ void k_h_cheb_step(long long n, int nvec, const T *__restrict__ dinv,
   d[i] = di;
   x[i] += di;
 }
-template <typename T>
-__global__ void k_h_add(long long n, T *x, const T *__restrict__ t) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] += t[i];
-}
 
 // ---------------------------------------------------------------------
-// Reductions: per-component sums of a.b (and c.d) in a fixed order:
-// block partials, then one block combines them.
-__global__ void __launch_bounds__(256)
-    k_h_dot2(long long n, int nvec, const double *__restrict__ a,
-             const double *__restrict__ b, const double *__restrict__ c,
-             const double *__restrict__ d, double *part) {
-  __shared__ double sh[2][HM_MAXVEC][8];
-  double s1[HM_MAXVEC], s2[HM_MAXVEC];
-  for (int v = 0; v < nvec; v++) s1[v] = s2[v] = 0.0;
+// Reductions: per-component sums in a fixed order: block partials, then one
+// block combines them.  NV components in registers (0: any number up to
+// HM_MAXVEC).
+template <int NV, typename F>
+__device__ __forceinline__ void h_block_sums(long long n, int nvec, double *part, F &&f) {
+  constexpr int MV = NV ? NV : HM_MAXVEC;
+  __shared__ double sh[2][MV][8];
+  double s1[MV], s2[MV];
+#pragma unroll
+  for (int v = 0; v < MV; v++) s1[v] = s2[v] = 0.0;
+  const int nv = NV ? NV : nvec;
   for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n;
        j += (long long)gridDim.x * blockDim.x) {
-    for (int v = 0; v < nvec; v++) {
-      long long i = j * nvec + v;
-      s1[v] = fma(a[i], b[i], s1[v]);
-      if (c) s2[v] = fma(c[i], d[i], s2[v]);
-    }
+#pragma unroll
+    for (int v = 0; v < MV; v++)
+      if (v < nv) f(j * nv + v, v, s1[v], s2[v]);
   }
-  int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  for (int v = 0; v < nvec; v++) {
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+#pragma unroll
+  for (int v = 0; v < MV; v++) {
     double x1 = s1[v], x2 = s2[v];
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -563,70 +753,105 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  if (threadIdx.x < 2 * nvec) {
-    int k = threadIdx.x / nvec, v = threadIdx.x % nvec;
+  if (threadIdx.x < 2 * nv) {
+    int k = threadIdx.x / nv, v = threadIdx.x % nv;
     double t = 0.0;
     for (int q = 0; q < 8; q++) t += sh[k][v][q];
-    part[((long long)blockIdx.x * 2 + k) * nvec + v] = t;
+    part[((long long)blockIdx.x * 2 + k) * nv + v] = t;
   }
 }
-// out[k*nvec + v] = sum over blocks of part (k = 0, 1): one warp per
-// output, lanes strided over the blocks, then a fixed shuffle tree.
-__global__ void k_h_dot_final(int nblocks, int nvec, const double *__restrict__ part,
-                              double *out) {
-  const int lane = threadIdx.x & 31;
-  for (int t = threadIdx.x >> 5; t < 2 * nvec; t += blockDim.x >> 5) {
-    int k = t / nvec, v = t % nvec;
-    double s = 0.0;
-    for (int b = lane; b < nblocks; b += 32) s += part[((long long)b * 2 + k) * nvec + v];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[k * nvec + v] = s;
-  }
+// a . b
+template <int NV>
+__global__ void __launch_bounds__(256)
+    k_h_dot(long long n, int nvec, const double *__restrict__ a, const double *__restrict__ b,
+            double *part) {
+  h_block_sums<NV>(n, nvec, part, [&](long long i, int, double &s1, double &) {
+    s1 = fma(a[i], b[i], s1);
+  });
 }
-
+// r . z and r . z_old of the FP32 preconditioner's results (zo null: 0)
+template <int NV>
+__global__ void __launch_bounds__(256)
+    k_h_cg_rz(long long n, int nvec, const double *__restrict__ r, const float *__restrict__ z,
+              const float *__restrict__ zo, double *part) {
+  h_block_sums<NV>(n, nvec, part, [&](long long i, int, double &s1, double &s2) {
+    const double ri = r[i];
+    s1 = fma(ri, (double)z[i], s1);
+    if (zo) s2 = fma(ri, (double)zo[i], s2);
+  });
+}
+// x += alpha p; r -= alpha q; r . r; the next preconditioner input in FP32
+template <int NV>
+__global__ void __launch_bounds__(256)
+    k_h_cg_update(long long n, int nvec, const double *__restrict__ sc,
+                  const double *__restrict__ p, const double *__restrict__ q, double *x,
+                  double *r, float *b32, double *part) {
+  h_block_sums<NV>(n, nvec, part, [&](long long i, int v, double &s1, double &) {
+    const double al = sc[8 * v + 2];
+    x[i] = fma(al, p[i], x[i]);
+    const double ri = fma(-al, q[i], r[i]);
+    r[i] = ri;
+    b32[i] = (float)ri;
+    s1 = fma(ri, ri, s1);
+  });
+}
 // Conjugate-gradient scalars, per component v at sc[8v]: [0] r.z, [2]
 // alpha, [3] beta, [4] done flag, [5] thr^2.
-// alpha = rz / pq (0 once the component has converged)
-__global__ void k_h_cg_alpha(int nvec, const double *__restrict__ dots, double *sc) {
-  int v = threadIdx.x;
-  if (v >= nvec) return;
+enum HScalar { HS_NONE, HS_ALPHA, HS_CHECK, HS_BETA };
+// out[k*nvec + v] = sum over blocks of part (k = 0..nk-1, nk per block): one
+// warp per output, lanes strided over the blocks, then a fixed shuffle tree;
+// then the scalars that follow:
+//   HS_ALPHA  alpha = rz / out (0 once the component has converged)
+//   HS_CHECK  done once out = r.r <= thr^2 (alpha and beta are 0 from then on)
+//   HS_BETA   out = (r.z_new, r.z_old): Polak-Ribiere beta = (r.z_new -
+//             r.z_old) / rz, then rz = r.z_new
+__global__ void __launch_bounds__(1024)
+    k_h_dot_final(int nblocks, int nk, int nvec, const double *__restrict__ part, double *out,
+                  int what, double *sc) {
+  const int lane = threadIdx.x & 31;
+  const int outs = nk * nvec;
+  // warps per output: all of them share a long list of blocks
+  const int wpo = max(1, (int)(blockDim.x >> 5) / outs);
+  __shared__ double sh[32];
+  for (int t0 = 0; t0 < outs; t0 += (int)(blockDim.x >> 5) / wpo) {
+    const int w = threadIdx.x >> 5, t = t0 + w / wpo;
+    double s = 0.0;
+    if (t < outs) {
+      const int k = t / nvec, v = t % nvec;
+      for (int b = (w % wpo) * 32 + lane; b < nblocks; b += 32 * wpo)
+        s += part[((long long)b * nk + k) * nvec + v];
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) sh[w] = s;
+    __syncthreads();
+    if (t < outs && w % wpo == 0 && lane == 0) {
+      double r = 0.0;
+      for (int q = 0; q < wpo; q++) r += sh[w + q];
+      out[t] = r;
+    }
+    __syncthreads();
+  }
+  const int v = threadIdx.x;
+  if (v >= nvec || what == HS_NONE) return;
   double *c = sc + 8 * v;
-  double pq = dots[v];
-  c[2] = (c[4] != 0.0 || pq == 0.0) ? 0.0 : c[0] / pq;
-}
-// a component is done once r.r <= thr^2 (alpha and beta are 0 from then on)
-__global__ void k_h_cg_check(int nvec, const double *__restrict__ dots, double *sc) {
-  int v = threadIdx.x;
-  if (v >= nvec) return;
-  if (dots[v] <= sc[8 * v + 5]) sc[8 * v + 4] = 1.0;
-}
-// after the preconditioner: dots = (r.z_new, r.z_old); Polak-Ribiere
-// beta = (r.z_new - r.z_old) / rz, then rz = r.z_new
-__global__ void k_h_cg_beta(int nvec, const double *__restrict__ dots, double *sc) {
-  int v = threadIdx.x;
-  if (v >= nvec) return;
-  double *c = sc + 8 * v;
-  double rz = dots[v], rzo = dots[nvec + v];
-  c[3] = (c[4] != 0.0 || c[0] == 0.0) ? 0.0 : (rz - rzo) / c[0];
-  c[0] = rz;
-}
-// x += alpha p; r -= alpha q
-__global__ void k_h_cg_update(long long n, int nvec, const double *__restrict__ sc,
-                              const double *__restrict__ p, const double *__restrict__ q,
-                              double *x, double *r) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * nvec) return;
-  double al = sc[8 * (i % nvec) + 2];
-  x[i] = fma(al, p[i], x[i]);
-  r[i] = fma(-al, q[i], r[i]);
+  if (what == HS_ALPHA) {
+    const double pq = out[v];
+    c[2] = (c[4] != 0.0 || pq == 0.0) ? 0.0 : c[0] / pq;
+  } else if (what == HS_CHECK) {
+    if (out[v] <= c[5]) c[4] = 1.0;
+  } else {
+    const double rz = out[v], rzo = nk > 1 ? out[nvec + v] : 0.0;
+    c[3] = (c[4] != 0.0 || c[0] == 0.0) ? 0.0 : (rz - rzo) / c[0];
+    c[0] = rz;
+  }
 }
 // p = z + beta p
 __global__ void k_h_cg_dir(long long n, int nvec, const double *__restrict__ sc,
-                           const double *__restrict__ z, double *p) {
+                           const float *__restrict__ z, double *p) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * nvec) return;
-  p[i] = fma(sc[8 * (i % nvec) + 3], p[i], z[i]);
+  p[i] = fma(sc[8 * (i % nvec) + 3], p[i], (double)z[i]);
 }
 
 // Lanczos helpers on D^-1/2 K D^-1/2.
@@ -666,7 +891,15 @@ template <typename T>
 static void ensure_work(HLevel &L, HWork<T> &W, int nvec, cudaStream_t s) {
   if (nvec <= W.cap) return;
   W.cap = nvec;
-  for (DBuf<T> *b : {&W.x, &W.b, &W.r, &W.d, &W.t}) b->alloc(std::max(1LL, L.nn * nvec), s);
+  // the FP32 levels on tiles need a second buffer for x and d, and no
+  // dependent or slot values; the FP64 operator needs only those
+  const bool tiles = std::is_same<T, float>::value && L.tiled.ok;
+  if (std::is_same<T, float>::value) {
+    for (DBuf<T> *b : {&W.x, &W.b, &W.r, &W.d}) b->alloc(std::max(1LL, L.nn * nvec), s);
+    if (tiles)
+      for (DBuf<T> *b : {&W.d2, &W.t}) b->alloc(std::max(1LL, L.nn * nvec), s);
+  }
+  if (tiles) return;
   W.xd.alloc(std::max(1LL, L.ndep * nvec), s);
   W.yE.alloc(std::max(1LL, L.ne * L.npe * nvec), s);
 }
@@ -696,8 +929,18 @@ struct LevelData<float> {
 // level's work vectors of precision T (xd, yE).
 template <typename T>
 static void h_apply(HLevel &L, bool stiff, int nvec, const T *x, T *y, const T *b, int mode,
-                    cudaStream_t s) {
+                    cudaStream_t s, double *part = nullptr) {
   using D = LevelData<T>;
+  if constexpr (std::is_same<T, double>::value) {
+    if (stiff && mode == 0 && L.k64.p) {
+      HtArgs<double> A{};
+      A.in = x;
+      A.r = y;
+      A.part = part;
+      ht_launch<double, HT_APPLY>(L.tiled, (const double *)L.k64.p, nvec, A, s);
+      return;
+    }
+  }
   HWork<T> &W = D::work(L);
   ensure_work(L, W, nvec, s);
   const long long sz = sizeof(T);
@@ -773,13 +1016,28 @@ static void h_apply(HLevel &L, bool stiff, int nvec, const T *x, T *y, const T *
            (const int *)L.sslot.p, D::sw(L), (const T *)yE, b, y, mode);
 }
 
-// per-component dot products (a.b, c.d) into dev_out[0..2 nvec)
+#define H_BY_NVEC(K, ...)                                      \
+  do {                                                         \
+    switch (nvec) {                                            \
+      case 1: launch(K<1>, __VA_ARGS__); break;                \
+      case 2: launch(K<2>, __VA_ARGS__); break;                \
+      case 3: launch(K<3>, __VA_ARGS__); break;                \
+      default: launch(K<0>, __VA_ARGS__);                      \
+    }                                                          \
+  } while (0)
+// Block partials (nk per component) to dev_out[0..nk nvec) and the scalars
+// that follow from them.
+static void h_final(Helmholtz &H, int nblocks, int nk, int nvec, double *dev_out,
+                    HScalar what = HS_NONE) {
+  launch(k_h_dot_final, 1, 1024, 0, H.s, nblocks, nk, nvec, (const double *)H.part.p, dev_out,
+         (int)what, H.sc.p);
+}
+// per-component dot products a.b into dev_out[0..2 nvec) (zeros behind them)
 static void h_dots(Helmholtz &H, long long n, int nvec, const double *a, const double *b,
-                   const double *c, const double *d, double *dev_out) {
-  cudaStream_t s = H.s;
-  prof_bytes(8LL * n * nvec * (c ? 4 : 2));
-  launch(k_h_dot2, HM_RED_BLOCKS, 256, 0, s, n, nvec, a, b, c, d, H.part.p);
-  launch(k_h_dot_final, 1, 256, 0, s, HM_RED_BLOCKS, nvec, (const double *)H.part.p, dev_out);
+                   double *dev_out) {
+  prof_bytes(8LL * n * nvec * 2);
+  H_BY_NVEC(k_h_dot, HM_RED_BLOCKS, 256, 0, H.s, n, nvec, a, b, H.part.p);
+  h_final(H, HM_RED_BLOCKS, 2, nvec, dev_out);
 }
 
 // Largest eigenvalue of the symmetric tridiagonal (alpha, beta) by
@@ -822,7 +1080,7 @@ static void lanczos_lmax(Helmholtz &H, HLevel &L) {
   vp.zero();
   launch(k_h_start, blocks_for(n, 256), 256, 0, s, n, v.p);
   double h2[2];
-  h_dots(H, n, 1, v.p, v.p, nullptr, nullptr, dots.p);
+  h_dots(H, n, 1, v.p, v.p, dots.p);
   TMRG_CUDA(cudaMemcpyAsync(h2, dots.p, sizeof(h2), cudaMemcpyDeviceToHost, s));
   TMRG_CUDA(cudaStreamSynchronize(s));
   launch(k_h_scale, blocks_for(n, 256), 256, 0, s, n, v.p, (const double *)v.p,
@@ -835,14 +1093,14 @@ static void lanczos_lmax(Helmholtz &H, HLevel &L) {
     h_apply<double>(L, true, 1, u.p, w.p, nullptr, 0, s);
     launch(k_h_scale_sqrt, blocks_for(n, 256), 256, 0, s, n, (const double *)L.dinv.p,
            (const double *)w.p, w.p);
-    h_dots(H, n, 1, w.p, v.p, nullptr, nullptr, dots.p);
+    h_dots(H, n, 1, w.p, v.p, dots.p);
     TMRG_CUDA(cudaMemcpyAsync(h2, dots.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     TMRG_CUDA(cudaStreamSynchronize(s));
     double alpha = h2[0];
     al.push_back(alpha);
     launch(k_h_lanczos_orth, blocks_for(n, 256), 256, 0, s, n, w.p, (const double *)v.p,
            (const double *)vp.p, alpha, beta);
-    h_dots(H, n, 1, w.p, w.p, nullptr, nullptr, dots.p);
+    h_dots(H, n, 1, w.p, w.p, dots.p);
     TMRG_CUDA(cudaMemcpyAsync(h2, dots.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     TMRG_CUDA(cudaStreamSynchronize(s));
     beta = std::sqrt(std::max(h2[0], 0.0));
@@ -885,17 +1143,84 @@ static void chebyshev(Helmholtz &H, HLevel &L, int nvec, const float *rin, bool 
   if (keep_r) h_apply<float>(L, true, nvec, W.d.p, W.r.p, nullptr, 2, s);
 }
 
-static void p_apply32(Helmholtz &H, int k, bool transpose, int nvec, const float *x, float *y) {
+// The smoother on tiles: from a zero guess with the residual kept, or from
+// the guess in W.x (the result is again in W.x).
+static void chebyshev_tiled(Helmholtz &H, HLevel &L, int nvec, const float *b, bool zero,
+                            bool keep_r) {
+  cudaStream_t s = H.s;
+  HWork<float> &W = L.w32;
+  const double lmax = H.cheb_upper * L.lam,
+               lmin = (L.o == 2 ? H.cheb_lower2 : H.cheb_lower3) * L.lam;
+  const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
+  const double sigma = theta / delta;
+  const int degree = L.o == 2 ? H.cheb_degree2 : H.cheb_degree3;
+  const float *val = L.k32.p;
+  double rho = 1.0 / sigma;
+  HtArgs<float> A{};
+  A.b = b;
+  A.dinv = L.dinv32.p;
+  A.r = W.r.p;
+  A.c1 = (float)(1.0 / theta);
+  int k = 1;
+  auto step = [&]() {
+    const double rn = 1.0 / (2.0 * sigma - rho);
+    A.a = (float)(rn * rho);
+    A.c = (float)(2.0 * rn / delta);
+    rho = rn;
+    k++;
+  };
+  if (zero) {
+    A.in = b;
+    A.x = W.x.p;
+    A.d2 = W.d.p;
+    if (degree > 1) {
+      step();
+      ht_launch<float, HT_START>(L.tiled, val, nvec, A, s);
+    } else {
+      ht_launch<float, HT_START1>(L.tiled, val, nvec, A, s);
+    }
+  } else {
+    A.in = W.x.p;
+    A.x2 = W.t.p;
+    A.d2 = W.d.p;
+    ht_launch<float, HT_FROM>(L.tiled, val, nvec, A, s);
+    W.x.swap(W.t);
+    A.x = W.x.p;
+  }
+  while (k < degree) {
+    step();
+    A.in = W.d.p;
+    A.d2 = W.d2.p;
+    if (k == degree && !keep_r) {
+      ht_launch<float, HT_END>(L.tiled, val, nvec, A, s);
+    } else {
+      ht_launch<float, HT_STEP>(L.tiled, val, nvec, A, s);
+      W.d.swap(W.d2);
+    }
+  }
+  // (degree 1 has formed b - K d already)
+  if (keep_r && degree > 1) {
+    A.in = W.d.p;
+    ht_launch<float, HT_RES>(L.tiled, val, nvec, A, s);
+  }
+}
+
+static void p_apply32(Helmholtz &H, int k, bool transpose, int nvec, const float *x, float *y,
+                      bool add) {
   Interp &I = *H.P[k];
   HInterp32 &F = *H.P32[k];
   const long long nout = transpose ? I.cols : I.rows;
   prof_bytes(8LL * I.nnz_nz + 4 * (nout + 1) + 4LL * nvec * (I.rows + I.cols));
+  // lanes by the mean row length, as for one vector of the P applies
+  const int lb = I.nnz_nz < 10 * nout ? 0 : I.nnz_nz < 24 * nout ? 1 : 2;
+  const unsigned g = blocks_for((nout * nvec) << lb, 256);
   if (transpose)
-    launch(k_h_csr<float>, blocks_for(nout * nvec, 256), 256, 0, H.s, nout, nvec,
-           (const int *)I.t_rowptr.p, (const int *)I.t_colidx.p, (const float *)F.pt.p, x, y);
+    launch(k_h_csr<float>, g, 256, 0, H.s, nout, nvec, lb,
+           (const int *)I.t_rowptr.p, (const int *)I.t_colidx.p, (const float *)F.pt.p, x, y,
+           (int)add);
   else
-    launch(k_h_csr<float>, blocks_for(nout * nvec, 256), 256, 0, H.s, nout, nvec,
-           I.ap_rowptr(), I.ap_colidx(), (const float *)F.p.p, x, y);
+    launch(k_h_csr<float>, g, 256, 0, H.s, nout, nvec, lb,
+           I.ap_rowptr(), I.ap_colidx(), (const float *)F.p.p, x, y, (int)add);
 }
 
 // x_k = B_k b in FP32 (one V-cycle from a zero guess); the result is left
@@ -910,6 +1235,9 @@ static void vcycle(Helmholtz &H, int k, int nvec, const float *b) {
       prof_bytes(4LL * n * n + 8LL * n * nvec);
       launch(k_h_dense_mv<float>, blocks_for(n * nvec * 32, 256), 256, 0, s, n, nvec,
              (const float *)H.Ainv32.p, b, W.x.p);
+    } else if (L.tiled.ok) {
+      chebyshev_tiled(H, L, nvec, b, true, false);
+      for (int it = 1; it < H.coarse_sweeps; it++) chebyshev_tiled(H, L, nvec, b, false, false);
     } else {
       chebyshev(H, L, nvec, b, true, false);
       for (int it = 1; it < H.coarse_sweeps; it++) {
@@ -920,44 +1248,44 @@ static void vcycle(Helmholtz &H, int k, int nvec, const float *b) {
     return;
   }
   HLevel &C = *H.L[k + 1];
-  chebyshev(H, L, nvec, b, true, true);
-  p_apply32(H, k, true, nvec, W.r.p, C.w32.b.p);
+  if (L.tiled.ok)
+    chebyshev_tiled(H, L, nvec, b, true, true);
+  else
+    chebyshev(H, L, nvec, b, true, true);
+  p_apply32(H, k, true, nvec, W.r.p, C.w32.b.p, false);
   vcycle(H, k + 1, nvec, C.w32.b.p);
-  p_apply32(H, k, false, nvec, C.w32.x.p, W.t.p);
-  prof_bytes(12LL * n * nvec);
-  launch(k_h_add<float>, blocks_for(n * nvec, 256), 256, 0, s, n * nvec, W.x.p,
-         (const float *)W.t.p);
-  h_apply<float>(L, true, nvec, W.x.p, W.r.p, b, 1, s);
-  chebyshev(H, L, nvec, W.r.p, false, false);
-}
-
-// z = B r: r (FP64) to FP32, V-cycle, result back to FP64.
-static void precondition(Helmholtz &H, int nvec, const double *r, double *z) {
-  HLevel &L = *H.L[0];
-  const long long len = L.nn * nvec;
-  prof_bytes(12LL * len);
-  launch((k_h_cvt<double, float>), blocks_for(len, 256), 256, 0, H.s, len, r, L.w32.b.p);
-  vcycle(H, 0, nvec, L.w32.b.p);
-  prof_bytes(12LL * len);
-  launch((k_h_cvt<float, double>), blocks_for(len, 256), 256, 0, H.s, len,
-         (const float *)L.w32.x.p, z);
+  p_apply32(H, k, false, nvec, C.w32.x.p, W.x.p, true);
+  if (L.tiled.ok) {
+    chebyshev_tiled(H, L, nvec, b, false, false);
+  } else {
+    h_apply<float>(L, true, nvec, W.x.p, W.r.p, b, 1, s);
+    chebyshev(H, L, nvec, W.r.p, false, false);
+  }
 }
 
 // Solve K x = b on the finest level (all components), flexible PCG with
-// the FP32 V-cycle; x and b are nvec-interleaved FP64 device vectors.
+// the FP32 V-cycle; x and b are nvec-interleaved FP64 device vectors.  The
+// preconditioner reads the residual from the finest level's w32.b, where the
+// update leaves it rounded to FP32, and its result z = w32.x is used from
+// there.
 static void solve(Helmholtz &H, int nvec, const double *b, double *x) {
   cudaStream_t s = H.s;
   HLevel &L = *H.L[0];
+  HWork<float> &W = L.w32;
   const long long n = L.nn;
   const long long len = n * nvec;
   const unsigned g = blocks_for(len, 256);
   for (auto &lv : H.L) ensure_work(*lv, lv->w32, nvec, s);
-  for (DBuf<double> *v : {&H.cg_r, &H.cg_p, &H.cg_q, &H.cg_z, &H.cg_zo}) ensure(*v, len, s);
+  for (DBuf<double> *v : {&H.cg_r, &H.cg_p, &H.cg_q}) ensure(*v, len, s);
+  // changes places with w32.x, which holds W.cap components
+  ensure(H.cg_zo, std::max(1LL, n * W.cap), s);
+  // partial sums: two per component of a reduction, or one of every tile
+  ensure(H.part, std::max(2LL * HM_RED_BLOCKS, L.tiled.tiles) * HM_MAXVEC, s);
   TMRG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * len, s));
   TMRG_CUDA(cudaMemcpyAsync(H.cg_r.p, b, sizeof(double) * len, cudaMemcpyDeviceToDevice, s));
   // thresholds from |b|
   std::vector<double> hd(2 * nvec), hsc(8 * nvec, 0.0);
-  h_dots(H, n, nvec, b, b, nullptr, nullptr, H.dots.p);
+  h_dots(H, n, nvec, b, b, H.dots.p);
   TMRG_CUDA(cudaMemcpyAsync(hd.data(), H.dots.p, sizeof(double) * 2 * nvec,
                             cudaMemcpyDeviceToHost, s));
   TMRG_CUDA(cudaStreamSynchronize(s));
@@ -978,22 +1306,37 @@ static void solve(Helmholtz &H, int nvec, const double *b, double *x) {
   if (all_done) return;
   TMRG_CUDA(cudaMemcpyAsync(H.sc.p, hsc.data(), sizeof(double) * 8 * nvec,
                             cudaMemcpyHostToDevice, s));
-  // z = B r ; p = z ; rz = r.z
-  precondition(H, nvec, H.cg_r.p, H.cg_z.p);
-  TMRG_CUDA(cudaMemcpyAsync(H.cg_p.p, H.cg_z.p, sizeof(double) * len, cudaMemcpyDeviceToDevice,
-                            s));
-  TMRG_CUDA(cudaMemsetAsync(H.cg_zo.p, 0, sizeof(double) * len, s));
-  h_dots(H, n, nvec, H.cg_r.p, H.cg_z.p, H.cg_r.p, H.cg_zo.p, H.dots.p);
-  launch(k_h_cg_beta, 1, 32, 0, s, nvec, (const double *)H.dots.p, H.sc.p);
+  // rz = r.z, beta from r.z_old (it > 0), p = z + beta p
+  auto direction = [&](const float *zo) {
+    prof_bytes(len * (zo ? 16 : 12));
+    H_BY_NVEC(k_h_cg_rz, HM_RED_BLOCKS, 256, 0, s, n, nvec, (const double *)H.cg_r.p,
+              (const float *)W.x.p, zo, H.part.p);
+    h_final(H, HM_RED_BLOCKS, 2, nvec, H.dots.p, HS_BETA);
+    prof_bytes(len * 20);
+    launch(k_h_cg_dir, g, 256, 0, s, n, nvec, (const double *)H.sc.p, (const float *)W.x.p,
+           H.cg_p.p);
+  };
+  // z = B r ; p = z
+  prof_bytes(12LL * len);
+  launch((k_h_cvt<double, float>), g, 256, 0, s, len, (const double *)H.cg_r.p, W.b.p);
+  vcycle(H, 0, nvec, W.b.p);
+  TMRG_CUDA(cudaMemsetAsync(H.cg_p.p, 0, sizeof(double) * len, s));
+  direction(nullptr);
   for (int it = 1; it <= H.max_iters; it++) {
-    h_apply<double>(L, true, nvec, H.cg_p.p, H.cg_q.p, nullptr, 0, s);
-    h_dots(H, n, nvec, H.cg_p.p, H.cg_q.p, nullptr, nullptr, H.dots.p);
-    launch(k_h_cg_alpha, 1, 32, 0, s, nvec, (const double *)H.dots.p, H.sc.p);
-    prof_bytes(8LL * len * 6);
-    launch(k_h_cg_update, g, 256, 0, s, n, nvec, (const double *)H.sc.p,
-           (const double *)H.cg_p.p, (const double *)H.cg_q.p, x, H.cg_r.p);
-    h_dots(H, n, nvec, H.cg_r.p, H.cg_r.p, nullptr, nullptr, H.dots.p);
-    launch(k_h_cg_check, 1, 32, 0, s, nvec, (const double *)H.dots.p, H.sc.p);
+    if (L.k64.p) {
+      h_apply<double>(L, true, nvec, H.cg_p.p, H.cg_q.p, nullptr, 0, s, H.part.p);
+      h_final(H, (int)L.tiled.tiles, 1, nvec, H.dots.p, HS_ALPHA);
+    } else {
+      h_apply<double>(L, true, nvec, H.cg_p.p, H.cg_q.p, nullptr, 0, s);
+      prof_bytes(16 * len);
+      H_BY_NVEC(k_h_dot, HM_RED_BLOCKS, 256, 0, s, n, nvec, (const double *)H.cg_p.p,
+                (const double *)H.cg_q.p, H.part.p);
+      h_final(H, HM_RED_BLOCKS, 2, nvec, H.dots.p, HS_ALPHA);
+    }
+    prof_bytes(len * 52);
+    H_BY_NVEC(k_h_cg_update, HM_RED_BLOCKS, 256, 0, s, n, nvec, (const double *)H.sc.p,
+              (const double *)H.cg_p.p, (const double *)H.cg_q.p, x, H.cg_r.p, W.b.p, H.part.p);
+    h_final(H, HM_RED_BLOCKS, 2, nvec, H.dots.p, HS_CHECK);
     TMRG_CUDA(cudaMemcpyAsync(hd.data(), H.dots.p, sizeof(double) * nvec,
                               cudaMemcpyDeviceToHost, s));
     TMRG_CUDA(cudaStreamSynchronize(s));
@@ -1007,13 +1350,9 @@ static void solve(Helmholtz &H, int nvec, const double *b, double *x) {
       fin = fin && done[v];
     }
     if (fin) break;
-    H.cg_zo.swap(H.cg_z);
-    precondition(H, nvec, H.cg_r.p, H.cg_z.p);
-    h_dots(H, n, nvec, H.cg_r.p, H.cg_z.p, H.cg_r.p, H.cg_zo.p, H.dots.p);
-    launch(k_h_cg_beta, 1, 32, 0, s, nvec, (const double *)H.dots.p, H.sc.p);
-    prof_bytes(8LL * len * 3);
-    launch(k_h_cg_dir, g, 256, 0, s, n, nvec, (const double *)H.sc.p,
-           (const double *)H.cg_z.p, H.cg_p.p);
+    W.x.swap(H.cg_zo);  // the previous z
+    vcycle(H, 0, nvec, W.b.p);
+    direction(H.cg_zo.p);
   }
 }
 
@@ -1127,6 +1466,21 @@ static void build_level(Helmholtz &H, const HSource &f, HLevel &L) {
     throw Error(TMRG_ERR_ARG, "Helmholtz filter: a node has a non-positive diagonal "
                               "(degenerate element geometry)");
 }
+// K of a level of linear elements on tiles; nothing where it cannot be held
+// there (assemble_rows, tsell_build), and the element operator runs.
+static void build_tiles(Helmholtz &H, HLevel &L, bool finest) {
+  if (L.o != 2 || L.nn == 0) return;
+  cudaStream_t s = H.s;
+  DBuf<int> err(1, s), rp, ci;
+  DBuf<double> v;
+  err.zero();
+  long long nnz = 0;
+  const ElemCtx c{L.econn.p, L.dptr.p, L.dconn.p, L.dw.p, err.p, L.npe};
+  if (!assemble_rows(c, make_helm_entry(L), L.nn, L.ne, false, rp, ci, v, nnz, s)) return;
+  if (!tsell_build(L.tiled, L.nn, rp.p, ci.p, s)) return;
+  tsell_values(L.tiled, rp.p, (const double *)v.p, L.k32, s);
+  if (finest) tsell_values(L.tiled, rp.p, (const double *)v.p, L.k64, s);
+}
 
 // The levels and the P between consecutive forests (octree or quadtree).
 template <typename F, typename MakeP>
@@ -1203,7 +1557,10 @@ static void helmholtz_finish(Helmholtz &H) {
            (const double *)A.p, H.Ainv32.p);
   }
   for (int k = 0; k < nlevels; k++)
-    if (!(H.dense && k == nlevels - 1)) lanczos_lmax(H, *H.L[k]);
+    if (!(H.dense && k == nlevels - 1)) {
+      build_tiles(H, *H.L[k], k == 0);
+      lanczos_lmax(H, *H.L[k]);
+    }
   TMRG_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -30,7 +30,7 @@ struct HBasisT {
 template <typename T>
 struct HWork {
   int cap = 0;  // components the vectors hold
-  DBuf<T> x, b, r, d, t, xd, yE;
+  DBuf<T> x, b, r, d, d2, t, xd, yE;
 };
 
 // One level of the filter hierarchy: the forest's element connectivity
@@ -47,6 +47,11 @@ struct HLevel {
   DBuf<int> econn, dptr, dconn, srp, sslot;
   DBuf<double> dw, geo, sw, dinv;
   DBuf<float> dw32, geo32, sw32, dinv32;
+  // K assembled on tiles (linear elements): FP32 values for the smoother and,
+  // on the finest level, FP64 values for the Krylov iteration
+  TSell tiled;
+  DBuf<float> k32;
+  DBuf<double> k64;
   double lam = 0.0;  // Lanczos estimate of the largest eigenvalue of D^-1 K
   HWork<double> w64;
   HWork<float> w32;
@@ -73,15 +78,16 @@ struct Helmholtz {
   int max_iters = 300;
   // Chebyshev smoother: interval [lower, upper] x lam; degree and lower
   // bound by level order
-  double cheb_lower2 = 0.05, cheb_lower3 = 0.1, cheb_upper = 1.1;
-  int cheb_degree2 = 5, cheb_degree3 = 6;
+  double cheb_lower2 = 0.2, cheb_lower3 = 0.1, cheb_upper = 1.1;
+  int cheb_degree2 = 3, cheb_degree3 = 6;
   int lanczos_steps = 16;
   int coarse_sweeps = 4;
   // last solve
   int last_iters = 0;
   std::vector<double> last_res;
   // finest-level Krylov vectors
-  DBuf<double> cg_r, cg_p, cg_q, cg_z, cg_zo, rhs, psi, part, dots, sc;
+  DBuf<double> cg_r, cg_p, cg_q, rhs, psi, part, dots, sc;
+  DBuf<float> cg_zo;  // the preconditioner's previous result
 };
 
 void helmholtz_create(Forest *const *forests, int nlevels, double r, Helmholtz &H);
