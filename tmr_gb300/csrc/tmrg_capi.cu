@@ -1479,33 +1479,34 @@ int tmrg_qforest_get_points(tmrg_qforest *f, double *X) {
 }
 
 // ---- iso-surface STL ----------------------------------------------------
-static long long stl_run(tmrg_forest *f, const double *x, bool device, int vpn,
-                         int x_offset, double cutoff, DBuf<double> &tris) {
+// The design values of `f` on the device: x itself, or a copy in `dx`.
+static const double *stl_values(tmrg_forest *f, const double *x, bool device, int vpn,
+                                DBuf<double> &dx) {
   Forest &F = f->f;
   if (!F.have_nodes) forest_create_nodes(F);
+  if (device) return x;
   const long long len = F.num_owned * vpn;
-  if (device) return stl_triangles(F, x, vpn, x_offset, cutoff, tris);
-  DBuf<double> dx(std::max(1LL, len), F.s);
+  dx.alloc(std::max(1LL, len), F.s);
   if (len)
     TMRG_CUDA(cudaMemcpyAsync(dx.p, x, sizeof(double) * len, cudaMemcpyHostToDevice, F.s));
-  return stl_triangles(F, dx.p, vpn, x_offset, cutoff, tris);
+  return dx.p;
 }
 static int stl_entry(tmrg_forest *f, const double *x, bool device, int vpn, int x_offset,
                      double cutoff, int64_t *ntris, double *tris, int64_t max_tris) {
   return guarded([&] {
     ARG(f && x && ntris && vpn > 0, "bad argument");
-    DBuf<double> d;
-    const long long n = stl_run(f, x, device, vpn, x_offset, cutoff, d);
-    *ntris = n;
-    if (tris && max_tris >= n && n) {
-      if (device) {
-        TMRG_CUDA(cudaMemcpyAsync(tris, d.p, sizeof(double) * 9 * n, cudaMemcpyDeviceToDevice,
-                                  f->f.s));
-        TMRG_CUDA(cudaStreamSynchronize(f->f.s));
-      } else {
-        copy_d2h(tris, d.p, sizeof(double) * 9 * n, f->f.s);
-      }
+    DBuf<double> dx;
+    const double *xd = stl_values(f, x, device, vpn, dx);
+    if (device) {
+      *ntris = stl_triangles(f->f, xd, vpn, x_offset, cutoff, tris, tris ? max_tris : 0);
+      return;
     }
+    const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, nullptr, 0);
+    *ntris = n;
+    if (!tris || max_tris < n || !n) return;
+    DBuf<double> d(9 * (size_t)n, f->f.s);
+    stl_triangles(f->f, xd, vpn, x_offset, cutoff, d.p, n);
+    copy_d2h(tris, d.p, sizeof(double) * 9 * n, f->f.s);
   });
 }
 int tmrg_stl_triangles(tmrg_forest *f, const double *x, int vpn, int x_offset, double cutoff,
@@ -1520,9 +1521,12 @@ int tmrg_generate_bin_file(const char *filename, tmrg_forest *f, const double *x
                            int x_offset, double cutoff) {
   return guarded([&] {
     ARG(filename && f && x && vpn > 0, "bad argument");
-    DBuf<double> d;
-    const long long n = stl_run(f, x, false, vpn, x_offset, cutoff, d);
+    DBuf<double> dx;
+    const double *xd = stl_values(f, x, false, vpn, dx);
+    const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, nullptr, 0);
     ARG(n < (1LL << 31), "more triangles than the binary format's int count holds");
+    DBuf<double> d(9 * (size_t)std::max(1LL, n), f->f.s);
+    if (n) stl_triangles(f->f, xd, vpn, x_offset, cutoff, d.p, n);
     std::vector<double> h((size_t)9 * n);
     copy_d2h(h.data(), d.p, sizeof(double) * h.size(), f->f.s);
     FILE *fp = fopen(filename, "wb");

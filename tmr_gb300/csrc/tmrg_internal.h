@@ -202,7 +202,12 @@ void forest_transform_nodes(Forest &f, tmrg_octant *d_octs, long long n, int edg
 void forest_find_enclosing(Forest &f, int order, const double *knots,
                            const tmrg_octant *d_nodes, long long n, long long *d_index);
 void forest_get_points(Forest &f, const double *boxes, double *d_X);
+// The first (element << 8 | local index) of every local node (num_local + 1
+// entries), which its position is taken from.
+void forest_first_refs(Forest &f, DBuf<unsigned long long> &rep);
+// Triangles: their number, and 9 doubles each to `out` (device) when it holds
+// at least that many (max_tris); out may be null.
 long long stl_triangles(Forest &f, const double *d_x, int vpn, int offset, double cutoff,
-                        DBuf<double> &tris);
+                        double *out, long long max_tris);
 
 }  // namespace tmrg

@@ -251,6 +251,37 @@ __device__ __forceinline__ void transform_node(const ConnDev &c, int32_t &block,
   if (z == hmax) z = hmax - 1;
 }
 
+// Position of a node from an element and its local index there: a block's
+// axis-aligned box (origin, extent) stands in for TMRVolume::evalPoint,
+// X = origin + extent * (u + 0.5 d (1 + knot)), u = x / 2^30, d = h / 2^30.
+struct PointCtx {
+  int order;
+  double knots[TMRG_MAX_ORDER];
+  const unsigned long long *rep;  // per local node: element << 8 | local index
+  const int *blk, *xs, *ys, *zs;
+  const int16_t *lev;
+  const double *boxes;  // null: every point is at 0
+};
+void forest_eval_points(Forest &f, const PointCtx &c, double *d_X);
+__device__ __forceinline__ void node_point(const PointCtx &c, long long i, double *p) {
+  p[0] = p[1] = p[2] = 0.0;
+  if (!c.boxes) return;
+  const unsigned long long r = c.rep[i];
+  if (r == ~0ULL) return;
+  const long long e = (long long)(r >> 8);
+  const int l = (int)(r & 255u), o = c.order;
+  const int ijk[3] = {l % o, (l / o) % o, l / (o * o)};
+  const int32_t x[3] = {c.xs[e], c.ys[e], c.zs[e]};
+  const double scale = 1.0 / (double)(1 << TMRG_MAX_LEVEL);
+  const double d = (double)side_of(c.lev[e]) * scale;
+  const double *bx = c.boxes + 6 * (long long)c.blk[e];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double u = (double)x[k] * scale + 0.5 * d * (1.0 + c.knots[ijk[k]]);
+    p[k] = bx[k] + bx[3 + k] * u;
+  }
+}
+
 // lower_bound over a sorted key array (uint64_t or U128).
 template <typename K>
 __device__ __forceinline__ long long lower_bound_key(const K *a, long long n, K v) {
