@@ -116,7 +116,25 @@ struct Interp {
   // FP32 pipe (GB300 issues FP64 at 1/64 of its FP32 rate), same 8 bytes
   // per weight as an FP64 copy.
   DBuf<float2> ap_w;
-  DBuf<int> perm;  // apply rows ordered by length inside windows
+  // P for the applies on tiles of 256 rows (k_tb_build): each tile's columns
+  // (tile_uoff, tile_ucol), every entry's place among them and the tile's rows
+  // by length; the most columns and entries of a tile
+  bool tile_ok = false;
+  int tile_maxu = 0, tile_maxe = 0;
+  DBuf<unsigned> tile_uoff;
+  DBuf<int> tile_ucol;
+  DBuf<uint16_t> tile_idx;
+  DBuf<uint8_t> tile_order;
+  // the transposed tiles (tile_t: used by the applies): runs of one column (row
+  // inside the tile, weight), one per (tile, column) pair, a tile's longest
+  // first: place among the pairs sorted by column, start in the tile and
+  // length; each column's pairs
+  bool tile_t = false;
+  DBuf<uint8_t> tile_row;
+  DBuf<float2> tile_w;
+  DBuf<uint2> tile_runs;
+  DBuf<unsigned> col_pairs;
+  DBuf<int> perm;  // apply rows ordered by length inside windows (without tiles)
   DBuf<int> t_rowptr, t_colidx;  // P^T (zero-free) as CSR, rows = coarse nodes
   DBuf<int> t_perm;  // P^T rows by input chunk of their last entry, then length
   std::vector<long long> t_chunk;  // t_perm range of each input chunk
@@ -128,7 +146,8 @@ struct Interp {
   // run in FP64); dfflag[1]: the same for the input vector of one apply
   DBuf<int> dfflag;
   bool have_colsum = false;
-  DBuf<double> colsum;  // P^T 1 (column sums of P), made on first use
+  DBuf<double> colsum;  // P^T 1 (column sums of P) and their reciprocals, made on
+                        // first use
 };
 
 struct Filter {

@@ -1002,35 +1002,11 @@ __device__ __forceinline__ void df_add(float &sh, float &sl, float oh, float ol)
   sh = t;
   df_renorm(sh, sl);
 }
-// sh + sl as a double, from the bits with integer operations (the FP64 pipe
-// carries no work of the applies but rare special cases).  (sh, sl) is
-// normalised, |sl| <= ulp(sh) / 2, so sl lies 24 or more binades below sh:
-// the double of sh plus sl in units of the double ulp at sh's exponent
-// (exact up to a gap of 29 binades, rounded half away from zero beyond;
-// when sh is a power of two and sl has the other sign the result falls
-// into the binade below, whose ulp is half as large).
+// sh + sl as a double, correctly rounded.  (Put together from the bits with
+// integer operations it took more time: the special cases were run in FP64 for
+// every value and selected from.)
 __device__ __forceinline__ double df_value(float sh, float sl) {
-  const unsigned bh = __float_as_uint(sh), bl = __float_as_uint(sl);
-  const int eh = (int)((bh >> 23) & 0xffu), el = (int)((bl >> 23) & 0xffu);
-  if (eh == 0 || eh == 255 || (el == 0 && (bl & 0x7fffffffu) != 0u) || el == 255)
-    return __dadd_rn((double)sh, (double)sl);  // zeros/subnormal sh, Inf, NaN
-  const unsigned long long hd = ((unsigned long long)(bh & 0x80000000u) << 32) |
-                                ((unsigned long long)(eh + 896) << 52) |
-                                ((unsigned long long)(bh & 0x7fffffu) << 29);
-  if (el == 0) return __longlong_as_double((long long)hd);  // sl = +-0
-  const int g = eh - el;
-  const bool neg = ((bh ^ bl) >> 31) != 0u;
-  const bool pow2 = (bh & 0x7fffffu) == 0u;
-  const int sft = (neg && pow2 ? 30 : 29) - g;
-  const unsigned long long ml = (unsigned long long)((bl & 0x7fffffu) | 0x800000u);
-  unsigned long long d;
-  if (sft >= 0)
-    d = ml << sft;
-  else if (sft > -26)
-    d = (ml + (1ULL << (-sft - 1))) >> (-sft);
-  else
-    d = 0;
-  return __longlong_as_double((long long)(neg ? hd - d : hd + d));
+  return __dadd_rn((double)sh, (double)sl);
 }
 
 // The apply copy's weights when it shares P's structure (nnz_nz == nnz).
@@ -1104,8 +1080,330 @@ __global__ void k_nz_fill(long long rows, const int *__restrict__ rp,
   if (have && g8 == 0 && r == rows - 1) nrp[rows] = (int)nzoff[rows];
 }
 
-// Transpose support.  Entries are keyed row << 32 | column; the stable
-// sort runs on the column bits only, so rows stay ascending inside each
+// ---------------------------------------------------------------------
+// The apply copy and P^T by tiles of TB_ROWS rows.  A tile's entries have few
+// distinct columns (115 of 2,170 entries for quadratic elements, 126 of 900
+// for linear ones: the fine nodes of a tile lie together on the curve), so a
+// tile is transposed in shared memory, and only its (column, run of entries)
+// pairs are sorted by column, stably; each run then moves to its place in
+// P^T.  Rows are ascending inside a run and tiles ascending inside a column:
+// the order of a stable sort of all entries by column.
+//
+// Bound by latency inside a tile (hash probes, bit masks, barriers): 664M
+// entries in 11.9 ms (2.7 TB/s of what must be moved), and 4.1 ms (3.6 TB/s) for
+// the runs' move.  The sort of all entries (key, place and row of each) took
+// three radix passes over them and a gather of the weights; with the applies by
+// tiles below, three levels of a quadratic mesh went from 143.8 to 121.4 ms.
+constexpr int TB_ROWS = 256;
+// Slots of a tile's column table (a power of two), columns it may hold and
+// entries it may have: the second size for tiles that need it, and beyond
+// that the sort of all entries.
+struct TbSize {
+  int slots, cols, entries;
+};
+constexpr TbSize TB_SIZES[2] = {{512, 384, 4096}, {2048, 1536, 8192}};
+__host__ __device__ inline size_t tb_smem(const TbSize &Z) {
+  return (size_t)Z.slots * (4 + 2) + (size_t)Z.cols * (32 + 8 + 4 + 4 + 2) + (size_t)Z.entries * 3;
+}
+// off: first kept entry of every row in the apply copy (rowptr itself when
+// every entry is kept: nci and nrp are null then).  Per tile, at its first
+// entry's place: pcol and pstart, its columns ascending and where their runs
+// start in it; trow and tw, the transposed entries (row inside the tile,
+// weight).  idx: every entry's place among its tile's columns; order: the
+// tile's rows, longest first (rows of one length in any order).  state[0]: a
+// tile does not fit, [1], [2]: the most columns and entries of a tile.
+template <bool ALL>
+__global__ void __launch_bounds__(TB_ROWS)
+    k_tb_build(long long rows, TbSize Z, const int *__restrict__ rp, const int *__restrict__ ci,
+               const double *__restrict__ v, const long long *__restrict__ keepoff, int *nrp,
+               int *nci, float2 *nw, int *flag, unsigned *ucount, int *pcol, unsigned *pstart,
+               uint8_t *trow, float2 *tw, uint16_t *idx, uint8_t *order, int *state) {
+  extern __shared__ __align__(16) unsigned char tb_mem[];
+  // per column: its rows as 8 words, and the number of rows before each word
+  // as 8 bytes (at most 224)
+  unsigned *mask = (unsigned *)tb_mem;
+  unsigned long long *before = (unsigned long long *)(mask + 8 * Z.cols);
+  int *tab = (int *)(before + Z.cols);                // per slot: its column
+  int *cols = tab + Z.slots;                          // columns as found
+  unsigned *start = (unsigned *)(cols + Z.cols);      // per column: its run
+  uint16_t *cslot = (uint16_t *)(start + Z.cols);     // slots of the columns as found
+  uint16_t *rank = cslot + Z.cols;                    // per slot: place of its column
+  uint16_t *eslot = rank + Z.slots;                   // per entry: slot, and row
+  uint8_t *erow = (uint8_t *)(eslot + Z.entries);
+  constexpr int LB = 64;  // row lengths told apart (longer ones are one class)
+  __shared__ int s_rp[TB_ROWS + 1], s_new, s_empty, s_kept[TB_ROWS / 32], s_len[LB];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const long long r0 = (long long)blockIdx.x * TB_ROWS;
+  const int nr = (int)min((long long)TB_ROWS, rows - r0);
+  const long long base = ALL ? (long long)__ldg(rp + r0) : __ldg(keepoff + r0);
+  const long long lim = ALL ? (long long)__ldg(rp + r0 + nr) : __ldg(keepoff + r0 + nr);
+  const int ne = (int)(lim - base);
+  if (ne > Z.entries) {  // uniform
+    if (t == 0) atomicOr(state, 1);
+    return;
+  }
+  for (int i = t; i <= nr; i += TB_ROWS) {
+    s_rp[i] = __ldg(rp + r0 + i);
+    if (!ALL) {
+      const int d = (int)__ldg(keepoff + r0 + i);
+      if (i < nr || r0 + nr == rows) nrp[r0 + i] = d;
+    }
+  }
+  for (int i = t; i < Z.slots; i += TB_ROWS) tab[i] = -1;
+  if (t == 0) s_new = s_empty = 0;
+  __syncthreads();
+  if (t < nr && s_rp[t] == s_rp[t + 1]) s_empty = 1;
+  int mylen = 0;
+  if (t < nr)
+    mylen = ALL ? s_rp[t + 1] - s_rp[t]
+                : (int)(__ldg(keepoff + r0 + t + 1) - __ldg(keepoff + r0 + t));
+  if (t < LB) s_len[t] = 0;
+  // each warp takes a run of the tile's entries of P; their kept ones are
+  // counted first, which gives the warp its place in the copy
+  const int f0 = s_rp[0], nf = s_rp[nr] - f0;
+  const int per = (nf + TB_ROWS - 1) / TB_ROWS * 32;
+  const int a0 = min(nf, warp * per), a1 = min(nf, a0 + per);
+  int at = a0;
+  if (!ALL) {
+    int kept = 0;
+#pragma unroll 4
+    for (int p = a0 + lane; p < a1; p += 32) kept += apply_keeps(__ldg(v + f0 + p));
+    kept = __reduce_add_sync(0xffffffffu, kept);
+    if (lane == 0) s_kept[warp] = kept;
+    __syncthreads();
+    at = 0;
+    for (int w = 0; w < warp; w++) at += s_kept[w];
+  } else {
+    __syncthreads();
+  }
+  // an entry's row is the last one that starts at or before it.  Without empty
+  // rows 32 entries begin at most 32 rows, whose starts make a bit mask.
+  const bool any_empty = s_empty != 0;
+  auto row_of = [&](int p) {
+    int lo = 0, hi = nr;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_rp[mid] <= f0 + p)
+        lo = mid;
+      else
+        hi = mid;
+    }
+    return lo;
+  };
+  int row0 = a0 < a1 ? row_of(a0) : 0;
+#pragma unroll 2
+  for (int q0 = a0; q0 < a1; q0 += 32) {
+    const int p = q0 + lane;
+    const bool on = p < a1;
+    const double w = on ? __ldg(v + f0 + p) : 0.0;
+    const int c = on ? __ldg(ci + f0 + p) : 0;
+    const bool keep = on && (ALL || apply_keeps(w));
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    int lr;
+    if (any_empty) {
+      lr = on ? row_of(p) : 0;
+    } else {
+      const int nx = row0 + 1 + lane, d = nx < nr ? s_rp[nx] - f0 - q0 : 32;
+      const unsigned sm = __reduce_or_sync(0xffffffffu, d < 32 ? 1u << d : 0u);
+      lr = row0 + __popc(sm & (0xffffffffu >> (31 - lane)));
+      row0 += __popc(sm);
+      // entry 32 may begin a row too: it is the next trip's first
+      if (row0 + 1 < nr && s_rp[row0 + 1] - f0 == q0 + 32) row0++;
+    }
+    if (keep) {
+      const int li = at + __popc(m & ((1u << lane) - 1u));
+      if (!ALL) nci[base + li] = c;
+      nw[base + li] = df_weight(w, flag);
+      unsigned h = ((unsigned)c * 0x9E3779B1u) >> 16 & (unsigned)(Z.slots - 1);
+      for (int k = 0; k < Z.slots; k++) {
+        int was = *(volatile int *)(tab + h);
+        if (was == -1) {
+          was = atomicCAS(tab + h, -1, c);
+          if (was == -1) {
+            const int u = atomicAdd(&s_new, 1);
+            if (u < Z.cols) {
+              cols[u] = c;
+              cslot[u] = (uint16_t)h;
+            }
+          }
+        }
+        if (was == -1 || was == c || *(volatile int *)&s_new > Z.cols) break;
+        h = (h + 1) & (unsigned)(Z.slots - 1);
+      }
+      eslot[li] = (uint16_t)h;
+      erow[li] = (uint8_t)lr;
+    }
+    at += __popc(m);
+  }
+  __syncthreads();
+  const int U = s_new;
+  if (U > Z.cols) {  // uniform
+    if (t == 0) atomicOr(state, 1);
+    return;
+  }
+  // row order: a counting sort on the length, longest first
+  const int bucket = LB - 1 - min(mylen, LB - 1);
+  atomicAdd(&s_len[bucket], 1);
+  __syncthreads();
+  if (warp == 0) {
+    const int a = s_len[2 * lane], b = s_len[2 * lane + 1];
+    int incl = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    s_len[2 * lane] = incl - a - b;
+    s_len[2 * lane + 1] = incl - b;
+  }
+  __syncthreads();
+  order[(long long)blockIdx.x * TB_ROWS + atomicAdd(&s_len[bucket], 1)] = (uint8_t)t;
+  // the columns' places in ascending order, by counting
+  for (int k = t; k < U; k += TB_ROWS) {
+    const int c = cols[k];
+    int r = 0;
+    for (int j = 0; j < U; j++) r += cols[j] < c;
+    rank[cslot[k]] = (uint16_t)r;
+    pcol[base + r] = c;
+  }
+  for (int i = t; i < 8 * U; i += TB_ROWS) mask[i] = 0u;
+  __syncthreads();
+  for (int li = t; li < ne; li += TB_ROWS) {
+    const int u = rank[eslot[li]], lr = erow[li];
+    const unsigned bit = 1u << (lr & 31);
+    eslot[li] = (uint16_t)u;
+    // (a row that names a column twice has no place of its own)
+    if (atomicOr(mask + 8 * u + (lr >> 5), bit) & bit) atomicOr(state, 1);
+  }
+  __syncthreads();
+  // the runs' starts
+  if (warp == 0) {
+    unsigned run = 0;
+    for (int k0 = 0; k0 < U; k0 += 32) {
+      const int k = k0 + lane;
+      unsigned c = 0;
+      if (k < U) {
+        unsigned long long b = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          b |= (unsigned long long)(c & 0xffu) << (8 * q);
+          c += __popc(mask[8 * k + q]);
+        }
+        before[k] = b;
+      }
+      unsigned incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (k < U) {
+        start[k] = run + incl - c;
+        pstart[base + k] = run + incl - c;
+      }
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+  }
+  if (t == 0) {
+    ucount[blockIdx.x] = (unsigned)U;
+    atomicMax(state + 1, U);
+    atomicMax(state + 2, ne);
+  }
+  __syncthreads();
+  // every entry to its run: its place there is the number of its column's
+  // rows before its own
+  for (int li = t; li < ne; li += TB_ROWS) {
+    const int u = eslot[li], lr = erow[li];
+    const unsigned place = start[u] + (unsigned)((uint8_t *)(before + u))[lr >> 5] +
+                           __popc(mask[8 * u + (lr >> 5)] & ((1u << (lr & 31)) - 1u));
+    trow[base + place] = (uint8_t)lr;
+    tw[base + place] = nw[base + li];
+    idx[base + li] = (uint16_t)u;
+  }
+}
+// The tiles' pairs side by side: column (twice: the tile's list, and the key
+// of the sort), place of the run and its length and tile; and every tile's
+// pairs with the longest runs first (runs[pos]; equal lengths in any order).
+__global__ void __launch_bounds__(128)
+    k_tb_pairs(long long rows, const long long *__restrict__ keepoff,
+               const int *__restrict__ rp, const unsigned *__restrict__ uoff,
+               const int *__restrict__ pcol, const unsigned *__restrict__ pstart,
+               int *ucol, uint32_t *key, uint32_t *pay, unsigned *src, unsigned *len,
+               unsigned *tile, unsigned *pos, uint2 *runs) {
+  __shared__ int s_cnt[64];
+  const long long r0 = (long long)blockIdx.x * TB_ROWS, r1 = min(rows, r0 + TB_ROWS);
+  const long long base = keepoff ? keepoff[r0] : rp[r0];
+  const unsigned ne = (unsigned)((keepoff ? keepoff[r1] : (long long)rp[r1]) - base);
+  const unsigned u0 = uoff[blockIdx.x], U = uoff[blockIdx.x + 1] - u0;
+  if (threadIdx.x < 64) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  for (unsigned k = threadIdx.x; k < U; k += blockDim.x) {
+    const int c = pcol[base + k];
+    const unsigned a = pstart[base + k], b = k + 1 < U ? pstart[base + k + 1] : ne;
+    ucol[u0 + k] = c;
+    key[u0 + k] = (uint32_t)c;
+    pay[u0 + k] = u0 + k;
+    src[u0 + k] = (unsigned)(base + a);
+    len[u0 + k] = b - a;
+    tile[u0 + k] = blockIdx.x;
+    atomicAdd(&s_cnt[63 - min((b - a) >> 1, 63u)], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int l = threadIdx.x, a = s_cnt[2 * l], b = s_cnt[2 * l + 1];
+    int incl = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (l >= o) incl += y;
+    }
+    s_cnt[2 * l] = incl - a - b;
+    s_cnt[2 * l + 1] = incl - b;
+  }
+  __syncthreads();
+  for (unsigned k = threadIdx.x; k < U; k += blockDim.x) {
+    const unsigned n = len[u0 + k];
+    const unsigned o = u0 + (unsigned)atomicAdd(&s_cnt[63 - min(n >> 1, 63u)], 1);
+    pos[u0 + k] = o;
+    runs[o].y = (pstart[base + k] << 16) | n;
+  }
+}
+__global__ void k_tb_gather(long long n, const uint32_t *__restrict__ pay,
+                            const unsigned *__restrict__ len, unsigned *out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = len[pay[i]];
+}
+// Runs to their places in P^T, 8 lanes each; the pairs' places in the sorted
+// order and the columns' starts in entries and in pairs.
+__global__ void k_tb_copy(long long n, const uint32_t *__restrict__ key,
+                          const uint32_t *__restrict__ pay, const unsigned *__restrict__ toff,
+                          const unsigned *__restrict__ src, const unsigned *__restrict__ tile,
+                          const uint8_t *__restrict__ trow, const float2 *__restrict__ tw,
+                          int *tcols, float2 *tvals, int *trowptr,
+                          const unsigned *__restrict__ pos, uint2 *runs, unsigned *cstart) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long i = t >> 3;
+  if (i >= n) return;
+  const int l = (int)(t & 7);
+  const uint32_t q = pay[i];
+  const unsigned o = toff[i], m = toff[i + 1] - o, s = src[q];
+  const int r0 = (int)(tile[q] * TB_ROWS);
+  for (unsigned k = l; k < m; k += 8) {
+    tcols[o + k] = r0 + (int)__ldg(trow + s + k);
+    tvals[o + k] = __ldg(tw + s + k);
+  }
+  if (l == 0) {
+    runs[pos[q]].x = (unsigned)i;
+    const int c = (int)key[i], cprev = i == 0 ? -1 : (int)key[i - 1];
+    for (int j = cprev + 1; j <= c; j++) {
+      trowptr[j] = (int)o;
+      cstart[j] = (unsigned)i;
+    }
+  }
+}
+
+// Transpose support where the tiles do not fit.  Entries are keyed row << 32 |
+// column; the stable sort runs on the column bits only, so rows stay ascending inside each
 // column (the entries arrive row-major) with a third of the passes a full
 // (column, row) key would take.  8 lanes per row write its entries.
 __global__ void k_t_keys(long long rows, const int *__restrict__ rowptr,
@@ -1135,12 +1433,15 @@ __global__ void k_t_fill(long long nnz, const uint32_t *__restrict__ keys,
   int cprev = (i == 0) ? -1 : (int)keys[i - 1];
   for (int j = cprev + 1; j <= c; j++) trowptr[j] = (int)i;
 }
-__global__ void k_t_tail(long long ncols, long long nnz, const uint32_t *__restrict__ keys,
-                         int *trowptr) {
+__global__ void k_t_tail(long long ncols, long long nnz, long long nkeys,
+                         const uint32_t *__restrict__ keys, int *trowptr, unsigned *cstart) {
   // columns after the last entry's column are empty
   long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int clast = nnz ? (int)keys[nnz - 1] : -1;
-  if (j > clast && j <= ncols) trowptr[j] = (int)nnz;
+  int clast = nkeys ? (int)keys[nkeys - 1] : -1;
+  if (j > clast && j <= ncols) {
+    trowptr[j] = (int)nnz;
+    if (cstart) cstart[j] = (unsigned)nkeys;
+  }
 }
 // Rows ordered by length inside windows of LO_WIN rows (one block per
 // window, counting sort on min(length, LO_BUCKETS - 1)); the order inside a
@@ -1213,6 +1514,8 @@ __global__ void k_chunk_bounds(long long n, const uint64_t *__restrict__ keys, i
   }
   bounds[k] = lo;
 }
+// sum[rows + r]: its reciprocal where the sum is within 2^+-64, else 0 (the
+// quotients of k_df_pair_sum are then divided).
 __global__ void k_rowsum(long long rows, const int *__restrict__ rowptr,
                          const float2 *__restrict__ vals, double *sum) {
   long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1223,6 +1526,8 @@ __global__ void k_rowsum(long long rows, const int *__restrict__ rowptr,
     s = __dadd_rn(s, __dadd_rn((double)w.x, (double)w.y));
   }
   sum[r] = s;
+  const double a = fabs(s);
+  sum[rows + r] = a >= 0x1p-64 && a <= 0x1p64 ? __ddiv_rn(1.0, s) : 0.0;
 }
 
 // findEnclosing (TMROctForest.cpp:6228-6377) for a batch of nodes: each
@@ -1832,12 +2137,134 @@ void interp_create(Forest &fine, Forest &coarse, Interp &I) {
   interp_finish(I, nonzeros, s, states ? keep.p : nullptr);
 }
 
+// The apply copy (I.ap_w, and I.nz_rowptr / I.nz_colidx where entries are
+// dropped) and P^T by tiles; false, with nothing usable written, where some
+// tile has too many columns or entries.
+static bool transpose_tiles(Interp &I, const long long *keepoff, cudaStream_t s) {
+  const long long rows = I.rows, nnz = I.nnz_nz;
+  I.tile_ok = I.tile_t = false;
+  if (rows == 0 || nnz == 0) return false;
+  const long long tiles = (rows + TB_ROWS - 1) / TB_ROWS;
+  DBuf<unsigned> &ucount = I.tile_uoff;
+  ucount.alloc(tiles + 1, s);
+  I.tile_order.alloc(tiles * TB_ROWS, s);
+  DBuf<int> pcol(nnz, s), state(3, s);
+  DBuf<unsigned> pstart(nnz, s);
+  DBuf<uint8_t> &trow = I.tile_row;
+  DBuf<float2> &tw = I.tile_w;
+  trow.alloc(nnz, s);
+  tw.alloc(nnz, s);
+  DBuf<uint16_t> &idx = I.tile_idx;
+  idx.alloc(nnz, s);
+  long long np = -1;
+  for (const TbSize &Z : TB_SIZES) {
+    const size_t smem = tb_smem(Z);
+    TMRG_CUDA(cudaFuncSetAttribute(k_tb_build<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)tb_smem(TB_SIZES[1])));
+    TMRG_CUDA(cudaFuncSetAttribute(k_tb_build<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)tb_smem(TB_SIZES[1])));
+    state.zero();
+    // compulsory traffic: P once; the copy and the transposed entries
+    prof_bytes(12 * I.nnz + 8 * rows + 21 * nnz + (keepoff ? 4 * nnz : 0));
+    if (keepoff)
+      launch(k_tb_build<false>, (unsigned)tiles, TB_ROWS, smem, s, rows, Z,
+             (const int *)I.rowptr.p, (const int *)I.colidx.p, (const double *)I.vals.p, keepoff,
+             I.nz_rowptr.p, I.nz_colidx.p, I.ap_w.p, I.dfflag.p, ucount.p, pcol.p, pstart.p,
+             trow.p, tw.p, idx.p, I.tile_order.p, state.p);
+    else
+      launch(k_tb_build<true>, (unsigned)tiles, TB_ROWS, smem, s, rows, Z,
+             (const int *)I.rowptr.p, (const int *)I.colidx.p, (const double *)I.vals.p,
+             (const long long *)nullptr, (int *)nullptr, (int *)nullptr, I.ap_w.p, I.dfflag.p,
+             ucount.p, pcol.p, pstart.p, trow.p, tw.p, idx.p, I.tile_order.p, state.p);
+    exclusive_scan<unsigned>(ucount.p, ucount.p, tiles, s);
+    const unsigned *pv[4] = {ucount.p + tiles, (const unsigned *)state.p,
+                             (const unsigned *)state.p + 1, (const unsigned *)state.p + 2};
+    unsigned hv[4];
+    read_scalars(pv, hv, s);
+    if (!hv[1]) {
+      np = hv[0];
+      I.tile_maxu = (int)hv[2];
+      I.tile_maxe = (int)hv[3];
+      break;
+    }
+  }
+  if (np < 0) {
+    ucount.release();
+    trow.release();
+    tw.release();
+    idx.release();
+    I.tile_order.release();
+    return false;
+  }
+  I.tile_ok = true;
+  // P^T applies by tiles keep a sum per pair and vector: no more of them than
+  // inputs (nested meshes have about half as many)
+  I.tile_t = np <= rows;
+  Stage st_t("tmrg_transpose");
+  DBuf<int> &ucol = I.tile_ucol;
+  ucol.alloc(np, s);
+  DBuf<uint32_t> key(np, s), pay(np, s);
+  DBuf<unsigned> tile(np, s), toff(np + 1, s), src(np, s), len(np, s), pos(np, s);
+  I.tile_runs.alloc(np, s);
+  I.col_pairs.alloc(I.cols + 1, s);
+  launch(k_tb_pairs, (unsigned)tiles, 128, 0, s, rows, keepoff, (const int *)I.rowptr.p,
+         (const unsigned *)ucount.p, (const int *)pcol.p, (const unsigned *)pstart.p, ucol.p,
+         key.p, pay.p, src.p, len.p, tile.p, pos.p,
+         I.tile_runs.p);
+  radix_sort(key, &pay, np, bits_for(I.cols + 1), s);
+  launch(k_tb_gather, blocks_for(np, 256), 256, 0, s, np, (const uint32_t *)pay.p,
+         (const unsigned *)len.p, toff.p);
+  exclusive_scan<unsigned>(toff.p, toff.p, np, s);
+  prof_bytes(21 * nnz + 24 * np);
+  launch(k_tb_copy, blocks_for(np * 8, 256), 256, 0, s, np, (const uint32_t *)key.p,
+         (const uint32_t *)pay.p, (const unsigned *)toff.p, (const unsigned *)src.p,
+         (const unsigned *)tile.p, (const uint8_t *)trow.p, (const float2 *)tw.p, I.t_colidx.p,
+         I.t_w.p, I.t_rowptr.p, (const unsigned *)pos.p, I.tile_runs.p, I.col_pairs.p);
+  launch(k_t_tail, blocks_for(I.cols + 1, 256), 256, 0, s, I.cols, nnz, np,
+         (const uint32_t *)key.p, I.t_rowptr.p, I.col_pairs.p);
+  if (!I.tile_t) {
+    trow.release();
+    tw.release();
+    I.tile_runs.release();
+    I.col_pairs.release();
+  }
+  return true;
+}
+
+// The same by a stable sort of all entries by column.
+static void transpose_sorted(Interp &I, const long long *keepoff, cudaStream_t s) {
+  const long long rows = I.rows, nnz = I.nnz_nz;
+  // sort records (column key, position, row) of every apply entry
+  DBuf<uint32_t> tk(nnz + 1, s);
+  DBuf<uint32_t> tp(nnz + 1, s);
+  DBuf<int> erow(nnz + 1, s);
+  if (!keepoff) {
+    launch(k_df_weights, blocks_for(nnz, 256), 256, 0, s, nnz, (const double *)I.vals.p,
+           I.ap_w.p, I.dfflag.p);
+    launch(k_t_keys, blocks_for(rows * 8, 256), 256, 0, s, rows, (const int *)I.rowptr.p,
+           (const int *)I.colidx.p, tk.p, tp.p, erow.p);
+  } else {
+    launch(k_nz_fill, blocks_for(((rows + 3) / 4) * 32, 256), 256, 0, s, rows,
+           (const int *)I.rowptr.p, (const int *)I.colidx.p, (const double *)I.vals.p,
+           keepoff, I.nz_rowptr.p, I.nz_colidx.p, I.ap_w.p, I.dfflag.p, tk.p, tp.p, erow.p);
+  }
+  Stage st_t("tmrg_transpose");
+  // the column bits only: a stable LSD sort keeps rows ascending per column
+  radix_sort(tk, &tp, nnz, bits_for(I.cols + 1), s);
+  launch(k_t_fill, blocks_for(nnz, 256), 256, 0, s, nnz, (const uint32_t *)tk.p,
+         (const uint32_t *)tp.p, (const int *)erow.p, (const float2 *)I.ap_w.p, I.t_colidx.p,
+         I.t_w.p, I.t_rowptr.p);
+  launch(k_t_tail, blocks_for(I.cols + 1, 256), 256, 0, s, I.cols, nnz, nnz,
+         (const uint32_t *)tk.p, I.t_rowptr.p, (unsigned *)nullptr);
+}
+
 // The apply structures of a finished P (rows, cols, nnz, rowptr, colidx,
 // vals set): the apply copy without numerically-zero entries, the length-ordered
 // row permutation and P^T.
 void interp_finish(Interp &I, long long nonzeros, cudaStream_t s, const long long *keepoff) {
   const long long rows = I.rows, nnz = I.nnz;
   I.win_maxcol.clear();  // made again by the first host-buffer prolongation
+  I.perm.release();      // made where the tiles do not fit
   // the apply copy (apply_keeps entries), worth a second copy only when the
   // dropped entries are a good part of P
   I.nnz_nz = (nnz - nonzeros) * 8 >= nnz ? nonzeros : nnz;
@@ -1845,18 +2272,11 @@ void interp_finish(Interp &I, long long nonzeros, cudaStream_t s, const long lon
   I.dfflag.alloc(3, s);  // [0] weights, [1] inputs outside the double-float window, [2] TMA wait
   I.dfflag.zero();
   I.ap_w.alloc(nnz_nz + 1, s);
-  // transpose sort records (column key, position, row) of every apply entry
-  DBuf<uint32_t> tk(nnz_nz + 1, s);
-  DBuf<uint32_t> tp(nnz_nz + 1, s);
-  DBuf<int> erow(nnz_nz + 1, s);
-  if (I.nnz_nz == nnz) {
-    launch(k_df_weights, blocks_for(nnz, 256), 256, 0, s, nnz, (const double *)I.vals.p,
-           I.ap_w.p, I.dfflag.p);
-    launch(k_t_keys, blocks_for(rows * 8, 256), 256, 0, s, rows, (const int *)I.rowptr.p,
-           (const int *)I.colidx.p, tk.p, tp.p, erow.p);
-  }
-  if (I.nnz_nz < nnz) {
-    DBuf<long long> nzoff;
+  // offsets of the rows' kept entries (null where all are kept)
+  DBuf<long long> nzoff;
+  if (nnz_nz == nnz) {
+    keepoff = nullptr;
+  } else {
     if (!keepoff) {
       nzoff.alloc(rows + 1, s);
       launch(k_nz_count, blocks_for(rows * 8, 256), 256, 0, s, rows, (const int *)I.rowptr.p,
@@ -1867,34 +2287,27 @@ void interp_finish(Interp &I, long long nonzeros, cudaStream_t s, const long lon
     I.nz_rowptr.alloc(rows + 1, s);
     I.nz_colidx.alloc(nnz_nz + 1, s);
     if (rows == 0) TMRG_CUDA(cudaMemsetAsync(I.nz_rowptr.p, 0, sizeof(int), s));
-    launch(k_nz_fill, blocks_for(((rows + 3) / 4) * 32, 256), 256, 0, s, rows,
-           (const int *)I.rowptr.p, (const int *)I.colidx.p, (const double *)I.vals.p,
-           keepoff, I.nz_rowptr.p, I.nz_colidx.p, I.ap_w.p, I.dfflag.p, tk.p, tp.p, erow.p);
   }
-
-  I.perm.alloc(rows + 1, s);
-  launch(k_len_order, blocks_for(rows, LO_WIN), LO_THREADS, 0, s, rows, I.ap_rowptr(),
-         (const int *)nullptr, I.perm.p);
-
-  // P^T by a stable sort on the column (rows stay ascending per column).
-  Stage st_t("tmrg_transpose");
   I.t_colidx.alloc(nnz_nz + 1, s);
   I.t_w.alloc(nnz_nz + 1, s);
   I.t_rowptr.alloc(I.cols + 1, s);
-  // the column bits only: a stable LSD sort keeps rows ascending per column
-  const int cbits = bits_for(I.cols + 1);
-  radix_sort(tk, &tp, nnz_nz, cbits, s);
-  launch(k_t_fill, blocks_for(nnz_nz, 256), 256, 0, s, nnz_nz, (const uint32_t *)tk.p,
-         (const uint32_t *)tp.p, (const int *)erow.p, (const float2 *)I.ap_w.p, I.t_colidx.p,
-         I.t_w.p, I.t_rowptr.p);
-  launch(k_t_tail, blocks_for(I.cols + 1, 256), 256, 0, s, I.cols, nnz_nz,
-         (const uint32_t *)tk.p, I.t_rowptr.p);
-  tk.release();
-  tp.release();
-  erow.release();
-  // P^T rows ordered by the input chunk their last entry needs (stable),
-  // then by length inside 4096-row windows of each chunk
-  {
+  if (!transpose_tiles(I, keepoff, s)) transpose_sorted(I, keepoff, s);
+  nzoff.release();
+
+  if (!I.tile_ok) {
+    I.perm.alloc(rows + 1, s);
+    launch(k_len_order, blocks_for(rows, LO_WIN), LO_THREADS, 0, s, rows, I.ap_rowptr(),
+           (const int *)nullptr, I.perm.p);
+  }
+
+  I.t_chunk.clear();
+  if (I.tile_t) {
+    I.t_perm.alloc(I.cols + 1, s);
+    launch(k_len_order, blocks_for(I.cols, LO_WIN), LO_THREADS, 0, s, I.cols,
+           (const int *)I.t_rowptr.p, (const int *)nullptr, I.t_perm.p);
+  } else {
+    // P^T rows ordered by the input chunk their last entry needs (stable),
+    // then by length inside 4096-row windows of each chunk
     DBuf<uint64_t> ck(I.cols + 1, s);
     DBuf<uint32_t> cv(I.cols + 1, s);
     launch(k_t_chunk_keys, blocks_for(I.cols, 256), 256, 0, s, I.cols, rows,
@@ -2129,7 +2542,7 @@ void topo_weights_create(Forest &filter, Forest &analysis, Interp &I) {
 // Column sums of P for the weight-normalised transpose, on first use.
 static void interp_colsum(Interp &I) {
   if (I.have_colsum) return;
-  I.colsum.alloc(I.cols + 1, I.s);
+  I.colsum.alloc(2 * I.cols + 1, I.s);
   launch(k_rowsum, blocks_for(I.cols, 256), 256, 0, I.s, I.cols,
          (const int *)I.t_rowptr.p, (const float2 *)I.t_w.p, I.colsum.p);
   I.have_colsum = true;
@@ -2146,9 +2559,7 @@ static void interp_colsum(Interp &I) {
 // Few vectors on a small matrix, in FP64 straight from the caller's vector:
 // 2^LB lanes per row take its entries in turn, each with all NV components,
 // and combine in a fixed tree.  One launch instead of a flag reset, a pass
-// that splits the input and an apply; no window on the values.  The weight is
-// put together from its two floats with integer operations, which leaves the
-// FP64 pipe NV instructions an entry.
+// that splits the input and an apply; no window on the values.
 template <int NV>
 __global__ void __launch_bounds__(256)
     k_f64_rows(long long rows, int LB, const int *__restrict__ rowptr,
@@ -2256,8 +2667,9 @@ __global__ void __launch_bounds__(256)
 // wait more arithmetic.
 // An odd number of vectors is carried as one more, zero, in the (hi, lo)
 // input (a lane per vector took 1.70 ms for 3 vectors and 117M entries, whole
-// pairs take 0.96 ms; 7 vectors 3.04 and 1.75 ms); SC: the caller's vectors then have no 16-byte rows (nor has an
-// unaligned buffer) and are read and written value by value.
+// pairs take 0.96 ms; 7 vectors 3.04 and 1.75 ms); SC: the caller's vectors
+// then have no 16-byte rows (nor has an unaligned buffer) and are read and
+// written value by value.
 template <int LPR, int NG, int PPL, bool SC>
 __global__ void __launch_bounds__(256)
     k_df_apply2(long long rows, int nvec2, int nvec, const int *__restrict__ rowptr,
@@ -2411,6 +2823,236 @@ __global__ void __launch_bounds__(256)
         }
       }
     }
+  }
+}
+
+// P and P^T by tiles (k_tb_build), in double-float, V = 2 L vectors at once:
+// L = 2^LB lanes per row or run hold one vector pair each.  The inputs of a
+// tile are split into (hi, lo) as they are loaded into shared memory, so no
+// split copy of the input is made and no input row is gathered more than once
+// per tile; an entry reads one row of 16 L bytes there.  A value outside the
+// double-float window (or a weight, flags[0]) sets flags[1]; the apply is then
+// run again by the FP64 kernels, which return at once when no flag is set.
+// (The flags are reset before the apply.)
+//
+// Bound by instruction issue (12 FP32 instructions an entry and vector, and
+// about half as many around them).  117M entries, 2 / 4 / 8 / 16 vectors: P 606
+// / 957 / 1728 / 2247 us from a split copy and gathers in L2 -> 582 / 774 / 918
+// / 1730 us; P^T 4 / 8 / 16 vectors 1059 / 1912 / 3003 -> 952 / 1290 / 2370 us,
+// 2 vectors 685 us against 808 (stays with k_df_apply2).  4.8M entries, 4 and 16
+// vectors: P 78 and 172 -> 55 and 144 us, P^T 83 and 215 -> 81 and 200 us.
+// Tried: the entries in shared memory too (P, 16 vectors 2100 us), two pairs a
+// lane (P^T 2840 us), the input split beforehand (P 1790 us).
+struct DfTiles {
+  long long rows, tiles, tile0;
+  int nvec, maxu;
+  const unsigned *uoff;
+  const int *ucol;
+  const float2 *w;  // the apply copy (P) or the tiles' runs (P^T)
+};
+__device__ __forceinline__ float2 df_in(double v, bool &out) {
+  float hi, lo;
+  out |= !df_split(v, DF_X_EMIN, DF_X_ERANGE, hi, lo);
+  return make_float2(hi, lo);
+}
+
+// y = P x.  Rows longest first.
+template <int LB>
+__global__ void __launch_bounds__(TB_ROWS)
+    k_df_tile(DfTiles D, bool scalar, const int *__restrict__ rp,
+              const uint16_t *__restrict__ idx, const uint8_t *__restrict__ order,
+              const double *__restrict__ x, double *__restrict__ y, int *flags) {
+  constexpr int L = 1 << LB, V = 2 * L;
+  extern __shared__ __align__(16) unsigned char dt_mem[];
+  float2 *sx = (float2 *)dt_mem;  // maxu x V
+  __shared__ int s_rp[TB_ROWS + 1];
+  __shared__ uint8_t s_ord[TB_ROWS];
+  if (flags[0] != 0) return;  // (no block may leave for flags[1], which others are setting)
+  const int t = threadIdx.x, nvec = D.nvec;
+  const long long tile = D.tile0 + blockIdx.x, r0 = tile * TB_ROWS;
+  const int nr = (int)min((long long)TB_ROWS, D.rows - r0);
+  const unsigned u0 = D.uoff[tile];
+  const int U = (int)(D.uoff[tile + 1] - u0);
+  for (int i = t; i <= nr; i += TB_ROWS) s_rp[i] = __ldg(rp + r0 + i);
+  s_ord[t] = __ldg(order + tile * TB_ROWS + t);
+  __syncthreads();
+  const int base = s_rp[0];
+  const int l = t & (L - 1);
+  bool out = false;
+  for (int c0 = 0; c0 < nvec; c0 += V) {
+#pragma unroll 4
+    for (int i = t; i < U * V; i += TB_ROWS) {
+      const int k = i >> (LB + 1), v = c0 + (i & (V - 1));
+      sx[i] = v < nvec ? df_in(__ldg(x + (long long)__ldg(D.ucol + u0 + k) * nvec + v), out)
+                       : make_float2(0.0f, 0.0f);
+    }
+    __syncthreads();
+    const float4 *xp = (const float4 *)sx + l;
+    for (int q = t >> LB; q < TB_ROWS; q += TB_ROWS >> LB) {
+      const int lr = s_ord[q];
+      if (lr >= nr) continue;
+      const int p0 = s_rp[lr] - base, p1 = s_rp[lr + 1] - base;
+      float ah = 0.0f, al = 0.0f, bh = 0.0f, bl = 0.0f;
+      auto entry = [&](int p) {
+        const float2 wv = __ldg(D.w + base + p);
+        const float4 xv = xp[(int)__ldg(idx + base + p) * L];
+        df_fma(wv.x, wv.y, xv.x, xv.y, ah, al);
+        df_fma(wv.x, wv.y, xv.z, xv.w, bh, bl);
+      };
+      int p = p0;
+      for (; p + 4 <= p1; p += 4) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) entry(p + k);
+        df_renorm(ah, al);
+        df_renorm(bh, bl);
+      }
+      for (; p < p1; p++) entry(p);
+      df_renorm(ah, al);
+      df_renorm(bh, bl);
+      const int v0 = c0 + 2 * l;
+      double *yp = y + (r0 + lr) * nvec + v0;
+      const double a = df_value(ah, al), b = df_value(bh, bl);
+      if (scalar) {
+        if (v0 < nvec) yp[0] = a;
+        if (v0 + 1 < nvec) yp[1] = b;
+      } else if (v0 < nvec) {
+        *(double2 *)yp = make_double2(a, b);
+      }
+    }
+    __syncthreads();
+  }
+  if (out) atomicOr(flags + 1, 1);
+}
+// The same tiles in FP64: a thread per row and vector.
+__global__ void __launch_bounds__(TB_ROWS)
+    k_df_tile_f64(DfTiles D, const int *__restrict__ rp, const uint16_t *__restrict__ idx,
+                  const double *__restrict__ x, double *__restrict__ y,
+                  const int *__restrict__ flags) {
+  if ((__ldg(flags) | __ldg(flags + 1)) == 0) return;
+  for (long long tile = D.tile0 + blockIdx.x; tile < D.tile0 + D.tiles; tile += gridDim.x) {
+    const long long r0 = tile * TB_ROWS;
+    const int nr = (int)min((long long)TB_ROWS, D.rows - r0);
+    const int *uc = D.ucol + D.uoff[tile];
+    for (int i = threadIdx.x; i < nr * D.nvec; i += TB_ROWS) {
+      const int lr = i / D.nvec, v = i - lr * D.nvec;
+      double a = 0.0;
+      for (int p = __ldg(rp + r0 + lr); p < __ldg(rp + r0 + lr + 1); p++) {
+        const float2 wv = __ldg(D.w + p);
+        a = __fma_rn(__dadd_rn((double)wv.x, (double)wv.y),
+                     __ldg(x + (long long)__ldg(uc + __ldg(idx + p)) * D.nvec + v), a);
+      }
+      y[(r0 + lr) * D.nvec + v] = a;
+    }
+  }
+}
+
+// y = P^T x in two parts: every tile sums its runs (the entries of one column
+// in the tile) over its own input rows, which are one block of memory, and
+// k_df_pair_sum adds a column's runs, tiles ascending.  Runs longest first.
+template <int LB>
+__global__ void __launch_bounds__(TB_ROWS)
+    k_df_tile_t(DfTiles D, const int *__restrict__ rp, const uint2 *__restrict__ runs,
+                const uint8_t *__restrict__ row, const double *__restrict__ x,
+                float2 *__restrict__ part, int *flags) {
+  constexpr int L = 1 << LB, V = 2 * L;
+  extern __shared__ __align__(16) unsigned char dt_mem[];
+  float2 *sx = (float2 *)dt_mem;  // TB_ROWS x V
+  if (flags[0] != 0) return;  // (no block may leave for flags[1], which others are setting)
+  const int t = threadIdx.x, nvec = D.nvec, tile = (int)D.tile0 + blockIdx.x;
+  const long long r0 = (long long)tile * TB_ROWS;
+  const int nr = (int)min((long long)TB_ROWS, D.rows - r0);
+  const unsigned u0 = D.uoff[tile];
+  const int U = (int)(D.uoff[tile + 1] - u0);
+  const int l = t & (L - 1);
+  bool out = false;
+  for (int c0 = 0; c0 < nvec; c0 += V) {
+#pragma unroll 4
+    for (int i = t; i < nr * V; i += TB_ROWS) {
+      const int k = i >> (LB + 1), v = c0 + (i & (V - 1));
+      sx[i] = v < nvec ? df_in(__ldg(x + (r0 + k) * nvec + v), out) : make_float2(0.0f, 0.0f);
+    }
+    __syncthreads();
+    const float4 *xp = (const float4 *)sx + l;
+    for (int q = t >> LB; q < U; q += TB_ROWS >> LB) {
+      const uint2 run = __ldg(runs + u0 + q);  // place, start and length
+      const unsigned s = __ldg(rp + r0) + (run.y >> 16);
+      const int n = (int)(run.y & 0xffffu);
+      float ah = 0.0f, al = 0.0f, bh = 0.0f, bl = 0.0f;
+      auto entry = [&](int p) {
+        const float2 wv = __ldg(D.w + s + p);
+        const float4 xv = xp[(int)__ldg(row + s + p) * L];
+        df_fma(wv.x, wv.y, xv.x, xv.y, ah, al);
+        df_fma(wv.x, wv.y, xv.z, xv.w, bh, bl);
+      };
+      int p = 0;
+      for (; p + 4 <= n; p += 4) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) entry(p + k);
+        df_renorm(ah, al);
+        df_renorm(bh, bl);
+      }
+      for (; p < n; p++) entry(p);
+      df_renorm(ah, al);
+      df_renorm(bh, bl);
+      const int v0 = c0 + 2 * l;
+      float2 *o = part + (long long)run.x * nvec + v0;
+      if (v0 < nvec) o[0] = make_float2(ah, al);
+      if (v0 + 1 < nvec) o[1] = make_float2(bh, bl);
+    }
+    __syncthreads();
+  }
+  if (out) atomicOr(flags + 1, 1);
+}
+__global__ void __launch_bounds__(256)
+    k_df_pair_sum(long long cols, int nvec, const unsigned *__restrict__ cstart,
+                  const float2 *__restrict__ part, double *__restrict__ y,
+                  const double *__restrict__ scale, const int *__restrict__ flags) {
+  if ((__ldg(flags) | __ldg(flags + 1)) != 0) return;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= cols * nvec) return;
+  const long long c = (unsigned long long)t >> 32 ? t / nvec : (unsigned)t / (unsigned)nvec;
+  const int v = (int)(t - c * nvec);
+  const unsigned a = __ldg(cstart + c), b = __ldg(cstart + c + 1);
+  float sh = 0.0f, sl = 0.0f;
+  for (unsigned i = a; i < b; i++) {
+    const float2 q = __ldg(part + (long long)i * nvec + v);
+    df_add(sh, sl, q.x, q.y);
+  }
+  double r = df_value(sh, sl);
+  if (scale) {
+    // r / sc from the column's reciprocal and one correction
+    const double sc = scale[c], inv = scale[cols + c];
+    if (inv != 0.0) {
+      const double q = __dmul_rn(r, inv);
+      r = __fma_rn(__fma_rn(-q, sc, r), inv, q);
+    } else {
+      r = sc != 0.0 ? __ddiv_rn(r, sc) : 0.0;
+    }
+  }
+  y[t] = r;
+}
+// P^T in FP64 by its own rows, where the flags ask for it.
+__global__ void __launch_bounds__(256)
+    k_df_rows_f64(long long rows, int nvec, const int *__restrict__ rp,
+                  const int *__restrict__ ci, const float2 *__restrict__ w,
+                  const double *__restrict__ x, double *__restrict__ y,
+                  const double *__restrict__ scale, const int *__restrict__ flags) {
+  if ((__ldg(flags) | __ldg(flags + 1)) == 0) return;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < rows * nvec;
+       t += (long long)gridDim.x * blockDim.x) {
+    const long long r = t / nvec;
+    const int v = (int)(t - r * nvec);
+    double a = 0.0;
+    for (int p = __ldg(rp + r); p < __ldg(rp + r + 1); p++) {
+      const float2 wv = __ldg(w + p);
+      a = __fma_rn(__dadd_rn((double)wv.x, (double)wv.y),
+                   __ldg(x + (long long)__ldg(ci + p) * nvec + v), a);
+    }
+    if (scale) {
+      const double sc = scale[r];
+      a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
+    }
+    y[t] = a;
   }
 }
 
@@ -2696,6 +3338,67 @@ static void df_apply2(int shape, long long rows, int nvec, const int *rp, const 
 #undef TMRG_DF2
 #undef TMRG_DF2S
 }
+// Vectors at once: 16, 8, 4 or 2.
+static int df_tile_lanes(int nvec) {
+  int lb = 0;
+  while (lb < 3 && (2 << lb) < nvec) lb++;
+  return lb;
+}
+static DfTiles df_tiles(const Interp &I, long long t0, long long t1, int nvec, const float2 *w) {
+  return DfTiles{I.rows, t1 - t0, t0, nvec, I.tile_maxu, I.tile_uoff.p, I.tile_ucol.p, w};
+}
+// y = P x on tiles [t0, t1).
+static void df_tile_apply(const Interp &I, long long t0, long long t1, int nvec, const double *x,
+                          double *y, cudaStream_t s) {
+  const bool scalar = nvec % 2 != 0 || ((uintptr_t)y % 16) != 0;
+  const DfTiles D = df_tiles(I, t0, t1, nvec, I.ap_w.p);
+  auto smem = [&](int lb) { return sizeof(float2) * ((size_t)I.tile_maxu << (lb + 1)); };
+  int lb = df_tile_lanes(nvec);
+  while (lb > 0 && smem(lb) > 100 * 1024) lb--;  // tiles with many columns
+#define TMRG_DT(B)                                                                              \
+  do {                                                                                          \
+    TMRG_CUDA(cudaFuncSetAttribute(k_df_tile<B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
+                                   (int)smem(B)));                                              \
+    launch(k_df_tile<B>, (unsigned)(t1 - t0), TB_ROWS, smem(B), s, D, scalar, I.ap_rowptr(),    \
+           (const uint16_t *)I.tile_idx.p, (const uint8_t *)I.tile_order.p, x, y, I.dfflag.p);  \
+  } while (0)
+  switch (lb) {
+    case 0: TMRG_DT(0); break;
+    case 1: TMRG_DT(1); break;
+    case 2: TMRG_DT(2); break;
+    default: TMRG_DT(3);
+  }
+#undef TMRG_DT
+  launch(k_df_tile_f64, (unsigned)std::min(t1 - t0, 152LL * 8), TB_ROWS, 0, s, D, I.ap_rowptr(),
+         (const uint16_t *)I.tile_idx.p, x, y, (const int *)I.dfflag.p);
+}
+// y = P^T x in two steps: the runs of tiles [t0, t1), then the columns
+// (divided by `scale` where given).
+static void df_tile_runs(const Interp &I, long long t0, long long t1, int nvec, const double *x,
+                         float2 *part, cudaStream_t s) {
+  if (t1 <= t0) return;
+  const DfTiles D = df_tiles(I, t0, t1, nvec, I.tile_w.p);
+#define TMRG_DT(B)                                                                             \
+  launch(k_df_tile_t<B>, (unsigned)(t1 - t0), TB_ROWS,                                         \
+         sizeof(float2) * ((size_t)TB_ROWS << (B + 1)), s, D, I.ap_rowptr(),                   \
+         (const uint2 *)I.tile_runs.p, (const uint8_t *)I.tile_row.p, x, part, I.dfflag.p)
+  switch (df_tile_lanes(nvec)) {
+    case 0: TMRG_DT(0); break;
+    case 1: TMRG_DT(1); break;
+    case 2: TMRG_DT(2); break;
+    default: TMRG_DT(3);
+  }
+#undef TMRG_DT
+}
+static void df_tile_columns(const Interp &I, int nvec, const float2 *part, const double *x,
+                            double *y, const double *scale, cudaStream_t s) {
+  launch(k_df_pair_sum, blocks_for(I.cols * nvec, 256), 256, 0, s, I.cols, nvec,
+         (const unsigned *)I.col_pairs.p, part, y, scale, (const int *)I.dfflag.p);
+  launch(k_df_rows_f64, std::min(blocks_for(I.cols * nvec, 256), 152u * 8), 256, 0, s, I.cols,
+         nvec, (const int *)I.t_rowptr.p, (const int *)I.t_colidx.p, (const float2 *)I.t_w.p, x,
+         y, scale, (const int *)I.dfflag.p);
+}
+
 // Size class of an apply: direction, vector pairs (8 = 8 or more), log2 of
 // the rows, mean row length in quarters (capped).
 static TuneKey df_key(int which, long long rows, long long nnz, int nvec2) {
@@ -2720,15 +3423,16 @@ static void df_split_input(Interp &I, const double *x, long long nrows, int nvec
 }
 
 // Transpose apply with the input in host memory: the input rows are copied
-// in TC_CHUNKS pieces on a second stream, and after piece k arrives (and is
-// split into (hi, lo) pairs) the output rows whose inputs all lie in pieces
-// <= k are computed (t_perm holds the rows grouped that way), so the copy
-// of the next piece overlaps them.  Same kernel, rows and summation order
+// in TC_CHUNKS pieces on a second stream.  With tiles, piece k's tiles are
+// summed as it arrives and the columns at the end.  Otherwise, after piece k
+// arrives (and is split into (hi, lo) pairs) the output rows whose inputs all
+// lie in pieces <= k are computed (t_perm holds the rows grouped that way), so
+// the copy of the next piece overlaps them.  Same kernel, rows and summation order
 // as the single apply; a piece with a value outside the double-float window
 // sends that piece's rows and every later piece's rows to FP64 (each row
 // only reads pieces already split, so a row never runs in double-float on
 // an input that was not represented).
-// Returns false (nothing done) where the grouped kernel does not apply.
+// Returns false (nothing done) where these kernels do not apply.
 // Reports (and clears) a TMA input stage of k_df_apply_tma that did not
 // complete within its wait limit; read where the host already waits.
 void interp_check_apply(Interp &I) {
@@ -2742,13 +3446,14 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
                                    double *y, int nvec) {
   if ((which != 1 && which != 2) || nvec % 2 != 0 || nvec / 2 < 8 ||
       ((uintptr_t)dx % 16) != 0 || ((uintptr_t)y % 16) != 0 ||
-      (long long)I.t_chunk.size() != TC_CHUNKS + 1)
+      (I.tile_t ? tune_forced(TUNE_PT) : (long long)I.t_chunk.size() != TC_CHUNKS + 1))
     return false;
   Stage st("tmrg_interp_mult_transpose_staged");
   cudaStream_t s = I.s;
   if (which == 2) interp_colsum(I);
   const long long nin = I.rows;
-  DBuf<float2> xs(nin * nvec + 1, s);
+  // the split input, or with tiles the runs' sums
+  DBuf<float2> xs((I.tile_t ? (long long)I.tile_runs.n : nin) * nvec + 1, s);
   TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
   cudaStream_t cs;
   TMRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -2773,6 +3478,12 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
   for (int k = 0; k < TC_CHUNKS; k++) {
     TMRG_CUDA(cudaStreamWaitEvent(s, ev[k], 0));
     const long long r0 = r0s[k], r1 = r0s[k + 1];
+    if (I.tile_t) {
+      // the tiles whose rows have all arrived with this piece
+      const long long t1 = (k + 1 < TC_CHUNKS ? r1 : nin + TB_ROWS - 1) / TB_ROWS;
+      df_tile_runs(I, r0 / TB_ROWS, t1, nvec, dx, xs.p, s);
+      continue;
+    }
     if (r1 > r0)
       launch(k_df_split_x, blocks_for((r1 - r0) * nvec, 256), 256, 0, s, (r1 - r0) * nvec,
              (const double *)(dx + r0 * nvec), xs.p + r0 * nvec, I.dfflag.p + 1);
@@ -2781,6 +3492,7 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
       df_apply2(shape, n, nvec, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, xs.p, dx, y, sc,
                 I.t_perm.p + a, I.dfflag.p, s, nin);
   }
+  if (I.tile_t) df_tile_columns(I, nvec, xs.p, dx, y, sc, s);
   TMRG_CUDA(cudaStreamSynchronize(s));
   for (int k = 0; k <= TC_CHUNKS; k++) cudaEventDestroy(ev[k]);
   cudaStreamDestroy(cs);
@@ -2821,7 +3533,8 @@ __global__ void k_win_maxcol(long long rows, const int *__restrict__ rp,
 constexpr int FC_CHUNKS = 16;
 bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double *yh,
                                  int nvec) {
-  if (nvec % 2 != 0 || ((uintptr_t)dx % 16) != 0 || I.rows < (long long)LO_WIN * FC_CHUNKS)
+  if (nvec % 2 != 0 || ((uintptr_t)dx % 16) != 0 || I.rows < (long long)LO_WIN * FC_CHUNKS ||
+      (I.tile_ok && tune_forced(TUNE_P)))
     return false;
   Stage st("tmrg_interp_mult_staged");
   cudaStream_t s = I.s;
@@ -2838,7 +3551,8 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
     TMRG_CUDA(cudaStreamSynchronize(s));
     g_host_syncs.fetch_add(1, std::memory_order_relaxed);
   }
-  DBuf<float2> xs(nin * nvec + 1, s);
+  const bool tiled = I.tile_ok;
+  DBuf<float2> xs(tiled ? 0 : nin * nvec + 1, s);
   TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
   DBuf<double> dy(rows * nvec + 2, s);
   double *y = dy.p;
@@ -2883,7 +3597,7 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
     for (; split < upto; split++) {
       TMRG_CUDA(cudaStreamWaitEvent(s, iev[split], 0));
       const long long a = c0[split], b = c0[split + 1];
-      if (b > a) {
+      if (b > a && !tiled) {
         prof_bytes(16 * (b - a) * nvec);
         launch(k_df_split_x, blocks_for((b - a) * nvec, 256), 256, 0, s, (b - a) * nvec,
                (const double *)(dx + a * nvec), xs.p + a * nvec, I.dfflag.p + 1);
@@ -2891,8 +3605,11 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
     }
     if (r1 > r0) {
       prof_bytes(12 * I.nnz_nz * (r1 - r0) / rows + 4 * (r1 - r0) + 8LL * nvec * (r1 - r0));
-      df_apply2(shape, r1 - r0, nvec, I.ap_rowptr(), I.ap_colidx(), I.ap_w.p, xs.p, dx, y,
-                nullptr, I.perm.p + r0, I.dfflag.p, s, nin);
+      if (tiled)
+        df_tile_apply(I, r0 / TB_ROWS, (r1 + TB_ROWS - 1) / TB_ROWS, nvec, dx, y, s);
+      else
+        df_apply2(shape, r1 - r0, nvec, I.ap_rowptr(), I.ap_colidx(), I.ap_w.p, xs.p, dx, y,
+                  nullptr, I.perm.p + r0, I.dfflag.p, s, nin);
     }
     TMRG_CUDA(cudaEventRecord(ev[k], s));
     TMRG_CUDA(cudaStreamWaitEvent(cs, ev[k], 0));
@@ -2964,9 +3681,26 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
   const long long bytes = 12 * I.nnz_nz + 4 * (nout + 1) + 8LL * nvec * (nin + nout) +
                           (which == 2 ? 8 * nout : 0);
   if (f64_rows(nvec, nout, I.nnz_nz, rp, ci, w, x, y, sc, bytes, s)) return;
+  TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
+  // tiles where they exist; P^T of 2 vectors is faster from its own rows (see
+  // k_df_tile), and a forced launch shape means the row kernels
+  const bool free_shape = !tune_forced(which == 0 ? TUNE_P : TUNE_PT);
+  if (which == 0 && nvec > 1 && I.tile_ok && free_shape) {
+    prof_bytes(bytes - 2 * I.nnz_nz);
+    df_tile_apply(I, 0, (nout + TB_ROWS - 1) / TB_ROWS, nvec, x, y, s);
+    return;
+  }
+  if (which != 0 && nvec > 2 && I.tile_t && free_shape) {
+    const long long np = (long long)I.tile_runs.n;
+    DBuf<float2> part((size_t)np * nvec, s);
+    prof_bytes(9 * I.nnz_nz + 8LL * nvec * (nin + np) + 14 * np);
+    df_tile_runs(I, 0, (nin + TB_ROWS - 1) / TB_ROWS, nvec, x, part.p, s);
+    prof_bytes(8LL * nvec * (np + nout) + (sc ? 8 * nout : 0));
+    df_tile_columns(I, nvec, part.p, x, y, sc, s);
+    return;
+  }
   const int n2 = (nvec + 1) / 2;
   DBuf<float2> xs(nin * (nvec == 1 ? 1 : 2 * n2) + 1, s);
-  TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
   df_split_input(I, x, nin, nvec, xs, s);
   prof_bytes(bytes);
   if (nvec == 1) {

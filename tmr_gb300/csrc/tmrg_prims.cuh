@@ -475,6 +475,7 @@ enum TuneKind {
 int tune_run(const TuneKey &k, int ncand, const std::function<void(int)> &run,
              cudaStream_t s);
 int tune_lookup(const TuneKey &k);
+bool tune_forced(int kind);  // a candidate is forced for the kind (tmrg_tune_force)
 
 template <typename K, bool VALS>
 inline void radix_scatter_shape(int shape, unsigned nb, cudaStream_t s, const K *kin,

@@ -92,6 +92,11 @@ int tune_lookup(const TuneKey &k) {
   return it != g_tune.end() ? it->second.choice : k.fallback;
 }
 
+bool tune_forced(int kind) {
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  return g_force.count(kind) != 0;
+}
+
 void tune_set_enabled(bool on) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune_on = on;
