@@ -601,11 +601,13 @@ static void launch_tile_term(const Filter &F, bool tr, bool first, int vpn, int 
   // once, B
   prof_bytes((long long)(sizeof(T) + 2) * F.nnz + (long long)sizeof(T) * F.n * (3LL * VPN + 1));
   prof_flops(2LL * VPN * F.nnz);
+  // the limit is the kernel's, for all threads: that of the largest tile
 #define TMRG_TILE(TR, FIRST)                                                                 \
   do {                                                                                       \
     if (smem > 48 * 1024)                                                                    \
       TMRG_CUDA(cudaFuncSetAttribute(k_fe_tile<T, VPN, TR, FIRST>,                           \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+                                     (int)(sizeof(T) * VPN * TS_SIZES[1].cols)));            \
     launch((k_fe_tile<T, VPN, TR, FIRST>), g, TS_ROWS, smem, s, M, vpn, c0, tile_vals<T>(F), B, \
            pre, t1, x, y, post);                                                             \
   } while (0)

@@ -599,12 +599,14 @@ static void ht_launch(const TSell &M, const T *val, int nvec, const HtArgs<T> &A
                       cudaStream_t s) {
   const TSellView V = M.view();
   const unsigned g = (unsigned)M.tiles;
+  // the limit is the kernel's, for all threads: that of the largest tile
 #define TMRG_HT(VPN)                                                                         \
   do {                                                                                       \
     const size_t smem = sizeof(T) * VPN * (size_t)M.maxu;                                    \
     if (smem > 48 * 1024)                                                                    \
       TMRG_CUDA(cudaFuncSetAttribute(k_ht<T, VPN, MODE>,                                     \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+                                     (int)(sizeof(T) * VPN * TS_SIZES[1].cols)));            \
     prof_bytes((long long)(sizeof(T) + 2) * M.entries + (long long)sizeof(T) * M.n *         \
                                                             (1 + 5LL * VPN));                \
     prof_flops(sizeof(T) == 8 ? 2LL * VPN * M.entries : 0);                                  \

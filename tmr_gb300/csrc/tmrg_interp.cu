@@ -3354,11 +3354,13 @@ static void df_tile_apply(const Interp &I, long long t0, long long t1, int nvec,
   const DfTiles D = df_tiles(I, t0, t1, nvec, I.ap_w.p);
   auto smem = [&](int lb) { return sizeof(float2) * ((size_t)I.tile_maxu << (lb + 1)); };
   int lb = df_tile_lanes(nvec);
-  while (lb > 0 && smem(lb) > 100 * 1024) lb--;  // tiles with many columns
+  constexpr int most = 100 * 1024;
+  while (lb > 0 && smem(lb) > most) lb--;  // tiles with many columns
+  // (the attribute is the kernel's, for all threads: always the same)
 #define TMRG_DT(B)                                                                              \
   do {                                                                                          \
     TMRG_CUDA(cudaFuncSetAttribute(k_df_tile<B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                   (int)smem(B)));                                              \
+                                   most));                                                      \
     launch(k_df_tile<B>, (unsigned)(t1 - t0), TB_ROWS, smem(B), s, D, scalar, I.ap_rowptr(),    \
            (const uint16_t *)I.tile_idx.p, (const uint8_t *)I.tile_order.p, x, y, I.dfflag.p);  \
   } while (0)

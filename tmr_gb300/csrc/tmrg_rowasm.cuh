@@ -135,16 +135,22 @@ static __global__ void k_fa_list(long long ne, const unsigned *__restrict__ hoff
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < ne && hoff[e + 1] != hoff[e]) list[hoff[e]] = (unsigned)e;
 }
+// total: entries of all blocks, which the 32-bit places of the scan must hold.
 template <typename Entry>
 __global__ void k_fa_count(long long nh, ElemCtx c, Entry ent,
                            const unsigned *__restrict__ list,
-                           unsigned *ucnt, unsigned *bcnt) {
+                           unsigned *ucnt, unsigned *bcnt, unsigned long long *total) {
   const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= nh) return;
-  int U[FMAXK];
-  const int K = element_block(c, ent, list[h], U, nullptr);
-  ucnt[h] = (unsigned)K;
-  bcnt[h] = (unsigned)(K * K);
+  unsigned kk = 0;
+  if (h < nh) {
+    int U[FMAXK];
+    const int K = element_block(c, ent, list[h], U, nullptr);
+    kk = (unsigned)(K * K);
+    ucnt[h] = (unsigned)K;
+    bcnt[h] = kk;
+  }
+  kk = __reduce_add_sync(0xffffffffu, kk);
+  if ((threadIdx.x & 31) == 0 && kk) atomicAdd(total, (unsigned long long)kk);
 }
 template <typename Entry>
 __global__ void __launch_bounds__(64)
@@ -369,13 +375,19 @@ inline bool assemble_rows(const ElemCtx &c, const Entry &ent, long long n, long 
   const long long nh = read_scalar(hoff.p + ne, s);
   DBuf<unsigned> list(nh + 1, s), ucnt(nh + 1, s), boff(nh + 1, s);
   launch(k_fa_list, blocks_for(ne, 256), 256, 0, s, ne, (const unsigned *)hoff.p, list.p);
+  DBuf<unsigned long long> total(1, s);
+  total.zero();
   launch(k_fa_count<Entry>, blocks_for(nh, 128), 128, 0, s, nh, c, ent, (const unsigned *)list.p,
-         ucnt.p, boff.p);
+         ucnt.p, boff.p, total.p);
   exclusive_scan<unsigned>(ucnt.p, ucnt.p, nh, s);
   exclusive_scan<unsigned>(boff.p, boff.p, nh, s);
-  const unsigned *hp[2] = {ucnt.p + nh, boff.p + nh};
-  unsigned hv[2];
+  const unsigned *tw = (const unsigned *)total.p;  // low word first
+  const unsigned *hp[5] = {ucnt.p + nh, boff.p + nh, tw, tw + 1, (const unsigned *)c.err};
+  unsigned hv[5];
   read_scalars(hp, hv, s);
+  // rows, each at its number of entries before equal columns are added
+  const long long E = (ne - nh) * c.npe * c.npe + ((long long)hv[3] << 32 | hv[2]);
+  if (E >= (1LL << 32) || hv[4]) return false;
   DBuf<int> unode((size_t)hv[0] + 1, s);
   DBuf<double> block((size_t)hv[1] + 1, s);
   launch(k_fa_blocks<Entry>, blocks_for(nh, 64), 64, 0, s, nh, c, ent, (const unsigned *)list.p,
@@ -401,9 +413,6 @@ inline bool assemble_rows(const ElemCtx &c, const Entry &ent, long long n, long 
   skey.release();
   A.srp = srp.p;
   A.slot = slot.p;
-  // rows, each at its number of entries before equal columns are added
-  const long long E = (long long)(ne - nh) * c.npe * c.npe + hv[1];
-  if (E >= (1LL << 32)) return false;
   DBuf<unsigned> coff(n + 1, s), large(n + 1, s), nlarge(1, s);
   nlarge.zero();
   launch(k_fa_candidates, blocks_for(n, 256), 256, 0, s, n, A, coff.p, large.p, nlarge.p);
