@@ -93,6 +93,21 @@ __device__ __forceinline__ int apply_keeps(double w) {
 }
 #endif
 
+// The expansion of every element (npe <= 27 nodes) onto independent nodes,
+// sorted by column (stably, in local-node order): column, dependent weight,
+// local node | KEY_INDEP for an independent one, and the element's kind (0: no
+// dependent node, 2: a column more than once).
+constexpr uint8_t KEY_INDEP = 0x80;
+struct ElemLists {
+  long long total = 0;  // entries of all lists
+  DBuf<long long> eoff;
+  DBuf<int> lcol;
+  DBuf<double> ldw;
+  DBuf<uint8_t> lkey, ekind;
+};
+void build_elists(long long n, int npe, const int *conn, const int *dptr, const int *dconn,
+                  const double *dw, ElemLists &L, int *err, cudaStream_t s);
+
 struct Interp {
   cudaStream_t s = 0;
   long long rows = 0, cols = 0, nnz = 0;

@@ -27,7 +27,6 @@ namespace tmrg {
 
 constexpr int IMAX_CO = 3;   // coarse orders built for createInterpolation
 constexpr int IMAX_E = 256;  // entries of one coarse element's expansion
-constexpr uint8_t KEY_INDEP = 0x80;  // list entry is an independent node
 
 struct InterpCtx {
   int fo, co;  // fine / coarse order
@@ -1902,30 +1901,19 @@ static void interp_rows_general(Forest &coarse, Interp &I, InterpCtx &c, GenInte
   interp_finish(I, nonzeros, s, nullptr);
 }
 
-// Sorted expansion lists of every element of `coarse` (k_elist_*).
-struct ElemLists {
-  long long total = 0;  // entries of all lists
-  DBuf<long long> eoff;
-  DBuf<int> lcol;
-  DBuf<double> ldw;
-  DBuf<uint8_t> lkey, ekind;
-};
-static void build_elists(Forest &coarse, ElemLists &L, int *err, cudaStream_t s) {
-  const int cnpe = coarse.order * coarse.order * coarse.order;
-  L.eoff.alloc(coarse.n + 1, s);
-  launch(k_elist_count, blocks_for(coarse.n, 256), 256, 0, s, coarse.n, cnpe,
-         (const int *)coarse.econn.p, (const int *)coarse.dep_ptr.p, L.eoff.p);
-  exclusive_scan<long long>(L.eoff.p, L.eoff.p, coarse.n, s);
-  const long long ne = read_scalar(L.eoff.p + coarse.n, s);
+void build_elists(long long n, int npe, const int *conn, const int *dptr, const int *dconn,
+                  const double *dw, ElemLists &L, int *err, cudaStream_t s) {
+  L.eoff.alloc(n + 1, s);
+  launch(k_elist_count, blocks_for(n, 256), 256, 0, s, n, npe, conn, dptr, L.eoff.p);
+  exclusive_scan<long long>(L.eoff.p, L.eoff.p, n, s);
+  const long long ne = read_scalar(L.eoff.p + n, s);
   L.total = ne;
   L.lcol.alloc(ne + 1, s);
   L.ldw.alloc(ne + 1, s);
   L.lkey.alloc(ne + 1, s);
-  L.ekind.alloc(coarse.n + 1, s);
-  launch(k_elist_fill, blocks_for(coarse.n, EL_WARPS), EL_WARPS * 32, 0, s, coarse.n, cnpe,
-         (const int *)coarse.econn.p, (const int *)coarse.dep_ptr.p,
-         (const int *)coarse.dep_conn.p, (const double *)coarse.dep_w.p,
-         (const long long *)L.eoff.p, L.lcol.p, L.ldw.p, L.lkey.p, L.ekind.p, err);
+  L.ekind.alloc(n + 1, s);
+  launch(k_elist_fill, blocks_for(n, EL_WARPS), EL_WARPS * 32, 0, s, n, npe, conn, dptr, dconn,
+         dw, (const long long *)L.eoff.p, L.lcol.p, L.ldw.p, L.lkey.p, L.ekind.p, err);
 }
 void interp_create(Forest &fine, Forest &coarse, Interp &I) {
   Stage st("tmrg_create_interpolation");
@@ -1997,7 +1985,8 @@ void interp_create(Forest &fine, Forest &coarse, Interp &I) {
   }
   // sorted expansion list of every coarse element
   ElemLists EL;
-  build_elists(coarse, EL, err.p, s);
+  build_elists(coarse.n, cnpe, coarse.econn.p, coarse.dep_ptr.p, coarse.dep_conn.p,
+               coarse.dep_w.p, EL, err.p, s);
   c.eoff = EL.eoff.p;
   c.lcol = EL.lcol.p;
   c.ldw = EL.ldw.p;
@@ -2502,7 +2491,8 @@ void topo_weights_create(Forest &filter, Forest &analysis, Interp &I) {
          (const int *)filter.z.p, (const int16_t *)filter.level.p, c4.p);
   c.c4 = c4.p;
   ElemLists EL;
-  build_elists(filter, EL, err.p, s);
+  build_elists(filter.n, filter.order * filter.order * filter.order, filter.econn.p,
+               filter.dep_ptr.p, filter.dep_conn.p, filter.dep_w.p, EL, err.p, s);
   c.eoff = EL.eoff.p;
   c.lcol = EL.lcol.p;
   c.ldw = EL.ldw.p;

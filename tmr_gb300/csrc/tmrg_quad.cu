@@ -1146,7 +1146,9 @@ __global__ void k_q_dep_info(long long n, QConnDev c, QKeyT<Key> K, const Key *_
     return;
   }
   auto exists = [&](const Quad &q) {
-    return contains_key(keys, n, K.make(q.block, q.x, q.y, q.level));
+    const Key v = K.make(q.block, q.x, q.y, q.level);
+    const long long j = lower_bound_near(keys, n, i, v);
+    return j < n && kldg(keys + j) == v;
   };
   const int32_t h = side_of(o.level);
   const int id = ((o.x & h) ? 1 : 0) | ((o.y & h) ? 2 : 0);
@@ -1264,10 +1266,12 @@ struct QKnots {
   double k[3];
   double r[3][3];
 };
+// The node with `key`, searched from the node `near`.
 template <typename Key>
-__device__ __forceinline__ long long q_find_node(const Key *ukeys, long long nl, Key key) {
-  long long i = lower_bound_key(ukeys, nl, key);
-  return (i < nl && ukeys[i] == key) ? i : -1;
+__device__ __forceinline__ long long q_find_node(const Key *ukeys, long long nl, long long near,
+                                                 Key key) {
+  const long long i = lower_bound_near(ukeys, nl, near, key);
+  return (i < nl && kldg(ukeys + i) == key) ? i : -1;
 }
 template <typename Key>
 __global__ void k_q_dep_rows(long long n, QConnDev c, QNodeKeyT<Key> NK, int order, QKnots kn,
@@ -1286,6 +1290,8 @@ __global__ void k_q_dep_rows(long long n, QConnDev c, QNodeKeyT<Key> NK, int ord
   for (int e = 0; e < 4; e++) {
     if (!(info[i] & (1 << e))) continue;
     int en[3];
+    // the parent edge's nodes lie near the edge's own first one
+    long long t = lconn[i * o * o + q_edge_offset(o, e, 0)];
     for (int ii = 0; ii < o; ii++) {
       // parent edge nodes at 2h (order 2) or h (order 3) steps
       int32_t step = (o == 2) ? 2 * h : h;
@@ -1298,7 +1304,7 @@ __global__ void k_q_dep_rows(long long n, QConnDev c, QNodeKeyT<Key> NK, int ord
         y = p.y + 2 * h * (e % 2);
       }
       q_transform_node(c, b, x, y);
-      long long t = q_find_node<Key>(ukeys, nl, NK.make(b, x, y));
+      t = q_find_node<Key>(ukeys, nl, t, NK.make(b, x, y));
       if (t < 0) {
         atomicExch(err, 1);
         return;
@@ -1456,10 +1462,17 @@ struct QInterpCtx {
   const int16_t *fl;
   long long cn;
   const int4 *c4;  // coarse (face | level << 26, x, y, 0)
-  const int *cconn, *cdptr, *cdconn;
-  const double *cdw;
   const unsigned long long *rep;
   int *err;
+  // direction states (null uv: none): the fine knots' 1 + k as 0, 1 or 2,
+  // those that are 2^-53 off it, and the products of two states' weights
+  int fk1i[3], fodd;
+  const double *uv;
+  // the coarse elements' expansion lists (ElemLists)
+  const long long *eoff;
+  const int *lcol;
+  const double *ldw;
+  const uint8_t *lkey;
 };
 __global__ void k_q_pack(long long n, const int *__restrict__ b, const int *__restrict__ x,
                          const int *__restrict__ y, const int16_t *__restrict__ l, int4 *out) {
@@ -1549,6 +1562,19 @@ __device__ __forceinline__ void q_range(const QInterpCtx &I, int i, int32_t nx, 
     e = co;
   }
 }
+// The coarse Lagrange basis at u (co is 2 or 3; places known when compiled
+// keep N in registers).
+__device__ __forceinline__ void q_weights(const QInterpCtx &I, double u, double *N) {
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    double v = 1.0;
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+      if (a != b && a < I.co && b < I.co)
+        v = __dmul_rn(v, __dmul_rn(__dsub_rn(u, I.ck[b]), I.crk[a][b]));
+    N[a] = v;
+  }
+}
 // one direction of computeElemInterp (:4486-4640, Lagrange branch)
 __device__ __forceinline__ void q_dir(const QInterpCtx &I, int i, int32_t nx, int nlev,
                                       int32_t ox, int clev, int &s, int &e, double *N) {
@@ -1561,7 +1587,7 @@ __device__ __forceinline__ void q_dir(const QInterpCtx &I, int i, int32_t nx, in
   } else if ((i == 0 && ox + hc == nx) || (i == mo - 1 && ox + hc == nx + h)) {
     s = co - 1;
     e = co;
-    N[co - 1] = 1.0;
+    N[1] = N[2] = 1.0;
   } else {
     s = 0;
     e = co;
@@ -1570,113 +1596,186 @@ __device__ __forceinline__ void q_dir(const QInterpCtx &I, int i, int32_t nx, in
     // expression does
     double t = __dadd_rn(q_exact(nx), __dmul_rn(q_pow2(TMRG_MAX_LEVEL - 1 - nlev), I.fk1[i]));
     double u = __dadd_rn(-1.0, __dmul_rn(__dsub_rn(t, q_exact(ox)), q_pow2(clev - TMRG_MAX_LEVEL + 1)));
-    for (int a = 0; a < co; a++) {
-      double v = 1.0;
-      for (int b = 0; b < co; b++)
-        if (a != b) v = __dmul_rn(v, __dmul_rn(__dsub_rn(u, I.ck[b]), I.crk[a][b]));
-      N[a] = v;
-    }
+    q_weights(I, u, N);
   }
 }
-// the row's entries (uniqueSort: stable by column, duplicates summed in
-// order); returns the count, and with WEIGHTS writes the columns and
-// weights (the count pass needs only the columns).  The enclosing coarse
-// element is searched when *tp < 0 and returned in *tp.
+// The octree's direction states (dir_state in tmrg_interp.cu): the u of a
+// direction is one of -1 + s / 2 for s = 0..4, the inexact middle knot's at the
+// block's side (6), or the row hits the element's side (5).  -1 where these do
+// not cover it (levels too far apart).  The weights of two states are then a
+// table's, computed by q_dir's sequence: the same bits, without the 45 FP64
+// operations a row that q_dir takes on a pipe of 1 / 64 of the FP32 rate.
+constexpr int Q_DIR = 7;
+__device__ __forceinline__ int q_dir_state(const QInterpCtx &I, int i, bool one, int32_t nx,
+                                           int lf, int32_t ox, int lc) {
+  if (one) return 5;
+  if (lf - lc > 1 || (lf < lc && I.fodd)) return -1;
+  if (((I.fodd >> i) & 1) && nx == 0 && lf == lc) return 6;
+  const long long num = 2LL * (nx - ox) + (long long)side_of(lf) * I.fk1i[i] - side_of(lc);
+  const int lm = max(lf, lc);
+  const int s = (int)(num >> (TMRG_MAX_LEVEL - lm)) * (1 << (1 - (lm - lc))) + 2;
+  return (unsigned)s < 5u ? s : -1;
+}
+// tab[(su * 7 + sv) * 9 + ii + co * jj] = Nu[ii] Nv[jj]; fk1odd is 1 + the
+// inexact knot.
+__global__ void k_q_uv_table(QInterpCtx I, double fk1odd, double *tab) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= Q_DIR * Q_DIR * 9) return;
+  const int ss[2] = {t / 9 / Q_DIR, t / 9 % Q_DIR}, ix[2] = {t % 9 % I.co, t % 9 / I.co};
+  double w[2];
+  for (int d = 0; d < 2; d++) {
+    double u = -1.0 + 0.5 * ss[d];
+    if (ss[d] == 6) {
+      // q_dir's sequence at nx = ox = 0, lf = lc = 10
+      const double x = __dadd_rn(0.0, __dmul_rn(q_pow2(TMRG_MAX_LEVEL - 11), fk1odd));
+      u = __dadd_rn(-1.0, __dmul_rn(__dsub_rn(x, 0.0), q_pow2(11 - TMRG_MAX_LEVEL)));
+    }
+    double N[3];
+    q_weights(I, u, N);
+    w[d] = ss[d] == 5 ? 1.0 : ix[d] == 0 ? N[0] : ix[d] == 1 ? N[1] : N[2];
+  }
+  tab[t] = __dmul_rn(w[0], w[1]);
+}
+// The row's enclosing coarse element (-1 with the error flag set, or no row),
+// and the mask of its local nodes in the row's box; with WEIGHTS also the
+// table place of its direction states (-1: none, and its weights in Nu and Nv).
 template <bool WEIGHTS>
-__device__ int q_row(const QInterpCtx &I, long long row, int *tp, int *cols, double *w) {
-  unsigned long long rr = I.rep[row];
-  long long e = (long long)(rr >> 8);
-  int info = (int)(rr & 255u);
-  Quad node{I.fb[e], I.fx[e], I.fy[e], I.fl[e]};
-  long long t = *tp;
-  if (t < 0) {
+__device__ __forceinline__ long long q_row_box(const QInterpCtx &I, long long row, long long t,
+                                               unsigned &bm, int &st, double *Nu, double *Nv) {
+  const unsigned long long rr = I.rep[row];
+  const long long e = (long long)(rr >> 8);
+  const int info = (int)(rr & 255u);
+  const Quad node{I.fb[e], I.fx[e], I.fy[e], I.fl[e]};
+  if (!WEIGHTS) {
     t = q_find_enclosing(I, node, info);
     if (t < 0) {
       atomicExch(I.err, 1);
-      return 0;
+      return -1;
     }
-    *tp = (int)t;
   }
-  int4 cq = I.c4[t];
-  const int mo = I.fo, co = I.co;
-  double Nu[3], Nv[3];
+  const int4 cq = I.c4[t];
+  const int mo = I.fo, co = I.co, ni = info % mo, nj = info / mo, lc = cq.x >> 26;
   int is, ie, js, je;
+  q_range(I, ni, node.x, node.level, cq.y, lc, is, ie);
+  q_range(I, nj, node.y, node.level, cq.z, lc, js, je);
+  const unsigned mu = ((1u << ie) - 1u) & ~((1u << is) - 1u);
+  bm = 0;
+  for (int jj = js; jj < je; jj++) bm |= mu << (jj * co);
   if (WEIGHTS) {
-    q_dir(I, info % mo, node.x, node.level, cq.y, cq.x >> 26, is, ie, Nu);
-    q_dir(I, info / mo, node.y, node.level, cq.z, cq.x >> 26, js, je, Nv);
-  } else {
-    q_range(I, info % mo, node.x, node.level, cq.y, cq.x >> 26, is, ie);
-    q_range(I, info / mo, node.y, node.level, cq.z, cq.x >> 26, js, je);
+    st = -1;
+    if (I.uv) {
+      const int su = q_dir_state(I, ni, ie - is == 1, node.x, node.level, cq.y, lc);
+      const int sv = q_dir_state(I, nj, je - js == 1, node.y, node.level, cq.z, lc);
+      if (su >= 0 && sv >= 0) st = (su * Q_DIR + sv) * 9;
+    }
+    if (st < 0) {
+      q_dir(I, ni, node.x, node.level, cq.y, lc, is, ie, Nu);
+      q_dir(I, nj, node.y, node.level, cq.z, lc, js, je, Nv);
+    }
   }
-  int ic[27];
-  double iw[WEIGHTS ? 27 : 1];
-  int m = 0;
-  const int *c = I.cconn + t * co * co;
-  for (int jj = js; jj < je; jj++)
-    for (int ii = is; ii < ie; ii++) {
-      double wt = WEIGHTS ? __dmul_rn(Nu[ii], Nv[jj]) : 0.0;
-      int g = c[ii + jj * co];
-      if (g >= 0) {
-        ic[m] = g;
-        if (WEIGHTS) iw[m] = wt;
-        m++;
-      } else {
-        int d = -g - 1;
-        for (int p = I.cdptr[d]; p < I.cdptr[d + 1] && m < 27; p++) {
-          ic[m] = I.cdconn[p];
-          if (WEIGHTS) iw[m] = __dmul_rn(wt, I.cdw[p]);
-          m++;
-        }
+  return t;
+}
+// A row is the in-box part of its element's sorted list (ElemLists), equal
+// columns summed in order (uniqueSort).  Quadratic meshes of 64 x 64 faces, 36M
+// rows on three levels: count 2.47 -> 2.05 ms, fill 6.17 -> 2.60 ms and 1.18 ms
+// for the lists, against every row sorting its own entries in local memory
+// with weights from q_dir (6.27 ms with the entries in shared memory, 5.00 with
+// the weights from the table); a third pass that counted the kept entries, 1.4
+// ms, is gone.
+constexpr int QR_THREADS = 128;
+// Entries of a warp's 32 rows that are staged in shared memory (quadratic
+// elements: 250 on average).
+constexpr int QR_STAGE = 416;
+__global__ void __launch_bounds__(QR_THREADS)
+    k_q_row_count(long long rows, QInterpCtx I, int *cnt, int *encl) {
+  const long long r = (long long)blockIdx.x * QR_THREADS + threadIdx.x;
+  if (r >= rows) return;
+  unsigned bm;
+  int st, m = 0, pcol = -1;
+  const long long t = q_row_box<false>(I, r, -1, bm, st, nullptr, nullptr);
+  encl[r] = (int)t;
+  if (t >= 0) {
+    const long long e1 = __ldg(I.eoff + t + 1);
+    for (long long a = __ldg(I.eoff + t); a < e1; a++) {
+      const int col = __ldg(I.lcol + a);
+      if ((bm >> (__ldg(I.lkey + a) & 31)) & 1u) {
+        m += col != pcol;
+        pcol = col;
       }
     }
-  // stable insertion sort by column
-  for (int a = 1; a < m; a++) {
-    int kc = ic[a];
-    double kw = WEIGHTS ? iw[a] : 0.0;
-    int b = a - 1;
-    while (b >= 0 && ic[b] > kc) {
-      ic[b + 1] = ic[b];
-      if (WEIGHTS) iw[b + 1] = iw[b];
-      b--;
-    }
-    ic[b + 1] = kc;
-    if (WEIGHTS) iw[b + 1] = kw;
   }
-  int k = 0;
-  for (int a = 0; a < m; a++) {
-    double sum = WEIGHTS ? iw[a] : 0.0;
-    while (a + 1 < m && ic[a + 1] == ic[a]) {
-      ++a;
-      if (WEIGHTS) sum = __dadd_rn(sum, iw[a]);
-    }
-    if (WEIGHTS) {
-      cols[k] = ic[a];
-      w[k] = sum;
-    }
-    k++;
-  }
-  return k;
+  cnt[r] = m;
 }
-__global__ void k_q_row_count(long long rows, QInterpCtx I, int *cnt, int *encl) {
-  long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  int t = -1;
-  cnt[r] = q_row<false>(I, r, &t, nullptr, nullptr);
-  encl[r] = t;
-}
-__global__ void k_q_row_fill(long long rows, QInterpCtx I, const int *__restrict__ rp,
-                             const int *__restrict__ encl, int *cols, double *w,
-                             unsigned long long *nonzero) {
-  long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned nz = 0;
+// A warp's rows are one run of the matrix: they are put together in shared
+// memory at their places in it and written together, or row by row where the
+// run is longer than QR_STAGE.  keep[r]: the row's entries that the applies
+// keep.  Bound by latency (list entry after list entry), hence by how many
+// warps the stage leaves room for.
+__global__ void __launch_bounds__(QR_THREADS)
+    k_q_row_fill(long long rows, QInterpCtx I, const int *__restrict__ rp,
+                 const int *__restrict__ encl, int *cols, double *w, long long *keep) {
+  __shared__ double s_w[QR_THREADS / 32][QR_STAGE];
+  __shared__ int s_c[QR_THREADS / 32][QR_STAGE];
+  __shared__ double s_uv[Q_DIR * Q_DIR * 9];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (I.uv)
+    for (int i = threadIdx.x; i < Q_DIR * Q_DIR * 9; i += QR_THREADS) s_uv[i] = I.uv[i];
+  __syncthreads();
+  const long long r = (long long)blockIdx.x * QR_THREADS + threadIdx.x;
+  const long long w0 = r - lane;
+  if (w0 >= rows) return;
+  const int base = rp[w0], total = rp[min(w0 + 32, rows)] - base;
+  const bool staged = total <= QR_STAGE;
+  int *oc = staged ? s_c[warp] : cols + base;
+  double *ow = staged ? s_w[warp] : w + base;
   if (r < rows) {
-    int t = encl[r];
-    int k = q_row<true>(I, r, &t, cols + rp[r], w + rp[r]);
-    for (int a = 0; a < k; a++) nz += apply_keeps(w[rp[r] + a]);
+    double Nu[3], Nv[3], acc = 0.0;
+    unsigned bm;
+    int st, nz = 0, pcol = -1;
+    const long long t = q_row_box<true>(I, r, encl[r], bm, st, Nu, Nv);
+    int k = rp[r] - base;
+    const int end = rp[r + 1] - base;
+    auto emit = [&]() {
+      if (pcol < 0) return;
+      if (k < end) {
+        oc[k] = pcol;
+        ow[k] = acc;
+        nz += apply_keeps(acc);
+      }
+      k++;
+    };
+    const long long e1 = __ldg(I.eoff + t + 1);
+#pragma unroll 2
+    for (long long a = __ldg(I.eoff + t); a < e1; a++) {
+      const int key = __ldg(I.lkey + a), li = key & 31, col = __ldg(I.lcol + a);
+      if (!((bm >> li) & 1u)) continue;
+      double v;
+      if (st >= 0) {
+        v = s_uv[st + li];
+      } else {
+        const int jj = li / I.co, ii = li - jj * I.co;
+        v = __dmul_rn(ii == 0 ? Nu[0] : ii == 1 ? Nu[1] : Nu[2],
+                      jj == 0 ? Nv[0] : jj == 1 ? Nv[1] : Nv[2]);
+      }
+      if (!(key & KEY_INDEP)) v = __dmul_rn(v, __ldg(I.ldw + a));
+      if (col == pcol) {
+        acc = __dadd_rn(acc, v);
+      } else {
+        emit();
+        pcol = col;
+        acc = v;
+      }
+    }
+    emit();
+    if (k != end) atomicExch(I.err, 3);  // never: the count pass took the same entries
+    keep[r] = nz;
   }
-  // one atomic per warp
-  for (int o = 16; o; o >>= 1) nz += __shfl_xor_sync(0xffffffffu, nz, o);
-  if ((threadIdx.x & 31) == 0 && nz) atomicAdd(nonzero, (unsigned long long)nz);
+  __syncwarp();
+  if (staged)
+    for (int p = lane; p < total; p += 32) {
+      cols[base + p] = s_c[warp][p];
+      w[base + p] = s_w[warp][p];
+    }
 }
 
 void qinterp_create(QForest &fine, QForest &coarse, Interp &I) {
@@ -1723,12 +1822,15 @@ void qinterp_create(QForest &fine, QForest &coarse, Interp &I) {
   c.fl = fine.level.p;
   c.cn = coarse.n;
   c.c4 = c4.p;
-  c.cconn = coarse.econn.p;
-  c.cdptr = coarse.dep_ptr.p;
-  c.cdconn = coarse.dep_conn.p;
-  c.cdw = coarse.dep_w.p;
   c.rep = rep.p;
   c.err = err.p;
+  ElemLists EL;
+  build_elists(coarse.n, coarse.order * coarse.order, coarse.econn.p, coarse.dep_ptr.p,
+               coarse.dep_conn.p, coarse.dep_w.p, EL, err.p, s);
+  c.eoff = EL.eoff.p;
+  c.lcol = EL.lcol.p;
+  c.ldw = EL.ldw.p;
+  c.lkey = EL.lkey.p;
   DBuf<int> cnt(rows + 1, s);
   // compulsory per row: its reference entry, the fine element fields, the
   // coarse element it lands in (packed quad and connectivity) and the row
@@ -1736,7 +1838,7 @@ void qinterp_create(QForest &fine, QForest &coarse, Interp &I) {
   const long long row_bytes = rows * (8LL + 14 + 16 + 4LL * coarse.order * coarse.order + 8);
   prof_bytes(row_bytes);
   DBuf<int> encl(std::max(1LL, rows), s);
-  launch(k_q_row_count, blocks_for(rows, 128), 128, 0, s, rows, c, cnt.p, encl.p);
+  launch(k_q_row_count, blocks_for(rows, QR_THREADS), QR_THREADS, 0, s, rows, c, cnt.p, encl.p);
   exclusive_scan<int>(cnt.p, cnt.p, rows, s);
   const long long nnz = read_scalar(cnt.p + rows, s);
   if (read_scalar(err.p, s))
@@ -1745,13 +1847,43 @@ void qinterp_create(QForest &fine, QForest &coarse, Interp &I) {
   I.rowptr = std::move(cnt);
   I.colidx.alloc(std::max(1LL, nnz), s);
   I.vals.alloc(std::max(1LL, nnz), s);
-  DBuf<unsigned long long> nzc(1, s);
-  nzc.zero();
-  prof_bytes(row_bytes + 12 * nnz);
-  launch(k_q_row_fill, blocks_for(rows, 128), 128, 0, s, rows, c, (const int *)I.rowptr.p,
-         (const int *)encl.p, I.colidx.p, I.vals.p, nzc.p);
-  const long long nonzeros = (long long)read_scalar(nzc.p, s);
-  interp_finish(I, nonzeros, s);
+  // direction states: 1 + each fine knot within 2^-53 of 0, 1 or 2, at most
+  // one inexact, and the tie of an inexact knot one level below rounding to
+  // -1/2 as on the device
+  bool states = true;
+  double fk1odd = 1.0;
+  for (int i = 0; i < fine.order; i++) {
+    const double k1 = c.fk1[i];
+    const double k = k1 < 0.5 ? 0.0 : (k1 < 1.5 ? 1.0 : 2.0);
+    c.fk1i[i] = (int)k;
+    if (std::fabs(k1 - k) > std::ldexp(1.0, -53)) states = false;
+    if (k1 != k) {
+      if (c.fodd) states = false;
+      c.fodd |= 1 << i;
+      fk1odd = k1;
+    }
+  }
+  if (c.fodd) {
+    volatile double tt = std::ldexp(1.0, TMRG_MAX_LEVEL - 12) * fk1odd;  // lf = 11
+    volatile double x = tt * std::ldexp(1.0, 11 - TMRG_MAX_LEVEL);        // lc = 10
+    volatile double u = -1.0 + x;
+    if (u != -0.5) states = false;
+  }
+  DBuf<double> uv;
+  if (states) {
+    uv.alloc(Q_DIR * Q_DIR * 9, s);
+    launch(k_q_uv_table, blocks_for(Q_DIR * Q_DIR * 9, 128), 128, 0, s, c, fk1odd, uv.p);
+    c.uv = uv.p;
+  }
+  DBuf<long long> keep(rows + 1, s);
+  prof_bytes(row_bytes + 12 * nnz + 8 * rows);
+  launch(k_q_row_fill, blocks_for(rows, QR_THREADS), QR_THREADS, 0, s, rows, c,
+         (const int *)I.rowptr.p, (const int *)encl.p, I.colidx.p, I.vals.p, keep.p);
+  exclusive_scan<long long>(keep.p, keep.p, rows, s);
+  const long long nonzeros = read_scalar(keep.p + rows, s);
+  if (read_scalar(err.p, s))
+    throw Error(TMRG_ERR_INTERNAL, "createInterpolation: a row outgrew its counted length");
+  interp_finish(I, nonzeros, s, keep.p);
   TMRG_CUDA(cudaStreamSynchronize(s));
 }
 
