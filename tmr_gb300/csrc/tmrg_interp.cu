@@ -727,8 +727,9 @@ __global__ void k_group_rows(long long rows, const int *__restrict__ trow,
 // row is one contiguous store, with no FP64 instruction.
 // Other elements walk the sorted list in step (broadcast shared-memory
 // reads), lane r <-> row r:
-//   stage: the in-box (row, entry) pairs of list entries k0.. in list
-//     order, with each entry's rows mask and first pair;
+//   stage: lane j <-> list entry k0 + j, whose rows are those that take its
+//     local node (27 ballots a batch of rows give them): the in-box (row,
+//     entry) pairs in list order, and each entry's rows and first pair;
 //   weights: the pairs' products on full warps (table value times the
 //     dependent weight, as in k_interp_rows; a masked FP64 warp
 //     instruction costs the GB300 FP64 pipe as much as a full one);
@@ -736,8 +737,17 @@ __global__ void k_group_rows(long long rows, const int *__restrict__ trow,
 //     that order; an add is issued only at list entries that repeat the
 //     previous entry's column (the list is sorted, so no other entry can
 //     continue a run).
-constexpr int EW_WARPS = 4;
-constexpr int EW_CAP = 256;  // staged pairs per warp
+// Bound by latency and FP64 issue.  Elements differ in their rows and lists, so
+// a block of few warps gives its place up earlier, and a short stage leaves
+// room for more blocks.  Fill of three quadratic matrices of 1.6G entries: 22.6
+// ms with 4 warps a block, every list entry kept staged and a ballot per
+// entry; 20.4 with 2 warps, 19.0 with a window of the list, 18.3 with entries
+// staged a lane each.  (1 warp a block, or 40 registers: 20.9.  Pairs staged
+// row by row and each row's equal columns summed by the lane of the first:
+// 39.5, every sum a masked FP64 instruction.)
+constexpr int EW_WARPS = 2;
+constexpr int EW_CAP = 256;  // staged pairs per warp, of at most
+constexpr int EW_WIN = 64;   // list entries
 template <bool FILL>
 __global__ void __launch_bounds__(EW_WARPS * 32)
     k_interp_elem(long long n, InterpCtx I, const unsigned *__restrict__ estart,
@@ -747,12 +757,13 @@ __global__ void __launch_bounds__(EW_WARPS * 32)
   constexpr int FW = FILL ? EW_WARPS : 1;
   __shared__ int s_col[EW_WARPS][IMAX_E];
   __shared__ uint8_t s_key[EW_WARPS][IMAX_E];
-  __shared__ unsigned s_mk[FW][IMAX_E];   // rows (lanes) taking entry k
-  __shared__ uint16_t s_bk[FW][IMAX_E];   // staged position of its first pair
-  __shared__ uint8_t s_pr[FW][EW_CAP];    // staged pair: row lane
-  __shared__ uint8_t s_pk[FW][EW_CAP];    // staged pair: list entry
-  __shared__ double s_pv[FW][EW_CAP];     // staged pair: weight
-  __shared__ int s_st[FW][32];            // row state * co^3
+  // staged list entry: rows (lanes) taking it, place of its first pair, column,
+  // and whether the entry before has the same one
+  __shared__ int4 s_en[FW][EW_WIN];
+  __shared__ uint16_t s_p[FW][EW_CAP];  // staged pair: row lane << 8 | list entry
+  __shared__ double s_pv[FW][EW_CAP];   // its weight
+  __shared__ int s_st[FW][32];          // row state * co^3
+  __shared__ unsigned s_km[FW][32];     // rows (lanes) taking local node l
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const long long t = (long long)blockIdx.x * EW_WARPS + warp;
@@ -838,41 +849,58 @@ __global__ void __launch_bounds__(EW_WARPS * 32)
         }
       }
     } else {
+      unsigned km = 0;
+      for (int l = 0; l < cn3; l++) {
+        const unsigned m = __ballot_sync(0xffffffffu, (bm >> l) & 1u);
+        if (lane == l) km = m;
+      }
+      s_km[fw][lane] = km;
       int pcol = -1;
       double acc = 0.0;
       for (int k0 = 0; k0 < E;) {
-        // stage entries k0..k1-1 (at most EW_CAP pairs)
+        // stage entries k0..k1-1, a lane each
         int k1 = k0, nst = 0;
         __syncwarp();
-        while (k1 < E && nst + 32 <= EW_CAP) {
-          const bool in = (bm >> (s_key[warp][k1] & 31)) & 1u;
-          const unsigned m = __ballot_sync(0xffffffffu, in);
-          if (in) {
-            const int p = nst + __popc(m & lt);
-            s_pr[fw][p] = (uint8_t)lane;
-            s_pk[fw][p] = (uint8_t)k1;
+        while (k1 < E && k1 - k0 <= EW_WIN - 32) {
+          const int k = k1 + lane;
+          unsigned m = k < E ? s_km[fw][s_key[warp][k] & 31] : 0u;
+          const int c = __popc(m);
+          int incl = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
           }
-          if (lane == 0) {
-            s_mk[fw][k1] = m;
-            s_bk[fw][k1] = (uint16_t)nst;
+          // (one entry always fits an empty stage)
+          const int nf = __popc(__ballot_sync(0xffffffffu, k < E && nst + incl <= EW_CAP));
+          if (lane < nf) {
+            int p = nst + incl - c;
+            const int col = s_col[warp][k];
+            s_en[fw][k - k0] =
+                make_int4((int)m, p, col, kind == 2 && k > 0 && s_col[warp][k - 1] == col);
+            for (; m; m &= m - 1)
+              s_p[fw][p++] = (uint16_t)((__ffs(m) - 1) << 8 | k);
           }
-          nst += __popc(m);
-          k1++;
+          if (nf == 0) break;
+          nst += __shfl_sync(0xffffffffu, incl, nf - 1);
+          k1 += nf;
+          if (nf < 32) break;
         }
         __syncwarp();
         for (int p = lane; p < nst; p += 32) {
-          const int k = s_pk[fw][p];
-          const double w = __ldg(I.uvw + s_st[fw][s_pr[fw][p]] + (s_key[warp][k] & 31));
-          s_pv[fw][p] = kind == 0 ? w : __dmul_rn(w, __ldg(ldw + k));
+          const int q = s_p[fw][p], k = q & 255;
+          const double w = __ldg(I.uvw + s_st[fw][q >> 8] + (s_key[warp][k] & 31));
+          s_pv[fw][p] = __dmul_rn(w, __ldg(ldw + k));
         }
         __syncwarp();
         for (int k = k0; k < k1; k++) {
-          const unsigned m = s_mk[fw][k];
-          const int col = s_col[warp][k];
+          const int4 en = s_en[fw][k - k0];
+          const unsigned m = (unsigned)en.x;
+          const int col = en.z;
           const bool in = (m >> lane) & 1u;
-          const bool cont = kind == 2 && k > 0 && s_col[warp][k - 1] == col;  // uniform
+          const bool cont = en.w != 0;  // uniform
           if (in) {
-            const double v = s_pv[fw][s_bk[fw][k] + __popc(m & lt)];
+            const double v = s_pv[fw][en.y + __popc(m & lt)];
             if (cont && col == pcol) {
               acc = __dadd_rn(acc, v);
             } else {
