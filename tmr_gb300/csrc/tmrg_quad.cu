@@ -1462,6 +1462,10 @@ struct QInterpCtx {
   const int16_t *fl;
   long long cn;
   const int4 *c4;  // coarse (face | level << 26, x, y, 0)
+  // their keys where those fit 64 bits and hold every fine quadrant's place too
+  // (else null)
+  const uint64_t *ckey;
+  int ckW, ckbb;
   const unsigned long long *rep;
   int *err;
   // direction states (null uv: none): the fine knots' 1 + k as 0, 1 or 2,
@@ -1479,6 +1483,13 @@ __global__ void k_q_pack(long long n, const int *__restrict__ b, const int *__re
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = make_int4(b[i] | ((int)l[i] << 26), x[i], y[i], 0);
 }
+__global__ void k_q_pack_keys(long long n, QKeyT<uint64_t> K, const int4 *__restrict__ c4,
+                              uint64_t *out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int4 q = c4[i];
+  out[i] = K.make(q.x & 0x3ffffff, q.y, q.z, q.x >> 26);
+}
 // 2^e as a double from its exponent (exact; e >= -1022).
 __device__ __forceinline__ double q_pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 // A non-negative int32 as a double assembled from its bits with integer
@@ -1495,14 +1506,14 @@ __device__ __forceinline__ double q_exact(int32_t v) {
 __device__ long long q_find_enclosing(const QInterpCtx &I, const Quad &node, int info) {
   const int order = I.fo;
   const int32_t h = side_of(node.level);
-  const int ii = info % order, jj = info / order;
+  const int jj = order_div(info, order), ii = info - jj * order;
   int32_t xi = -1, yi = -1;
   if (ii == 0 || ii == order - 1)
-    xi = node.x + (ii / (order - 1)) * h;
+    xi = node.x + (ii ? h : 0);
   else if (order % 2 == 1 && ii == order / 2)
     xi = node.x + h / 2;
   if (jj == 0 || jj == order - 1)
-    yi = node.y + (jj / (order - 1)) * h;
+    yi = node.y + (jj ? h : 0);
   else if (order % 2 == 1 && jj == order / 2)
     yi = node.y + h / 2;
   int32_t xl = xi, xh = xi, yl = yi, yh = yi;
@@ -1517,20 +1528,35 @@ __device__ long long q_find_enclosing(const QInterpCtx &I, const Quad &node, int
     yh = (int32_t)ceil(yd);
   }
   long long low = 0, high = I.cn - 1, mid = low + (high - low) / 2;
-  while (mid != low) {
-    int4 q = I.c4[mid];
-    int32_t hm = side_of(q.x >> 26);
-    int32_t ab = q.x & 0x3ffffff;
-    if (node.block == ab && node.x >= q.y && node.x < q.y + hm && node.y >= q.z &&
-        node.y < q.z + hm)
-      break;
-    int st = cmp_position2(ab, q.y, q.z, node.block, node.x, node.y);
-    if (st == 0) break;
-    if (st < 0)
-      low = mid + 1;
-    else
-      high = mid - 1;
-    mid = low + (high - low) / 2;
+  if (I.ckey) {  // the same steps on keys (find_enclosing in tmrg_interp.cu)
+    const uint64_t at = QKeyT<uint64_t>{I.ckW, I.ckbb}.make(node.block, node.x, node.y, 0) >> 5;
+    int lo = 0, hi = (int)I.cn - 1, m = hi / 2;
+    while (m != lo) {
+      const uint64_t k = __ldg(I.ckey + m), p = k >> 5;
+      if (((at ^ p) >> (2 * (I.ckW - (int)(k & 31)))) == 0) break;
+      if (p < at)
+        lo = m + 1;
+      else
+        hi = m - 1;
+      m = lo + (hi - lo) / 2;
+    }
+    mid = m;
+  } else {
+    while (mid != low) {
+      int4 q = I.c4[mid];
+      int32_t hm = side_of(q.x >> 26);
+      int32_t ab = q.x & 0x3ffffff;
+      if (node.block == ab && node.x >= q.y && node.x < q.y + hm && node.y >= q.z &&
+          node.y < q.z + hm)
+        break;
+      int st = cmp_position2(ab, q.y, q.z, node.block, node.x, node.y);
+      if (st == 0) break;
+      if (st < 0)
+        low = mid + 1;
+      else
+        high = mid - 1;
+      mid = low + (high - low) / 2;
+    }
   }
   const int32_t bx = node.x + h, by = node.y + h;
   while (mid < I.cn) {
@@ -1654,7 +1680,7 @@ __device__ __forceinline__ long long q_row_box(const QInterpCtx &I, long long ro
     }
   }
   const int4 cq = I.c4[t];
-  const int mo = I.fo, co = I.co, ni = info % mo, nj = info / mo, lc = cq.x >> 26;
+  const int mo = I.fo, co = I.co, nj = order_div(info, mo), ni = info - nj * mo, lc = cq.x >> 26;
   int is, ie, js, je;
   q_range(I, ni, node.x, node.level, cq.y, lc, is, ie);
   q_range(I, nj, node.y, node.level, cq.z, lc, js, je);
@@ -1677,7 +1703,7 @@ __device__ __forceinline__ long long q_row_box(const QInterpCtx &I, long long ro
 }
 // A row is the in-box part of its element's sorted list (ElemLists), equal
 // columns summed in order (uniqueSort).  Quadratic meshes of 64 x 64 faces, 36M
-// rows on three levels: count 2.47 -> 2.05 ms, fill 6.17 -> 2.60 ms and 1.18 ms
+// rows on three levels: count 2.47 -> 1.5 ms, fill 6.17 -> 2.6 ms and 1.2 ms
 // for the lists, against every row sorting its own entries in local memory
 // with weights from q_dir (6.27 ms with the entries in shared memory, 5.00 with
 // the weights from the table); a third pass that counted the kept entries, 1.4
@@ -1822,6 +1848,17 @@ void qinterp_create(QForest &fine, QForest &coarse, Interp &I) {
   c.fl = fine.level.p;
   c.cn = coarse.n;
   c.c4 = c4.p;
+  DBuf<uint64_t> ckey;
+  const QKeyT<uint64_t> K{std::max({fine.maxlev, coarse.maxlev, 1}),
+                          std::max(fine.conn->block_bits, coarse.conn->block_bits)};
+  if (K.total_bits() <= 64 && coarse.n > 0 && coarse.n < (1LL << 31)) {
+    ckey.alloc(std::max(1LL, coarse.n), s);
+    launch(k_q_pack_keys, blocks_for(coarse.n, 256), 256, 0, s, coarse.n, K,
+           (const int4 *)c4.p, ckey.p);
+    c.ckey = ckey.p;
+    c.ckW = K.W;
+    c.ckbb = K.bb;
+  }
   c.rep = rep.p;
   c.err = err.p;
   ElemLists EL;

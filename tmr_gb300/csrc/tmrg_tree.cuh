@@ -282,6 +282,15 @@ __device__ __forceinline__ void node_point(const PointCtx &c, long long i, doubl
   }
 }
 
+// i / o for an order o from 2 to 8: a local index (i < 256) by a multiply (a
+// division by a number not known when compiled is some 20 instructions).
+__device__ __forceinline__ int order_div(int i, int o) {
+  if ((unsigned)i >= 256u) return i / o;
+  const unsigned r = o == 2 ? 32769u : o == 3 ? 21846u : o == 4 ? 16385u : o == 5 ? 13108u
+                   : o == 6 ? 10923u : o == 7 ? 9363u : 8193u;
+  return (int)((unsigned)i * r >> 16);
+}
+
 // lower_bound over a sorted key array (uint64_t or U128).
 template <typename K>
 __device__ __forceinline__ long long lower_bound_key(const K *a, long long n, K v) {
