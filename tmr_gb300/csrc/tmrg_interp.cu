@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(EL_WARPS * 32, 16)
                  const int *__restrict__ dptr, const int *__restrict__ dconn,
                  const double *__restrict__ dw, const long long *__restrict__ eoff,
                  int *lcol, double *ldw, uint8_t *lkey, uint8_t *ekind, int *err) {
-  __shared__ int s_col[EL_WARPS][IMAX_E];
+  __shared__ __align__(16) int s_col[EL_WARPS][IMAX_E];
   __shared__ double s_dw[EL_WARPS][IMAX_E];
   __shared__ uint8_t s_key[EL_WARPS][IMAX_E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -157,18 +157,71 @@ __global__ void __launch_bounds__(EL_WARPS * 32, 16)
   }
   const bool anydep = __any_sync(0xffffffffu, lane < cnpe && cv < 0);
   __syncwarp();
-  bool dup = false;
-  for (int a = lane; a < E; a += 32) {
-    const int col = s_col[warp][a];
-    int rk = 0;
-    for (int b = 0; b < E; b++) {
-      const int cb = s_col[warp][b];
-      rk += (cb < col) || (cb == col && b < a);
-      dup |= (cb == col && b != a);
+  // Ranks by comparing every entry with all others.  Lists longer than a warp
+  // do so on words of a column (from the least one) and a place, all different,
+  // four to a load: 4.84 -> 2.80 ms for the lists of three quadratic levels.  A
+  // list of one entry a lane is ranked as fast without (quadtrees: 1.18 against
+  // 1.63 ms).
+  int cmin = 0x7fffffff, cmax = 0;
+  if (E > 32) {
+    for (int a = lane; a < E; a += 32) {
+      const int col = s_col[warp][a];
+      cmin = min(cmin, col);
+      cmax = max(cmax, col);
     }
-    lcol[eo + rk] = col;
-    ldw[eo + rk] = s_dw[warp][a];
-    lkey[eo + rk] = s_key[warp][a];
+    cmin = __reduce_min_sync(0xffffffffu, cmin);
+    cmax = __reduce_max_sync(0xffffffffu, cmax);
+  }
+  bool dup = false;
+  if (E > 32 && cmax - cmin < (1 << 24)) {
+    unsigned *s_k = (unsigned *)s_col[warp];
+    for (int a = lane; a < ((E + 3) & ~3); a += 32)
+      s_k[a] = a < E ? (unsigned)(s_col[warp][a] - cmin) << 8 | (unsigned)a : 0xffffffffu;
+    __syncwarp();
+    unsigned my[IMAX_E / 32];
+    int rk[IMAX_E / 32];
+#pragma unroll
+    for (int j = 0; j < IMAX_E / 32; j += 2) {
+      if (32 * j >= E) break;  // uniform
+      const int a = 32 * j + lane;
+      const unsigned m0 = a < E ? s_k[a] : 0u, m1 = a + 32 < E ? s_k[a + 32] : 0u;
+      int r0 = 0, r1 = 0;
+      for (int b = 0; b < E; b += 4) {
+        const uint4 q = *(const uint4 *)(s_k + b);
+        r0 += (q.x < m0) + (q.y < m0) + (q.z < m0) + (q.w < m0);
+        r1 += (q.x < m1) + (q.y < m1) + (q.z < m1) + (q.w < m1);
+      }
+      my[j] = m0;
+      my[j + 1] = m1;
+      rk[j] = r0;
+      rk[j + 1] = r1;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < IMAX_E / 32; j++) {
+      if (32 * j >= E) break;
+      const int a = 32 * j + lane;
+      if (a >= E) continue;
+      lcol[eo + rk[j]] = cmin + (int)(my[j] >> 8);
+      ldw[eo + rk[j]] = s_dw[warp][a];
+      lkey[eo + rk[j]] = s_key[warp][a];
+      s_k[rk[j]] = my[j] >> 8;
+    }
+    __syncwarp();
+    for (int a = lane + 1; a < E; a += 32) dup |= s_k[a] == s_k[a - 1];
+  } else {
+    for (int a = lane; a < E; a += 32) {
+      const int col = s_col[warp][a];
+      int rk = 0;
+      for (int b = 0; b < E; b++) {
+        const int cb = s_col[warp][b];
+        rk += (cb < col) || (cb == col && b < a);
+        dup |= (cb == col && b != a);
+      }
+      lcol[eo + rk] = col;
+      ldw[eo + rk] = s_dw[warp][a];
+      lkey[eo + rk] = s_key[warp][a];
+    }
   }
   const bool anydup = __any_sync(0xffffffffu, dup);
   if (lane == 0) ekind[t] = anydup ? 2 : (anydep ? 1 : 0);
