@@ -1691,6 +1691,7 @@ int tmrg_helmholtz_set_smoother(tmrg_helmholtz *H, int degree_order2, int degree
     ARG(lower_order2 > 0.0 && lower_order3 > 0.0 && upper > lower_order2 &&
             upper > lower_order3,
         "bad smoother interval");
+    H->H.cheb_auto = false;
     H->H.cheb_degree2 = degree_order2;
     H->H.cheb_degree3 = degree_order3;
     H->H.cheb_lower2 = lower_order2;

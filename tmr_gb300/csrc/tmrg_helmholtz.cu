@@ -30,10 +30,8 @@
 //   FP32 at 64 times its FP64 rate, and the FP64 outer iteration still
 //   drives the true residual to the reference's tolerance.  The smoother is
 //   Chebyshev on D^-1 K over [lower, 1.1] lmax (lmax from Lanczos; degree
-//   3 and lower 0.2 for order-2 levels, degree 6 and lower 0.1 for order 3;
-//   per solve of 2.1M nodes, degree 5 from 0.05 against 3 from 0.2: r = 2 h
-//   12.3 and 7.5 ms, r = 32 h 12.3 and 8.7 ms, with 7 and 6 or 7 iterations;
-//   on scattered refinement at r = 32 h 4.1 and 4.6 ms, all else faster),
+//   3 and lower 0.2, or 5 and 0.05, for order-2 levels (smoother_of), degree
+//   6 and lower 0.1 for order 3),
 //   which is parallel where SOR is sequential.  Restriction and prolongation are the forests' own
 //   createInterpolation operators (P^T and P); coarse levels are
 //   rediscretised, as in the reference (use_galerkin = 0).  The coarsest
@@ -1117,6 +1115,29 @@ static void lanczos_lmax(Helmholtz &H, HLevel &L) {
   L.w64 = HWork<double>();
 }
 
+// Degree and lower end (as a fraction of lam) of a level's smoother, where the
+// caller set none: for linear levels by the finest one's lam, which tells how
+// far the mass matrix rules there.  Where r is about the element size or more
+// everywhere, lam is 1.5 to 2.2 and the short modes lie above a fifth of it;
+// where some elements are much larger than r it comes to 3.4, short modes go
+// down to lam / 27, and a short interval costs iterations.  2.56M nodes, element
+// sides r / 2 to 16 r (lam above 2.6): 3 steps from 0.2 take 15 iterations, 19.4
+// ms, 5 from 0.05 take 7, 13.2 ms; r four times as large (2.2): 8 and 7
+// iterations, 10.6 and 13.2 ms.
+constexpr double HM_MASS_LAM = 2.6;
+static void smoother_of(const Helmholtz &H, const HLevel &L, int &degree, double &lower) {
+  degree = L.o == 2 ? H.cheb_degree2 : H.cheb_degree3;
+  lower = L.o == 2 ? H.cheb_lower2 : H.cheb_lower3;
+  if (!H.cheb_auto || L.o != 2) return;
+  for (const auto &F : H.L) {
+    if (F->o != 2) continue;  // (quadratic levels come first)
+    if (F->lam > HM_MASS_LAM) {
+      degree = 5;
+      lower = 0.05;
+    }
+    return;
+  }
+}
 // Chebyshev smoothing of level L in FP32: on entry r = b - A x (zero: x = 0
 // and r = rin = b); keeps r = b - A x on exit when keep_r.
 static void chebyshev(Helmholtz &H, HLevel &L, int nvec, const float *rin, bool zero,
@@ -1125,15 +1146,16 @@ static void chebyshev(Helmholtz &H, HLevel &L, int nvec, const float *rin, bool 
   HWork<float> &W = L.w32;
   const long long n = L.nn;
   const unsigned g = blocks_for(n * nvec, 256);
-  const double lmax = H.cheb_upper * L.lam,
-               lmin = (L.o == 2 ? H.cheb_lower2 : H.cheb_lower3) * L.lam;
+  int degree;
+  double lower;
+  smoother_of(H, L, degree, lower);
+  const double lmax = H.cheb_upper * L.lam, lmin = lower * L.lam;
   const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
   const double sigma = theta / delta;
   double rho = 1.0 / sigma;
   prof_bytes(4LL * n * nvec * 4 + 4LL * n);
   launch(k_h_cheb_first<float>, g, 256, 0, s, n, nvec, (const float *)L.dinv32.p, rin, W.r.p,
          W.d.p, W.x.p, (float)(1.0 / theta), zero ? 1 : 0);
-  const int degree = L.o == 2 ? H.cheb_degree2 : H.cheb_degree3;
   for (int k = 1; k < degree; k++) {
     h_apply<float>(L, true, nvec, W.d.p, W.r.p, nullptr, 2, s);
     double rn = 1.0 / (2.0 * sigma - rho);
@@ -1151,11 +1173,12 @@ static void chebyshev_tiled(Helmholtz &H, HLevel &L, int nvec, const float *b, b
                             bool keep_r) {
   cudaStream_t s = H.s;
   HWork<float> &W = L.w32;
-  const double lmax = H.cheb_upper * L.lam,
-               lmin = (L.o == 2 ? H.cheb_lower2 : H.cheb_lower3) * L.lam;
+  int degree;
+  double lower;
+  smoother_of(H, L, degree, lower);
+  const double lmax = H.cheb_upper * L.lam, lmin = lower * L.lam;
   const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
   const double sigma = theta / delta;
-  const int degree = L.o == 2 ? H.cheb_degree2 : H.cheb_degree3;
   const float *val = L.k32.p;
   double rho = 1.0 / sigma;
   HtArgs<float> A{};

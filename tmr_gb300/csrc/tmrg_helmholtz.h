@@ -78,6 +78,7 @@ struct Helmholtz {
   int max_iters = 300;
   // Chebyshev smoother: interval [lower, upper] x lam; degree and lower
   // bound by level order
+  bool cheb_auto = true;  // no smoother set by the caller: chosen per level
   double cheb_lower2 = 0.2, cheb_lower3 = 0.1, cheb_upper = 1.1;
   int cheb_degree2 = 3, cheb_degree3 = 6;
   int lanczos_steps = 16;
