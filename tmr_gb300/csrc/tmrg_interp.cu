@@ -3778,6 +3778,13 @@ static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, con
   return true;
 }
 
+// Rows below which P, and P^T with the wide shapes (15 vectors or more), go by
+// rows: a tile is a block, and fewer of them than SMs leave some idle.  16
+// vectors by tiles and by rows: 27K entries P 18.4 and 15.9 us, P^T 24.9 and
+// 15.7; 80K entries 23.6 and 15.7, 36.1 and 28.1; above the line, 610K entries,
+// 28.8 and 34.4, 42 and 106.  P^T of 10 vectors, 80K entries, takes 86 us by rows.
+constexpr long long DF_TILE_ROWS = 152LL * TB_ROWS;
+
 void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
   Stage st(which == 0 ? "tmrg_interp_mult" : "tmrg_interp_mult_transpose");
   if (nvec <= 0) throw Error(TMRG_ERR_ARG, "interp apply: nvec <= 0");
@@ -3796,9 +3803,10 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
                           (which == 2 ? 8 * nout : 0);
   if (f64_rows(nvec, nout, I.nnz_nz, rp, ci, w, x, y, sc, bytes, s)) return;
   TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
-  // tiles where they exist; P^T of 2 vectors is faster from its own rows (see
-  // k_df_tile), and a forced launch shape means the row kernels
-  const bool free_shape = !tune_forced(which == 0 ? TUNE_P : TUNE_PT);
+  // tiles where they exist and one for every SM; P^T of 2 vectors is faster from
+  // its own rows (see k_df_tile), and a forced launch shape means the row kernels
+  const bool free_shape = (I.rows >= DF_TILE_ROWS || (which != 0 && nvec < 15)) &&
+                          !tune_forced(which == 0 ? TUNE_P : TUNE_PT);
   if (which == 0 && nvec > 1 && I.tile_ok && free_shape) {
     prof_bytes(bytes - 2 * I.nnz_nz);
     df_tile_apply(I, 0, (nout + TB_ROWS - 1) / TB_ROWS, nvec, x, y, s);
