@@ -3522,6 +3522,20 @@ static TuneKey df_key(int which, long long rows, long long nnz, int nvec2) {
   return TuneKey{which == 0 ? TUNE_P : TUNE_PT, std::min(nvec2, 8), lr, q, 0, 0};
 }
 
+// The FP64 apply (k_f64_rows) where it is the faster one: up to 8 vectors and
+// F64_ROWS_MAX entries x vectors, where launches count and the FP64 pipe does
+// not yet.  Measured per apply, split pass and double-float apply against
+// this kernel: 27K entries, 1 to 8 vectors 16-20 -> 10-12 us; 476K entries, 1
+// vector 16 -> 12 us, 2 vectors 19 -> 16 us, 3 vectors 20 -> 19 us, 4 vectors
+// 19 against 23 us; 4.8M entries, 1 vector 37 against 65 us.
+constexpr long long F64_ROWS_MAX = 1000000;
+// Rows below which P, and P^T with the wide shapes (15 vectors or more), go by
+// rows: a tile is a block, and fewer of them than SMs leave some idle.  16
+// vectors by tiles and by rows: 27K entries P 18.4 and 15.9 us, P^T 24.9 and
+// 15.7; 80K entries 23.6 and 15.7, 36.1 and 28.1; above the line, 610K entries,
+// 28.8 and 34.4, 42 and 106.  P^T of 10 vectors, 80K entries, takes 86 us by rows.
+constexpr long long DF_TILE_ROWS = 152LL * TB_ROWS;
+
 // The input as (hi, lo) pairs in pool memory, with its window flag; an odd
 // number of vectors gets one more, zero.
 static void df_split_input(Interp &I, const double *x, long long nrows, int nvec,
@@ -3546,7 +3560,8 @@ static void df_split_input(Interp &I, const double *x, long long nrows, int nvec
 // sends that piece's rows and every later piece's rows to FP64 (each row
 // only reads pieces already split, so a row never runs in double-float on
 // an input that was not represented).
-// Returns false (nothing done) where these kernels do not apply.
+// Returns false (nothing done) where these kernels do not apply, or the apply of
+// device vectors takes others (the results are the same bits).
 // Reports (and clears) a TMA input stage of k_df_apply_tma that did not
 // complete within its wait limit; read where the host already waits.
 void interp_check_apply(Interp &I) {
@@ -3560,7 +3575,8 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
                                    double *y, int nvec) {
   if ((which != 1 && which != 2) || nvec % 2 != 0 || nvec / 2 < 8 ||
       ((uintptr_t)dx % 16) != 0 || ((uintptr_t)y % 16) != 0 ||
-      (I.tile_t ? tune_forced(TUNE_PT) : (long long)I.t_chunk.size() != TC_CHUNKS + 1))
+      (I.tile_t ? I.rows < DF_TILE_ROWS || tune_forced(TUNE_PT)
+                : (long long)I.t_chunk.size() != TC_CHUNKS + 1))
     return false;
   Stage st("tmrg_interp_mult_transpose_staged");
   cudaStream_t s = I.s;
@@ -3648,7 +3664,7 @@ constexpr int FC_CHUNKS = 16;
 bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double *yh,
                                  int nvec) {
   if (nvec % 2 != 0 || ((uintptr_t)dx % 16) != 0 || I.rows < (long long)LO_WIN * FC_CHUNKS ||
-      (I.tile_ok && tune_forced(TUNE_P)))
+      (nvec <= 8 && I.nnz_nz * nvec <= F64_ROWS_MAX) || (I.tile_ok && tune_forced(TUNE_P)))
     return false;
   Stage st("tmrg_interp_mult_staged");
   cudaStream_t s = I.s;
@@ -3743,13 +3759,6 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
   return true;
 }
 
-// The FP64 apply (k_f64_rows) where it is the faster one: up to 8 vectors and
-// F64_ROWS_MAX entries x vectors, where launches count and the FP64 pipe does
-// not yet.  Measured per apply, split pass and double-float apply against
-// this kernel: 27K entries, 1 to 8 vectors 16-20 -> 10-12 us; 476K entries, 1
-// vector 16 -> 12 us, 2 vectors 19 -> 16 us, 3 vectors 20 -> 19 us, 4 vectors
-// 19 against 23 us; 4.8M entries, 1 vector 37 against 65 us.
-constexpr long long F64_ROWS_MAX = 1000000;
 static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, const int *ci,
                      const float2 *w, const double *x, double *y, const double *scale,
                      long long bytes, cudaStream_t s) {
@@ -3777,13 +3786,6 @@ static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, con
   }
   return true;
 }
-
-// Rows below which P, and P^T with the wide shapes (15 vectors or more), go by
-// rows: a tile is a block, and fewer of them than SMs leave some idle.  16
-// vectors by tiles and by rows: 27K entries P 18.4 and 15.9 us, P^T 24.9 and
-// 15.7; 80K entries 23.6 and 15.7, 36.1 and 28.1; above the line, 610K entries,
-// 28.8 and 34.4, 42 and 106.  P^T of 10 vectors, 80K entries, takes 86 us by rows.
-constexpr long long DF_TILE_ROWS = 152LL * TB_ROWS;
 
 void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
   Stage st(which == 0 ? "tmrg_interp_mult" : "tmrg_interp_mult_transpose");
