@@ -87,3 +87,21 @@ def test_vector_counts_in_turn(gpu_lib):
         r, s = _solves(H, vpn, 10 + vpn)
         assert r <= 2e-12 and s <= 1e-11
         assert first.setdefault(vpn, (r, s)) == (r, s)  # the same bits again
+
+
+@pytest.mark.parametrize("vpn,k", [(1, 1533), (1, 1534), (1, 1535), (2, 766), (2, 767), (2, 768)])
+def test_largest_tile_about_the_shared_memory_limit(gpu_lib, vpn, k):
+    # k blocks around an edge: every node is a column of the first tile, and
+    # its FP64 inputs with the sums beside them end just below, at and above
+    # 48 KB (4 k + 2 columns of 8 vpn bytes, and 64 bytes)
+    from tests.test_gpu_filter_rows import _fan
+    from tmr_gb300 import TMR
+    f = TMR.OctForest(order=2)
+    f.setConnectivity(_fan(k))
+    f.createTrees(0)
+    f.createNodes()
+    n = int(f.getNodeRange()[1])
+    assert n == 4 * k + 2 and abs(8 * vpn * n + 64 - 48 * 1024) < 150
+    f.setBlockBoxes(np.tile([0.0, 0.0, 0.0, 1.0, 1.0, 1.0], (k, 1)))
+    r, s = _solves(TMR.HelmholtzFilter(0.3, None, [f]), vpn, 6)
+    assert r <= 2e-12 and s <= 1e-11

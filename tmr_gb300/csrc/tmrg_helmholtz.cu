@@ -597,11 +597,13 @@ static void ht_launch(const TSell &M, const T *val, int nvec, const HtArgs<T> &A
                       cudaStream_t s) {
   const TSellView V = M.view();
   const unsigned g = (unsigned)M.tiles;
+  // 48 KB without the opt-in, the sums of HT_APPLY (static) among them
+  constexpr size_t most = 48 * 1024 - (MODE == HT_APPLY ? sizeof(double) * TS_SLICES : 0);
   // the limit is the kernel's, for all threads: that of the largest tile
 #define TMRG_HT(VPN)                                                                         \
   do {                                                                                       \
     const size_t smem = sizeof(T) * VPN * (size_t)M.maxu;                                    \
-    if (smem > 48 * 1024)                                                                    \
+    if (smem > most)                                                                         \
       TMRG_CUDA(cudaFuncSetAttribute(k_ht<T, VPN, MODE>,                                     \
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                                      (int)(sizeof(T) * VPN * TS_SIZES[1].cols)));            \
