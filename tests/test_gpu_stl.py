@@ -73,3 +73,34 @@ def test_stl_files_and_empty_level_set(gpu_lib, tmp_path):
         assert fa.read() == fb.read()
     with pytest.raises(ValueError):
         TMR.getSTLTriangles(f, x[:-1], vpn=sc["vpn"])
+
+
+def test_host_calls_count_once(gpu_lib, tmp_path):
+    # a call that fills a host array, and one that writes a file, launch what
+    # a call that fills a device array does: one count and one write
+    import ctypes
+
+    import torch
+    sc, case, g, f, X, x, TMR = _gpu_case("brick_o2")
+    xd = torch.tensor(x, device="cuda")
+    pts = TMR.getSTLTriangles(f, xd, offset=sc["offset"], cutoff=sc["cutoff"], vpn=sc["vpn"])
+    n = pts.shape[0] // 3
+    out, outd = np.empty(9 * n), torch.empty(9 * n, dtype=torch.float64, device="cuda")
+    xh = np.ascontiguousarray(x, dtype=np.float64)
+
+    def fill(name, src, dst):
+        m = ctypes.c_int64(0)
+        k = TMR.kernel_launch_count()
+        TMR.call(name, f.ptr, ctypes.c_void_p(src), sc["vpn"], sc["offset"], float(sc["cutoff"]),
+                 ctypes.byref(m), ctypes.c_void_p(dst), n)
+        assert m.value == n
+        return TMR.kernel_launch_count() - k
+
+    kd = fill("tmrg_stl_triangles_device", xd.data_ptr(), outd.data_ptr())
+    kh = fill("tmrg_stl_triangles", xh.ctypes.data, out.ctypes.data)
+    k = TMR.kernel_launch_count()
+    TMR.writeSTLToBin(str(tmp_path / "a.bin"), f, x, index=sc["offset"], cutoff=sc["cutoff"],
+                      vpn=sc["vpn"])
+    assert kh == kd and TMR.kernel_launch_count() - k == kd
+    np.testing.assert_array_equal(out, pts.reshape(-1))
+    np.testing.assert_array_equal(outd.cpu().numpy(), out)

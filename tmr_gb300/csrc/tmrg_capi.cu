@@ -1497,16 +1497,20 @@ static int stl_entry(tmrg_forest *f, const double *x, bool device, int vpn, int 
     ARG(f && x && ntris && vpn > 0, "bad argument");
     DBuf<double> dx;
     const double *xd = stl_values(f, x, device, vpn, dx);
-    if (device) {
-      *ntris = stl_triangles(f->f, xd, vpn, x_offset, cutoff, tris, tris ? max_tris : 0);
-      return;
-    }
-    const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, nullptr, 0);
+    // one count a call: the buffer is found between it and the write
+    DBuf<double> d;
+    std::function<double *(long long)> room;
+    if (tris && max_tris > 0)
+      room = [&](long long n) -> double * {
+        *ntris = n;
+        if (max_tris < n) return nullptr;
+        if (device) return tris;
+        d.alloc(9 * (size_t)n, f->f.s);
+        return d.p;
+      };
+    const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, room);
     *ntris = n;
-    if (!tris || max_tris < n || !n) return;
-    DBuf<double> d(9 * (size_t)n, f->f.s);
-    stl_triangles(f->f, xd, vpn, x_offset, cutoff, d.p, n);
-    copy_d2h(tris, d.p, sizeof(double) * 9 * n, f->f.s);
+    if (d.p) copy_d2h(tris, d.p, sizeof(double) * 9 * n, f->f.s);
   });
 }
 int tmrg_stl_triangles(tmrg_forest *f, const double *x, int vpn, int x_offset, double cutoff,
@@ -1523,10 +1527,12 @@ int tmrg_generate_bin_file(const char *filename, tmrg_forest *f, const double *x
     ARG(filename && f && x && vpn > 0, "bad argument");
     DBuf<double> dx;
     const double *xd = stl_values(f, x, false, vpn, dx);
-    const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, nullptr, 0);
-    ARG(n < (1LL << 31), "more triangles than the binary format's int count holds");
-    DBuf<double> d(9 * (size_t)std::max(1LL, n), f->f.s);
-    if (n) stl_triangles(f->f, xd, vpn, x_offset, cutoff, d.p, n);
+    DBuf<double> d;
+    const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, [&](long long m) {
+      ARG(m < (1LL << 31), "more triangles than the binary format's int count holds");
+      d.alloc(9 * (size_t)m, f->f.s);
+      return d.p;
+    });
     std::vector<double> h((size_t)9 * n);
     copy_d2h(h.data(), d.p, sizeof(double) * h.size(), f->f.s);
     FILE *fp = fopen(filename, "wb");

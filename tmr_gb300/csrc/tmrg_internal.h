@@ -239,9 +239,9 @@ void forest_get_points(Forest &f, const double *boxes, double *d_X);
 // The first (element << 8 | local index) of every local node (num_local + 1
 // entries), which its position is taken from.
 void forest_first_refs(Forest &f, DBuf<unsigned long long> &rep);
-// Triangles: their number, and 9 doubles each to `out` (device) when it holds
-// at least that many (max_tris); out may be null.
+// Triangles: their number, and 9 doubles each to the device buffer that `room`
+// returns for that number (null: none are written; no `room`: only counted).
 long long stl_triangles(Forest &f, const double *d_x, int vpn, int offset, double cutoff,
-                        double *out, long long max_tris);
+                        const std::function<double *(long long)> &room);
 
 }  // namespace tmrg

@@ -379,9 +379,9 @@ static void bernstein(int o, double u, double *N) {
 
 // Triangles of the level set x[offset] = cutoff on forest f (x: device,
 // vpn interleaved values per independent node).  Returns the count and
-// leaves 9 doubles per triangle in `out` where it has room for them all.
+// leaves 9 doubles per triangle in the buffer that `room` gives for it.
 long long stl_triangles(Forest &f, const double *d_x, int vpn, int offset, double cutoff,
-                        double *out, long long max_tris) {
+                        const std::function<double *(long long)> &room) {
   Stage st("tmrg_stl_triangles");
   if (!f.have_nodes) forest_create_nodes(f);
   if (f.order < 2 || f.order > 3)
@@ -455,7 +455,7 @@ long long stl_triangles(Forest &f, const double *d_x, int vpn, int offset, doubl
   else
     launch(k_stl_count<3>, blocks_for(n, 128), 128, 0, s, c, cnt.p, pos.p);
   exclusive_scan<long long>(cnt.p, cnt.p, n, s);
-  if (!out || max_tris <= 0) return read_scalar(cnt.p + n, s);
+  if (!room) return read_scalar(cnt.p + n, s);
   exclusive_scan<unsigned>(pos.p, pos.p, n, s);
   long long ntri = 0;
   unsigned na = 0;
@@ -463,7 +463,8 @@ long long stl_triangles(Forest &f, const double *d_x, int vpn, int offset, doubl
   TMRG_CUDA(cudaMemcpyAsync(&ntri, cnt.p + n, sizeof(ntri), cudaMemcpyDeviceToHost, s));
   TMRG_CUDA(cudaMemcpyAsync(&na, pos.p + n, sizeof(na), cudaMemcpyDeviceToHost, s));
   TMRG_CUDA(cudaStreamSynchronize(s));
-  if (ntri == 0 || max_tris < ntri) return ntri;
+  double *out = ntri ? room(ntri) : nullptr;
+  if (!out) return ntri;
   if (!C.boxes.empty()) {
     forest_first_refs(f, first);
     c.pts.rep = first.p;
