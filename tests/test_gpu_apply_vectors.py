@@ -105,3 +105,27 @@ def test_applies_outside_the_window(operators, size, nvec):
             fn(_on_device(x, 0), y)
             np.testing.assert_allclose(y.cpu().numpy().reshape(-1, nvec) / scale,
                                        (A @ x) / scale, rtol=1e-13, atol=1e-13)
+
+
+@pytest.mark.parametrize("size", ["small", "large"])
+@pytest.mark.parametrize("nvec", [1, 2, 3, 8, 9, 16])
+@pytest.mark.parametrize("shift", [0, 3])
+def test_input_and_output_in_one_buffer(operators, size, nvec, shift):
+    # the output written over the input, from its start or a few values on
+    import torch
+    I, P = operators[size]
+    rows, cols = P.shape
+    rng = np.random.default_rng(60 + nvec)
+    for scale in (1.0, 1e-30):
+        for fn, nin, nout in ((I.mult, cols, rows), (I.multTranspose, rows, cols),
+                              (I.multWeightTranspose, rows, cols)):
+            x = _on_device(rng.standard_normal(nin * nvec) * scale, 0)
+            want = torch.empty(nout * nvec, dtype=torch.float64, device="cuda")
+            fn(x, want)
+            both = torch.zeros(max(nin, nout) * nvec + shift, dtype=torch.float64, device="cuda")
+            both[:nin * nvec] = x
+            got = both[shift:shift + nout * nvec]
+            fn(both[:nin * nvec], got)
+            # an unaligned output may take another launch shape
+            assert torch.equal(got, want) if shift == 0 else torch.allclose(
+                got, want, rtol=0, atol=1e-13 * scale * 8)

@@ -35,6 +35,12 @@ struct Error : public std::runtime_error {
   } while (0)
 #define TMRG_CHECK_LAUNCH() TMRG_CUDA(cudaGetLastError())
 
+// Whether `na` bytes from `a` and `nb` bytes from `b` share any.
+inline bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+  const uintptr_t p = (uintptr_t)a, q = (uintptr_t)b;
+  return p < q + nb && q < p + na;
+}
+
 HD int32_t side_of(int level) { return (int32_t)1 << (TMRG_MAX_LEVEL - level); }
 
 // Corner nodes of block edge e: edges 0-3 run along x, 4-7 along y,

@@ -618,10 +618,6 @@ static void launch_tile_term(const Filter &F, bool tr, bool first, int vpn, int 
   }
 #undef TMRG_TILE
 }
-static bool overlap(const void *a, const void *b, size_t bytes) {
-  const uintptr_t p = (uintptr_t)a, q = (uintptr_t)b;
-  return p < q + bytes && q < p + bytes;
-}
 // applyFilter / applyTranspose on the tiled copy (F.N > 0); t1 and tmp hold
 // n * vpn values.  Where `in` and `out` overlap t1 is formed before any term
 // writes.
@@ -632,7 +628,7 @@ static void horner_tiled(const Filter &F, bool tr, int vpn, const T *in, T *out,
   const T *pre = tr ? Tinv : Ainv, *post = tr ? Ainv : Tinv;
   const T *x = in;
   bool first = true;
-  if (overlap(in, out, sizeof(T) * len)) {
+  if (overlap(in, sizeof(T) * len, out, sizeof(T) * len)) {
     prof_bytes(2LL * sizeof(T) * len + (long long)sizeof(T) * F.n);
     launch(k_fe_scale<T>, blocks_for(len, 256), 256, 0, s, F.n, vpn, pre, in, t1);
     x = t1;

@@ -3794,6 +3794,14 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
   if (which == 2) interp_colsum(I);
   const long long nin = (which == 0) ? I.cols : I.rows;
   const long long nout = (which == 0) ? I.rows : I.cols;
+  // the kernels read the caller's input while they write: one that shares
+  // memory with the output is copied first
+  DBuf<double> own;
+  if (overlap(x, sizeof(double) * nin * nvec, y, sizeof(double) * nout * nvec)) {
+    own.alloc(nin * nvec, s);
+    TMRG_CUDA(cudaMemcpyAsync(own.p, x, sizeof(double) * nin * nvec, cudaMemcpyDeviceToDevice, s));
+    x = own.p;
+  }
   const int *rp = which == 0 ? I.ap_rowptr() : I.t_rowptr.p;
   const int *ci = which == 0 ? I.ap_colidx() : I.t_colidx.p;
   const float2 *w = which == 0 ? (const float2 *)I.ap_w.p : (const float2 *)I.t_w.p;
