@@ -105,3 +105,22 @@ def test_largest_tile_about_the_shared_memory_limit(gpu_lib, vpn, k):
     f.setBlockBoxes(np.tile([0.0, 0.0, 0.0, 1.0, 1.0, 1.0], (k, 1)))
     r, s = _solves(TMR.HelmholtzFilter(0.3, None, [f]), vpn, 6)
     assert r <= 2e-12 and s <= 1e-11
+
+
+@pytest.mark.parametrize("vpn", [1, 3])
+@pytest.mark.parametrize("level", [0, 1])
+def test_operators_in_place(gpu_lib, vpn, level):
+    # K x and M x written over x
+    import torch
+
+    from tmr_gb300 import TMR
+    H = _filter(TMR, 3, 2)
+    n = int(H.sizes()[level][0])
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(n * vpn, dtype=torch.float64, device="cuda", generator=g)
+    for which in (0, 1):
+        want = torch.empty_like(x)
+        H.mult(level, which, x, want, vpn)
+        same = x.clone()
+        H.mult(level, which, same, same, vpn)
+        assert torch.equal(same, want)

@@ -1617,7 +1617,16 @@ void helmholtz_operator(Helmholtz &H, int level, bool stiff, int nvec, const dou
                         double *out) {
   if (level < 0 || level >= H.nlevels) throw Error(TMRG_ERR_ARG, "level out of range");
   if (nvec < 1 || nvec > HM_MAXVEC) throw Error(TMRG_ERR_ARG, "nvec out of range");
-  h_apply<double>(*H.L[level], stiff, nvec, in, out, nullptr, 0, H.s);
+  HLevel &L = *H.L[level];
+  const size_t bytes = sizeof(double) * L.nn * nvec;
+  DBuf<double> own;
+  // K on tiles reads `in` while it writes (the element operator does not)
+  if (stiff && L.k64.p && overlap(in, bytes, out, bytes)) {
+    own.alloc(L.nn * nvec, H.s);
+    TMRG_CUDA(cudaMemcpyAsync(own.p, in, bytes, cudaMemcpyDeviceToDevice, H.s));
+    in = own.p;
+  }
+  h_apply<double>(L, stiff, nvec, in, out, nullptr, 0, H.s);
 }
 
 }  // namespace tmrg
