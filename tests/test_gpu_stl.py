@@ -104,3 +104,22 @@ def test_host_calls_count_once(gpu_lib, tmp_path):
     assert kh == kd and TMR.kernel_launch_count() - k == kd
     np.testing.assert_array_equal(out, pts.reshape(-1))
     np.testing.assert_array_equal(outd.cpu().numpy(), out)
+
+
+def test_triangles_over_the_values(gpu_lib):
+    # device triangles written over the design values they come from
+    import ctypes
+
+    import torch
+    sc, case, g, f, X, x, TMR = _gpu_case("brick_o2")
+    xd = torch.tensor(x, device="cuda")
+    pts = TMR.getSTLTriangles(f, xd, offset=sc["offset"], cutoff=sc["cutoff"], vpn=sc["vpn"])
+    n = pts.shape[0] // 3
+    both = torch.zeros(max(9 * n, xd.numel()) + 5, dtype=torch.float64, device="cuda")
+    for at in (0, 5):
+        both[:xd.numel()] = xd
+        m = ctypes.c_int64(0)
+        TMR.call("tmrg_stl_triangles_device", f.ptr, ctypes.c_void_p(both.data_ptr()), sc["vpn"],
+                 sc["offset"], float(sc["cutoff"]), ctypes.byref(m),
+                 ctypes.c_void_p(both[at:].data_ptr()), n)
+        np.testing.assert_array_equal(both[at:at + 9 * n].cpu().numpy(), pts.reshape(-1))

@@ -1497,20 +1497,28 @@ static int stl_entry(tmrg_forest *f, const double *x, bool device, int vpn, int 
     ARG(f && x && ntris && vpn > 0, "bad argument");
     DBuf<double> dx;
     const double *xd = stl_values(f, x, device, vpn, dx);
-    // one count a call: the buffer is found between it and the write
+    // one count a call: the buffer is found between it and the write, and is one
+    // of its own where the triangles would go over the values they come from
     DBuf<double> d;
+    const size_t xbytes = sizeof(double) * f->f.num_owned * vpn;
     std::function<double *(long long)> room;
     if (tris && max_tris > 0)
       room = [&](long long n) -> double * {
         *ntris = n;
         if (max_tris < n) return nullptr;
-        if (device) return tris;
+        if (device && !overlap(x, xbytes, tris, sizeof(double) * 9 * n)) return tris;
         d.alloc(9 * (size_t)n, f->f.s);
         return d.p;
       };
     const long long n = stl_triangles(f->f, xd, vpn, x_offset, cutoff, room);
     *ntris = n;
-    if (d.p) copy_d2h(tris, d.p, sizeof(double) * 9 * n, f->f.s);
+    if (d.p && device) {
+      TMRG_CUDA(cudaMemcpyAsync(tris, d.p, sizeof(double) * 9 * n, cudaMemcpyDeviceToDevice,
+                                f->f.s));
+      TMRG_CUDA(cudaStreamSynchronize(f->f.s));
+    } else if (d.p) {
+      copy_d2h(tris, d.p, sizeof(double) * 9 * n, f->f.s);
+    }
   });
 }
 int tmrg_stl_triangles(tmrg_forest *f, const double *x, int vpn, int x_offset, double cutoff,
