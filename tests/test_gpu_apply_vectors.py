@@ -129,3 +129,28 @@ def test_input_and_output_in_one_buffer(operators, size, nvec, shift):
             # an unaligned output may take another launch shape
             assert torch.equal(got, want) if shift == 0 else torch.allclose(
                 got, want, rtol=0, atol=1e-13 * scale * 8)
+
+
+def test_unaligned_vectors_are_tuned_by_themselves(operators):
+    # vectors off the 16-byte grid run other kernels: a class of their own
+    import ctypes
+    import json
+
+    import torch
+
+    from tmr_gb300 import TMR
+    I, P = operators["large"]
+    rows, cols = P.shape
+    lib = TMR.lib()
+    assert lib.tmrg_tune_reset(1) == 0
+    try:
+        x = np.random.default_rng(3).standard_normal(rows * 2)
+        for shift in (1, 0, 1):
+            y = torch.empty(cols * 2 + shift, dtype=torch.float64, device="cuda")[shift:]
+            I.multTranspose(_on_device(x, shift), y)
+        buf = ctypes.create_string_buffer(1 << 16)
+        assert lib.tmrg_tune_report(buf, len(buf)) == 0
+        keys = [tuple(e["key"]) for e in json.loads(buf.value.decode()) if e["kind"] == 2]
+        assert len(keys) == 2 and len({k[:2] for k in keys}) == 1
+    finally:
+        lib.tmrg_tune_reset(1)

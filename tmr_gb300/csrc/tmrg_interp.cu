@@ -3404,12 +3404,17 @@ static bool tma_apply(long long rows, long long nin, const int *rp, const int *c
 // (k_df_apply_tma); fewer pairs: LPR = pairs rounded down to a power of
 // two, NG 1 or 2
 constexpr int DF2_SHAPES_WIDE = 7, DF2_SHAPES_NARROW = 2;
+// Whether the pair kernels take the caller's vectors value by value: an odd
+// number of them, or buffers off the 16-byte grid.
+static bool df_scalar(int nvec, const double *x, const double *y) {
+  return nvec % 2 != 0 || ((uintptr_t)x % 16) != 0 || ((uintptr_t)y % 16) != 0;
+}
 static void df_apply2(int shape, long long rows, int nvec, const int *rp, const int *ci,
                       const float2 *w, const float2 *xs, const double *x, double *y,
                       const double *scale, const int *perm, int *flags, cudaStream_t s,
                       long long nin) {
   const int nvec2 = (nvec + 1) / 2;
-  const bool scalar = nvec % 2 != 0 || ((uintptr_t)x % 16) != 0 || ((uintptr_t)y % 16) != 0;
+  const bool scalar = df_scalar(nvec, x, y);
   if (shape == 6 && nvec2 == 8 && !scalar &&
       tma_apply(rows, nin, rp, ci, w, xs, x, y, scale, perm, flags, s))
     return;
@@ -3514,12 +3519,13 @@ static void df_tile_columns(const Interp &I, int nvec, const float2 *part, const
 }
 
 // Size class of an apply: direction, vector pairs (8 = 8 or more), log2 of
-// the rows, mean row length in quarters (capped).
-static TuneKey df_key(int which, long long rows, long long nnz, int nvec2) {
+// the rows, mean row length in quarters (capped), and whether the vectors go
+// value by value (other kernels, and shape 6 is none of them).
+static TuneKey df_key(int which, long long rows, long long nnz, int nvec2, bool scalar) {
   int lr = 0;
   while ((1LL << (lr + 1)) <= rows) lr++;
   const int q = rows ? (int)std::min(4096LL, (4 * nnz) / rows) : 0;
-  return TuneKey{which == 0 ? TUNE_P : TUNE_PT, std::min(nvec2, 8), lr, q, 0, 0};
+  return TuneKey{which == 0 ? TUNE_P : TUNE_PT, std::min(nvec2, 8), lr, q, scalar ? 1 : 0, 0};
 }
 
 // The FP64 apply (k_f64_rows) where it is the faster one: up to 8 vectors and
@@ -3604,7 +3610,7 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
   }
   const double *sc = which == 2 ? (const double *)I.colsum.p : (const double *)nullptr;
   // the tuned shape of the whole apply's class (the pieces are not tuned)
-  const int shape = tune_lookup(df_key(1, I.cols, I.nnz_nz, nvec / 2));
+  const int shape = tune_lookup(df_key(1, I.cols, I.nnz_nz, nvec / 2, false));
   for (int k = 0; k < TC_CHUNKS; k++) {
     TMRG_CUDA(cudaStreamWaitEvent(s, ev[k], 0));
     const long long r0 = r0s[k], r1 = r0s[k + 1];
@@ -3688,7 +3694,7 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
   double *y = dy.p;
   if ((uintptr_t)y % 16) y++;
   const int n2 = nvec / 2;
-  const int shape = tune_lookup(df_key(0, rows, I.nnz_nz, n2));
+  const int shape = tune_lookup(df_key(0, rows, I.nnz_nz, n2, false));
   cudaStream_t is, cs;
   TMRG_CUDA(cudaStreamCreateWithFlags(&is, cudaStreamNonBlocking));
   TMRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -3844,7 +3850,8 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
            (const float2 *)xs.p, x, y, sc, (const int *)I.dfflag.p);
     return;
   }
-  tune_run(df_key(which, nout, I.nnz_nz, n2), n2 >= 8 ? DF2_SHAPES_WIDE : DF2_SHAPES_NARROW,
+  tune_run(df_key(which, nout, I.nnz_nz, n2, df_scalar(nvec, x, y)),
+           n2 >= 8 ? DF2_SHAPES_WIDE : DF2_SHAPES_NARROW,
            [&](int shape) {
              df_apply2(shape, nout, nvec, rp, ci, w, xs.p, x, y, sc, perm, I.dfflag.p, s, nin);
            },
