@@ -172,3 +172,49 @@ def test_terms_of_a_tile_with_too_many_columns(gpu_lib):
                 torch.from_numpy(x.reshape(-1)).cuda(), y, vpn)
             assert np.abs(y.cpu().numpy().reshape(n, vpn) - want).max() <= (
                 1e-12 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("k", [2040, 2047, 2048, 2100])
+def test_rows_of_more_columns_than_any_table(gpu_lib, k):
+    # a node in k blocks has 4 k + 2 columns; above 8192 the entries are
+    # sorted.  M 1 is the volume around each node
+    from tmr_gb300 import TMR
+    f = TMR.OctForest(order=2)
+    f.setConnectivity(_fan(k))
+    f.createTrees(0)
+    f.createNodes()
+    n = int(f.getNodeRange()[1])
+    F = TMR.MatrixFilter(0.5, 3, None, [f])
+    rp, c, v, _, _, _ = F.getMatrix()
+    assert n == 4 * k + 2 and rp[1] - rp[0] == n
+    assert all(np.all(np.diff(c[rp[i]:rp[i + 1]]) > 0) for i in range(0, n, 97))
+    D = np.add.reduceat(v, rp[:-1])
+    vol = np.bincount(f.getMeshConn().reshape(-1), minlength=n) / 8.0
+    # sums of at most 8 k + 4 products of positive numbers
+    np.testing.assert_allclose(D, vol, rtol=1e-12)
+    # the entry of the axis with itself: k corners of 1/27
+    np.testing.assert_allclose(v[rp[0]], k / 27.0, rtol=1e-12)
+
+
+def test_filter_of_many_quadrants(gpu_lib):
+    # 2^27 quadrants: one more than the row assembly's places take
+    import torch
+
+    from tmr_gb300 import TMR
+    if torch.cuda.mem_get_info()[0] < (200 << 30):
+        pytest.skip("needs 200 GB of device memory")
+    f = TMR.QuadForest(order=2)
+    f.setConnectivity(W.brick2d(2, 1))
+    f.createTrees(13)
+    assert f.getNumQuadrants() == 1 << 27
+    f.createNodes()
+    F = TMR.MatrixFilter(1e-4, 1, None, [f])
+    n, nnz = F.size()
+    side = 1 << 13
+    assert n == (2 * side + 1) * (side + 1)
+    assert nnz == (3 * (2 * side + 1) - 2) * (3 * (side + 1) - 2)
+    x = torch.ones(n, dtype=torch.float64, device="cuda")
+    y = torch.empty_like(x)
+    F.applyFilter(x, y)
+    # the filter keeps constants: rounding of a two-term sum
+    assert float((y - 1).abs().max()) < 1e-12

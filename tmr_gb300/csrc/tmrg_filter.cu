@@ -826,11 +826,37 @@ void filter_create_quad(QForest &f, double len, double r, int N, Filter &F) {
                len, r, N, F);
 }
 
-// M with every block entry sorted by (row, column) and equal ones summed in
-// element order (orders 3 and 4).
+// M from its E block entries: sorted by (row, column), equal ones summed in
+// element order.
+static void sum_entries(DBuf<uint64_t> &keys, DBuf<uint32_t> &perm, DBuf<double> &ev, long long E,
+                        int cb, Filter &F) {
+  cudaStream_t s = F.s;
+  const long long n = F.n;
+  radix_sort(keys, &perm, E, 2 * cb, s);
+  DBuf<unsigned> pos(E + 1, s);
+  launch(k_fe_first, blocks_for(E, 256), 256, 0, s, E, (const uint64_t *)keys.p,
+         pos.p);
+  exclusive_scan<unsigned>(pos.p, pos.p, E, s);
+  const long long nnz = read_scalar(pos.p + E, s);
+  F.nnz = nnz;
+  F.colidx.alloc(nnz + 1, s);
+  F.vals.alloc(nnz + 1, s);
+  F.rowptr.alloc(n + 1, s);
+  F.rowptr.zero();
+  launch(k_fe_reduce, blocks_for(E, 256), 256, 0, s, E, (const uint64_t *)keys.p,
+         (const uint32_t *)perm.p, (const double *)ev.p, (const unsigned *)pos.p,
+         cb, F.colidx.p, F.vals.p, F.rowptr.p);
+  keys.release();
+  perm.release();
+  ev.release();
+  pos.release();
+  exclusive_scan<int>(F.rowptr.p, F.rowptr.p, n, s);
+}
+
+// The entries of orders 3 and 4.
 static void assemble_sorted(const FSource &f, const FilterCtx &c, int cb, Filter &F) {
   cudaStream_t s = f.s;
-  const long long n = f.nn, ne = f.ne;
+  const long long ne = f.ne;
   long long E = 0;
   DBuf<uint64_t> keys;
   DBuf<uint32_t> perm;
@@ -878,25 +904,7 @@ static void assemble_sorted(const FSource &f, const FilterCtx &c, int cb, Filter
                                  (int)smem));
   launch(k_fe_gen_write, blocks_for(ne, FG_WARPS), FG_WARPS * 32, smem, s, ne, c, g, cb,
          (const long long *)cnt.p, keys.p, perm.p, ev.p);
-  radix_sort(keys, &perm, E, 2 * cb, s);
-  DBuf<unsigned> pos(E + 1, s);
-  launch(k_fe_first, blocks_for(E, 256), 256, 0, s, E, (const uint64_t *)keys.p,
-         pos.p);
-  exclusive_scan<unsigned>(pos.p, pos.p, E, s);
-  const long long nnz = read_scalar(pos.p + E, s);
-  F.nnz = nnz;
-  F.colidx.alloc(nnz + 1, s);
-  F.vals.alloc(nnz + 1, s);
-  F.rowptr.alloc(n + 1, s);
-  F.rowptr.zero();
-  launch(k_fe_reduce, blocks_for(E, 256), 256, 0, s, E, (const uint64_t *)keys.p,
-         (const uint32_t *)perm.p, (const double *)ev.p, (const unsigned *)pos.p,
-         cb, F.colidx.p, F.vals.p, F.rowptr.p);
-  keys.release();
-  perm.release();
-  ev.release();
-  pos.release();
-  exclusive_scan<int>(F.rowptr.p, F.rowptr.p, n, s);
+  sum_entries(keys, perm, ev, E, cb, F);
 }
 
 static void filter_build(const FSource &f, double len, double r, int N, Filter &F) {
@@ -918,12 +926,22 @@ static void filter_build(const FSource &f, double len, double r, int N, Filter &
     // near the ends of the exponent's range an entry of a deep level might
     // not be the scaled one (3 x 30 levels and nd <= 3)
     const int ex = (int)((ent.m0 >> 52) & 0x7ff);
-    if (!assemble_rows(ElemCtx{c.conn, c.dptr, c.dconn, c.dw, c.err, c.npe}, ent, n, ne,
-                       ex < 128 || ex == 0x7ff, F.rowptr, F.colidx, F.vals, F.nnz, s)) {
-      if (read_scalar(err.p, s))
-        throw Error(TMRG_ERR_INTERNAL, "matrix filter: element touches too many nodes");
-      throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
+    const ElemCtx ec{c.conn, c.dptr, c.dconn, c.dw, c.err, c.npe};
+    AsmResult res = assemble_rows(ec, ent, n, ne, ex < 128 || ex == 0x7ff, F.rowptr, F.colidx,
+                                  F.vals, F.nnz, s);
+    if (res == ASM_PLACES) {
+      DBuf<uint64_t> keys;
+      DBuf<uint32_t> perm;
+      DBuf<double> ev;
+      long long E = 0;
+      err.zero();
+      res = assemble_entries(ec, ent, ne, cb, keys, perm, ev, E, s);
+      if (res == ASM_DONE) sum_entries(keys, perm, ev, E, cb, F);
     }
+    if (res == ASM_NODES)
+      throw Error(TMRG_ERR_INTERNAL, "matrix filter: element touches too many nodes");
+    if (res == ASM_ENTRIES)
+      throw Error(TMRG_ERR_ARG, "matrix filter: more than 2^32 element-matrix entries");
   } else {
     assemble_sorted(f, c, cb, F);
   }

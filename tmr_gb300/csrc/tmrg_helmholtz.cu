@@ -1503,7 +1503,8 @@ static void build_tiles(Helmholtz &H, HLevel &L, bool finest) {
   err.zero();
   long long nnz = 0;
   const ElemCtx c{L.econn.p, L.dptr.p, L.dconn.p, L.dw.p, err.p, L.npe};
-  if (!assemble_rows(c, make_helm_entry(L), L.nn, L.ne, false, rp, ci, v, nnz, s)) return;
+  if (assemble_rows(c, make_helm_entry(L), L.nn, L.ne, false, rp, ci, v, nnz, s) != ASM_DONE)
+    return;
   if (!tsell_build(L.tiled, L.nn, rp.p, ci.p, s)) return;
   tsell_values(L.tiled, rp.p, (const double *)v.p, L.k32, s);
   if (finest) tsell_values(L.tiled, rp.p, (const double *)v.p, L.k64, s);

@@ -355,15 +355,20 @@ static __global__ void k_fa_compact(long long n, const unsigned *__restrict__ co
 }
 
 // The n x n matrix of the elements' entries as CSR (columns ascending).  `all`:
-// every element stores its block.  False, with nothing in the outputs, where
-// there are too many elements or entries for the 32-bit places, an element
-// touches more than FMAXK nodes or a row outgrows every table (c.err is set
-// in the last two cases).
+// every element stores its block.  Anything but ASM_DONE leaves nothing in the
+// outputs.
+enum AsmResult {
+  ASM_DONE,
+  ASM_NODES,    // an element touches more than FMAXK nodes
+  ASM_ENTRIES,  // 2^32 element-matrix entries or more
+  ASM_PLACES    // too many elements for their 32-bit places, or a row of more
+                // than FA_HUGE columns: assemble_entries has no such limit
+};
 template <typename Entry>
-inline bool assemble_rows(const ElemCtx &c, const Entry &ent, long long n, long long ne, bool all,
+inline AsmResult assemble_rows(const ElemCtx &c, const Entry &ent, long long n, long long ne, bool all,
                           DBuf<int> &rowptr, DBuf<int> &colidx, DBuf<double> &vals,
                           long long &nnz, cudaStream_t s) {
-  if (ne >= (1LL << 27)) return false;
+  if (ne >= (1LL << 27)) return ASM_PLACES;
   const int cb = bits_for(n + 1);
   RowAsm A{};
   A.conn = c.conn;
@@ -387,7 +392,8 @@ inline bool assemble_rows(const ElemCtx &c, const Entry &ent, long long n, long 
   read_scalars(hp, hv, s);
   // rows, each at its number of entries before equal columns are added
   const long long E = (ne - nh) * c.npe * c.npe + ((long long)hv[3] << 32 | hv[2]);
-  if (E >= (1LL << 32) || hv[4]) return false;
+  if (hv[4]) return ASM_NODES;
+  if (E >= (1LL << 32)) return ASM_ENTRIES;
   DBuf<int> unode((size_t)hv[0] + 1, s);
   DBuf<double> block((size_t)hv[1] + 1, s);
   launch(k_fa_blocks<Entry>, blocks_for(nh, 64), 64, 0, s, nh, c, ent, (const unsigned *)list.p,
@@ -445,14 +451,59 @@ inline bool assemble_rows(const ElemCtx &c, const Entry &ent, long long n, long 
   }
   if (err) {
     rowptr.release();
-    return false;
+    return err == FA_FULL ? ASM_PLACES : ASM_NODES;
   }
   colidx.alloc(nnz + 1, s);
   vals.alloc(nnz + 1, s);
   launch(k_fa_compact, blocks_for(n * 8, 256), 256, 0, s, n, (const unsigned *)coff.p,
          (const int *)rowptr.p, (const int *)col.p, (const double *)val.p, colidx.p,
          vals.p);
-  return true;
+  return ASM_DONE;
+}
+
+// The block entries of every element as records (row << cb | column, place,
+// value) for a sort, and their number in E.
+template <typename Entry>
+__global__ void k_fa_entry_count(long long ne, ElemCtx c, Entry ent, long long *cnt) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  int U[FMAXK];
+  const int K = element_block(c, ent, e, U, nullptr);
+  cnt[e] = K * K;
+}
+template <typename Entry>
+__global__ void __launch_bounds__(64)
+    k_fa_entries(long long ne, ElemCtx c, Entry ent, int cb, const long long *__restrict__ off,
+                 uint64_t *keys, uint32_t *perm, double *vals) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  int U[FMAXK];
+  double L[FMAXK][FMAXK];
+  const int K = element_block(c, ent, e, U, L);
+  long long o = off[e];
+  for (int u = 0; u < K; u++)
+    for (int v = 0; v < K; v++, o++) {
+      keys[o] = (uint64_t)(uint32_t)U[u] << cb | (uint64_t)(uint32_t)U[v];
+      perm[o] = (uint32_t)o;
+      vals[o] = L[u][v];
+    }
+}
+template <typename Entry>
+inline AsmResult assemble_entries(const ElemCtx &c, const Entry &ent, long long ne, int cb,
+                                  DBuf<uint64_t> &keys, DBuf<uint32_t> &perm, DBuf<double> &vals,
+                                  long long &E, cudaStream_t s) {
+  DBuf<long long> cnt(ne + 1, s);
+  launch(k_fa_entry_count<Entry>, blocks_for(ne, 128), 128, 0, s, ne, c, ent, cnt.p);
+  exclusive_scan<long long>(cnt.p, cnt.p, ne, s);
+  E = read_scalar(cnt.p + ne, s);
+  if (read_scalar(c.err, s)) return ASM_NODES;
+  if (E >= (1LL << 32)) return ASM_ENTRIES;
+  keys.alloc(E, s);
+  perm.alloc(E, s);
+  vals.alloc(E, s);
+  launch(k_fa_entries<Entry>, blocks_for(ne, 64), 64, 0, s, ne, c, ent, cb,
+         (const long long *)cnt.p, keys.p, perm.p, vals.p);
+  return ASM_DONE;
 }
 
 }  // namespace tmrg
