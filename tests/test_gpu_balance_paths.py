@@ -145,3 +145,36 @@ def test_nodes_of_tiles_equal_nodes_of_entries(gpu_lib, order, interp):
     assert got[0][1] < 16384 <= got[1][1] and got[1][1] % 256 != 0
     for a, b in zip(got[0][2:], got[1][2:]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("dim,blocks,nrand,lo,hi", [(3, (8, 8, 4), 2000, 5, 7), (3, (4, 4, 2), 3000, 6, 9),
+                                                    (2, (8, 8), 20000, 6, 12)])
+def test_a_set_that_outgrows_its_list_is_given_up_early(gpu_lib, dim, blocks, nrand, lo, hi):
+    # the balance that gave its set up takes no more than a few times the
+    # balance of its result, which fits one (1 to 2 times; 10 where every
+    # level goes on adding to the full table)
+    import time
+
+    import torch
+
+    from tmr_gb300 import TMR
+    f = _forest(TMR, dim, _brick(dim, *blocks), 0)
+    f.createRandomTrees(nrand, lo, hi, 4)
+
+    def best(g):
+        out, t = None, []
+        for _ in range(4):
+            out = g.duplicate()
+            torch.cuda.synchronize()
+            a = time.perf_counter()
+            out.balance(1)
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - a)
+        return out, min(t)
+
+    a, ta = best(f)
+    b, tb = best(a)
+    num = (lambda g: g.getNumOctants()) if dim == 3 else (lambda g: g.getNumQuadrants())
+    n0 = num(f)
+    assert num(a) > (8 if dim == 3 else 4) * (n0 + n0 // 4 + 4096) and num(b) == num(a)
+    assert ta <= 5 * tb + 1e-3

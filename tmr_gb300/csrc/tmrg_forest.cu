@@ -733,7 +733,9 @@ static void balance_impl(Forest &f, int corner, const OctKeyT<Key> K) {
 // to about 3M octants.  Measured with the in-place refine, refine + balance +
 // createNodes of a linear forest: 1.42 -> 0.68 ms at 3,000 octants (140 -> 70
 // launches), 9.75 -> 7.22 ms at 5.9M octants.  The sorting path stays for
-// 128-bit keys and for a closure that outgrows the set.
+// 128-bit keys and for a closure that outgrows the set (seeds far apart: 1.0M
+// random octants that close to 28.6M 5.9 ms, 96K to 11.4M 3.5 ms; 10.9 and 5.3
+// with 26 targets a family sorted and no set tried).
 
 // Families of the octants, each once per run of siblings.
 __global__ void __launch_bounds__(256)
@@ -763,6 +765,7 @@ __global__ void __launch_bounds__(256)
     const unsigned i = b0 + (threadIdx.x >> 3);
     const uint64_t k = i < m ? S.list[i] : 0;
     const bool mine = i < m && (int)(k & 31) == level && (corner || g != 7);
+    if (S.full()) return;
     if (!__any_sync(0xffffffffu, mine)) continue;
     // the first target is added by the whole warp; a face, edge or corner
     // shared by several trees gives some lanes more
@@ -792,6 +795,7 @@ __global__ void __launch_bounds__(256)
 // Leaves: the siblings of every family that no finer family refines.
 __global__ void __launch_bounds__(256)
     k_fam_leaves(int gens, OctKey K, KeySet S, uint64_t *out, unsigned cap) {
+  if (S.full()) return;
   const unsigned m = S.before(gens);
   const int j = threadIdx.x & 7, lane = threadIdx.x & 31;
   const unsigned stride = gridDim.x * 32;

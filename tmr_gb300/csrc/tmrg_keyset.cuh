@@ -28,6 +28,12 @@ struct KeySet {
   }
   __device__ __forceinline__ unsigned *overflow() const { return count + KEYSET_GENS; }
   __device__ __forceinline__ unsigned *counter() const { return count + KEYSET_GENS + 1; }
+  // The set overflowed: it is given up, and nothing more need be added (a full
+  // table would take KEYSET_PROBES steps a key).  A whole warp asks and gets
+  // one answer.
+  __device__ __forceinline__ bool full() const {
+    return __any_sync(0xffffffffu, __ldcg(overflow()) != 0u);
+  }
   // True when `k` was not in the set (it is now).
   __device__ __forceinline__ bool insert(uint64_t k) const {
     const unsigned mask = 0xffffffffu >> (shift - 32);

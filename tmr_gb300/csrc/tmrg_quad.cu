@@ -1029,6 +1029,7 @@ __global__ void __launch_bounds__(256)
     const unsigned i = b0 + (threadIdx.x >> 2);
     const uint64_t k = i < m ? S.list[i] : 0;
     const bool mine = i < m && (int)(k & 31) == level && (corner || g != 3);
+    if (S.full()) return;
     if (!__any_sync(0xffffffffu, mine)) continue;
     uint64_t first = 0;
     int cnt = 0;
@@ -1055,6 +1056,7 @@ __global__ void __launch_bounds__(256)
 }
 __global__ void __launch_bounds__(256)
     k_q_fam_leaves(int gens, QKey K, KeySet S, uint64_t *out, unsigned cap) {
+  if (S.full()) return;
   const unsigned m = S.before(gens);
   const int j = threadIdx.x & 3, lane = threadIdx.x & 31;
   const unsigned stride = gridDim.x * 64;
