@@ -97,3 +97,91 @@ def test_host_buffers_equal_device_buffers(operator):
         xd = torch.from_numpy(x).cuda()
         fn(xd, y)
         np.testing.assert_array_equal(yh, y.cpu().numpy())
+
+
+@pytest.mark.parametrize("nvec", [2, 5, 17])
+@pytest.mark.parametrize("where", ["all", "first", "last", "inf"])
+def test_values_outside_the_window_at_the_ends(operator, nvec, where):
+    # values the (hi, lo) pairs do not hold everywhere, at the first or the last
+    # input that is read, or one infinity: the whole result in FP64, infinite
+    # where a row reads it
+    import torch
+    I, P = operator
+    if P.nnz > 20 * P.shape[0]:
+        pytest.skip("tiles that do not fit")
+    rows, cols = P.shape
+    T = P.T.tocsr()
+    rng = np.random.default_rng(80 + nvec)
+    one = np.asarray(T @ np.ones(rows))[:, None]
+    # the column sums' own rounding and that of the weights in them
+    sums = (np.diff(T.indptr)[:, None] + 4) * 2.0 ** -48 * np.asarray(abs(T) @ np.ones(rows))[:, None]
+    sums = np.where(one == 0.0, 0.0, sums / np.where(one == 0.0, 1.0, abs(one)))
+    one[one == 0.0] = np.inf
+    for fn, A, scale, den in ((I.mult, P, 1.0, 0.0), (I.multTranspose, T, 1.0, 0.0),
+                              (I.multWeightTranspose, T, one, sums)):
+        x = rng.standard_normal((A.shape[1], nvec))
+        read = np.unique(A.indices)
+        if where == "all":
+            x *= 1e-30
+        else:
+            i = (read[0], 0) if where == "first" else (read[-1], nvec - 1)
+            x[i] = np.inf if where == "inf" else 1e-30
+        want = (A @ np.where(np.isinf(x), 0.0, x)) / scale
+        bound = (abs(A) @ np.where(np.isinf(x), 0.0, abs(x))) / abs(scale)
+        # rounding of a row's products, its sum and the weights (2^-48 each)
+        n = np.diff(A.indptr)[:, None]
+        bound = bound * ((n + 4) * 2.0 ** -52 + 2.0 ** -47 + den) + 1e-300
+        for shift in (0, 1):
+            xd = torch.empty(x.size + shift, dtype=torch.float64, device="cuda")[shift:]
+            xd.copy_(torch.from_numpy(x.reshape(-1)))
+            y = torch.full((A.shape[0] * nvec + shift,), float("nan"), dtype=torch.float64,
+                           device="cuda")[shift:]
+            fn(xd, y)
+            got = y.cpu().numpy().reshape(-1, nvec)
+            fin = np.ones(got.shape, bool)
+            if where == "inf":
+                fin[:, nvec - 1] = np.asarray(A[:, read[-1]].todense())[:, 0] == 0.0
+                if fn != I.multWeightTranspose:  # (a column of no weight gives 0)
+                    assert not fin.all() and not np.isfinite(got[~fin]).any()
+            assert np.all(np.abs(got - want)[fin] <= bound[fin])
+
+
+def test_tile_applies_outside_the_window_take_no_second_apply(gpu_lib):
+    # small values everywhere: a few times the double-float apply (2 to 4; 12
+    # where it ran in full before a thread per row and vector)
+    import time
+
+    import torch
+
+    from tmr_gb300 import TMR
+    from tmr_gb300 import workloads as W
+    f = TMR.OctForest(order=3)
+    f.setConnectivity(W.brick(4, 4, 2))
+    f.createTrees(2)
+    for p in range(3):
+        f.refine(W.random_indicator(f.getNumOctants(), 7, p, 0.3), 0, 9)
+        f.balance(1)
+    f.createNodes()
+    c = f.coarsen()
+    c.balance(1)
+    c.createNodes()
+    I = TMR.VecInterp()
+    f.createInterpolation(c, I)
+    rows, cols, _ = I.sizes()
+
+    def best(fn, x, y):
+        t = []
+        for _ in range(7):
+            torch.cuda.synchronize()
+            a = time.perf_counter()
+            for _ in range(10):
+                fn(x, y)
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - a)
+        return min(t[2:])
+
+    for nvec in (4, 16):
+        for fn, nin, nout in ((I.mult, cols, rows), (I.multTranspose, rows, cols)):
+            x = torch.randn(nin * nvec, dtype=torch.float64, device="cuda")
+            y = torch.empty(nout * nvec, dtype=torch.float64, device="cuda")
+            assert best(fn, x * 1e-20, y) <= 7 * best(fn, x, y)

@@ -2668,10 +2668,10 @@ static void interp_colsum(Interp &I) {
 // input and rebuilds each weight as hi + lo).  With `scale` the result is
 // divided by scale[row] (weight-normalised transpose).
 
-// Few vectors on a small matrix, in FP64 straight from the caller's vector:
-// 2^LB lanes per row take its entries in turn, each with all NV components,
-// and combine in a fixed tree.  One launch instead of a flag reset, a pass
-// that splits the input and an apply; no window on the values.
+// A small matrix, in FP64 straight from the caller's vectors: 2^LB lanes per
+// row take its entries in turn, each with all NV components, and combine in a
+// fixed tree.  One launch instead of a flag reset, a pass that splits the input
+// and an apply; no window on the values.
 template <int NV>
 __global__ void __launch_bounds__(256)
     k_f64_rows(long long rows, int LB, const int *__restrict__ rowptr,
@@ -2705,6 +2705,96 @@ __global__ void __launch_bounds__(256)
     double a = acc[v];
     if (scale) a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
     y[r * NV + v] = a;
+  }
+}
+
+// The whole apply in FP64 where the double-float one before it met a value
+// outside its window (else a return at once, hence a grid of a few blocks an SM
+// that takes the rows in turn).  LPR lanes per row hold PPL vector pairs each,
+// LPR apart; each lane makes the FP64 weight of one entry in LPR and the others
+// get it by shuffles, for a weight costs the FP64 pipe as much as a pair's
+// products.  A warp's rows are of one length: by `order` inside tiles of TB_ROWS
+// (P) or by `perm` (P^T).  SC: vectors read and written value by value.
+// (all blocks at once: the rows are dealt out in turn)
+constexpr int F64P_BLOCKS = 5;
+template <int LPR, int PPL, bool SC>
+__global__ void __launch_bounds__(256, F64P_BLOCKS)
+    k_f64_pairs(long long rows, int nvec, const int *__restrict__ rowptr,
+                const int *__restrict__ cols, const float2 *__restrict__ w,
+                const uint8_t *__restrict__ order, const int *__restrict__ perm,
+                const double *__restrict__ x, double *__restrict__ y,
+                const double *__restrict__ scale, const int *__restrict__ flags) {
+  if ((__ldg(flags) | __ldg(flags + 1)) == 0) return;
+  constexpr int RPW = 32 / LPR;
+  const int lane = threadIdx.x & 31, v = lane % LPR, nvec2 = (nvec + 1) / 2;
+  const long long slots = order ? (rows + TB_ROWS - 1) / TB_ROWS * TB_ROWS : rows;
+  const long long step = (long long)gridDim.x * 8 * RPW;
+  for (long long s0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW; s0 < slots;
+       s0 += step) {  // uniform per warp
+    long long r = s0 + lane / LPR;
+    if (order) {
+      // another place in every tile (step may be whole tiles): each warp has
+      // its share of the long rows, which come first
+      const long long tile = r / TB_ROWS;
+      const int at = ((int)(r & (TB_ROWS - 1)) + (int)(tile & 255) * (11 * RPW)) & (TB_ROWS - 1);
+      r = tile * TB_ROWS + __ldg(order + tile * TB_ROWS + at);
+    } else if (r < rows) {
+      r = __ldg(perm + r);
+    }
+    const bool have = r < rows;
+    const int p0 = have ? __ldg(rowptr + r) : 0, len = have ? __ldg(rowptr + r + 1) - p0 : 0;
+    const int trips = __reduce_max_sync(0xffffffffu, len);
+    const double sc = scale && have ? scale[r] : 1.0;
+    for (int vb = v; vb - v < nvec2; vb += LPR * PPL) {
+      double ax[PPL], ay[PPL];
+#pragma unroll
+      for (int j = 0; j < PPL; j++) ax[j] = ay[j] = 0.0;
+#pragma unroll 2
+      for (int t = 0; t < trips; t += LPR) {
+        const int own = t + v;
+        const int c = own < len ? __ldg(cols + p0 + own) : 0;
+        const float2 wv = own < len ? __ldg(w + p0 + own) : make_float2(0.0f, 0.0f);
+        const double wd = df_value(wv.x, wv.y);
+#pragma unroll
+        for (int k = 0; k < LPR; k++) {
+          const int ck = LPR == 1 ? c : __shfl_sync(0xffffffffu, c, k, LPR);
+          const double dk = LPR == 1 ? wd : __shfl_sync(0xffffffffu, wd, k, LPR);
+          const double *xr = x + (long long)ck * nvec;
+#pragma unroll
+          for (int j = 0; j < PPL; j++) {
+            const int q = vb + j * LPR;
+            double2 xv = make_double2(0.0, 0.0);
+            if (q < nvec2 && t + k < len) {
+              if (SC) {
+                xv.x = __ldg(xr + 2 * q);
+                if (2 * q + 1 < nvec) xv.y = __ldg(xr + 2 * q + 1);
+              } else {
+                xv = __ldg((const double2 *)xr + q);
+              }
+            }
+            ax[j] = __fma_rn(dk, xv.x, ax[j]);
+            ay[j] = __fma_rn(dk, xv.y, ay[j]);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < PPL; j++) {
+        const int q = vb + j * LPR;
+        if (q >= nvec2 || !have) continue;
+        double a = ax[j], b = ay[j];
+        if (scale) {
+          a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
+          b = (sc != 0.0) ? __ddiv_rn(b, sc) : 0.0;
+        }
+        double *yp = y + r * nvec + 2 * q;
+        if (SC) {
+          yp[0] = a;
+          if (2 * q + 1 < nvec) yp[1] = b;
+        } else {
+          *(double2 *)yp = make_double2(a, b);
+        }
+      }
+    }
   }
 }
 
@@ -2943,9 +3033,9 @@ __global__ void __launch_bounds__(256)
 // tile are split into (hi, lo) as they are loaded into shared memory, so no
 // split copy of the input is made and no input row is gathered more than once
 // per tile; an entry reads one row of 16 L bytes there.  A value outside the
-// double-float window (or a weight, flags[0]) sets flags[1]; the apply is then
-// run again by the FP64 kernels, which return at once when no flag is set.
-// (The flags are reset before the apply.)
+// double-float window (or a weight, flags[0]) sets flags[1], blocks that see it
+// leave, and k_f64_pairs, which returns at once when no flag is set, makes the
+// whole result.  (The flags are reset before the apply.)
 //
 // Bound by instruction issue (12 FP32 instructions an entry and vector, and
 // about half as many around them).  117M entries, 2 / 4 / 8 / 16 vectors: P 606
@@ -2979,8 +3069,9 @@ __global__ void __launch_bounds__(TB_ROWS)
   float2 *sx = (float2 *)dt_mem;  // maxu x V
   __shared__ int s_rp[TB_ROWS + 1];
   __shared__ uint8_t s_ord[TB_ROWS];
-  if (flags[0] != 0) return;  // (no block may leave for flags[1], which others are setting)
+  __shared__ int s_stop;
   const int t = threadIdx.x, nvec = D.nvec;
+  if (t == 0) s_stop = flags[0] | *(volatile int *)(flags + 1);
   const long long tile = D.tile0 + blockIdx.x, r0 = tile * TB_ROWS;
   const int nr = (int)min((long long)TB_ROWS, D.rows - r0);
   const unsigned u0 = D.uoff[tile];
@@ -2988,6 +3079,7 @@ __global__ void __launch_bounds__(TB_ROWS)
   for (int i = t; i <= nr; i += TB_ROWS) s_rp[i] = __ldg(rp + r0 + i);
   s_ord[t] = __ldg(order + tile * TB_ROWS + t);
   __syncthreads();
+  if (s_stop) return;
   const int base = s_rp[0];
   const int l = t & (L - 1);
   bool out = false;
@@ -3035,29 +3127,6 @@ __global__ void __launch_bounds__(TB_ROWS)
   }
   if (out) atomicOr(flags + 1, 1);
 }
-// The same tiles in FP64: a thread per row and vector.
-__global__ void __launch_bounds__(TB_ROWS)
-    k_df_tile_f64(DfTiles D, const int *__restrict__ rp, const uint16_t *__restrict__ idx,
-                  const double *__restrict__ x, double *__restrict__ y,
-                  const int *__restrict__ flags) {
-  if ((__ldg(flags) | __ldg(flags + 1)) == 0) return;
-  for (long long tile = D.tile0 + blockIdx.x; tile < D.tile0 + D.tiles; tile += gridDim.x) {
-    const long long r0 = tile * TB_ROWS;
-    const int nr = (int)min((long long)TB_ROWS, D.rows - r0);
-    const int *uc = D.ucol + D.uoff[tile];
-    for (int i = threadIdx.x; i < nr * D.nvec; i += TB_ROWS) {
-      const int lr = i / D.nvec, v = i - lr * D.nvec;
-      double a = 0.0;
-      for (int p = __ldg(rp + r0 + lr); p < __ldg(rp + r0 + lr + 1); p++) {
-        const float2 wv = __ldg(D.w + p);
-        a = __fma_rn(__dadd_rn((double)wv.x, (double)wv.y),
-                     __ldg(x + (long long)__ldg(uc + __ldg(idx + p)) * D.nvec + v), a);
-      }
-      y[(r0 + lr) * D.nvec + v] = a;
-    }
-  }
-}
-
 // y = P^T x in two parts: every tile sums its runs (the entries of one column
 // in the tile) over its own input rows, which are one block of memory, and
 // k_df_pair_sum adds a column's runs, tiles ascending.  Runs longest first.
@@ -3069,8 +3138,11 @@ __global__ void __launch_bounds__(TB_ROWS)
   constexpr int L = 1 << LB, V = 2 * L;
   extern __shared__ __align__(16) unsigned char dt_mem[];
   float2 *sx = (float2 *)dt_mem;  // TB_ROWS x V
-  if (flags[0] != 0) return;  // (no block may leave for flags[1], which others are setting)
+  __shared__ int s_stop;
   const int t = threadIdx.x, nvec = D.nvec, tile = (int)D.tile0 + blockIdx.x;
+  if (t == 0) s_stop = flags[0] | *(volatile int *)(flags + 1);
+  __syncthreads();
+  if (s_stop) return;
   const long long r0 = (long long)tile * TB_ROWS;
   const int nr = (int)min((long long)TB_ROWS, D.rows - r0);
   const unsigned u0 = D.uoff[tile];
@@ -3142,30 +3214,6 @@ __global__ void __launch_bounds__(256)
     }
   }
   y[t] = r;
-}
-// P^T in FP64 by its own rows, where the flags ask for it.
-__global__ void __launch_bounds__(256)
-    k_df_rows_f64(long long rows, int nvec, const int *__restrict__ rp,
-                  const int *__restrict__ ci, const float2 *__restrict__ w,
-                  const double *__restrict__ x, double *__restrict__ y,
-                  const double *__restrict__ scale, const int *__restrict__ flags) {
-  if ((__ldg(flags) | __ldg(flags + 1)) == 0) return;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < rows * nvec;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long r = t / nvec;
-    const int v = (int)(t - r * nvec);
-    double a = 0.0;
-    for (int p = __ldg(rp + r); p < __ldg(rp + r + 1); p++) {
-      const float2 wv = __ldg(w + p);
-      a = __fma_rn(__dadd_rn((double)wv.x, (double)wv.y),
-                   __ldg(x + (long long)__ldg(ci + p) * nvec + v), a);
-    }
-    if (scale) {
-      const double sc = scale[r];
-      a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
-    }
-    y[t] = a;
-  }
 }
 
 // ---------------------------------------------------------------------
@@ -3455,6 +3503,31 @@ static void df_apply2(int shape, long long rows, int nvec, const int *rp, const 
 #undef TMRG_DF2
 #undef TMRG_DF2S
 }
+// k_f64_pairs on `rows` rows (`order` begins with theirs).
+static void f64_pairs(int nvec, long long rows, const int *rp, const int *ci, const float2 *w,
+                      const uint8_t *order, const int *perm, const double *x, double *y,
+                      const double *scale, const int *flags, cudaStream_t s) {
+  const int nvec2 = (nvec + 1) / 2;
+#define TMRG_F64P(L, P)                                                                      \
+  do {                                                                                       \
+    const unsigned g = std::min(blocks_for(rows * (L), 256), 152u * F64P_BLOCKS);            \
+    if (df_scalar(nvec, x, y))                                                               \
+      launch((k_f64_pairs<L, P, true>), g, 256, 0, s, rows, nvec, rp, ci, w, order, perm, x, \
+             y, scale, flags);                                                               \
+    else                                                                                     \
+      launch((k_f64_pairs<L, P, false>), g, 256, 0, s, rows, nvec, rp, ci, w, order, perm, x, \
+             y, scale, flags);                                                               \
+  } while (0)
+  if (nvec2 == 1)
+    TMRG_F64P(1, 1);
+  else if (nvec2 == 2)
+    TMRG_F64P(2, 1);
+  else if (nvec2 <= 4)
+    TMRG_F64P(2, 2);
+  else
+    TMRG_F64P(4, 2);
+#undef TMRG_F64P
+}
 // Vectors at once: 16, 8, 4 or 2.
 static int df_tile_lanes(int nvec) {
   int lb = 0;
@@ -3488,8 +3561,9 @@ static void df_tile_apply(const Interp &I, long long t0, long long t1, int nvec,
     default: TMRG_DT(3);
   }
 #undef TMRG_DT
-  launch(k_df_tile_f64, (unsigned)std::min(t1 - t0, 152LL * 8), TB_ROWS, 0, s, D, I.ap_rowptr(),
-         (const uint16_t *)I.tile_idx.p, x, y, (const int *)I.dfflag.p);
+  const long long r0 = t0 * TB_ROWS, nr = std::min(I.rows, t1 * TB_ROWS) - r0;
+  f64_pairs(nvec, nr, I.ap_rowptr() + r0, I.ap_colidx(), I.ap_w.p, I.tile_order.p + r0, nullptr,
+            x, y + r0 * nvec, nullptr, I.dfflag.p, s);
 }
 // y = P^T x in two steps: the runs of tiles [t0, t1), then the columns
 // (divided by `scale` where given).
@@ -3502,7 +3576,7 @@ static void df_tile_runs(const Interp &I, long long t0, long long t1, int nvec, 
          sizeof(float2) * ((size_t)TB_ROWS << (B + 1)), s, D, I.ap_rowptr(),                   \
          (const uint2 *)I.tile_runs.p, (const uint8_t *)I.tile_row.p, x, part, I.dfflag.p)
   switch (df_tile_lanes(nvec)) {
-    case 0: TMRG_DT(0); break;
+    case 0:  // (fewer than 3 vectors go by rows)
     case 1: TMRG_DT(1); break;
     case 2: TMRG_DT(2); break;
     default: TMRG_DT(3);
@@ -3513,9 +3587,8 @@ static void df_tile_columns(const Interp &I, int nvec, const float2 *part, const
                             double *y, const double *scale, cudaStream_t s) {
   launch(k_df_pair_sum, blocks_for(I.cols * nvec, 256), 256, 0, s, I.cols, nvec,
          (const unsigned *)I.col_pairs.p, part, y, scale, (const int *)I.dfflag.p);
-  launch(k_df_rows_f64, std::min(blocks_for(I.cols * nvec, 256), 152u * 8), 256, 0, s, I.cols,
-         nvec, (const int *)I.t_rowptr.p, (const int *)I.t_colidx.p, (const float2 *)I.t_w.p, x,
-         y, scale, (const int *)I.dfflag.p);
+  f64_pairs(nvec, I.cols, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, nullptr, I.t_perm.p, x, y, scale,
+            I.dfflag.p, s);
 }
 
 // Size class of an apply: direction, vector pairs (8 = 8 or more), log2 of
@@ -3535,6 +3608,9 @@ static TuneKey df_key(int which, long long rows, long long nnz, int nvec2, bool 
 // vector 16 -> 12 us, 2 vectors 19 -> 16 us, 3 vectors 20 -> 19 us, 4 vectors
 // 19 against 23 us; 4.8M entries, 1 vector 37 against 65 us.
 constexpr long long F64_ROWS_MAX = 1000000;
+static bool f64_small(int nvec, long long nnz) {
+  return nvec <= 8 && nnz * nvec <= F64_ROWS_MAX;
+}
 // Rows below which P, and P^T with the wide shapes (15 vectors or more), go by
 // rows: a tile is a block, and fewer of them than SMs leave some idle.  16
 // vectors by tiles and by rows: 27K entries P 18.4 and 15.9 us, P^T 24.9 and
@@ -3670,7 +3746,7 @@ constexpr int FC_CHUNKS = 16;
 bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double *yh,
                                  int nvec) {
   if (nvec % 2 != 0 || ((uintptr_t)dx % 16) != 0 || I.rows < (long long)LO_WIN * FC_CHUNKS ||
-      (nvec <= 8 && I.nnz_nz * nvec <= F64_ROWS_MAX) || (I.tile_ok && tune_forced(TUNE_P)))
+      f64_small(nvec, I.nnz_nz) || (I.tile_ok && tune_forced(TUNE_P)))
     return false;
   Stage st("tmrg_interp_mult_staged");
   cudaStream_t s = I.s;
@@ -3768,7 +3844,7 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
 static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, const int *ci,
                      const float2 *w, const double *x, double *y, const double *scale,
                      long long bytes, cudaStream_t s) {
-  if (nvec > 8 || nnz * nvec > F64_ROWS_MAX) return false;
+  if (!f64_small(nvec, nnz)) return false;
   // lanes per row: about a third of the mean row length
   int lb = 0;
   while (lb < 4 && (6LL << lb) * rows <= 2 * nnz) lb++;
