@@ -185,3 +185,74 @@ def test_tile_applies_outside_the_window_take_no_second_apply(gpu_lib):
             x = torch.randn(nin * nvec, dtype=torch.float64, device="cuda")
             y = torch.empty(nout * nvec, dtype=torch.float64, device="cuda")
             assert best(fn, x * 1e-20, y) <= 7 * best(fn, x, y)
+
+
+def _refined(TMR, order, grid, depth, passes):
+    from tmr_gb300 import workloads as W
+    f = TMR.OctForest(order=order)
+    f.setConnectivity(W.brick(*grid))
+    f.createTrees(depth)
+    for p in range(passes):
+        f.refine(W.random_indicator(f.getNumOctants(), 7, p, 0.3), 0, 9)
+        f.balance(1)
+    f.createNodes()
+    c = f.coarsen()
+    c.balance(1)
+    c.createNodes()
+    I = TMR.VecInterp()
+    f.createInterpolation(c, I)
+    return I
+
+
+@pytest.mark.parametrize("grid", [(2, 2, 2), (4, 3, 2), (4, 4, 4)])
+def test_host_buffers_of_any_count_equal_device_buffers(gpu_lib, grid):
+    # one, two and more pieces; pageable and page-locked buffers; and values
+    # that send the apply to FP64, from the first or the last piece on
+    import torch
+
+    from tmr_gb300 import TMR
+    I = _refined(TMR, 2, grid, 3, 2)
+    rows, cols, _ = I.sizes()
+    for nvec in (2, 3, 4, 9, 16, 17, 18):
+        for fn, nin, nout in ((I.mult, cols, rows), (I.multTranspose, rows, cols),
+                              (I.multWeightTranspose, rows, cols)):
+            for where in (None, 0, -1):
+                x = np.random.default_rng(nvec).standard_normal(nin * nvec)
+                if where is not None:
+                    x[where] = 1e-30
+                y = torch.empty(nout * nvec, dtype=torch.float64, device="cuda")
+                fn(torch.from_numpy(x).cuda(), y)
+                want = y.cpu().numpy()
+                got = np.full(nout * nvec, np.nan)
+                fn(x, got)
+                pin = torch.full((nout * nvec,), float("nan"), dtype=torch.float64).pin_memory()
+                fn(torch.from_numpy(x).pin_memory().numpy(), pin.numpy())
+                for a in (got, pin.numpy()):
+                    if where is None:
+                        np.testing.assert_array_equal(a, want)
+                    else:
+                        # pieces before the value stay double-float
+                        np.testing.assert_allclose(a, want, rtol=1e-13, atol=1e-13)
+
+
+def test_page_locked_odd_counts_cost_what_even_ones_do(gpu_lib):
+    # 3 vectors into page-locked memory: no more than 4 (twice as much where the
+    # rows went over the link in order of length)
+    import time
+
+    import torch
+
+    from tmr_gb300 import TMR
+    I = _refined(TMR, 2, (4, 4, 4), 3, 3)
+    rows, cols, _ = I.sizes()
+    t = {}
+    for nvec in (3, 4):
+        x = torch.randn(cols * nvec, dtype=torch.float64).pin_memory().numpy()
+        y = torch.empty(rows * nvec, dtype=torch.float64).pin_memory().numpy()
+        best = []
+        for _ in range(12):
+            a = time.perf_counter()
+            I.mult(x, y)
+            best.append(time.perf_counter() - a)
+        t[nvec] = min(best[4:])
+    assert t[3] <= 1.3 * t[4]

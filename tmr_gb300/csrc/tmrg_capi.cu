@@ -1074,7 +1074,7 @@ static int interp_host(tmrg_interp *I, int which, const double *x, double *y,
     if (ym) {
       // page-locked output: the apply writes it over the host link while
       // it computes, instead of a copy after it
-      interp_apply(P, which, dx.p, ym, nvec);
+      interp_apply(P, which, dx.p, ym, nvec, true);
       TMRG_CUDA(cudaStreamSynchronize(P.s));
       interp_check_apply(P);
       return;

@@ -153,9 +153,10 @@ struct Interp {
   DBuf<int> t_rowptr, t_colidx;  // P^T (zero-free) as CSR, rows = coarse nodes
   DBuf<int> t_perm;  // P^T rows by input chunk of their last entry, then length
   std::vector<long long> t_chunk;  // t_perm range of each input chunk
-  // largest column read by each LO_WIN-row window of the apply copy (host
-  // copy, made by the first host-buffer prolongation)
-  std::vector<int> win_maxcol;
+  // largest column read by each LO_WIN-row window of the apply copy, and largest
+  // row that a window of columns gets anything from (host copies, made by the
+  // first host-buffer applies that need them)
+  std::vector<int> win_maxcol, win_maxrow;
   DBuf<float2> t_w;  // P^T weights (hi, lo)
   // dfflag[0]: a weight outside the double-float window (the applies then
   // run in FP64); dfflag[1]: the same for the input vector of one apply
@@ -199,7 +200,8 @@ void forest_duplicate(Forest &f, Forest &out);
 void forest_balance(Forest &f, int corner);
 void forest_create_nodes(Forest &f);
 void interp_create(Forest &fine, Forest &coarse, Interp &I);
-void interp_apply(Interp &I, int which, const double *x, double *y, int nvec);
+// host: y is page-locked host memory.
+void interp_apply(Interp &I, int which, const double *x, double *y, int nvec, bool host = false);
 // The apply structures of a finished P with `nonzeros` apply_keeps entries;
 // keepoff (optional, device) holds their exclusive per-row offsets.
 void interp_finish(Interp &I, long long nonzeros, cudaStream_t s,

@@ -2374,7 +2374,8 @@ static void transpose_sorted(Interp &I, const long long *keepoff, cudaStream_t s
 // row permutation and P^T.
 void interp_finish(Interp &I, long long nonzeros, cudaStream_t s, const long long *keepoff) {
   const long long rows = I.rows, nnz = I.nnz;
-  I.win_maxcol.clear();  // made again by the first host-buffer prolongation
+  I.win_maxcol.clear();  // made again by the first host-buffer applies
+  I.win_maxrow.clear();
   I.perm.release();      // made where the tiles do not fit
   // the apply copy (apply_keeps entries), worth a second copy only when the
   // dropped entries are a good part of P
@@ -3058,8 +3059,11 @@ __device__ __forceinline__ float2 df_in(double v, bool &out) {
   return make_float2(hi, lo);
 }
 
-// y = P x.  Rows longest first.
-template <int LB>
+// y = P x.  Rows longest first.  HOST: the output lies in host memory, and the
+// tile's rows are put together in shared memory and written in their order
+// (scattered by length, 3 vectors of 1.4M rows took 0.90 ms with the input's copy,
+// a copy of the result after the apply 0.33, this 0.30).
+template <int LB, bool HOST>
 __global__ void __launch_bounds__(TB_ROWS)
     k_df_tile(DfTiles D, bool scalar, const int *__restrict__ rp,
               const uint16_t *__restrict__ idx, const uint8_t *__restrict__ order,
@@ -3116,7 +3120,9 @@ __global__ void __launch_bounds__(TB_ROWS)
       const int v0 = c0 + 2 * l;
       double *yp = y + (r0 + lr) * nvec + v0;
       const double a = df_value(ah, al), b = df_value(bh, bl);
-      if (scalar) {
+      if (HOST) {
+        ((double2 *)(sx + (size_t)D.maxu * V))[lr * L + l] = make_double2(a, b);
+      } else if (scalar) {
         if (v0 < nvec) yp[0] = a;
         if (v0 + 1 < nvec) yp[1] = b;
       } else if (v0 < nvec) {
@@ -3124,6 +3130,14 @@ __global__ void __launch_bounds__(TB_ROWS)
       }
     }
     __syncthreads();
+    if (HOST) {
+      const double *so = (const double *)(sx + (size_t)D.maxu * V);
+      for (int i = t; i < nr * V; i += TB_ROWS) {
+        const int v = c0 + (i & (V - 1));
+        if (v < nvec) y[(r0 + (i >> (LB + 1))) * nvec + v] = so[i];
+      }
+      __syncthreads();
+    }
   }
   if (out) atomicOr(flags + 1, 1);
 }
@@ -3190,7 +3204,8 @@ __global__ void __launch_bounds__(TB_ROWS)
 __global__ void __launch_bounds__(256)
     k_df_pair_sum(long long cols, int nvec, const unsigned *__restrict__ cstart,
                   const float2 *__restrict__ part, double *__restrict__ y,
-                  const double *__restrict__ scale, const int *__restrict__ flags) {
+                  const double *__restrict__ scale, const double *__restrict__ recip,
+                  const int *__restrict__ flags) {
   if ((__ldg(flags) | __ldg(flags + 1)) != 0) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cols * nvec) return;
@@ -3205,7 +3220,7 @@ __global__ void __launch_bounds__(256)
   double r = df_value(sh, sl);
   if (scale) {
     // r / sc from the column's reciprocal and one correction
-    const double sc = scale[c], inv = scale[cols + c];
+    const double sc = scale[c], inv = recip[c];
     if (inv != 0.0) {
       const double q = __dmul_rn(r, inv);
       r = __fma_rn(__fma_rn(-q, sc, r), inv, q);
@@ -3537,29 +3552,37 @@ static int df_tile_lanes(int nvec) {
 static DfTiles df_tiles(const Interp &I, long long t0, long long t1, int nvec, const float2 *w) {
   return DfTiles{I.rows, t1 - t0, t0, nvec, I.tile_maxu, I.tile_uoff.p, I.tile_ucol.p, w};
 }
-// y = P x on tiles [t0, t1).
+// y = P x on tiles [t0, t1); host: y is page-locked host memory.
 static void df_tile_apply(const Interp &I, long long t0, long long t1, int nvec, const double *x,
-                          double *y, cudaStream_t s) {
+                          double *y, bool host, cudaStream_t s) {
   const bool scalar = nvec % 2 != 0 || ((uintptr_t)y % 16) != 0;
   const DfTiles D = df_tiles(I, t0, t1, nvec, I.ap_w.p);
   auto smem = [&](int lb) { return sizeof(float2) * ((size_t)I.tile_maxu << (lb + 1)); };
+  auto out = [&](int lb) { return host ? sizeof(double) * ((size_t)TB_ROWS << (lb + 1)) : 0; };
   int lb = df_tile_lanes(nvec);
   constexpr int most = 100 * 1024;
   while (lb > 0 && smem(lb) > most) lb--;  // tiles with many columns
   // (the attribute is the kernel's, for all threads: always the same)
-#define TMRG_DT(B)                                                                              \
-  do {                                                                                          \
-    TMRG_CUDA(cudaFuncSetAttribute(k_df_tile<B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                   most));                                                      \
-    launch(k_df_tile<B>, (unsigned)(t1 - t0), TB_ROWS, smem(B), s, D, scalar, I.ap_rowptr(),    \
-           (const uint16_t *)I.tile_idx.p, (const uint8_t *)I.tile_order.p, x, y, I.dfflag.p);  \
+#define TMRG_DT(B, H)                                                                            \
+  do {                                                                                           \
+    TMRG_CUDA(cudaFuncSetAttribute((k_df_tile<B, H>),                                            \
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
+                                   most + (H ? (int)sizeof(double) * TB_ROWS * 16 : 0)));        \
+    launch((k_df_tile<B, H>), (unsigned)(t1 - t0), TB_ROWS, smem(B) + out(B), s, D, scalar,      \
+           I.ap_rowptr(), (const uint16_t *)I.tile_idx.p, (const uint8_t *)I.tile_order.p, x, y, \
+           I.dfflag.p);                                                                          \
+  } while (0)
+#define TMRG_DTH(B) \
+  do {              \
+    if (host) TMRG_DT(B, true); else TMRG_DT(B, false); \
   } while (0)
   switch (lb) {
-    case 0: TMRG_DT(0); break;
-    case 1: TMRG_DT(1); break;
-    case 2: TMRG_DT(2); break;
-    default: TMRG_DT(3);
+    case 0: TMRG_DTH(0); break;
+    case 1: TMRG_DTH(1); break;
+    case 2: TMRG_DTH(2); break;
+    default: TMRG_DTH(3);
   }
+#undef TMRG_DTH
 #undef TMRG_DT
   const long long r0 = t0 * TB_ROWS, nr = std::min(I.rows, t1 * TB_ROWS) - r0;
   f64_pairs(nvec, nr, I.ap_rowptr() + r0, I.ap_colidx(), I.ap_w.p, I.tile_order.p + r0, nullptr,
@@ -3583,10 +3606,16 @@ static void df_tile_runs(const Interp &I, long long t0, long long t1, int nvec, 
   }
 #undef TMRG_DT
 }
-static void df_tile_columns(const Interp &I, int nvec, const float2 *part, const double *x,
-                            double *y, const double *scale, cudaStream_t s) {
-  launch(k_df_pair_sum, blocks_for(I.cols * nvec, 256), 256, 0, s, I.cols, nvec,
-         (const unsigned *)I.col_pairs.p, part, y, scale, (const int *)I.dfflag.p);
+static void df_tile_columns(const Interp &I, long long c0, long long c1, int nvec,
+                            const float2 *part, double *y, const double *scale, cudaStream_t s) {
+  if (c1 <= c0) return;
+  launch(k_df_pair_sum, blocks_for((c1 - c0) * nvec, 256), 256, 0, s, c1 - c0, nvec,
+         (const unsigned *)I.col_pairs.p + c0, part, y + c0 * nvec, scale ? scale + c0 : nullptr,
+         scale ? scale + I.cols + c0 : nullptr, (const int *)I.dfflag.p);
+}
+// The whole of y in FP64 where a flag asks for it.
+static void df_tile_columns_f64(const Interp &I, int nvec, const double *x, double *y,
+                                const double *scale, cudaStream_t s) {
   f64_pairs(nvec, I.cols, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, nullptr, I.t_perm.p, x, y, scale,
             I.dfflag.p, s);
 }
@@ -3632,86 +3661,23 @@ static void df_split_input(Interp &I, const double *x, long long nrows, int nvec
            I.dfflag.p + 1);
 }
 
-// Transpose apply with the input in host memory: the input rows are copied
-// in TC_CHUNKS pieces on a second stream.  With tiles, piece k's tiles are
-// summed as it arrives and the columns at the end.  Otherwise, after piece k
-// arrives (and is split into (hi, lo) pairs) the output rows whose inputs all
-// lie in pieces <= k are computed (t_perm holds the rows grouped that way), so
-// the copy of the next piece overlaps them.  Same kernel, rows and summation order
-// as the single apply; a piece with a value outside the double-float window
-// sends that piece's rows and every later piece's rows to FP64 (each row
-// only reads pieces already split, so a row never runs in double-float on
-// an input that was not represented).
-// Returns false (nothing done) where these kernels do not apply, or the apply of
-// device vectors takes others (the results are the same bits).
-// Reports (and clears) a TMA input stage of k_df_apply_tma that did not
-// complete within its wait limit; read where the host already waits.
-void interp_check_apply(Interp &I) {
-  if (read_scalar(I.dfflag.p + 2, I.s)) {
-    TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 2, 0, sizeof(int), I.s));
-    throw Error(TMRG_ERR_INTERNAL, "P apply: a staged input batch did not arrive");
-  }
-}
-
-bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, double *dx,
-                                   double *y, int nvec) {
-  if ((which != 1 && which != 2) || nvec % 2 != 0 || nvec / 2 < 8 ||
-      ((uintptr_t)dx % 16) != 0 || ((uintptr_t)y % 16) != 0 ||
-      (I.tile_t ? I.rows < DF_TILE_ROWS || tune_forced(TUNE_PT)
-                : (long long)I.t_chunk.size() != TC_CHUNKS + 1))
+// Whether the apply takes the tiles.
+static bool by_tiles(const Interp &I, int which, int nvec) {
+  if (f64_small(nvec, I.nnz_nz)) return false;
+  // tiles where they exist and one for every SM; P^T of 2 vectors is faster from
+  // its own rows (see k_df_tile), and a forced launch shape means the row kernels
+  if (!(I.rows >= DF_TILE_ROWS || (which != 0 && nvec < 15)) ||
+      tune_forced(which == 0 ? TUNE_P : TUNE_PT))
     return false;
-  Stage st("tmrg_interp_mult_transpose_staged");
-  cudaStream_t s = I.s;
-  if (which == 2) interp_colsum(I);
-  const long long nin = I.rows;
-  // the split input, or with tiles the runs' sums
-  DBuf<float2> xs((I.tile_t ? (long long)I.tile_runs.n : nin) * nvec + 1, s);
-  TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
-  cudaStream_t cs;
-  TMRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  cudaEvent_t ev[TC_CHUNKS + 1];
-  for (int k = 0; k <= TC_CHUNKS; k++)
-    TMRG_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
-  // the copies start after the work already queued on the forest stream
-  TMRG_CUDA(cudaEventRecord(ev[TC_CHUNKS], s));
-  TMRG_CUDA(cudaStreamWaitEvent(cs, ev[TC_CHUNKS], 0));
-  long long r0s[TC_CHUNKS + 1];
-  for (int k = 0; k <= TC_CHUNKS; k++) r0s[k] = (k * nin + TC_CHUNKS - 1) / TC_CHUNKS;
-  for (int k = 0; k < TC_CHUNKS; k++) {
-    const long long r0 = r0s[k], r1 = r0s[k + 1];
-    if (r1 > r0)
-      TMRG_CUDA(cudaMemcpyAsync(dx + r0 * nvec, xh + r0 * nvec, sizeof(double) * (r1 - r0) * nvec,
-                                cudaMemcpyHostToDevice, cs));
-    TMRG_CUDA(cudaEventRecord(ev[k], cs));
-  }
-  const double *sc = which == 2 ? (const double *)I.colsum.p : (const double *)nullptr;
-  // the tuned shape of the whole apply's class (the pieces are not tuned)
-  const int shape = tune_lookup(df_key(1, I.cols, I.nnz_nz, nvec / 2, false));
-  for (int k = 0; k < TC_CHUNKS; k++) {
-    TMRG_CUDA(cudaStreamWaitEvent(s, ev[k], 0));
-    const long long r0 = r0s[k], r1 = r0s[k + 1];
-    if (I.tile_t) {
-      // the tiles whose rows have all arrived with this piece
-      const long long t1 = (k + 1 < TC_CHUNKS ? r1 : nin + TB_ROWS - 1) / TB_ROWS;
-      df_tile_runs(I, r0 / TB_ROWS, t1, nvec, dx, xs.p, s);
-      continue;
-    }
-    if (r1 > r0)
-      launch(k_df_split_x, blocks_for((r1 - r0) * nvec, 256), 256, 0, s, (r1 - r0) * nvec,
-             (const double *)(dx + r0 * nvec), xs.p + r0 * nvec, I.dfflag.p + 1);
-    const long long a = I.t_chunk[k], n = I.t_chunk[k + 1] - a;
-    if (n > 0)
-      df_apply2(shape, n, nvec, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, xs.p, dx, y, sc,
-                I.t_perm.p + a, I.dfflag.p, s, nin);
-  }
-  if (I.tile_t) df_tile_columns(I, nvec, xs.p, dx, y, sc, s);
-  TMRG_CUDA(cudaStreamSynchronize(s));
-  for (int k = 0; k <= TC_CHUNKS; k++) cudaEventDestroy(ev[k]);
-  cudaStreamDestroy(cs);
-  interp_check_apply(I);
-  return true;
+  return which == 0 ? nvec > 1 && I.tile_ok : nvec > 2 && I.tile_t;
 }
 
+// Pieces of a host-buffer apply by tiles: four tiles for every SM in each (16
+// vectors in page-locked buffers, 366K rows: P 0.44 ms in two pieces, 0.43 in
+// four, 0.51 in 16; pageable ones 0.50, 0.59 and 1.08).
+static int tile_pieces(long long rows) {
+  return (int)std::min(64LL, (rows + TB_ROWS - 1) / TB_ROWS / (152 * 4));
+}
 // Largest column of each LO_WIN-row window of a column-sorted CSR (the last
 // entry of each row), -1 for a window of empty rows; wmax starts at -1.
 __global__ void k_win_maxcol(long long rows, const int *__restrict__ rp,
@@ -3728,9 +3694,115 @@ __global__ void k_win_maxcol(long long rows, const int *__restrict__ rp,
   if ((threadIdx.x & 31) == 0 && r < rows && m >= 0) atomicMax(wmax + r / LO_WIN, m);
 }
 
+// The same on the host, made on first use.
+static void window_last(long long rows, const int *rp, const int *ci, std::vector<int> &out,
+                        cudaStream_t s) {
+  const long long nwin = (rows + LO_WIN - 1) / LO_WIN;
+  if ((long long)out.size() == nwin) return;
+  DBuf<int> wm(nwin, s);
+  TMRG_CUDA(cudaMemsetAsync(wm.p, 0xff, sizeof(int) * nwin, s));
+  launch(k_win_maxcol, blocks_for(rows, 256), 256, 0, s, rows, rp, ci, wm.p);
+  out.resize(nwin);
+  TMRG_CUDA(cudaMemcpyAsync(out.data(), wm.p, sizeof(int) * nwin, cudaMemcpyDeviceToHost, s));
+  TMRG_CUDA(cudaStreamSynchronize(s));
+  g_host_syncs.fetch_add(1, std::memory_order_relaxed);
+}
+
+// Reports (and clears) a TMA input stage of k_df_apply_tma that did not
+// complete within its wait limit; read where the host already waits.
+void interp_check_apply(Interp &I) {
+  if (read_scalar(I.dfflag.p + 2, I.s)) {
+    TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 2, 0, sizeof(int), I.s));
+    throw Error(TMRG_ERR_INTERNAL, "P apply: a staged input batch did not arrive");
+  }
+}
+
+// Transpose apply with the input in host memory: the input rows are copied
+// in up to TC_CHUNKS pieces on a second stream.  With tiles, piece k's tiles are
+// summed as it arrives, and then the windows of columns that have all their
+// runs, so a page-locked result goes over the link meanwhile (1.4M rows, 16
+// vectors: all columns at the end 1.29 ms, so 1.17).  Otherwise, after piece k
+// arrives (and is split into (hi, lo) pairs) the output rows whose inputs all
+// lie in pieces <= k are computed (t_perm holds the rows grouped that way), so
+// the copy of the next piece overlaps them.  Same kernel, rows and summation order
+// as the single apply; a piece with a value outside the double-float window
+// sends that piece's rows and every later piece's rows to FP64 (each row
+// only reads pieces already split, so a row never runs in double-float on
+// an input that was not represented), with tiles all rows.
+// Returns false (nothing done) where these kernels do not apply, the apply of
+// device vectors takes others (the results are the same bits), or there are fewer
+// than two pieces.
+bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, double *dx,
+                                   double *y, int nvec) {
+  if (which != 1 && which != 2) return false;
+  const int pieces = I.tile_t ? std::min(TC_CHUNKS, tile_pieces(I.rows)) : TC_CHUNKS;
+  if (nvec < 16 || (I.tile_t ? pieces < 2 || !by_tiles(I, which, nvec)
+                             : df_scalar(nvec, dx, y) ||
+                                   (long long)I.t_chunk.size() != TC_CHUNKS + 1))
+    return false;
+  Stage st("tmrg_interp_mult_transpose_staged");
+  cudaStream_t s = I.s;
+  if (which == 2) interp_colsum(I);
+  const long long nin = I.rows;
+  // the split input, or with tiles the runs' sums
+  DBuf<float2> xs((I.tile_t ? (long long)I.tile_runs.n : nin) * nvec + 1, s);
+  TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
+  cudaStream_t cs;
+  TMRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+  cudaEvent_t ev[TC_CHUNKS + 1];
+  for (int k = 0; k <= pieces; k++)
+    TMRG_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
+  // the copies start after the work already queued on the forest stream
+  TMRG_CUDA(cudaEventRecord(ev[pieces], s));
+  TMRG_CUDA(cudaStreamWaitEvent(cs, ev[pieces], 0));
+  long long r0s[TC_CHUNKS + 1];
+  for (int k = 0; k <= pieces; k++) r0s[k] = (k * nin + pieces - 1) / pieces;
+  for (int k = 0; k < pieces; k++) {
+    const long long r0 = r0s[k], r1 = r0s[k + 1];
+    if (r1 > r0)
+      TMRG_CUDA(cudaMemcpyAsync(dx + r0 * nvec, xh + r0 * nvec, sizeof(double) * (r1 - r0) * nvec,
+                                cudaMemcpyHostToDevice, cs));
+    TMRG_CUDA(cudaEventRecord(ev[k], cs));
+  }
+  const double *sc = which == 2 ? (const double *)I.colsum.p : (const double *)nullptr;
+  // columns whose runs all lie in the pieces so far, window by window
+  const long long nwin = (I.cols + LO_WIN - 1) / LO_WIN;
+  long long summed = 0;
+  if (I.tile_t)
+    window_last(I.cols, I.t_rowptr.p, I.t_colidx.p, I.win_maxrow, s);
+  // the tuned shape of the whole apply's class (the pieces are not tuned)
+  const int shape = tune_lookup(df_key(1, I.cols, I.nnz_nz, nvec / 2, false));
+  for (int k = 0; k < pieces; k++) {
+    TMRG_CUDA(cudaStreamWaitEvent(s, ev[k], 0));
+    const long long r0 = r0s[k], r1 = r0s[k + 1];
+    if (I.tile_t) {
+      // the tiles whose rows have all arrived with this piece
+      const long long t1 = (k + 1 < pieces ? r1 : nin + TB_ROWS - 1) / TB_ROWS;
+      df_tile_runs(I, r0 / TB_ROWS, t1, nvec, dx, xs.p, s);
+      const long long w0 = summed;
+      while (summed < nwin && I.win_maxrow[summed] < t1 * TB_ROWS) summed++;
+      df_tile_columns(I, w0 * LO_WIN, std::min(I.cols, summed * LO_WIN), nvec, xs.p, y, sc, s);
+      continue;
+    }
+    if (r1 > r0)
+      launch(k_df_split_x, blocks_for((r1 - r0) * nvec, 256), 256, 0, s, (r1 - r0) * nvec,
+             (const double *)(dx + r0 * nvec), xs.p + r0 * nvec, I.dfflag.p + 1);
+    const long long a = I.t_chunk[k], n = I.t_chunk[k + 1] - a;
+    if (n > 0)
+      df_apply2(shape, n, nvec, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, xs.p, dx, y, sc,
+                I.t_perm.p + a, I.dfflag.p, s, nin);
+  }
+  if (I.tile_t) df_tile_columns_f64(I, nvec, dx, y, sc, s);
+  TMRG_CUDA(cudaStreamSynchronize(s));
+  for (int k = 0; k <= pieces; k++) cudaEventDestroy(ev[k]);
+  cudaStreamDestroy(cs);
+  interp_check_apply(I);
+  return true;
+}
+
 // Prolongation with the input and the output in host memory: the input
-// (coarse values) is copied in FC_CHUNKS column ranges on a second stream,
-// and the rows are computed in FC_CHUNKS pieces of whole 4096-row windows
+// (coarse values) is copied in column ranges on a second stream, and the rows are
+// computed in as many pieces (up to FC_CHUNKS) of whole 4096-row windows
 // (the length-ordered permutation stays inside a window, so a piece of
 // slots is exactly a piece of rows) into device memory, each piece as soon
 // as the input range holding its largest column has arrived and been split
@@ -3741,29 +3813,23 @@ __global__ void k_win_maxcol(long long rows, const int *__restrict__ rp,
 // it at less than half).  Same kernel, rows and summation order as the
 // single apply; as in the transpose, a range with a value outside the
 // double-float window sends the rows computed after its split to FP64.
-// Returns false (nothing done) where the pair kernel does not apply.
+// Returns false (nothing done) where the pair kernel or the tiles do not apply, or
+// there are fewer than two pieces.
 constexpr int FC_CHUNKS = 16;
 bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double *yh,
                                  int nvec) {
-  if (nvec % 2 != 0 || ((uintptr_t)dx % 16) != 0 || I.rows < (long long)LO_WIN * FC_CHUNKS ||
-      f64_small(nvec, I.nnz_nz) || (I.tile_ok && tune_forced(TUNE_P)))
+  const bool tiled = I.tile_ok;
+  if (nvec % 2 != 0 || I.rows < (long long)LO_WIN * FC_CHUNKS || f64_small(nvec, I.nnz_nz) ||
+      (tiled ? !by_tiles(I, 0, nvec) : ((uintptr_t)dx % 16) != 0))
     return false;
+  const long long rows = I.rows;
+  const int pieces = tiled ? std::min(FC_CHUNKS, tile_pieces(rows)) : FC_CHUNKS;
+  if (pieces < 2) return false;
   Stage st("tmrg_interp_mult_staged");
   cudaStream_t s = I.s;
-  const long long nin = I.cols, rows = I.rows;
+  const long long nin = I.cols;
   const long long nwin = (rows + LO_WIN - 1) / LO_WIN;
-  if ((long long)I.win_maxcol.size() != nwin) {
-    DBuf<int> wm(nwin, s);
-    TMRG_CUDA(cudaMemsetAsync(wm.p, 0xff, sizeof(int) * nwin, s));
-    launch(k_win_maxcol, blocks_for(rows, 256), 256, 0, s, rows, I.ap_rowptr(), I.ap_colidx(),
-           wm.p);
-    I.win_maxcol.resize(nwin);
-    TMRG_CUDA(cudaMemcpyAsync(I.win_maxcol.data(), wm.p, sizeof(int) * nwin,
-                              cudaMemcpyDeviceToHost, s));
-    TMRG_CUDA(cudaStreamSynchronize(s));
-    g_host_syncs.fetch_add(1, std::memory_order_relaxed);
-  }
-  const bool tiled = I.tile_ok;
+  window_last(rows, I.ap_rowptr(), I.ap_colidx(), I.win_maxcol, s);
   DBuf<float2> xs(tiled ? 0 : nin * nvec + 1, s);
   TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
   DBuf<double> dy(rows * nvec + 2, s);
@@ -3775,17 +3841,17 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
   TMRG_CUDA(cudaStreamCreateWithFlags(&is, cudaStreamNonBlocking));
   TMRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaEvent_t iev[FC_CHUNKS + 1], ev[FC_CHUNKS];
-  for (int k = 0; k <= FC_CHUNKS; k++)
+  for (int k = 0; k <= pieces; k++)
     TMRG_CUDA(cudaEventCreateWithFlags(&iev[k], cudaEventDisableTiming));
-  for (int k = 0; k < FC_CHUNKS; k++)
+  for (int k = 0; k < pieces; k++)
     TMRG_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
   // input ranges: columns [c0[j], c0[j + 1]), copied in order after the work
   // already queued on the forest stream
   long long c0[FC_CHUNKS + 1];
-  for (int j = 0; j <= FC_CHUNKS; j++) c0[j] = nin * j / FC_CHUNKS;
-  TMRG_CUDA(cudaEventRecord(iev[FC_CHUNKS], s));
-  TMRG_CUDA(cudaStreamWaitEvent(is, iev[FC_CHUNKS], 0));
-  for (int j = 0; j < FC_CHUNKS; j++) {
+  for (int j = 0; j <= pieces; j++) c0[j] = nin * j / pieces;
+  TMRG_CUDA(cudaEventRecord(iev[pieces], s));
+  TMRG_CUDA(cudaStreamWaitEvent(is, iev[pieces], 0));
+  for (int j = 0; j < pieces; j++) {
     if (c0[j + 1] > c0[j])
       TMRG_CUDA(cudaMemcpyAsync(dx + c0[j] * nvec, xh + c0[j] * nvec,
                                 sizeof(double) * (c0[j + 1] - c0[j]) * nvec,
@@ -3793,15 +3859,15 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
     TMRG_CUDA(cudaEventRecord(iev[j], is));
   }
   int split = 0;  // input ranges [0, split) are on the device and split
-  for (int k = 0; k < FC_CHUNKS; k++) {
-    const long long w0 = nwin * k / FC_CHUNKS, w1 = nwin * (k + 1) / FC_CHUNKS;
+  for (int k = 0; k < pieces; k++) {
+    const long long w0 = nwin * k / pieces, w1 = nwin * (k + 1) / pieces;
     const long long r0 = std::min(rows, w0 * LO_WIN), r1 = std::min(rows, w1 * LO_WIN);
     int need = -1;  // largest column the piece reads
     for (long long w = w0; w < w1; w++) need = std::max(need, I.win_maxcol[w]);
     // ranges up to the one holding `need` (all of them if a column were
     // out of range)
-    int upto = need < 0 ? 0 : FC_CHUNKS;
-    for (int j = 0; j < FC_CHUNKS && need >= 0; j++)
+    int upto = need < 0 ? 0 : pieces;
+    for (int j = 0; j < pieces && need >= 0; j++)
       if (need < c0[j + 1]) {
         upto = j + 1;
         break;
@@ -3818,7 +3884,7 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
     if (r1 > r0) {
       prof_bytes(12 * I.nnz_nz * (r1 - r0) / rows + 4 * (r1 - r0) + 8LL * nvec * (r1 - r0));
       if (tiled)
-        df_tile_apply(I, r0 / TB_ROWS, (r1 + TB_ROWS - 1) / TB_ROWS, nvec, dx, y, s);
+        df_tile_apply(I, r0 / TB_ROWS, (r1 + TB_ROWS - 1) / TB_ROWS, nvec, dx, y, false, s);
       else
         df_apply2(shape, r1 - r0, nvec, I.ap_rowptr(), I.ap_colidx(), I.ap_w.p, xs.p, dx, y,
                   nullptr, I.perm.p + r0, I.dfflag.p, s, nin);
@@ -3830,11 +3896,11 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
                                 cudaMemcpyDeviceToHost, cs));
   }
   // every input range is waited for before the call returns
-  for (; split < FC_CHUNKS; split++) TMRG_CUDA(cudaStreamWaitEvent(s, iev[split], 0));
+  for (; split < pieces; split++) TMRG_CUDA(cudaStreamWaitEvent(s, iev[split], 0));
   TMRG_CUDA(cudaStreamSynchronize(cs));
   TMRG_CUDA(cudaStreamSynchronize(s));
-  for (int k = 0; k <= FC_CHUNKS; k++) cudaEventDestroy(iev[k]);
-  for (int k = 0; k < FC_CHUNKS; k++) cudaEventDestroy(ev[k]);
+  for (int k = 0; k <= pieces; k++) cudaEventDestroy(iev[k]);
+  for (int k = 0; k < pieces; k++) cudaEventDestroy(ev[k]);
   cudaStreamDestroy(is);
   cudaStreamDestroy(cs);
   interp_check_apply(I);
@@ -3869,7 +3935,7 @@ static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, con
   return true;
 }
 
-void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
+void interp_apply(Interp &I, int which, const double *x, double *y, int nvec, bool host) {
   Stage st(which == 0 ? "tmrg_interp_mult" : "tmrg_interp_mult_transpose");
   if (nvec <= 0) throw Error(TMRG_ERR_ARG, "interp apply: nvec <= 0");
   cudaStream_t s = I.s;
@@ -3895,22 +3961,20 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec) {
                           (which == 2 ? 8 * nout : 0);
   if (f64_rows(nvec, nout, I.nnz_nz, rp, ci, w, x, y, sc, bytes, s)) return;
   TMRG_CUDA(cudaMemsetAsync(I.dfflag.p + 1, 0, sizeof(int), s));
-  // tiles where they exist and one for every SM; P^T of 2 vectors is faster from
-  // its own rows (see k_df_tile), and a forced launch shape means the row kernels
-  const bool free_shape = (I.rows >= DF_TILE_ROWS || (which != 0 && nvec < 15)) &&
-                          !tune_forced(which == 0 ? TUNE_P : TUNE_PT);
-  if (which == 0 && nvec > 1 && I.tile_ok && free_shape) {
+  const bool tiles = by_tiles(I, which, nvec);
+  if (tiles && which == 0) {
     prof_bytes(bytes - 2 * I.nnz_nz);
-    df_tile_apply(I, 0, (nout + TB_ROWS - 1) / TB_ROWS, nvec, x, y, s);
+    df_tile_apply(I, 0, (nout + TB_ROWS - 1) / TB_ROWS, nvec, x, y, host, s);
     return;
   }
-  if (which != 0 && nvec > 2 && I.tile_t && free_shape) {
+  if (tiles) {
     const long long np = (long long)I.tile_runs.n;
     DBuf<float2> part((size_t)np * nvec, s);
     prof_bytes(9 * I.nnz_nz + 8LL * nvec * (nin + np) + 14 * np);
     df_tile_runs(I, 0, (nin + TB_ROWS - 1) / TB_ROWS, nvec, x, part.p, s);
     prof_bytes(8LL * nvec * (np + nout) + (sc ? 8 * nout : 0));
-    df_tile_columns(I, nvec, part.p, x, y, sc, s);
+    df_tile_columns(I, 0, nout, nvec, part.p, y, sc, s);
+    df_tile_columns_f64(I, nvec, x, y, sc, s);
     return;
   }
   const int n2 = (nvec + 1) / 2;
