@@ -154,3 +154,94 @@ def test_unaligned_vectors_are_tuned_by_themselves(operators):
         assert len(keys) == 2 and len({k[:2] for k in keys}) == 1
     finally:
         lib.tmrg_tune_reset(1)
+
+
+def _applied(P):
+    """P without the numerically-zero weights, which the applies leave out."""
+    P = P.copy()
+    P.data[abs(P.data) < 2.0 ** -40] = 0.0
+    P.eliminate_zeros()
+    return P
+
+
+@pytest.mark.parametrize("nvec", [2, 3, 4, 5, 6, 7, 8, 9, 14])
+@pytest.mark.parametrize("shape", [0, 1, 2, 3])
+def test_narrow_launch_shapes(operators, nvec, shape):
+    # one to seven pairs, all at once in one to eight groups of lanes
+    import torch
+
+    from tests.test_gpu_apply_tiles import _bound
+    from tmr_gb300 import TMR
+    I, P = operators["large"]
+    P = _applied(P)
+    rng = np.random.default_rng(70 + nvec)
+    lib = TMR.lib()
+    try:
+        assert lib.tmrg_tune_force(1, shape) == 0 and lib.tmrg_tune_force(2, shape) == 0
+        for fn, A in ((I.mult, P), (I.multTranspose, P.T.tocsr())):
+            x = rng.standard_normal((A.shape[1], nvec))
+            for shift in (0, 1):
+                y = torch.full((A.shape[0] * nvec + shift,), float("nan"), dtype=torch.float64,
+                               device="cuda")[shift:]
+                fn(_on_device(x, shift), y)
+                assert np.all(abs(y.cpu().numpy().reshape(-1, nvec) - A @ x) <= _bound(A, x))
+    finally:
+        lib.tmrg_tune_force(1, -1)
+        lib.tmrg_tune_force(2, -1)
+
+
+@pytest.mark.parametrize("size", ["small", "large"])
+@pytest.mark.parametrize("nvec", [9, 15, 16, 17, 24, 31, 33])
+def test_counts_beyond_eight(operators, size, nvec):
+    # the FP64 rows in parts, and nine or more pairs at once
+    import torch
+
+    from tests.test_gpu_apply_tiles import _bound
+    I, P = operators[size]
+    P = _applied(P)
+    rng = np.random.default_rng(90 + nvec)
+    one = np.asarray(P.T @ np.ones(P.shape[0]))[:, None]
+    for fn, A, s in ((I.mult, P, 1.0), (I.multTranspose, P.T.tocsr(), 1.0),
+                     (I.multWeightTranspose, P.T.tocsr(), one)):
+        x = rng.standard_normal((A.shape[1], nvec))
+        y = torch.full((A.shape[0] * nvec,), float("nan"), dtype=torch.float64, device="cuda")
+        fn(_on_device(x, 0), y)
+        assert np.all(abs(y.cpu().numpy().reshape(-1, nvec) - (A @ x) / s) <= _bound(A, x) / s)
+
+
+def test_few_long_rows_cost_no_more_for_odd_counts(gpu_lib):
+    # P^T of quartic elements, 160 entries a row: 5 vectors within twice 4 (2.3
+    # times where the pairs were taken two at a time by two lanes)
+    import time
+
+    import torch
+
+    from tmr_gb300 import TMR
+    from tmr_gb300 import workloads as W
+    f = TMR.OctForest(order=4)
+    f.setConnectivity(W.brick(3, 2, 2))
+    f.createTrees(1)
+    for p in range(2):
+        f.refine(W.random_indicator(f.getNumOctants(), 7, p, 0.3), 0, 9)
+        f.balance(1)
+    f.createNodes()
+    c = f.coarsen()
+    c.balance(1)
+    c.createNodes()
+    I = TMR.VecInterp()
+    f.createInterpolation(c, I)
+    rows, cols, _ = I.sizes()
+    t = {}
+    for nvec in (4, 5):
+        x = torch.randn(rows * nvec, dtype=torch.float64, device="cuda")
+        y = torch.empty(cols * nvec, dtype=torch.float64, device="cuda")
+        best = []
+        for _ in range(8):
+            torch.cuda.synchronize()
+            a = time.perf_counter()
+            for _ in range(20):
+                I.multTranspose(x, y)
+            torch.cuda.synchronize()
+            best.append(time.perf_counter() - a)
+        t[nvec] = min(best[2:])
+    assert t[5] <= 2 * t[4] and t[5] < 20 * 250e-6

@@ -149,7 +149,8 @@ struct Interp {
   DBuf<float2> tile_w;
   DBuf<uint2> tile_runs;
   DBuf<unsigned> col_pairs;
-  DBuf<int> perm;  // apply rows ordered by length inside windows (without tiles)
+  DBuf<int> perm;  // apply rows ordered by length inside windows (where the pair
+                   // kernels may take them)
   DBuf<int> t_rowptr, t_colidx;  // P^T (zero-free) as CSR, rows = coarse nodes
   DBuf<int> t_perm;  // P^T rows by input chunk of their last entry, then length
   std::vector<long long> t_chunk;  // t_perm range of each input chunk

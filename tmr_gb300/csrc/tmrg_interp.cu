@@ -1140,7 +1140,8 @@ __global__ void k_df_split_odd(long long rows, int nvec, const double *__restric
                                int *flag) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * (nvec + 1)) return;
-  const long long r = i / (nvec + 1);
+  const long long r = (unsigned long long)i >> 32 ? i / (nvec + 1)
+                                                  : (unsigned)i / (unsigned)(nvec + 1);
   const int v = (int)(i - r * (nvec + 1));
   float hi = 0.0f, lo = 0.0f;
   if (v < nvec && !df_split(__ldg(x + r * nvec + v), DF_X_EMIN, DF_X_ERANGE, hi, lo))
@@ -1205,6 +1206,18 @@ __global__ void k_nz_fill(long long rows, const int *__restrict__ rp,
 // three radix passes over them and a gather of the weights; with the applies by
 // tiles below, three levels of a quadratic mesh went from 143.8 to 121.4 ms.
 constexpr int TB_ROWS = 256;
+// Rows from which the tiles are taken: a tile is a block, and fewer of them than
+// the SMs can hold leave the chip idle where the pair kernels' rows fill it.  By
+// rows (d) against by tiles (t), us: P of 2 to 8 vectors, one tile an SM: 72K
+// rows, 4 vectors d 18.2, t 15.2; 17K rows, 8 vectors d 16.1, t 17.8.  P of more,
+// five: 138K rows, 16 vectors d 26.4, t 29.2; 233K rows d 36.1, t 35.4.  P^T, eight:
+// 233K rows, 4 and 16 vectors d 20.2 and 40.4, t 25.6 and 39.9; 365K rows d 48.3
+// and 133.5, t 47.0 and 98.3.
+constexpr long long DF_TILE_ROWS = 152LL * TB_ROWS;
+static long long df_tile_rows(int which, int nvec) {
+  return DF_TILE_ROWS * (which != 0 ? 8 : nvec > 8 ? 5 : 1);
+}
+
 // Slots of a tile's column table (a power of two), columns it may hold and
 // entries it may have: the second size for tiles that need it, and beyond
 // that the sort of all entries.
@@ -2406,7 +2419,8 @@ void interp_finish(Interp &I, long long nonzeros, cudaStream_t s, const long lon
   if (!transpose_tiles(I, keepoff, s)) transpose_sorted(I, keepoff, s);
   nzoff.release();
 
-  if (!I.tile_ok) {
+  // (for the pair kernels, see df_tile_rows)
+  if (!I.tile_ok || rows < df_tile_rows(0, 9)) {
     I.perm.alloc(rows + 1, s);
     launch(k_len_order, blocks_for(rows, LO_WIN), LO_THREADS, 0, s, rows, I.ap_rowptr(),
            (const int *)nullptr, I.perm.p);
@@ -2670,18 +2684,21 @@ static void interp_colsum(Interp &I) {
 // divided by scale[row] (weight-normalised transpose).
 
 // A small matrix, in FP64 straight from the caller's vectors: 2^LB lanes per
-// row take its entries in turn, each with all NV components, and combine in a
-// fixed tree.  One launch instead of a flag reset, a pass that splits the input
-// and an apply; no window on the values.
-template <int NV>
+// row take its entries in turn, each with NV components (of nvec, from NV
+// blockIdx.y; PART: the last of them may be fewer), and combine in a fixed tree.
+// One launch instead of a flag reset, a pass that splits the input and an
+// apply; no window on the values.
+template <int NV, bool PART>
 __global__ void __launch_bounds__(256)
-    k_f64_rows(long long rows, int LB, const int *__restrict__ rowptr,
+    k_f64_rows(long long rows, int LB, int nvec, const int *__restrict__ rowptr,
                const int *__restrict__ cols, const float2 *__restrict__ w,
                const double *__restrict__ x, double *__restrict__ y,
                const double *__restrict__ scale) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long r = t >> LB;
   const int L = 1 << LB, l = (int)t & (L - 1);
+  const int nv = PART ? nvec : NV, c0 = PART ? NV * (int)blockIdx.y : 0;
+  const int nc = PART ? min(NV, nv - c0) : NV;
   const bool have = r < rows;
   const int p0 = have ? __ldg(rowptr + r) : 0, p1 = have ? __ldg(rowptr + r + 1) : 0;
   double acc[NV];
@@ -2690,10 +2707,11 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 2
   for (int p = p0 + l; p < p1; p += L) {
     const float2 wv = __ldg(w + p);
-    const double *xr = x + (long long)__ldg(cols + p) * NV;
+    const double *xr = x + (long long)__ldg(cols + p) * nv + c0;
     const double wd = df_value(wv.x, wv.y);
 #pragma unroll
-    for (int v = 0; v < NV; v++) acc[v] = __fma_rn(wd, __ldg(xr + v), acc[v]);
+    for (int v = 0; v < NV; v++)
+      if (v < nc) acc[v] = __fma_rn(wd, __ldg(xr + v), acc[v]);
   }
   for (int o = L >> 1; o > 0; o >>= 1)
 #pragma unroll
@@ -2705,7 +2723,7 @@ __global__ void __launch_bounds__(256)
   for (int v = 0; v < NV; v++) {
     double a = acc[v];
     if (scale) a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
-    y[r * NV + v] = a;
+    if (v < nc) y[r * nv + c0 + v] = a;
   }
 }
 
@@ -3464,9 +3482,10 @@ static bool tma_apply(long long rows, long long nin, const int *rp, const int *c
 // come from the length-ordered permutation.
 // 8 or more pairs (16+ vectors): {8,1,1} {8,2,1} {8,4,1} {4,1,2} {2,1,4}
 // {1,1,8}, and for exactly 8 pairs {2,1,4} with TMA-staged inputs
-// (k_df_apply_tma); fewer pairs: LPR = pairs rounded down to a power of
-// two, NG 1 or 2
-constexpr int DF2_SHAPES_WIDE = 7, DF2_SHAPES_NARROW = 2;
+// (k_df_apply_tma); fewer pairs: LPR PPL pairs at once, all of them, NG 1, 2, 4
+// or 8 (few long rows: P^T of 157 entries a row, 8K rows: 5 vectors 515 -> 83 us
+// with two more NG and all three pairs at once)
+constexpr int DF2_SHAPES_WIDE = 7, DF2_SHAPES_NARROW = 4;
 // Whether the pair kernels take the caller's vectors value by value: an odd
 // number of them, or buffers off the 16-byte grid.
 static bool df_scalar(int nvec, const double *x, const double *y) {
@@ -3491,29 +3510,36 @@ static void df_apply2(int shape, long long rows, int nvec, const int *rp, const 
     if (scalar) TMRG_DF2S(L, N, P, true); else TMRG_DF2S(L, N, P, false); \
   } while (0)
   if (nvec2 >= 8) {
+    // 9 to 16 pairs at once
+    const bool two = nvec2 > 8;
     switch (shape) {
-      case 0: TMRG_DF2(8, 1, 1); break;
-      case 1: TMRG_DF2(8, 2, 1); break;
-      case 2: TMRG_DF2(8, 4, 1); break;
+      case 0: if (two) TMRG_DF2(8, 1, 2); else TMRG_DF2(8, 1, 1); break;
+      case 1: if (two) TMRG_DF2(8, 2, 2); else TMRG_DF2(8, 2, 1); break;
+      case 2: if (two) TMRG_DF2(8, 4, 2); else TMRG_DF2(8, 4, 1); break;
       case 3: TMRG_DF2(4, 1, 2); break;
       case 5: TMRG_DF2(1, 1, 8); break;
       default: TMRG_DF2(2, 1, 4);  // 4, and 6 where the staged kernel does not apply
     }
-  } else if (nvec2 >= 4) {
-    if (shape == 0)
-      TMRG_DF2(4, 1, 1);
-    else
-      TMRG_DF2(4, 2, 1);
-  } else if (nvec2 >= 2) {
-    if (shape == 0)
-      TMRG_DF2(2, 1, 1);
-    else
-      TMRG_DF2(2, 2, 1);
   } else {
-    if (shape == 0)
-      TMRG_DF2(1, 1, 1);
-    else
-      TMRG_DF2(1, 2, 1);
+#define TMRG_DF2N(L, P)                    \
+  switch (shape) {                         \
+    case 0: TMRG_DF2(L, 1, P); break;      \
+    case 1: TMRG_DF2(L, 2, P); break;      \
+    case 2: TMRG_DF2(L, 4, P); break;      \
+    default: TMRG_DF2(L, 8, P);            \
+  }
+    if (nvec2 == 1) {
+      TMRG_DF2N(1, 1);
+    } else if (nvec2 == 2) {
+      TMRG_DF2N(2, 1);
+    } else if (nvec2 == 3) {
+      TMRG_DF2N(2, 2);
+    } else if (nvec2 == 4) {
+      TMRG_DF2N(4, 1);
+    } else {
+      TMRG_DF2N(4, 2);
+    }
+#undef TMRG_DF2N
   }
 #undef TMRG_DF2
 #undef TMRG_DF2S
@@ -3630,23 +3656,14 @@ static TuneKey df_key(int which, long long rows, long long nnz, int nvec2, bool 
   return TuneKey{which == 0 ? TUNE_P : TUNE_PT, std::min(nvec2, 8), lr, q, scalar ? 1 : 0, 0};
 }
 
-// The FP64 apply (k_f64_rows) where it is the faster one: up to 8 vectors and
-// F64_ROWS_MAX entries x vectors, where launches count and the FP64 pipe does
-// not yet.  Measured per apply, split pass and double-float apply against
-// this kernel: 27K entries, 1 to 8 vectors 16-20 -> 10-12 us; 476K entries, 1
-// vector 16 -> 12 us, 2 vectors 19 -> 16 us, 3 vectors 20 -> 19 us, 4 vectors
-// 19 against 23 us; 4.8M entries, 1 vector 37 against 65 us.
+// The FP64 apply (k_f64_rows) where it is the faster one: entries x (vectors + 1
+// for the weight) up to a line, where launches count and the FP64 pipe does not
+// yet.  Per apply, one after another, split pass and double-float apply against
+// this kernel: 53K entries, 1 / 9 / 17 vectors 14.3 / 15.6 / 15.9 -> 9.7 / 10.0 /
+// 14.8 us; 478K entries, 1 vector 15.9 -> 12.9 us; above the line, 610K entries, 1
+// vector 15.6 against 20.8 us, 478K entries, 2 vectors 16.0 against 18.9 us.
 constexpr long long F64_ROWS_MAX = 1000000;
-static bool f64_small(int nvec, long long nnz) {
-  return nvec <= 8 && nnz * nvec <= F64_ROWS_MAX;
-}
-// Rows below which P, and P^T with the wide shapes (15 vectors or more), go by
-// rows: a tile is a block, and fewer of them than SMs leave some idle.  16
-// vectors by tiles and by rows: 27K entries P 18.4 and 15.9 us, P^T 24.9 and
-// 15.7; 80K entries 23.6 and 15.7, 36.1 and 28.1; above the line, 610K entries,
-// 28.8 and 34.4, 42 and 106.  P^T of 10 vectors, 80K entries, takes 86 us by rows.
-constexpr long long DF_TILE_ROWS = 152LL * TB_ROWS;
-
+static bool f64_small(int nvec, long long nnz) { return nnz * (nvec + 1) <= F64_ROWS_MAX; }
 // The input as (hi, lo) pairs in pool memory, with its window flag; an odd
 // number of vectors gets one more, zero.
 static void df_split_input(Interp &I, const double *x, long long nrows, int nvec,
@@ -3664,10 +3681,9 @@ static void df_split_input(Interp &I, const double *x, long long nrows, int nvec
 // Whether the apply takes the tiles.
 static bool by_tiles(const Interp &I, int which, int nvec) {
   if (f64_small(nvec, I.nnz_nz)) return false;
-  // tiles where they exist and one for every SM; P^T of 2 vectors is faster from
-  // its own rows (see k_df_tile), and a forced launch shape means the row kernels
-  if (!(I.rows >= DF_TILE_ROWS || (which != 0 && nvec < 15)) ||
-      tune_forced(which == 0 ? TUNE_P : TUNE_PT))
+  // (P^T of 2 vectors is faster from its own rows, see k_df_tile; a forced launch
+  // shape means the row kernels)
+  if (I.rows < df_tile_rows(which, nvec) || tune_forced(which == 0 ? TUNE_P : TUNE_PT))
     return false;
   return which == 0 ? nvec > 1 && I.tile_ok : nvec > 2 && I.tile_t;
 }
@@ -3915,21 +3931,24 @@ static bool f64_rows(int nvec, long long rows, long long nnz, const int *rp, con
   int lb = 0;
   while (lb < 4 && (6LL << lb) * rows <= 2 * nnz) lb++;
   prof_bytes(bytes);
-  const unsigned g = blocks_for(rows << lb, 256);
-  switch (nvec) {
-#define TMRG_F64(V)                                                                     \
-  case V:                                                                               \
-    launch(k_f64_rows<V>, g, 256, 0, s, rows, lb, rp, ci, w, x, y, scale);              \
-    break
-    TMRG_F64(1);
-    TMRG_F64(2);
-    TMRG_F64(3);
-    TMRG_F64(4);
-    TMRG_F64(5);
-    TMRG_F64(6);
-    TMRG_F64(7);
-    default:
-      launch(k_f64_rows<8>, g, 256, 0, s, rows, lb, rp, ci, w, x, y, scale);
+  // more than 8 vectors in equal parts of at most 8
+  const int parts = (nvec + 7) / 8;
+  const dim3 g(blocks_for(rows << lb, 256), (unsigned)parts);
+  switch ((nvec + parts - 1) / parts) {
+#define TMRG_F64(V)                                                                       \
+  if (parts == 1)                                                                         \
+    launch((k_f64_rows<V, false>), g, 256, 0, s, rows, lb, nvec, rp, ci, w, x, y, scale); \
+  else                                                                                    \
+    launch((k_f64_rows<V, true>), g, 256, 0, s, rows, lb, nvec, rp, ci, w, x, y, scale);  \
+  break
+    case 1: TMRG_F64(1);
+    case 2: TMRG_F64(2);
+    case 3: TMRG_F64(3);
+    case 4: TMRG_F64(4);
+    case 5: TMRG_F64(5);
+    case 6: TMRG_F64(6);
+    case 7: TMRG_F64(7);
+    default: TMRG_F64(8);
 #undef TMRG_F64
   }
   return true;
@@ -3985,7 +4004,10 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec, bo
     // lanes per row by the mean row length: 1 below 10 entries (8.5: 471 us
     // against 514 with 2, 117M entries), 2 below 24 (13.9: 35 us against 47
     // with 1), then 4 (35.5: 593 us against 645 with 2 and 629 with 8)
-    const int lb = I.nnz_nz < 10 * nout ? 0 : I.nnz_nz < 24 * nout ? 1 : 2;
+    int lb = I.nnz_nz < 10 * nout ? 0 : I.nnz_nz < 24 * nout ? 1 : 2;
+    // few long rows: more lanes each, while they do not fill the chip (P^T of
+    // 157 entries a row, 8K rows: 109 -> 26 us; 38 a row, 16K rows: 26 -> 18)
+    while (lb < 5 && nout << lb < 152LL * 2048 && I.nnz_nz > (8LL << lb) * nout) lb++;
     launch(k_df_one, blocks_for(nout << lb, 256), 256, 0, s, nout, lb, rp, ci, w,
            (const float2 *)xs.p, x, y, sc, (const int *)I.dfflag.p);
     return;
