@@ -256,3 +256,32 @@ def test_page_locked_odd_counts_cost_what_even_ones_do(gpu_lib):
             best.append(time.perf_counter() - a)
         t[nvec] = min(best[4:])
     assert t[3] <= 1.3 * t[4]
+
+
+def test_rows_too_long_for_any_tile_are_sorted_at_once(gpu_lib):
+    # quartic elements: over 32 entries a row, which no tile holds; the tiles
+    # are not tried
+    import ctypes
+    import json
+
+    from tmr_gb300 import TMR
+    from tmr_gb300 import workloads as W
+    f = TMR.OctForest(order=4)
+    f.setConnectivity(W.brick(3, 2, 2))
+    f.createTrees(1)
+    for p in range(2):
+        f.refine(W.random_indicator(f.getNumOctants(), 7, p, 0.3), 0, 9)
+        f.balance(1)
+    f.createNodes()
+    c = f.coarsen()
+    c.balance(1)
+    c.createNodes()
+    I = TMR.VecInterp()
+    lib = TMR.lib()
+    lib.tmrg_profile_begin()
+    f.createInterpolation(c, I)
+    buf = ctypes.create_string_buffer(1 << 20)
+    assert lib.tmrg_profile_end(buf, len(buf)) == 0
+    rows, cols, nnz = I.sizes()
+    assert I.applyNnz() > 32 * rows
+    assert not [k for k in json.loads(buf.value.decode()) if "k_tb_build" in k]

@@ -1254,7 +1254,7 @@ __global__ void __launch_bounds__(TB_ROWS)
   uint16_t *eslot = rank + Z.slots;                   // per entry: slot, and row
   uint8_t *erow = (uint8_t *)(eslot + Z.entries);
   constexpr int LB = 64;  // row lengths told apart (longer ones are one class)
-  __shared__ int s_rp[TB_ROWS + 1], s_new, s_empty, s_kept[TB_ROWS / 32], s_len[LB];
+  __shared__ int s_rp[TB_ROWS + 1], s_new, s_empty, s_kept[TB_ROWS / 32], s_len[LB], s_stop;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const long long r0 = (long long)blockIdx.x * TB_ROWS;
   const int nr = (int)min((long long)TB_ROWS, rows - r0);
@@ -1273,8 +1273,12 @@ __global__ void __launch_bounds__(TB_ROWS)
     }
   }
   for (int i = t; i < Z.slots; i += TB_ROWS) tab[i] = -1;
-  if (t == 0) s_new = s_empty = 0;
+  if (t == 0) {
+    s_new = s_empty = 0;
+    s_stop = *(volatile int *)state;  // some tile does not fit: all for nothing
+  }
   __syncthreads();
+  if (s_stop) return;
   if (t < nr && s_rp[t] == s_rp[t + 1]) s_empty = 1;
   int mylen = 0;
   if (t < nr)
@@ -2269,6 +2273,8 @@ static bool transpose_tiles(Interp &I, const long long *keepoff, cudaStream_t s)
   I.tile_ok = I.tile_t = false;
   if (rows == 0 || nnz == 0) return false;
   const long long tiles = (rows + TB_ROWS - 1) / TB_ROWS;
+  // more entries than that many tiles hold: some tile has too many
+  if (nnz > tiles * TB_SIZES[1].entries) return false;
   DBuf<unsigned> &ucount = I.tile_uoff;
   ucount.alloc(tiles + 1, s);
   I.tile_order.alloc(tiles * TB_ROWS, s);
@@ -2282,6 +2288,7 @@ static bool transpose_tiles(Interp &I, const long long *keepoff, cudaStream_t s)
   idx.alloc(nnz, s);
   long long np = -1;
   for (const TbSize &Z : TB_SIZES) {
+    if (nnz > tiles * Z.entries) continue;
     const size_t smem = tb_smem(Z);
     TMRG_CUDA(cudaFuncSetAttribute(k_tb_build<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)tb_smem(TB_SIZES[1])));
