@@ -127,10 +127,14 @@ __device__ __forceinline__ int refine_target(const RefineArgs &a, int r,
 }
 
 // state[0]: finest target level, state[1]: some octant coarsens or refines
-// by more than one level.
+// by more than one level, state[2]: octants that the general path emits.
 __global__ void k_refine_levels(long long n, RefineArgs a, const int16_t *__restrict__ lev,
                                 int *state) {
+  __shared__ int s_ml;
+  __shared__ unsigned s_total;
+  if (threadIdx.x == 0) s_ml = 0, s_total = 0u;
   int ml = 0;
+  unsigned total = 0;
   bool general = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -138,12 +142,20 @@ __global__ void k_refine_levels(long long n, RefineArgs a, const int16_t *__rest
     const int l = lev[i], nl = refine_target(a, a.ref ? a.ref[i] : 1, l, reps);
     ml = max(ml, nl);
     general |= nl < l || reps > 1;
+    total += (unsigned)(reps * reps * reps);
   }
   ml = __reduce_max_sync(0xffffffffu, ml);
-  general = __any_sync(0xffffffffu, general);
+  total = __reduce_add_sync(0xffffffffu, total);
+  general = __syncthreads_or(general);
   if ((threadIdx.x & 31) == 0) {
-    if (ml > 0) atomicMax(state, ml);
+    atomicMax(&s_ml, ml);
+    atomicAdd(&s_total, total);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_ml > 0) atomicMax(state, s_ml);
     if (general) atomicOr(state + 1, 1);
+    atomicAdd((unsigned *)state + 2, s_total);
   }
 }
 // Every octant stays or becomes the child-0 seed of its refinement, which
@@ -285,20 +297,18 @@ void forest_refine(Forest &f, const int *d_ref, long long nref, int min_level,
   if (n == 0) return;
   cudaStream_t s = f.s;
   RefineArgs a{d_ref, min_level, max_level};
-  DBuf<int> state(2, s);
+  DBuf<int> state(4, s);
   state.zero();
   launch(k_refine_levels, std::min(blocks_for(n, 256), 152u * 8), 256, 0, s, n, a,
          (const int16_t *)f.level.p, state.p);
-  const int *dst[2] = {state.p, state.p + 1};
-  int hst[2];
-  read_scalars(dst, hst, s);
-  f.maxlev = std::max(hst[0], 0);
+  const int4 hst = read_scalar((const int4 *)state.p, s);  // one wait for all of it
+  f.maxlev = std::max(hst.x, 0);
   const OctKey K = f.oct_key();
   // Nothing coarsens and nothing refines by several levels (an indicator of
   // zeros and ones, or no indicator): one pass over levels and infos, 10
   // bytes an octant.  The general path sorts every emitted key and costs
   // about 100 bytes an octant and 20 launches.
-  if (!hst[1]) {
+  if (!hst.y) {
     launch(k_refine_in_place, blocks_for(n, 256), 256, 0, s, n, a, f.level.p, f.info.p);
     return;
   }
@@ -306,7 +316,7 @@ void forest_refine(Forest &f, const int *d_ref, long long nref, int min_level,
   launch(k_refine_count, blocks_for(n, 256), 256, 0, s, n, a, (const int16_t *)f.level.p,
          cnt.p);
   exclusive_scan<unsigned>(cnt.p, cnt.p, n, s);
-  unsigned total = read_scalar(cnt.p + n, s);
+  const unsigned total = (unsigned)hst.z;
   if (K.total_bits() > 64)
     refine_sort_compact<U128>(f, a, key_as<U128>(K), cnt, total);
   else

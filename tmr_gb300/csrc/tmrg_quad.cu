@@ -454,10 +454,15 @@ __device__ __forceinline__ int q_refine_target(const QRefineArgs &a, int r, int 
   return level;
 }
 // state[0]: finest target level, state[1]: some quadrant coarsens or refines
-// by more than one level (the octree's k_refine_levels).
+// by more than one level, state[2]: quadrants that the general path emits (the
+// octree's k_refine_levels).
 __global__ void k_q_refine_levels(long long n, QRefineArgs a, const int16_t *__restrict__ lev,
                                   int *state) {
+  __shared__ int s_ml;
+  __shared__ unsigned s_total;
+  if (threadIdx.x == 0) s_ml = 0, s_total = 0u;
   int ml = 0;
+  unsigned total = 0;
   bool general = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -465,12 +470,20 @@ __global__ void k_q_refine_levels(long long n, QRefineArgs a, const int16_t *__r
     const int l = lev[i], nl = q_refine_target(a, a.ref ? a.ref[i] : 1, l, reps);
     ml = max(ml, nl);
     general |= nl < l || reps > 1;
+    total += (unsigned)(reps * reps);
   }
   ml = __reduce_max_sync(0xffffffffu, ml);
-  general = __any_sync(0xffffffffu, general);
+  total = __reduce_add_sync(0xffffffffu, total);
+  general = __syncthreads_or(general);
   if ((threadIdx.x & 31) == 0) {
-    if (ml > 0) atomicMax(state, ml);
+    atomicMax(&s_ml, ml);
+    atomicAdd(&s_total, total);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_ml > 0) atomicMax(state, s_ml);
     if (general) atomicOr(state + 1, 1);
+    atomicAdd((unsigned *)state + 2, s_total);
   }
 }
 // Every quadrant stays or becomes the child-0 seed of its refinement, at its
@@ -587,17 +600,15 @@ void qforest_refine(QForest &f, const int *d_ref, long long nref, int min_level,
   if (n == 0) return;
   cudaStream_t s = f.s;
   QRefineArgs a{d_ref, min_level, max_level};
-  DBuf<int> state(2, s);
+  DBuf<int> state(4, s);
   state.zero();
   launch(k_q_refine_levels, std::min(blocks_for(n, 256), 152u * 8), 256, 0, s, n, a,
          (const int16_t *)f.level.p, state.p);
-  const int *dst[2] = {state.p, state.p + 1};
-  int hst[2];
-  read_scalars(dst, hst, s);
-  f.maxlev = std::max(f.maxlev, std::max(hst[0], 0));
+  const int4 hst = read_scalar((const int4 *)state.p, s);  // one wait for all of it
+  f.maxlev = std::max(f.maxlev, std::max(hst.x, 0));
   const QKey K = f.key();
   // as in the octree's refine: no sort where every quadrant keeps its anchor
-  if (!hst[1]) {
+  if (!hst.y) {
     launch(k_q_refine_in_place, blocks_for(n, 256), 256, 0, s, n, a, f.level.p, f.info.p);
     return;
   }
@@ -605,7 +616,7 @@ void qforest_refine(QForest &f, const int *d_ref, long long nref, int min_level,
   launch(k_q_refine_count, blocks_for(n, 256), 256, 0, s, n, a, (const int16_t *)f.level.p,
          cnt.p);
   exclusive_scan<unsigned>(cnt.p, cnt.p, n, s);
-  const unsigned total = read_scalar(cnt.p + n, s);
+  const unsigned total = (unsigned)hst.z;
   if (K.total_bits() > 64)
     q_refine_sort_compact<U128>(f, a, qkey_as<U128>(K), cnt, total);
   else
