@@ -174,22 +174,37 @@ def test_terms_of_a_tile_with_too_many_columns(gpu_lib):
                 1e-12 * np.abs(want).max())
 
 
-@pytest.mark.parametrize("k", [2040, 2047, 2048, 2100])
-def test_rows_of_more_columns_than_any_table(gpu_lib, k):
+def _fan_forest(TMR, k, extra):
+    """k blocks around an edge, and `extra` beside them: 8 uniform blocks of
+    4096 octants, which take the matrix over the line to the row assembly."""
+    from tests.test_gpu_balance_paths import _union
+    f = TMR.OctForest(order=2)
+    f.setConnectivity(_union([_fan(k), W.brick(2, 2, 2)]) if extra else _fan(k))
+    f.createTrees(0)
+    for _ in range(4 if extra else 0):
+        f.refine((f.getOctantsArray()[:, 0] >= k).astype(np.intc), 0, 4)
+        f.balance(1)
+    f.createNodes()
+    assert (f.getNumOctants() * 64 > 2_000_000) == extra
+    return f
+
+
+@pytest.mark.parametrize("extra", [False, True])
+@pytest.mark.parametrize("k", [7, 100, 300, 2040, 2047, 2048, 2100])
+def test_rows_of_more_columns_than_any_table(gpu_lib, k, extra):
     # a node in k blocks has 4 k + 2 columns; above 8192 the entries are
     # sorted.  M 1 is the volume around each node
     from tmr_gb300 import TMR
-    f = TMR.OctForest(order=2)
-    f.setConnectivity(_fan(k))
-    f.createTrees(0)
-    f.createNodes()
-    n = int(f.getNodeRange()[1])
+    f = _fan_forest(TMR, k, extra)
+    n = 4 * k + 2
     F = TMR.MatrixFilter(0.5, 3, None, [f])
     rp, c, v, _, _, _ = F.getMatrix()
-    assert n == 4 * k + 2 and rp[1] - rp[0] == n
+    assert rp[1] - rp[0] == n
     assert all(np.all(np.diff(c[rp[i]:rp[i + 1]]) > 0) for i in range(0, n, 97))
     D = np.add.reduceat(v, rp[:-1])
-    vol = np.bincount(f.getMeshConn().reshape(-1), minlength=n) / 8.0
+    conn = f.getMeshConn()
+    lev = f.getOctantsArray()[:, 5]
+    vol = np.bincount(conn.reshape(-1), np.repeat(0.125 ** lev, 8), minlength=len(D)) / 8.0
     # sums of at most 8 k + 4 products of positive numbers
     np.testing.assert_allclose(D, vol, rtol=1e-12)
     # the entry of the axis with itself: k corners of 1/27
@@ -218,3 +233,37 @@ def test_filter_of_many_quadrants(gpu_lib):
     F.applyFilter(x, y)
     # the filter keeps constants: rounding of a two-term sum
     assert float((y - 1).abs().max()) < 1e-12
+
+
+@pytest.mark.parametrize("dim", [3, 2])
+def test_sorted_and_row_assembly_agree(gpu_lib, dim):
+    # a small mesh, whose entries are sorted, beside uniform blocks that take
+    # the matrix over the line to the rows: the same bits
+    from tests.test_gpu_balance_paths import _union
+    from tmr_gb300 import TMR
+    base = W.rotate_blocks(W.brick(2, 2, 1), 4) if dim == 3 else W.brick2d(3, 2)
+    extra = W.brick(2, 2, 2) if dim == 3 else W.brick2d(3, 3)
+    depth = 4 if dim == 3 else 7
+    got = []
+    for conn in (base, _union([base, extra])):
+        f = (TMR.OctForest if dim == 3 else TMR.QuadForest)(order=2)
+        f.setConnectivity(conn)
+        f.createTrees(1)
+        for p in range(depth - 1):
+            a = f.getOctantsArray() if dim == 3 else f.getQuadrantsArray()
+            mine = a[:, 0] < len(base)
+            flags = np.zeros(len(a), np.intc)
+            flags[mine] = W.uniform(21, p, int(mine.sum())) < (0.3 if p < 3 else 0.0)
+            flags[~mine] = 1
+            f.refine(flags, 0, depth)
+            f.balance(1)
+        f.createNodes()
+        a = f.getOctantsArray() if dim == 3 else f.getQuadrantsArray()
+        ne = len(a)
+        n = int(f.getMeshConn()[a[:, 0] < len(base)].max()) + 1
+        rp, c, v, A, B, T = TMR.MatrixFilter(0.1, 3, None, [f]).getMatrix()
+        got.append((ne, rp[:n + 1], c[:rp[n]], v[:rp[n]]))
+    line = 2_000_000 // (64 if dim == 3 else 16)
+    assert got[0][0] < line < got[1][0]
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert np.array_equal(a, b)

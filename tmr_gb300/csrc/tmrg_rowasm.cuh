@@ -495,8 +495,12 @@ inline AsmResult assemble_entries(const ElemCtx &c, const Entry &ent, long long 
   DBuf<long long> cnt(ne + 1, s);
   launch(k_fa_entry_count<Entry>, blocks_for(ne, 128), 128, 0, s, ne, c, ent, cnt.p);
   exclusive_scan<long long>(cnt.p, cnt.p, ne, s);
-  E = read_scalar(cnt.p + ne, s);
-  if (read_scalar(c.err, s)) return ASM_NODES;
+  const unsigned *w = (const unsigned *)(cnt.p + ne);  // low word first
+  const unsigned *pv[3] = {w, w + 1, (const unsigned *)c.err};
+  unsigned hv[3];
+  read_scalars(pv, hv, s);
+  E = (long long)hv[1] << 32 | hv[0];
+  if (hv[2]) return ASM_NODES;
   if (E >= (1LL << 32)) return ASM_ENTRIES;
   keys.alloc(E, s);
   perm.alloc(E, s);

@@ -54,18 +54,22 @@ static __global__ void __launch_bounds__(TS_ROWS)
   extern __shared__ __align__(16) int ts_smem[];
   int *tab = ts_smem, *cols = ts_smem + Z.slots;
   __shared__ int slen[TS_ROWS];
-  __shared__ int s_n;
+  __shared__ int s_n, s_stop;
   const int t = threadIdx.x;
   const long long r0 = (long long)blockIdx.x * TS_ROWS;
   for (int i = t; i < Z.slots; i += TS_ROWS) tab[i] = -1;
   const long long r = r0 + t;
   const int a = r < n ? rp[r] : 0, b = r < n ? rp[r + 1] : 0;
   slen[t] = r < n ? b - a : -1;
-  if (t == 0) s_n = 0;
+  if (t == 0) {
+    s_n = 0;
+    s_stop = *(volatile int *)state;  // some tile has too many: all for nothing
+  }
   __syncthreads();
+  if (s_stop) return;
   // the tile's entries are one run; threads take them in turn
   const int e0 = rp[min(n, r0)], e1 = rp[min(n, r0 + TS_ROWS)];
-  for (int e = e0 + t; e < e1; e += TS_ROWS) {
+  for (int e = e0 + t; e < e1 && *(volatile int *)&s_n <= Z.cols; e += TS_ROWS) {
     const int c = __ldg(ci + e);
     unsigned h = ((unsigned)c * 0x9E3779B1u) >> 16 & (unsigned)(Z.slots - 1);
     // an empty slot always ends a probe: threads stop adding past Z.cols
