@@ -1,0 +1,98 @@
+"""Paths that need more memory than the ones they replaced give way to them where
+the memory does not suffice: the balance's set of families, and K on tiles.  A
+child process limits the device's allocator (its own memory pool)."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+CHILD = r"""
+import ctypes, sys
+import numpy as np, torch
+from tmr_gb300 import TMR, workloads as W
+rt = ctypes.CDLL("libcudart.so.%s" % torch.version.cuda.split(".")[0])
+torch.zeros(1, device="cuda")
+
+class Props(ctypes.Structure):
+    _fields_ = [("alloc", ctypes.c_int), ("handles", ctypes.c_int), ("loc", ctypes.c_int * 2),
+                ("win", ctypes.c_void_p), ("max", ctypes.c_size_t), ("usage", ctypes.c_ushort),
+                ("reserved", ctypes.c_ubyte * 54)]
+
+pool = ctypes.c_void_p()
+assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+def attr(a, put=None):
+    torch.cuda.synchronize()
+    v = ctypes.c_uint64(0)
+    if put is not None:
+        assert rt.cudaMemPoolSetAttribute(pool, a, ctypes.byref(v)) == 0
+    assert rt.cudaMemPoolGetAttribute(pool, a, ctypes.byref(v)) == 0
+    return v.value
+
+def limited(peak):
+    p = Props(1, 0, (ctypes.c_int * 2)(1, 0), None, peak)
+    h = ctypes.c_void_p()
+    assert rt.cudaMemPoolCreate(ctypes.byref(h), ctypes.byref(p)) == 0
+    assert rt.cudaDeviceSetMemPool(0, h) == 0
+
+def mesh(dim):
+    f = (TMR.OctForest if dim == 3 else TMR.QuadForest)(order=2)
+    f.setConnectivity(W.brick(4, 4, 2) if dim == 3 else W.brick2d(16, 16))
+    f.createTrees(2 if dim == 3 else 4)
+    num = (lambda g: g.getNumOctants()) if dim == 3 else (lambda g: g.getNumQuadrants())
+    for p in range(3):
+        f.refine(W.random_indicator(num(f), 7, p, 0.3), 0, 9)
+        if p < 2:
+            f.balance(1)
+    return f
+
+def balance(dim):
+    base = mesh(dim)
+    def run():
+        g = base.duplicate()
+        g.balance(1)
+        return g.getOctantsArray() if dim == 3 else g.getQuadrantsArray()
+    return run
+
+def helmholtz(_):
+    f = mesh(3)
+    f.balance(1)
+    c = f.coarsen()
+    c.balance(1)
+    for g in (f, c):
+        g.createNodes()
+        g.setBlockBoxes(np.array([[b % 4, b // 4 % 4, b // 16, 1, 1, 1] for b in range(32)], float))
+    n = int(f.getNodeRange()[1])
+    x = W.uniform(5, 0, n)
+    def run():
+        y = np.empty(n)
+        TMR.HelmholtzFilter(0.02, None, [f, c]).applyFilter(x, y)
+        return y
+    return run
+
+run = {"balance": balance, "helmholtz": helmholtz}[sys.argv[1]](int(sys.argv[2]))
+want = run()
+held = attr(8, 0)
+want = run()
+peak = attr(8) - held
+limited(int(float(sys.argv[3]) * peak))
+got = run()
+d = float(np.abs(got - want).max() / np.abs(want).max())
+print("peak %.1f MB, difference %.3g" % (peak / 1e6, d))
+assert d <= float(sys.argv[4])
+"""
+
+
+@pytest.mark.parametrize("what,dim,share,tol", [
+    # the sort of octants needs about two thirds of the set's memory, the element
+    # operator's filter two fifths; solves end at a residual of 1e-12 |b|
+    ("balance", 3, 0.85, 0.0)])
+def test_too_little_memory_for_the_larger_path(gpu_lib, what, dim, share, tol):
+    r = subprocess.run([sys.executable, "-c", CHILD, what, str(dim), str(share), str(tol)],
+                       cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr[-3000:]

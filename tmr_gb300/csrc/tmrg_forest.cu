@@ -830,33 +830,41 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// False (the forest unchanged) when the families outgrew the set.
+// False (the forest unchanged) when the families outgrew the set, or it the
+// memory (about 120 bytes an octant, the sorting path about 80).
 static bool balance_hashed(Forest &f, int corner, const OctKey K) {
   const long long n = f.n;
   cudaStream_t s = f.s;
   const ConnDev c = f.conn->dev;
-  // A refinement pass and its closure leave about half as many families as
-  // octants; a set of that size with room to spare, and the sorting path
-  // where a forest needs more.
-  const long long cap = n + n / 4 + 4096;
-  KeySetBuf B(cap, s);
-  const KeySet S = B.set;
-  launch(k_fam_seeds, blocks_for(n, 256), 256, 0, s, n, K, S, (const int *)f.block.p,
-         (const int *)f.x.p, (const int *)f.y.p, (const int *)f.z.p,
-         (const int16_t *)f.level.p);
-  const unsigned grid = std::min(blocks_for(cap, 32), 152u * 8);
-  int gens = 1;
-  for (int l = f.maxlev; l >= 2; l--, gens++)
-    launch(k_fam_close, grid, 256, 0, s, l, gens, corner, c, K, S);
-  DBuf<uint64_t> leaves(8 * cap, s);
-  launch(k_fam_leaves, grid, 256, 0, s, gens, K, S, leaves.p, (unsigned)(8 * cap));
-  const unsigned *dv[2] = {B.count.p + KEYSET_GENS + 1, B.count.p + KEYSET_GENS};
-  unsigned hv[2];
-  read_scalars(dv, hv, s);
-  if (hv[1]) return false;
-  const long long m = hv[0];
-  // positions are distinct: the level field need not be sorted
-  radix_sort(leaves, nullptr, m, K.total_bits(), s, 5);
+  DBuf<uint64_t> leaves;
+  long long m = 0;
+  try {
+    // A refinement pass and its closure leave about half as many families as
+    // octants; a set of that size with room to spare, and the sorting path
+    // where a forest needs more.
+    const long long cap = n + n / 4 + 4096;
+    KeySetBuf B(cap, s);
+    const KeySet S = B.set;
+    launch(k_fam_seeds, blocks_for(n, 256), 256, 0, s, n, K, S, (const int *)f.block.p,
+           (const int *)f.x.p, (const int *)f.y.p, (const int *)f.z.p,
+           (const int16_t *)f.level.p);
+    const unsigned grid = std::min(blocks_for(cap, 32), 152u * 8);
+    int gens = 1;
+    for (int l = f.maxlev; l >= 2; l--, gens++)
+      launch(k_fam_close, grid, 256, 0, s, l, gens, corner, c, K, S);
+    leaves.alloc(8 * cap, s);
+    launch(k_fam_leaves, grid, 256, 0, s, gens, K, S, leaves.p, (unsigned)(8 * cap));
+    const unsigned *dv[2] = {B.count.p + KEYSET_GENS + 1, B.count.p + KEYSET_GENS};
+    unsigned hv[2];
+    read_scalars(dv, hv, s);
+    if (hv[1]) return false;
+    m = hv[0];
+    // positions are distinct: the level field need not be sorted
+    radix_sort(leaves, nullptr, m, K.total_bits(), s, 5);
+  } catch (const Error &e) {
+    if (e.status != TMRG_ERR_NOMEM) throw;
+    return false;
+  }
   alloc_octs(f, m);
   launch(k_decode_octs<uint64_t>, blocks_for(m, 256), 256, 0, s, m, K,
          (const uint64_t *)leaves.p, f.block.p, f.x.p, f.y.p, f.z.p, f.level.p, f.info.p);
