@@ -91,7 +91,7 @@ assert d <= float(sys.argv[4])
 @pytest.mark.parametrize("what,dim,share,tol", [
     # the sort of octants needs about two thirds of the set's memory, the element
     # operator's filter two fifths; solves end at a residual of 1e-12 |b|
-    ("balance", 3, 0.85, 0.0)])
+    ("balance", 3, 0.85, 0.0), ("helmholtz", 3, 0.7, 1e-9)])
 def test_too_little_memory_for_the_larger_path(gpu_lib, what, dim, share, tol):
     r = subprocess.run([sys.executable, "-c", CHILD, what, str(dim), str(share), str(tol)],
                        cwd=ROOT, capture_output=True, text=True, timeout=300)

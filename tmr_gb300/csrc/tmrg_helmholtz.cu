@@ -1494,20 +1494,32 @@ static void build_level(Helmholtz &H, const HSource &f, HLevel &L) {
                               "(degenerate element geometry)");
 }
 // K of a level of linear elements on tiles; nothing where it cannot be held
-// there (assemble_rows, tsell_build), and the element operator runs.
+// there (assemble_rows, tsell_build, or too little memory: the assembly needs about
+// 1.8 KB a node at its peak, the element operator's filter 0.8), and the element
+// operator runs.
 static void build_tiles(Helmholtz &H, HLevel &L, bool finest) {
   if (L.o != 2 || L.nn == 0) return;
   cudaStream_t s = H.s;
-  DBuf<int> err(1, s), rp, ci;
-  DBuf<double> v;
-  err.zero();
-  long long nnz = 0;
-  const ElemCtx c{L.econn.p, L.dptr.p, L.dconn.p, L.dw.p, err.p, L.npe};
-  if (assemble_rows(c, make_helm_entry(L), L.nn, L.ne, false, rp, ci, v, nnz, s) != ASM_DONE)
+  try {
+    DBuf<int> err(1, s), rp, ci;
+    DBuf<double> v;
+    err.zero();
+    long long nnz = 0;
+    const ElemCtx c{L.econn.p, L.dptr.p, L.dconn.p, L.dw.p, err.p, L.npe};
+    if (assemble_rows(c, make_helm_entry(L), L.nn, L.ne, false, rp, ci, v, nnz, s) != ASM_DONE)
+      return;
+    if (!tsell_build(L.tiled, L.nn, rp.p, ci.p, s)) return;
+    tsell_values(L.tiled, rp.p, (const double *)v.p, L.k32, s);
+    if (finest) tsell_values(L.tiled, rp.p, (const double *)v.p, L.k64, s);
+  } catch (const Error &e) {
+    if (e.status != TMRG_ERR_NOMEM) throw;
+    L.tiled = TSell();
+    L.k32.release();
+    L.k64.release();
     return;
-  if (!tsell_build(L.tiled, L.nn, rp.p, ci.p, s)) return;
-  tsell_values(L.tiled, rp.p, (const double *)v.p, L.k32, s);
-  if (finest) tsell_values(L.tiled, rp.p, (const double *)v.p, L.k64, s);
+  }
+  // the element operator in FP32 is not run any more
+  for (DBuf<float> *b : {&L.geo32, &L.dw32, &L.sw32}) b->release();
 }
 
 // The levels and the P between consecutive forests (octree or quadtree).
