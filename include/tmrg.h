@@ -453,7 +453,8 @@ int tmrg_helmholtz_set_tolerances(tmrg_helmholtz *H, double rtol, double atol,
    levels and `degree_order3` over [lower_order3, upper] x lam on order-3
    levels, lam the Lanczos estimate of the largest eigenvalue of D^-1 K.
    A new filter has 3, 6, 0.2, 0.1, 1.1, with 5 and 0.05 on the order-2
-   levels where the lam of the finest of them is above 2.6.  The reference's
+   levels of an octree filter where the lam of the finest of them is above
+   2.6.  The reference's
    TACS multigrid uses symmetric SOR or, optionally, degree-3 Chebyshev over
    [1/30, 1.1] (TMR_RefinementTools.cpp:44-50); the smoother changes only the iteration
    count, not the converged result. */

@@ -1125,12 +1125,15 @@ static void lanczos_lmax(Helmholtz &H, HLevel &L) {
 // down to lam / 27, and a short interval costs iterations.  2.56M nodes, element
 // sides r / 2 to 16 r (lam above 2.6): 3 steps from 0.2 take 15 iterations, 19.4
 // ms, 5 from 0.05 take 7, 13.2 ms; r four times as large (2.2): 8 and 7
-// iterations, 10.6 and 13.2 ms.
+// iterations, 10.6 and 13.2 ms.  On quadrilaterals lam is at most 2.25 and short
+// modes go down to lam / 9 only: 3 steps from 0.2 take 9 iterations where the
+// mass rules, 5 from 0.05 take 7, in 20.2 against 22.9 ms (8.5M nodes) and 1.58
+// against 1.60 ms (16K), and fewer elsewhere; they stay.
 constexpr double HM_MASS_LAM = 2.6;
 static void smoother_of(const Helmholtz &H, const HLevel &L, int &degree, double &lower) {
   degree = L.o == 2 ? H.cheb_degree2 : H.cheb_degree3;
   lower = L.o == 2 ? H.cheb_lower2 : H.cheb_lower3;
-  if (!H.cheb_auto || L.o != 2) return;
+  if (!H.cheb_auto || L.o != 2 || L.dim != 3) return;
   for (const auto &F : H.L) {
     if (F->o != 2) continue;  // (quadratic levels come first)
     if (F->lam > HM_MASS_LAM) {
