@@ -83,6 +83,7 @@ struct Helmholtz {
   int cheb_degree2 = 3, cheb_degree3 = 6;
   int lanczos_steps = 16;
   int coarse_sweeps = 4;
+  bool coarse_smooth = false;  // a coarsest level in need of the longer smoother
   // last solve
   int last_iters = 0;
   std::vector<double> last_res;
