@@ -768,6 +768,7 @@ __global__ void __launch_bounds__(256)
 // Targets of the families of `level`: 8 lanes per family, one group each.
 __global__ void __launch_bounds__(256)
     k_fam_close(int level, int gen, int corner, ConnDev c, OctKey K, KeySet S) {
+  if (S.full()) return;
   const unsigned m = S.before(gen);
   const int g = threadIdx.x & 7;
   const unsigned stride = gridDim.x * 32;
@@ -775,7 +776,6 @@ __global__ void __launch_bounds__(256)
     const unsigned i = b0 + (threadIdx.x >> 3);
     const uint64_t k = i < m ? S.list[i] : 0;
     const bool mine = i < m && (int)(k & 31) == level && (corner || g != 7);
-    if (S.full()) return;
     if (!__any_sync(0xffffffffu, mine)) continue;
     // the first target is added by the whole warp; a face, edge or corner
     // shared by several trees gives some lanes more
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(256)
         if (cnt++ == 0) first = K.make(r.block, r.x, r.y, r.z, r.level);
       });
     }
-    S.add(first, cnt > 0, gen, m);
+    if (S.add(first, cnt > 0, gen, m)) return;
     const int most = __reduce_max_sync(0xffffffffu, cnt);
     for (int j = 1; j < most; j++) {
       uint64_t key = 0;
@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(256)
           if (at++ == j) key = K.make(r.block, r.x, r.y, r.z, r.level);
         });
       }
-      S.add(key, j < cnt, gen, m);
+      if (S.add(key, j < cnt, gen, m)) return;
     }
   }
 }

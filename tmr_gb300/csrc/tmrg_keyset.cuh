@@ -28,9 +28,7 @@ struct KeySet {
   }
   __device__ __forceinline__ unsigned *overflow() const { return count + KEYSET_GENS; }
   __device__ __forceinline__ unsigned *counter() const { return count + KEYSET_GENS + 1; }
-  // The set overflowed: it is given up, and nothing more need be added (a full
-  // table would take KEYSET_PROBES steps a key).  A whole warp asks and gets
-  // one answer.
+  // The set overflowed and is given up.  A whole warp asks and gets one answer.
   __device__ __forceinline__ bool full() const {
     return __any_sync(0xffffffffu, __ldcg(overflow()) != 0u);
   }
@@ -69,21 +67,22 @@ struct KeySet {
     return min(t, cap);
   }
   // Adds one key per lane where `on`, new members appended as generation g
-  // from list position `base` = before(g); a whole warp calls it.
-  __device__ __forceinline__ void add(uint64_t k, bool on, int g, unsigned base) const {
+  // from list position `base` = before(g); a whole warp calls it.  True once the
+  // list has no room for what the warp adds: the set is given up then, and a
+  // caller that goes on would fill the table (KEYSET_PROBES steps a key).
+  __device__ __forceinline__ bool add(uint64_t k, bool on, int g, unsigned base) const {
     const bool fresh = on && insert(k);
     const unsigned m = __ballot_sync(0xffffffffu, fresh);
-    if (m == 0u) return;
+    if (m == 0u) return false;
     const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
     unsigned o = 0;
     if (lane == lead) o = atomicAdd(count + g, (unsigned)__popc(m));
-    o = __shfl_sync(0xffffffffu, o, lead) + base + __popc(m & ((1u << lane) - 1u));
-    if (fresh) {
-      if (o < cap)
-        list[o] = k;
-      else
-        atomicOr(overflow(), 1u);
-    }
+    o = __shfl_sync(0xffffffffu, o, lead) + base;
+    const unsigned at = o + __popc(m & ((1u << lane) - 1u));
+    if (fresh && at < cap) list[at] = k;
+    const bool none = o + __popc(m) > cap;
+    if (none && lane == lead) atomicOr(overflow(), 1u);
+    return none;
   }
 };
 

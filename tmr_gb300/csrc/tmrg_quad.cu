@@ -1033,6 +1033,7 @@ __global__ void __launch_bounds__(256)
 // 4 lanes per family, one group each
 __global__ void __launch_bounds__(256)
     k_q_fam_close(int level, int gen, int corner, QConnDev c, QKey K, KeySet S) {
+  if (S.full()) return;
   const unsigned m = S.before(gen);
   const int g = threadIdx.x & 3;
   const unsigned stride = gridDim.x * 64;
@@ -1040,7 +1041,6 @@ __global__ void __launch_bounds__(256)
     const unsigned i = b0 + (threadIdx.x >> 2);
     const uint64_t k = i < m ? S.list[i] : 0;
     const bool mine = i < m && (int)(k & 31) == level && (corner || g != 3);
-    if (S.full()) return;
     if (!__any_sync(0xffffffffu, mine)) continue;
     uint64_t first = 0;
     int cnt = 0;
@@ -1051,7 +1051,7 @@ __global__ void __launch_bounds__(256)
         if (cnt++ == 0) first = K.make(r.block, r.x, r.y, r.level);
       });
     }
-    S.add(first, cnt > 0, gen, m);
+    if (S.add(first, cnt > 0, gen, m)) return;
     const int most = __reduce_max_sync(0xffffffffu, cnt);
     for (int j = 1; j < most; j++) {
       uint64_t key = 0;
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(256)
           if (at++ == j) key = K.make(r.block, r.x, r.y, r.level);
         });
       }
-      S.add(key, j < cnt, gen, m);
+      if (S.add(key, j < cnt, gen, m)) return;
     }
   }
 }
