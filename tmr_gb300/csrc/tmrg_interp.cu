@@ -2883,6 +2883,17 @@ __global__ void __launch_bounds__(256)
   y[r] = acc;
 }
 
+// r / sc from the correctly rounded reciprocal `inv` of sc by one correction of
+// the quotient with the exact remainder (P. Markstein, IBM J. Res. Dev. 34(1),
+// 1990: the quotient step of a division by multiply-adds), where the reciprocal is
+// kept (inv != 0: sc within 2^+-64), else by a division, some ten times as many
+// operations of the FP64 pipe.  r is finite.
+__device__ __forceinline__ double df_quotient(double r, double sc, double inv) {
+  if (inv == 0.0) return sc != 0.0 ? __ddiv_rn(r, sc) : 0.0;
+  const double q = __dmul_rn(r, inv);
+  return __fma_rn(__fma_rn(-q, sc, r), inv, q);
+}
+
 // Vector pairs: LPR lanes per row, lane v holds PPL consecutive vector
 // pairs (16-byte loads of (hi, lo, hi, lo) each), and NG groups of LPR
 // lanes split a row's entries; the warp runs one trip count with per-entry
@@ -2904,7 +2915,8 @@ __global__ void __launch_bounds__(256)
                 const int *__restrict__ cols, const float2 *__restrict__ w,
                 const float4 *__restrict__ xs, const double *__restrict__ x,
                 double *__restrict__ y, const double *__restrict__ scale,
-                const int *__restrict__ perm, const int *__restrict__ flags) {
+                const double *__restrict__ recip, const int *__restrict__ perm,
+                const int *__restrict__ flags) {
   constexpr int RPW = 32 / (LPR * NG);
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -3034,13 +3046,14 @@ __global__ void __launch_bounds__(256)
     }
     if (g == 0) {
       const double sc = scale && have ? scale[r] : 1.0;
+      const double inv = scale && have && !f64 ? recip[r] : 0.0;
 #pragma unroll
       for (int j = 0; j < PPL; j++) {
         if (!act[j]) continue;
         double a = ax[j], b = ay[j];
         if (scale) {
-          a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
-          b = (sc != 0.0) ? __ddiv_rn(b, sc) : 0.0;
+          a = df_quotient(a, sc, inv);
+          b = df_quotient(b, sc, inv);
         }
         if (SC) {
           double *yp = y + r * nvec + 2 * (q0 + j);
@@ -3244,14 +3257,7 @@ __global__ void __launch_bounds__(256)
   }
   double r = df_value(sh, sl);
   if (scale) {
-    // r / sc from the column's reciprocal and one correction
-    const double sc = scale[c], inv = recip[c];
-    if (inv != 0.0) {
-      const double q = __dmul_rn(r, inv);
-      r = __fma_rn(__fma_rn(-q, sc, r), inv, q);
-    } else {
-      r = sc != 0.0 ? __ddiv_rn(r, sc) : 0.0;
-    }
+    r = df_quotient(r, scale[c], recip[c]);
   }
   y[t] = r;
 }
@@ -3317,7 +3323,7 @@ __global__ void __launch_bounds__(TG_WARPS * 32)
                    const int *__restrict__ rowptr, const int *__restrict__ cols,
                    const float2 *__restrict__ w, const double2 *__restrict__ x,
                    double2 *__restrict__ y, const double *__restrict__ scale,
-                   const int *__restrict__ perm, int *flags) {
+                   const double *__restrict__ recip, const int *__restrict__ perm, int *flags) {
   extern __shared__ __align__(128) uint8_t tg_smem[];
   constexpr int PPL = 4, NV2 = 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -3426,12 +3432,13 @@ __global__ void __launch_bounds__(TG_WARPS * 32)
   }
   if (have) {
     const double sc = scale ? scale[r] : 1.0;
+    const double inv = scale && !f64 ? recip[r] : 0.0;
 #pragma unroll
     for (int j = 0; j < PPL; j++) {
       double a = ax[j], bv = ay[j];
       if (scale) {
-        a = (sc != 0.0) ? __ddiv_rn(a, sc) : 0.0;
-        bv = (sc != 0.0) ? __ddiv_rn(bv, sc) : 0.0;
+        a = df_quotient(a, sc, inv);
+        bv = df_quotient(bv, sc, inv);
       }
       y[r * NV2 + q0 + j] = make_double2(a, bv);
     }
@@ -3458,7 +3465,8 @@ static EncodeTiledFn encode_tiled() {
 }
 static bool tma_apply(long long rows, long long nin, const int *rp, const int *ci,
                       const float2 *w, const float2 *xs, const double *x, double *y,
-                      const double *scale, const int *perm, int *flags, cudaStream_t s) {
+                      const double *scale, const double *recip, const int *perm, int *flags,
+                      cudaStream_t s) {
   EncodeTiledFn enc = encode_tiled();
   if (!enc || nin <= 0 || nin >= (1LL << 31) || ((uintptr_t)xs % 16) != 0) return false;
   CUtensorMap map;
@@ -3479,7 +3487,7 @@ static bool tma_apply(long long rows, long long nin, const int *rp, const int *c
   const long long rows_per_block = 16LL * TG_WARPS;
   launch(k_df_apply_tma, (unsigned)((rows + rows_per_block - 1) / rows_per_block),
          TG_WARPS * 32, TG_SMEM, s, map, rows, rp, ci, w, (const double2 *)x, (double2 *)y,
-         scale, perm, flags);
+         scale, recip, perm, flags);
   return true;
 }
 
@@ -3500,18 +3508,18 @@ static bool df_scalar(int nvec, const double *x, const double *y) {
 }
 static void df_apply2(int shape, long long rows, int nvec, const int *rp, const int *ci,
                       const float2 *w, const float2 *xs, const double *x, double *y,
-                      const double *scale, const int *perm, int *flags, cudaStream_t s,
-                      long long nin) {
+                      const double *scale, const double *recip, const int *perm, int *flags,
+                      cudaStream_t s, long long nin) {
   const int nvec2 = (nvec + 1) / 2;
   const bool scalar = df_scalar(nvec, x, y);
   if (shape == 6 && nvec2 == 8 && !scalar &&
-      tma_apply(rows, nin, rp, ci, w, xs, x, y, scale, perm, flags, s))
+      tma_apply(rows, nin, rp, ci, w, xs, x, y, scale, recip, perm, flags, s))
     return;
   const float4 *x4 = (const float4 *)xs;
 #define TMRG_DF2S(L, N, P, SC)                                                             \
   launch((k_df_apply2<L, N, P, SC>),                                                       \
          blocks_for(((rows + 32 / ((L) * (N)) - 1) / (32 / ((L) * (N)))) * 32, 256), 256, 0, s, \
-         rows, nvec2, nvec, rp, ci, w, x4, x, y, scale, perm, flags)
+         rows, nvec2, nvec, rp, ci, w, x4, x, y, scale, recip, perm, flags)
 #define TMRG_DF2(L, N, P)                                     \
   do {                                                        \
     if (scalar) TMRG_DF2S(L, N, P, true); else TMRG_DF2S(L, N, P, false); \
@@ -3813,7 +3821,7 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
     const long long a = I.t_chunk[k], n = I.t_chunk[k + 1] - a;
     if (n > 0)
       df_apply2(shape, n, nvec, I.t_rowptr.p, I.t_colidx.p, I.t_w.p, xs.p, dx, y, sc,
-                I.t_perm.p + a, I.dfflag.p, s, nin);
+                sc ? sc + I.cols : nullptr, I.t_perm.p + a, I.dfflag.p, s, nin);
   }
   if (I.tile_t) df_tile_columns_f64(I, nvec, dx, y, sc, s);
   TMRG_CUDA(cudaStreamSynchronize(s));
@@ -3910,7 +3918,7 @@ bool interp_apply_forward_staged(Interp &I, const double *xh, double *dx, double
         df_tile_apply(I, r0 / TB_ROWS, (r1 + TB_ROWS - 1) / TB_ROWS, nvec, dx, y, false, s);
       else
         df_apply2(shape, r1 - r0, nvec, I.ap_rowptr(), I.ap_colidx(), I.ap_w.p, xs.p, dx, y,
-                  nullptr, I.perm.p + r0, I.dfflag.p, s, nin);
+                  nullptr, nullptr, I.perm.p + r0, I.dfflag.p, s, nin);
     }
     TMRG_CUDA(cudaEventRecord(ev[k], s));
     TMRG_CUDA(cudaStreamWaitEvent(cs, ev[k], 0));
@@ -3980,7 +3988,8 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec, bo
   const int *ci = which == 0 ? I.ap_colidx() : I.t_colidx.p;
   const float2 *w = which == 0 ? (const float2 *)I.ap_w.p : (const float2 *)I.t_w.p;
   const double *sc = which == 2 ? (const double *)I.colsum.p : (const double *)nullptr;
-  const int *perm = which == 0 ? (const int *)I.perm.p : (const int *)I.t_perm.p;
+  // (rows in their order where the result goes over the host link)
+  const int *perm = host ? nullptr : which == 0 ? (const int *)I.perm.p : (const int *)I.t_perm.p;
   // compulsory traffic: 12 B per nonzero entry, the row pointers, one read
   // of the input (its (hi, lo) copy) and one write of the output vectors
   const long long bytes = 12 * I.nnz_nz + 4 * (nout + 1) + 8LL * nvec * (nin + nout) +
@@ -4022,7 +4031,8 @@ void interp_apply(Interp &I, int which, const double *x, double *y, int nvec, bo
   tune_run(df_key(which, nout, I.nnz_nz, n2, df_scalar(nvec, x, y)),
            n2 >= 8 ? DF2_SHAPES_WIDE : DF2_SHAPES_NARROW,
            [&](int shape) {
-             df_apply2(shape, nout, nvec, rp, ci, w, xs.p, x, y, sc, perm, I.dfflag.p, s, nin);
+             df_apply2(shape, nout, nvec, rp, ci, w, xs.p, x, y, sc, sc ? sc + nout : nullptr,
+                       perm, I.dfflag.p, s, nin);
            },
            s);
 }
