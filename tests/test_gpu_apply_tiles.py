@@ -235,6 +235,45 @@ def test_host_buffers_of_any_count_equal_device_buffers(gpu_lib, grid):
                         np.testing.assert_allclose(a, want, rtol=1e-13, atol=1e-13)
 
 
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("grid", [(6, 4, 4), (8, 8, 4)])
+def test_host_buffers_in_pieces(gpu_lib, grid, pinned):
+    # two and seven pieces: input and output apart, and the output over the
+    # input, from the buffer's start or to its end
+    import torch
+
+    from tmr_gb300 import TMR
+    I = _refined(TMR, 2, grid, 3, 2)
+    rows, cols, _ = I.sizes()
+    assert rows >= 2 * 4 * 152 * 256
+
+    def host(n):
+        a = torch.zeros(n, dtype=torch.float64)
+        return (a.pin_memory() if pinned else a).numpy()
+
+    for nvec in (2, 16):
+        for fn, nin, nout in ((I.mult, cols, rows), (I.multTranspose, rows, cols),
+                              (I.multWeightTranspose, rows, cols)):
+            x = np.random.default_rng(nvec).standard_normal(nin * nvec)
+            for where in (None, 0, -1):
+                if where is not None:
+                    x[where] = 1e-30
+                y = torch.empty(nout * nvec, dtype=torch.float64, device="cuda")
+                fn(torch.from_numpy(x).cuda(), y)
+                want = y.cpu().numpy()
+                n = max(nin, nout) * nvec
+                for at in (n, 0, n - nout * nvec):
+                    both = host(n + (nout * nvec if at == n else 0))
+                    both[:nin * nvec] = x
+                    got = both[at:at + nout * nvec]
+                    fn(both[:nin * nvec], got)
+                    if where is None:
+                        np.testing.assert_array_equal(got, want)
+                    else:
+                        # pieces before the value stay double-float
+                        np.testing.assert_allclose(got, want, rtol=1e-13, atol=1e-13)
+
+
 def test_page_locked_odd_counts_cost_what_even_ones_do(gpu_lib):
     # 3 vectors into page-locked memory: no more than 4 (twice as much where the
     # rows went over the link in order of length)

@@ -1056,7 +1056,9 @@ static int interp_host(tmrg_interp *I, int which, const double *x, double *y,
     double *ym = (double *)host_mapped(y);
     host_warm(x, sizeof(double) * nin);
     host_warm(y, sizeof(double) * nout);
-    if (which != 0) {
+    // (pieces of an output over an input that is still being read: not at once)
+    const bool apart = !overlap(x, sizeof(double) * nin, y, sizeof(double) * nout);
+    if (which != 0 && apart) {
       // restriction: copy the input in pieces overlapped with the rows
       // they complete
       DBuf<double> dy;
@@ -1068,7 +1070,7 @@ static int interp_host(tmrg_interp *I, int which, const double *x, double *y,
     }
     // prolongation: rows computed in pieces, each piece copied back while
     // the next one computes
-    if (which == 0 && interp_apply_forward_staged(P, x, dx.p, y, nvec)) return;
+    if (which == 0 && apart && interp_apply_forward_staged(P, x, dx.p, y, nvec)) return;
     TMRG_CUDA(cudaMemcpyAsync(dx.p, x, sizeof(double) * nin,
                               cudaMemcpyHostToDevice, P.s));
     if (ym && (which != 0 || nvec <= 8 || nvec % 2 == 0)) {
