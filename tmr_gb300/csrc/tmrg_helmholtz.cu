@@ -10,9 +10,10 @@
 // the quadratic Bernstein hexahedron for order 3.
 //
 // Design:
-// * Matrix-free operator.  Forest geometry is a box per block, so every
-//   element is an axis-aligned box and its matrices are tensor products of
-//   exact 1-D reference matrices: K_e = V (cx Kx My Mz + cy Mx Ky Mz +
+// * Element operator, matrix-free: quadratic levels, the mass products, and
+//   linear levels whose K does not go on tiles.  Forest geometry is a box per
+//   block, so every element is an axis-aligned box and its matrices are tensor
+//   products of exact 1-D reference matrices: K_e = V (cx Kx My Mz + cy Mx Ky Mz +
 //   cz Mx My Kz + Mx My Mz) with V the element's Jacobian determinant and
 //   c_d = r^2 / s_d^2 (s_d the half side).  One thread per element gathers
 //   its node values (dependent nodes through their weights), applies K_e
@@ -31,9 +32,9 @@
 //   drives the true residual to the reference's tolerance.  The smoother is
 //   Chebyshev on D^-1 K over [lower, 1.1] lmax (lmax from Lanczos; degree
 //   3 and lower 0.2, or 5 and 0.05, for order-2 levels (smoother_of), degree
-//   6 and lower 0.1 for order 3),
-//   which is parallel where SOR is sequential.  Restriction and prolongation are the forests' own
-//   createInterpolation operators (P^T and P); coarse levels are
+//   6 and lower 0.1 for order 3), which is parallel where SOR is sequential.
+//   Restriction and prolongation are the forests' own createInterpolation
+//   operators (P^T and P); coarse levels are
 //   rediscretised, as in the reference (use_galerkin = 0).  The coarsest
 //   level is solved with its explicit dense inverse (Gauss-Jordan on the
 //   GPU) when it has at most HM_DENSE_MAX nodes, else by Chebyshev sweeps.
@@ -491,7 +492,7 @@ static HelmEntry make_helm_entry(const HLevel &L) {
 // A block loads its tile's distinct inputs into shared memory (HT_START forms
 // d as it loads) and its rows read them by 16-bit places; d2 and x2 are other
 // buffers than the gathered d and x.  Bound by the matrix (6 or 10 bytes an
-// entry, 5.0 TB/s) on the finest level and by latency on the small ones (8 us
+// entry, 4.4 TB/s) on the finest level and by latency on the small ones (8 us
 // for 6,000 nodes).
 enum HtMode { HT_APPLY, HT_START, HT_START1, HT_STEP, HT_END, HT_RES, HT_FROM };
 template <typename T>
@@ -1537,7 +1538,7 @@ static void build_level(Helmholtz &H, const HSource &f, HLevel &L) {
 }
 // K of a level of linear elements on tiles; nothing where it cannot be held
 // there (assemble_rows, tsell_build, or too little memory: the assembly needs about
-// 1.8 KB a node at its peak, the element operator's filter 0.8), and the element
+// 1.8 KB a node at its peak, the element operator's filter 0.7), and the element
 // operator runs.
 static void build_tiles(Helmholtz &H, HLevel &L, bool finest) {
   if (L.o != 2 || L.nn == 0) return;

@@ -14,9 +14,9 @@
 // subsequence, so each coarse element's expansion is stably sorted by
 // column once, and a row is the in-box filter of that list with adjacent
 // equal columns summed in order.  Rows are written in two passes (exact
-// count, then write at the scanned offsets).  P^T is the apply copy
-// re-sorted by (column, row), so transpose applies gather without atomics
-// and sum in a fixed order.
+// count, then write at the scanned offsets).  P^T is the apply copy in order
+// of (column, row), so transpose applies gather without atomics and sum in a
+// fixed order.
 #include <cuda.h>  // CUtensorMap (the encoder is fetched from the driver at run time)
 
 #include <algorithm>
@@ -1642,7 +1642,7 @@ __global__ void k_chunk_bounds(long long n, const uint64_t *__restrict__ keys, i
   bounds[k] = lo;
 }
 // sum[rows + r]: its reciprocal where the sum is within 2^+-64, else 0 (the
-// quotients of k_df_pair_sum are then divided).
+// applies then divide: df_quotient).
 __global__ void k_rowsum(long long rows, const int *__restrict__ rowptr,
                          const float2 *__restrict__ vals, double *sum) {
   long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -3748,7 +3748,7 @@ void interp_check_apply(Interp &I) {
   }
 }
 
-// Transpose apply with the input in host memory: the input rows are copied
+// Transpose apply with the input in host memory (apart from the output): it is copied
 // in up to TC_CHUNKS pieces on a second stream.  With tiles, piece k's tiles are
 // summed as it arrives, and then the windows of columns that have all their
 // runs, so a page-locked result goes over the link meanwhile (1.4M rows, 16
@@ -3831,19 +3831,19 @@ bool interp_apply_transpose_staged(Interp &I, int which, const double *xh, doubl
   return true;
 }
 
-// Prolongation with the input and the output in host memory: the input
-// (coarse values) is copied in column ranges on a second stream, and the rows are
-// computed in as many pieces (up to FC_CHUNKS) of whole 4096-row windows
-// (the length-ordered permutation stays inside a window, so a piece of
-// slots is exactly a piece of rows) into device memory, each piece as soon
-// as the input range holding its largest column has arrived and been split
-// (rows and columns follow the same node order, so piece k mostly needs
-// the first ranges), and each piece is copied to the host on a third
+// Prolongation with the input and the output in host memory, which share none of
+// it: the input (coarse values) is copied in column ranges on a second stream, and
+// the rows are computed in as many pieces (up to FC_CHUNKS) of whole 4096-row
+// windows (without tiles the length-ordered permutation stays inside a window, so
+// a piece of slots is exactly a piece of rows) into device memory, each piece as
+// soon as the input range holding its largest column has arrived and, without
+// tiles, been split (rows and columns follow the same node order, so piece k mostly
+// needs the first ranges), and each piece is copied to the host on a third
 // stream while the next piece computes.  One bulk copy per piece runs the
 // host link at its copy rate (the kernel writing host memory directly ran
 // it at less than half).  Same kernel, rows and summation order as the
-// single apply; as in the transpose, a range with a value outside the
-// double-float window sends the rows computed after its split to FP64.
+// single apply; as in the transpose, a value outside the double-float window
+// sends the rows computed after it was seen to FP64.
 // Returns false (nothing done) where the pair kernel or the tiles do not apply, or
 // there are fewer than two pieces.
 constexpr int FC_CHUNKS = 16;
