@@ -397,6 +397,11 @@ def base_name(k):
     return k.split("<")[0]
 
 
+def is_apply(k):
+    """Kernels of the P / P^T applies (double-float and FP64)."""
+    return base_name(k).startswith(("k_df_", "k_f64_"))
+
+
 def ncu_traffic(kernel, alg_bytes_per_launch):
     """DRAM bytes per launch of `kernel`: the ratio of ncu-measured DRAM
     traffic to algorithmic bytes of a captured launch (committed in
@@ -603,7 +608,7 @@ def run_gpu(args):
                 a[i] += v[i]
         top = max(fam.items(), key=lambda kv: kv[1][1])
         roof = roofline_entry(top[0], top[1], peak, peak_kind, fp64_peak, tot_ms)
-        apply = [(k, v) for k, v in prof.items() if "df_apply" in k]
+        apply = [(k, v) for k, v in prof.items() if is_apply(k)]
         if apply:
             nl2 = sum(v[0] for _, v in apply)
             tms2 = sum(v[1] for _, v in apply)
@@ -1520,8 +1525,8 @@ def filter_chain_metrics(TMR, steps=5):
     fb = sum(v[2] for k, v in prof.items() if k.startswith("(k_fe_") or k.startswith("k_fe_"))
     fms = sum(v[1] for k, v in prof.items() if k.startswith("(k_fe_") or k.startswith("k_fe_"))
     ffl = sum(v[3] for k, v in prof.items() if k.startswith("(k_fe_") or k.startswith("k_fe_"))
-    pb = sum(v[2] for k, v in prof.items() if "csr_apply" in k)
-    pms = sum(v[1] for k, v in prof.items() if "csr_apply" in k)
+    pb = sum(v[2] for k, v in prof.items() if is_apply(k))
+    pms = sum(v[1] for k, v in prof.items() if is_apply(k))
     peak, _ = measured_peaks()
     x32 = x.float()
     r32 = torch.empty_like(x32)
